@@ -575,7 +575,8 @@ int vb200_lm::make_state() {
 
 /* ------------------------------------------------------------------ activations */
 int vb200_lm::splits_of(const Linear &l, int M) const {
-    if (f32() || l.swiglu || fused_act(l, M)) return 1;
+    if (l.swiglu || fused_act(l, M)) return 1;
+    if (f32()) return lm_gemm_f32_splits(M, l.N, l.K, n_sm);
     if (M <= 64) return tc_pick_splits(l.N, l.Kp, n_sm);
     /* row-block kernel: a CTA per pair of weight tiles and 128 rows */
     const int tiles = (l.N + kTcTileN - 1) / kTcTileN, ctas = (tiles + 1) / 2 * ((M + 127) / 128);
@@ -738,8 +739,9 @@ int vb200_lm::gemm(const Linear &l, Acts *in, int M, float *part, Acts *swiglu_o
     if (f32()) {
         float *y = l.swiglu ? swiglu_out->rows : part;
         const int ld = l.swiglu ? swiglu_out->Kp : l.N;
-        if (out) *out = {part, 1, l.N, 0};
-        return lm_gemm_f32(y, ld, in->rows, in->Kp, l.W, l.Kp, M, l.N, l.K, l.swiglu ? LM_ACT_SWIGLU : LM_ACT_NONE, st);
+        const int splits = splits_of(l, M);
+        if (out) *out = {part, splits, l.N, (size_t)M * l.N};
+        return lm_gemm_f32(y, ld, in->rows, in->Kp, l.W, l.Kp, M, l.N, l.K, l.swiglu ? LM_ACT_SWIGLU : LM_ACT_NONE, st, splits);
     }
     TcActs *a = map_of(in, M);
     if (!a) return -1;
@@ -862,9 +864,9 @@ int vb200_lm::experts(const Layer &l, const LmMlp &m, int M, LmMix *mix) {
     LM_DO(lm_moe_plan(e, M, st));
     LM_DO(lm_moe_gather(e, to, M, st));
     if (f32()) {
-        LM_DO(lm_gemm_f32(ff->rows, ff->Kp, to.rows, to.ld, l.up.W, l.up.Kp, blocks * 128, m.ff, cfg.width, LM_ACT_RELU2, st, route_table,
+        LM_DO(lm_gemm_f32(ff->rows, ff->Kp, to.rows, to.ld, l.up.W, l.up.Kp, blocks * 128, m.ff, cfg.width, LM_ACT_RELU2, st, 1, route_table,
                           l.expert_rows));
-        LM_DO(lm_gemm_f32(expert_y, y_ld, ff->rows, ff->Kp, l.down.W, l.down.Kp, blocks * 128, cfg.width, m.ff, LM_ACT_NONE, st, route_table,
+        LM_DO(lm_gemm_f32(expert_y, y_ld, ff->rows, ff->Kp, l.down.W, l.down.Kp, blocks * 128, cfg.width, m.ff, LM_ACT_NONE, st, 1, route_table,
                           l.expert_rows_down));
         return 0;
     }

@@ -1,6 +1,6 @@
 /*
- * vb_lm_kernels.cu - decoder language models: residual stream and norms, weight repacking, the
- * fp32 GEMM of the 32-bit mode, greedy choice of the next token.
+ * vb_lm_kernels.cu - decoder language models: residual stream and norms, weight repacking, greedy
+ * choice of the next token.
  */
 #include "vb_lm_kernels.cuh"
 
@@ -179,67 +179,6 @@ __global__ void lm_fill_random_kernel(uint16_t *dst, size_t n, uint32_t seed, fl
     dst[i] = __bfloat16_as_ushort(__float2bfloat16_rn(mean + scale * 1.7320508f * s));
 }
 
-/* 64 x 64 tile, 16 columns of K per step, 4 x 4 results per thread. The sum over K is taken in two
- * levels, so that its rounding error grows with the step length and the number of steps, not with K. */
-constexpr int kFgT = 64, kFgK = 16;
-__global__ void __launch_bounds__(256)
-lm_gemm_f32_kernel(float *y, int ld_out, const float *x, int ldx, const uint16_t *W, int ldw, int M, int N, int K, int act,
-                   const int4 *table, int group_rows) {
-    __shared__ __align__(16) float xs[kFgK][kFgT + 4], ws[kFgK][kFgT + 4];
-    pdl_launch_dependents();
-    pdl_wait();
-    const int n0 = blockIdx.x * kFgT;
-    int m0 = blockIdx.y * kFgT;
-    if (table) {                       /* two tiles of rows per block of 128 */
-        const int4 g = __ldcg(table + (blockIdx.y >> 1));
-        m0 = g.y + (int)(blockIdx.y & 1) * kFgT;
-        M = g.y + g.z;
-        if (g.x < 0 || m0 >= M) return;
-        W += (size_t)g.x * group_rows * ldw;
-    }
-    const int tid = threadIdx.x, tm = (tid >> 4) * 4, tn = (tid & 15) * 4;
-    float sum[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += kFgK) {
-        for (int i = tid; i < kFgT * kFgK; i += 256) {
-            const int r = i / kFgK, k = i % kFgK;
-            const bool kin = k0 + k < K;
-            xs[k][r] = kin && m0 + r < M ? x[(size_t)(m0 + r) * ldx + k0 + k] : 0.0f;
-            ws[k][r] = kin && n0 + r < N ? __uint_as_float((uint32_t)W[(size_t)(n0 + r) * ldw + k0 + k] << 16) : 0.0f;
-        }
-        __syncthreads();
-        float acc[4][4] = {};
-#pragma unroll
-        for (int k = 0; k < kFgK; k++) {
-            const float4 a = *(const float4 *)&xs[k][tm], b = *(const float4 *)&ws[k][tn];
-            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) sum[i][j] += acc[i][j];
-        __syncthreads();
-    }
-    for (int i = 0; i < 4; i++) {
-        const int m = m0 + tm + i;
-        if (m >= M) break;
-        if (act == LM_ACT_SWIGLU) {
-            for (int j = 0; j < 4; j += 2) {
-                const int n = n0 + tn + j;
-                if (n + 1 < N) y[(size_t)m * ld_out + n / 2] = sum[i][j] / (1.0f + expf(-sum[i][j])) * sum[i][j + 1];
-            }
-        } else {
-            for (int j = 0; j < 4; j++) {
-                const float v = act == LM_ACT_RELU2 ? fmaxf(sum[i][j], 0.0f) * fmaxf(sum[i][j], 0.0f) : sum[i][j];
-                if (n0 + tn + j < N) y[(size_t)m * ld_out + n0 + tn + j] = v;
-            }
-        }
-    }
-}
-
 __global__ void __launch_bounds__(1024)
 lm_argmax_advance_kernel(LmDyn *dyn, int *tokens, int *log, int log_cap, const LmPart lg, int vocab, int rows) {
     __shared__ float rv[32];
@@ -311,13 +250,6 @@ int lm_fill_random(uint16_t *dst, size_t n, uint32_t seed, float mean, float sca
     if (n == 0) return 0;
     lm_fill_random_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(dst, n, seed, mean, scale);
     return ok(cudaGetLastError());
-}
-
-int lm_gemm_f32(float *y, int ld_out, const float *x, int ldx, const uint16_t *W, int ldw, int M, int N, int K, LmAct act,
-                cudaStream_t st, const int4 *table, int group_rows) {
-    const dim3 g((N + kFgT - 1) / kFgT, (M + kFgT - 1) / kFgT);
-    return ok(launch_pdl(lm_gemm_f32_kernel, g, dim3(256), 0, st, y, ld_out, x, ldx, W, ldw, M, N, K, (int)act,
-                         table, group_rows));
 }
 
 int lm_argmax_advance(LmDyn *dyn, int *tokens, int *log, int log_cap, LmPart logits, int vocab, int rows, cudaStream_t st) {
