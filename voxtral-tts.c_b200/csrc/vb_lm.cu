@@ -578,9 +578,7 @@ int vb200_lm::splits_of(const Linear &l, int M) const {
     if (l.swiglu || fused_act(l, M)) return 1;
     if (f32()) return lm_gemm_f32_splits(M, l.N, l.K, n_sm);
     if (M <= 64) return tc_pick_splits(l.N, l.Kp, n_sm);
-    /* row-block kernel: a CTA per pair of weight tiles and 128 rows */
-    const int tiles = (l.N + kTcTileN - 1) / kTcTileN, ctas = (tiles + 1) / 2 * ((M + 127) / 128);
-    return std::max(1, std::min({n_sm / ctas, kTcMaxSplits, l.Kp / kTcBlockK}));
+    return tc_row_splits(l.N, l.Kp, M, n_sm);
 }
 
 size_t vb200_lm::part_floats(const Linear &l, int max_rows) const {

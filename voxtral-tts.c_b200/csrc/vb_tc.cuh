@@ -49,8 +49,7 @@ struct TcWeight {
 
 /* Activation rows split into BF16 terms: [terms][rows_pad][K], rows_pad = 16, 64 or 256. */
 struct TcActs {
-    CUtensorMap map;
-    CUtensorMap map_rows;   /* rows_pad == 256 only: box of 128 rows (row-block kernel) */
+    CUtensorMap map;        /* rows_pad <= 256 */
     uint16_t *buf;
     int rows_pad, K;
     bool ok;
@@ -130,6 +129,12 @@ void tc_prepare(const TcActs &acts, const float *x, int ldx, int M, const float 
                 cudaStream_t st, const TcWait &wait = TcWait(), float *tap = nullptr);
 
 int tc_gemm(const TcWeight &w, const TcActs &acts, const TcGemm &g, cudaStream_t st);
+/* rows_pad >= 256 (vb_tc_rows.cu; two terms of the activations are read): what tc_gemm calls for them, and the K splits
+ * that suit M rows. */
+int tc_gemm_rows(const TcWeight &w, const TcActs &acts, const TcGemm &g, cudaStream_t st);
+int tc_row_splits(int N, int K, int M, int n_sm);
+/* [rows, cols] BF16 row-major as a tensor map; box = 64 columns x box_rows rows, 128-byte swizzle. */
+int tc_map(CUtensorMap *m, const void *base, uint64_t rows, uint64_t cols, uint32_t box_rows);
 
 /* Grouped GEMM: several weight matrices of equal size stacked in one TcWeight (each padded to whole
  * 128-row tiles), and rows sorted by matrix in blocks of 128. table[b] = {matrix or -1, first row, rows,
