@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 
 import lm_plain as plain
-from lm_models import LIMIT, Case, attention, config, delta, error, feed, tokens
+from lm_models import LIMIT, Case, attention, config, delta, error, feed, latent, tokens
 
 pytestmark = pytest.mark.gpu
 
@@ -18,3 +18,58 @@ def test_float32_gemm_rows(pkg, tmp_path, rows):
     with c.open("float32") as lm:
         s = lm.open()
         assert error(feed(lm, s, toks, [rows, 70]), want) < LIMIT["float32"]
+
+
+@pytest.mark.parametrize("rows", [65, 96, 97, 128, 129, 255, 256, 257, 300])
+def test_row_block_gemm_rows(pkg, tmp_path, rows):
+    """Rows on both sides of the row blocks' edges; matrices of one tile, of odd numbers of tiles and of tiles that are
+    not full, alone and with an activation in the epilogue. The limit is the two-term products'."""
+    c = Case(pkg, tmp_path, config([attention(ff=60, window=0), delta(ff=330)], width=392, vocab=301), seed=rows)
+    toks = tokens(c.cfg, rows, rows)
+    want = plain.forward(c.w, c.cfg, toks)[0]
+    with c.open("bfloat16") as lm:
+        assert error(lm.step(lm.open(), toks, range(rows)), want) < LIMIT["bfloat16"]
+
+
+PROMPT_ATTENTION = {
+    # heads of one, two and three 64-column blocks, sizes that end inside a step of 16; pairs that fill a tile of 128
+    # unevenly; windows and kept tokens on both sides of a 64-key tile
+    "128": attention(heads=8, kv_heads=2, dim=128, vdim=128, window=0, rot=64, scale=0.09, softcap=0, ff=0),
+    "64_8": attention(heads=4, kv_heads=4, dim=64, vdim=8, window=65, keep=3, ff=0),
+    "72_128": attention(heads=6, kv_heads=2, dim=72, vdim=128, window=64, keep=64, scale=0.12, ff=0),
+    "24_72": attention(heads=5, kv_heads=1, dim=24, vdim=72, window=63, keep=1, ff=0),
+    "8_64": attention(heads=3, kv_heads=3, dim=8, vdim=64, window=130, keep=70, rot=8, ff=0),
+    "latent_192_128": latent(heads=2, dim=128, rot_dim=64, vdim=128, kv_rank=64, window=0, scale=0.08, ff=0),
+    "latent_136_72": latent(heads=3, dim=72, rot_dim=64, vdim=72, window=65, scale=0.09, ff=0),
+    "latent_176_16": latent(heads=2, dim=168, rot_dim=8, vdim=16, window=64, scale=0.08, ff=0),
+    "latent_88_64": latent(heads=3, dim=80, rot_dim=8, vdim=64, window=127, scale=0.1, ff=0),
+    "latent_16_8": latent(heads=7, dim=8, rot_dim=8, vdim=8, window=129, ff=0),
+}
+
+
+@pytest.mark.parametrize("name", list(PROMPT_ATTENTION))
+def test_prompt_attention_tiles(pkg, tmp_path, name):
+    """Row tiles, key tiles and head sizes of the prompt attention. The limit is the two-term products'."""
+    c = Case(pkg, tmp_path, config([PROMPT_ATTENTION[name]]), seed=len(name))
+    toks = tokens(c.cfg, 420, 4)
+    want = plain.forward(c.w, c.cfg, toks)[0]
+    with c.open("bfloat16", block_rows=256) as lm:
+        for sizes in ([420], [65, 128, 17, 33], [31, 63]):
+            s = lm.open()
+            assert error(feed(lm, s, toks, sizes), want) < LIMIT["bfloat16"], sizes
+            lm.release(s)
+
+
+@pytest.mark.parametrize("first,rows", [(1, 64), (65, 31), (100, 129), (7, 300)])
+def test_prefill_attention_tiles(pkg, engine, synth_model, first, rows):
+    """A prompt in two calls against the same rows at once. Both are two-term products; a row's sums end in other
+    orders, and what that does to a layer's rows grows over the layers that follow: the limit of the chunking test."""
+    x = pkg.synth_f32((first + rows, 3072), 51, "edge.rows", 0.0, 0.5)
+    engine.prefill(x, 0)
+    whole = [engine.kv_read(l, 0, first + rows) for l in (0, 1, 25)]
+    if first:
+        engine.prefill(x[:first], 0)
+    engine.prefill(x[first:], first)
+    for (k1, v1), l in zip(whole, (0, 1, 25)):
+        k2, v2 = engine.kv_read(l, 0, first + rows)
+        assert np.linalg.norm(k2 - k1) < 1e-4 * np.linalg.norm(k1) and np.linalg.norm(v2 - v1) < 1e-4 * np.linalg.norm(v1), l

@@ -1,0 +1,457 @@
+/*
+ * vb_attn_tc.cuh - softmax attention of many query rows on the 5th-generation tensor cores: prompts of the speech
+ * decoder (vb_prefill.cu) and of the language models (vb_lm_attn.cu).
+ *
+ * A CTA owns one KV head and 128 (row, query head) pairs, so that the heads of a group share every key and value that
+ * is brought in, and walks the visible keys 64 at a time. Every product a.b is taken as a_hi.b_hi + a_hi.b_lo +
+ * a_lo.b_hi on BF16 halves (16 mantissa bits each side), summed in fp32 in TMEM:
+ *
+ *   S [128 x 64]    = Q . K^T   Q high halves in TMEM (A operand), low halves too, or in shared memory for heads over 128
+ *   O [128 x vdim] += P . V     P as halves in TMEM, in S's own columns; V rows [key][dim] are an MN-major B operand
+ *
+ * Scores, softcap, running maximum, weights and sums are fp32, a thread owns a row. Two warpgroups take alternate key
+ * tiles with a maximum, sum and accumulator each (merged at the end), so that the tensor pipe works on one tile while
+ * the other is in its softmax. An accumulator is rescaled only when a row's maximum has risen by more than 2^8: the
+ * reference a row is taken against cancels in the quotient.
+ *
+ * Warps: 0-3, 4-7 softmax, 8-11 bring keys and values into two rings (K slots are free after S, V slots after O), 12
+ * issues the MMAs. All waits are bounded.
+ *
+ * What bounds it: a 64-key tile of 128-wide heads costs the tensor pipe 8 x 3 x 32 + 4 x 3 x 64 = 1536 clocks and the
+ * softmax about as much; the warp-level MMAs used before (mma.sync, 16 rows per warp) ran at 44 useful TFLOP/s.
+ */
+#ifndef VB_ATTN_TC_CUH
+#define VB_ATTN_TC_CUH
+
+#include "vb_lm_attn.cuh"
+#include "vb_umma.cuh"
+
+namespace vb {
+
+constexpr int kAtRows = 128, kAtKeys = 64;
+constexpr int kAtSoft = 256, kAtLoaders = 128, kAtThreads = kAtSoft + kAtLoaders + 32;
+constexpr int kAtBlock = kAtKeys * 128;            /* 64 keys x 64 columns */
+constexpr int kAtStatus = 52;
+constexpr uint32_t kAtTmemCols = 512, kAtO = 128, kAtQ = 384;
+
+/* What every use has in common. */
+struct AtArgs {
+    int M, heads, kv_heads, dim, vdim;
+    int window, keep;
+    float scale, softcap;
+    int *status;
+};
+
+template <int DK, int DV>
+struct AtCfg {
+    static constexpr bool kQlTmem = DK <= 2;
+    static constexpr int kSlots = DK <= 2 ? 3 : 2;
+    static constexpr int kSlotK = 2 * DK * kAtBlock, kSlotV = 2 * DV * kAtBlock;
+    static constexpr int kQl = kQlTmem ? 0 : DK * kAtRows * 128;
+    static constexpr int kSmem = kQl + kSlots * (kSlotK + kSlotV) + 1024 + 256;
+    static_assert(kSmem <= 232448, "over the 227 KB a CTA may use");
+    static_assert(kAtQ + (kQlTmem ? 2 : 1) * DK * 32 <= kAtTmemCols, "Q does not fit TMEM");
+};
+
+VB_DEVINL void at_mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+#define VB_AT_R8(r, o) "r"((r)[o]), "r"((r)[o + 1]), "r"((r)[o + 2]), "r"((r)[o + 3]), "r"((r)[o + 4]), "r"((r)[o + 5]), "r"((r)[o + 6]), "r"((r)[o + 7])
+#define VB_AT_W8(r, o) "=r"((r)[o]), "=r"((r)[o + 1]), "=r"((r)[o + 2]), "=r"((r)[o + 3]), "=r"((r)[o + 4]), "=r"((r)[o + 5]), "=r"((r)[o + 6]), "=r"((r)[o + 7])
+/* 32 columns of this thread's TMEM lane; at_ld_wait before the values are used, at_st_wait before they are handed on */
+VB_DEVINL void at_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : VB_AT_W8(r, 0), VB_AT_W8(r, 8), VB_AT_W8(r, 16), VB_AT_W8(r, 24)
+        : "r"(taddr)
+        : "memory");
+}
+VB_DEVINL void at_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31};"
+        ::VB_AT_R8(r, 0), VB_AT_R8(r, 8), VB_AT_R8(r, 16), VB_AT_R8(r, 24), "r"(taddr)
+        : "memory");
+}
+VB_DEVINL void at_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+VB_DEVINL void at_proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+VB_DEVINL float at_ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+/* vb_mbar_wait with one answer for the warp: no lane leaves the others alone in a warp-wide instruction */
+VB_DEVINL bool at_warp_wait(uint64_t *bar, uint32_t parity, volatile int *cta_abort) {
+    return __all_sync(0xffffffffu, vb_mbar_wait(bar, parity, cta_abort));
+}
+/* Two values as packed BF16 high halves and packed remainders. */
+VB_DEVINL void at_split2(float a, float b, uint32_t &hi, uint32_t &lo) {
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(b), "f"(a));
+    const float ra = a - __uint_as_float(hi << 16), rb = b - __uint_as_float(hi & 0xffff0000u);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(rb), "f"(ra));
+}
+
+/* cap * tanh(x / cap), the hyperbolic tangent through one exponential (absolute error about 1e-7 of cap) */
+VB_DEVINL float soft_cap(float x, float cap, float two_over_cap) {
+    return cap - 2.0f * cap * __fdividef(1.0f, 1.0f + __expf(x * two_over_cap));
+}
+
+/* Rows [key][64 dims] as the B operand of P . V, read along the dims (MN-major): groups of eight keys 1024 bytes apart,
+ * blocks of 64 dims kAtBlock apart. */
+VB_DEVINL uint64_t at_desc_mn(uint32_t addr) {
+    uint64_t d = (uint64_t)((addr >> 4) & 0x3FFF);
+    d |= (uint64_t)(kAtBlock >> 4) << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
+    return d;
+}
+VB_DEVINL uint32_t at_idesc(int n, bool mn_major) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (mn_major ? 1u << 16 : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kAtRows >> 4) << 24);
+}
+/* Byte offset of 16-byte chunk `chunk` (0..7) of a 128-byte row, as the 128-byte swizzle has it */
+VB_DEVINL uint32_t at_off(int row, int chunk) { return (uint32_t)(row * 128 + (((chunk ^ row) & 7) << 4)); }
+
+/* A use (SRC) says where things come from and go:
+ *   kAsync                       keys and values are copied with cp.async (else: stored by the loading threads)
+ *   start()                      after the wait for the previous kernel: resolves what lies in device memory
+ *   pos0()                       position of row 0
+ *   q8(row, head, d, v)          eight query values (zeros beyond the head)
+ *   keys(...) / values(...)      a loading warp's 16 keys of a tile, into blocks of 64 columns: high halves, then low ones
+ *   gate(row, head)              factor of a result row
+ *   put4(row, column, v)         four results */
+template <int DK, int DV, class SRC>
+__global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const AtArgs a, const SRC src_arg) {
+    using Cfg = AtCfg<DK, DV>;
+    extern __shared__ unsigned char at_smem_raw[];
+    unsigned char *base = (unsigned char *)(((uintptr_t)at_smem_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char *ql_s = base, *k_s = ql_s + Cfg::kQl, *v_s = k_s + Cfg::kSlots * Cfg::kSlotK;
+    uint64_t *bars = (uint64_t *)(v_s + Cfg::kSlots * Cfg::kSlotV);
+    uint64_t *k_full = bars, *k_empty = k_full + Cfg::kSlots, *v_full = k_empty + Cfg::kSlots, *v_empty = v_full + Cfg::kSlots;
+    uint64_t *s_full = v_empty + Cfg::kSlots, *p_full = s_full + 2, *o_done = p_full + 2, *q_full = o_done + 2;
+    uint32_t *tmem_slot = (uint32_t *)(q_full + 1);
+    int *abort_flag = (int *)(tmem_slot + 1);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int i = 0; i < Cfg::kSlots; i++) {
+            vb_mbar_init(&k_full[i], kAtLoaders);
+            vb_mbar_init(&v_full[i], kAtLoaders);
+            vb_mbar_init(&k_empty[i], 1);
+            vb_mbar_init(&v_empty[i], 1);
+        }
+        for (int i = 0; i < 2; i++) {
+            vb_mbar_init(&s_full[i], 1);
+            vb_mbar_init(&p_full[i], 128);
+            vb_mbar_init(&o_done[i], 1);
+        }
+        vb_mbar_init(q_full, kAtSoft);
+        *abort_flag = 0;
+        vb_mbar_init_fence();
+    }
+    if (warp == 12) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(vb_smem_u32(tmem_slot)), "r"(kAtTmemCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *(volatile uint32_t *)tmem_slot;
+    pdl_launch_dependents();       /* not before the allocation: a GEMM that starts early must not take columns this kernel needs */
+    pdl_wait();
+
+    SRC src = src_arg;
+    src.start();
+    const int group = a.heads / a.kv_heads, g = blockIdx.x;
+    const int pairs = a.M * group, pos0 = src.pos0();
+    const int P0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kAtRows;           /* the latest rows see the most keys: they go first */
+    const int last = P0 + kAtRows < pairs ? P0 + kAtRows - 1 : pairs - 1;
+    const int imin = pos0 + P0 / group, imax = pos0 + last / group;
+    const KeyTiles kt = key_tiles<kAtKeys>(imin, imax, a.window, a.keep);
+    const int n_tiles = kt.n_tiles;
+
+    auto give_up = [&]() {
+        atomicCAS(a.status, 0, kAtStatus);
+        *(volatile int *)abort_flag = 1;
+    };
+
+    if (warp < 8) {
+        /* ---- softmax: warpgroup w takes key tiles w, w + 2, ...; a thread owns pair P0 + r ---- */
+        const int w = warp >> 2, r = tid & 127, P = P0 + r;
+        const bool valid = P < pairs;
+        const int row = valid ? P / group : 0, head = g * group + (valid ? P - row * group : 0), i = pos0 + row;
+        const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16, tS = tmem + lanes + (uint32_t)(w * kAtKeys), tO = tmem + lanes + kAtO + (uint32_t)(w * 128);
+        /* the query row: its high halves go to TMEM by the first warpgroup, its low ones by the second */
+#pragma unroll 1
+        for (int kb = 0; kb < DK; kb++) {
+            uint32_t reg[32];
+#pragma unroll
+            for (int c = 0; c < 8; c++) {
+                float e[8];
+                if (valid) src.q8(row, head, kb * 64 + c * 8, e);
+                else
+#pragma unroll
+                    for (int j = 0; j < 8; j++) e[j] = 0.0f;
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    uint32_t hi, lo;
+                    at_split2(e[2 * j], e[2 * j + 1], hi, lo);
+                    reg[c * 4 + j] = w == 0 ? hi : lo;
+                }
+            }
+            if (w == 0 || Cfg::kQlTmem) {
+                at_st32(tmem + lanes + kAtQ + (uint32_t)((w * DK + kb) * 32), reg);
+            } else {
+#pragma unroll
+                for (int c = 0; c < 8; c++)
+                    *reinterpret_cast<uint4 *>(ql_s + kb * kAtRows * 128 + at_off(r, c)) = make_uint4(reg[c * 4], reg[c * 4 + 1], reg[c * 4 + 2], reg[c * 4 + 3]);
+            }
+        }
+        at_st_wait();
+        at_proxy_fence();
+        tc_fence_before();
+        vb_mbar_arrive(q_full);
+
+        const float kLog2eHi = 1.44269502f, kLog2eLo = 1.92596303e-8f;
+        const float two_over_cap = a.softcap > 0.0f ? 2.0f / a.softcap : 0.0f;
+        float ref = -INFINITY, sum = 0.0f;      /* the row's reference (in powers of two), its sum of weights against it */
+        int it = 0;
+        for (int t = w; t < n_tiles; t += 2, it++) {
+            int j0, n;
+            key_tile<kAtKeys>(kt, t, &j0, &n);
+            if (!at_warp_wait(&s_full[w], (uint32_t)it & 1u, abort_flag)) { give_up(); break; }
+            tc_fence_after();
+            float s[kAtKeys];
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                uint32_t reg[32];
+                at_ld32(tS + (uint32_t)(c * 32), reg);
+#pragma unroll
+                for (int k = 0; k < 32; k++) s[c * 32 + k] = __uint_as_float(reg[k]) * a.scale;
+            }
+            if (a.softcap > 0.0f) {
+#pragma unroll
+                for (int k = 0; k < kAtKeys; k++) s[k] = soft_cap(s[k], a.softcap, two_over_cap);
+            }
+            const bool all_seen = n == kAtKeys && j0 + kAtKeys - 1 <= imin && (a.window <= 0 || imax - j0 < a.window || j0 + kAtKeys <= a.keep);
+            if (!all_seen) {
+                const int k_end = n - 1 < i - j0 ? n - 1 : i - j0;               /* last one not too late */
+                const int k_win = a.window > 0 ? i - a.window + 1 - j0 : 0, k_keep = a.keep - j0;
+#pragma unroll
+                for (int k = 0; k < kAtKeys; k++)
+                    if (k > k_end || (k < k_win && k >= k_keep)) s[k] = -INFINITY;
+            }
+            float top4[4] = {s[0], s[1], s[2], s[3]};
+#pragma unroll
+            for (int k = 4; k < kAtKeys; k++) top4[k & 3] = fmaxf(top4[k & 3], s[k]);
+            const float top = fmaxf(fmaxf(top4[0], top4[1]), fmaxf(top4[2], top4[3])) * kLog2eHi;
+            const bool rise = top > ref + 8.0f;
+            if (__any_sync(0xffffffffu, rise)) {
+                const float now = rise ? top : ref, f = rise ? at_ex2(ref - now) : 1.0f;     /* the first time: 0 */
+                if (it > 0) {
+                    if (!at_warp_wait(&o_done[w], (uint32_t)(it - 1) & 1u, abort_flag)) { give_up(); break; }
+                    tc_fence_after();
+#pragma unroll 1
+                    for (int c = 0; c < 2 * DV; c++) {
+                        uint32_t reg[32];
+                        at_ld32(tO + (uint32_t)(c * 32), reg);
+#pragma unroll
+                        for (int k = 0; k < 32; k++) reg[k] = __float_as_uint(__uint_as_float(reg[k]) * f);
+                        at_st32(tO + (uint32_t)(c * 32), reg);
+                    }
+                }
+                sum *= f;
+                ref = now;
+            }
+            const float m = ref > -INFINITY ? ref : 0.0f;         /* no key seen yet: every weight below is 2^-inf = 0 */
+            float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                uint32_t reg[32];
+#pragma unroll
+                for (int k = 0; k < 32; k += 2) {
+                    float p[2];
+#pragma unroll
+                    for (int u = 0; u < 2; u++) {
+                        const float x = s[c * 32 + k + u];
+                        p[u] = at_ex2(fmaf(x, kLog2eLo, fmaf(x, kLog2eHi, -m)));
+                        sum4[(k + u) & 3] += p[u];
+                    }
+                    at_split2(p[0], p[1], reg[k / 2], reg[16 + k / 2]);
+                }
+                at_st32(tS + (uint32_t)(c * 32), reg);            /* 16 columns of high halves, 16 of low ones */
+            }
+            sum += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+            at_st_wait();
+            tc_fence_before();
+            vb_mbar_arrive(&p_full[w]);
+        }
+        if (it > 0 && !at_warp_wait(&o_done[w], (uint32_t)(it - 1) & 1u, abort_flag)) give_up();
+        /* both halves of the keys, merged: each warpgroup writes half of the columns */
+        vb_named_bar(1, kAtSoft);                                 /* every product is done: the rings are free */
+        float2 *ml = reinterpret_cast<float2 *>(k_s);
+        ml[w * kAtRows + r] = make_float2(ref, sum);
+        tc_fence_before();
+        vb_named_bar(1, kAtSoft);
+        tc_fence_after();
+        const float2 A = ml[r], B = ml[kAtRows + r];
+        const float top = fmaxf(A.x, B.x);
+        const float fa = A.y > 0.0f ? at_ex2(A.x - top) : 0.0f, fb = B.y > 0.0f ? at_ex2(B.x - top) : 0.0f;
+        const float inv = 1.0f / (A.y * fa + B.y * fb) * (valid ? src.gate(row, head) : 1.0f);
+        const float ra = fa * inv, rb = fb * inv;
+#pragma unroll 1
+        for (int c = w * DV; c < w * DV + DV; c++) {
+            if (c * 32 >= a.vdim) break;
+            uint32_t oa[32], ob[32];
+            at_ld32(tmem + lanes + kAtO + (uint32_t)(c * 32), oa);
+            if (n_tiles > 1) {
+                at_ld32(tmem + lanes + kAtO + 128u + (uint32_t)(c * 32), ob);
+#pragma unroll
+                for (int k = 0; k < 32; k++)
+                    oa[k] = __float_as_uint(__uint_as_float(oa[k]) * ra + __uint_as_float(ob[k]) * rb);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 32; k++) oa[k] = __float_as_uint(__uint_as_float(oa[k]) * ra);
+            }
+            if (valid) {
+#pragma unroll
+                for (int k = 0; k < 32; k += 4) {
+                    const float v[4] = {__uint_as_float(oa[k]), __uint_as_float(oa[k + 1]), __uint_as_float(oa[k + 2]), __uint_as_float(oa[k + 3])};
+                    if (c * 32 + k < a.vdim) src.put4(row, head * a.vdim + c * 32 + k, v);
+                }
+            }
+        }
+    } else if (warp < 12) {
+        /* ---- keys and values: K0, K1, V0, K2, V1, ... as the MMAs take them ---- */
+        const int lw = warp - 8;
+        if (a.dim % 16) {          /* the last 16 columns of a product reach beyond the head: zeros there, for good */
+            const int chunk = a.dim / 8;
+            for (int x = tid - kAtSoft; x < Cfg::kSlots * 2 * kAtKeys; x += kAtLoaders) {
+                const int key = x % kAtKeys, plane = x / kAtKeys;
+                *reinterpret_cast<uint4 *>(k_s + (plane * DK + (chunk >> 3)) * kAtBlock + at_off(key, chunk)) = make_uint4(0u, 0u, 0u, 0u);
+            }
+        }
+        int told = 0;              /* steps before this one are handed over */
+        auto hand_over = [&](int upto) {
+            if (told >= upto) return;
+            at_proxy_fence();
+            for (; told < upto; told++) {
+                if (told == 2 * n_tiles - 1) continue;
+                const bool is_k = told == 0 || (told & 1);
+                const int t = is_k ? (told + 1) / 2 : told / 2 - 1;
+                vb_mbar_arrive(is_k ? &k_full[t % Cfg::kSlots] : &v_full[t % Cfg::kSlots]);
+            }
+        };
+        for (int step = 0; step <= 2 * n_tiles; step++) {
+            if (step != 2 * n_tiles - 1) {
+                const bool is_k = step == 0 || (step & 1);
+                const int t = is_k ? (step + 1) / 2 : step / 2 - 1, slot = t % Cfg::kSlots;
+                uint64_t *empty = is_k ? &k_empty[slot] : &v_empty[slot];
+                const uint32_t parity = ((uint32_t)(t / Cfg::kSlots) & 1u) ^ 1u;
+                if (!__all_sync(0xffffffffu, vb_mbar_try_wait(empty, parity))) {
+                    if constexpr (SRC::kAsync) {         /* what waits for the slot may wait for what is on its way */
+                        lm_cp_wait_all();
+                        hand_over(step);
+                    }
+                    if (!at_warp_wait(empty, parity, abort_flag)) { give_up(); break; }
+                }
+                int j0, n;
+                key_tile<kAtKeys>(kt, t, &j0, &n);
+                if (is_k) src.template keys<DK>(a, k_s + slot * Cfg::kSlotK, g, lw, lane, j0, n);
+                else src.template values<DV>(a, v_s + slot * Cfg::kSlotV, g, lw, lane, j0, n);
+            }
+            if constexpr (SRC::kAsync) {
+                lm_cp_commit();
+                asm volatile("cp.async.wait_group 2;" ::: "memory");
+                hand_over(step - 1);
+            } else {
+                hand_over(step + 1);
+            }
+        }
+        if constexpr (SRC::kAsync) lm_cp_wait_all();
+        if (!*(volatile int *)abort_flag) hand_over(2 * n_tiles + 1);
+    } else if (lane == 0) {
+        /* ---- MMA issuer ---- */
+        const int k_steps = (a.dim + 15) / 16;
+        const uint32_t idesc_s = at_idesc(kAtKeys, false), idesc_o = at_idesc((a.vdim + 15) & ~15, true);
+        bool ok = vb_mbar_wait(q_full, 0u, abort_flag);
+        tc_fence_after();
+        auto scores = [&](int t) {
+            const int slot = t % Cfg::kSlots;
+            if (!vb_mbar_wait(&k_full[slot], (uint32_t)(t / Cfg::kSlots) & 1u, abort_flag)) return false;
+            tc_fence_after();
+            const unsigned char *kp = k_s + slot * Cfg::kSlotK;
+            const uint32_t d = tmem + (uint32_t)((t & 1) * kAtKeys);
+            for (int ks = 0; ks < k_steps; ks++) {
+                const uint64_t hi = umma_desc_k_sw128(kp + (ks >> 2) * kAtBlock) + 2 * (ks & 3);
+                const uint64_t lo = umma_desc_k_sw128(kp + (DK + (ks >> 2)) * kAtBlock) + 2 * (ks & 3);
+                const uint32_t qh = tmem + kAtQ + (uint32_t)(ks * 8);
+                at_mma_ts(d, qh, hi, idesc_s, ks != 0 ? 1u : 0u);
+                at_mma_ts(d, qh, lo, idesc_s, 1u);
+                if constexpr (Cfg::kQlTmem) at_mma_ts(d, qh + DK * 32, hi, idesc_s, 1u);
+                else umma_bf16(d, umma_desc_k_sw128(ql_s + (ks >> 2) * kAtRows * 128) + 2 * (ks & 3), hi, idesc_s, 1u);
+            }
+            umma_commit(&k_empty[slot]);
+            umma_commit(&s_full[t & 1]);
+            return true;
+        };
+        ok = ok && n_tiles > 0 && scores(0);
+        if (ok && n_tiles > 1) ok = scores(1);
+        for (int t = 0; t < n_tiles && ok; t++) {
+            const int w = t & 1, slot = t % Cfg::kSlots;
+            ok = vb_mbar_wait(&v_full[slot], (uint32_t)(t / Cfg::kSlots) & 1u, abort_flag) &&
+                 vb_mbar_wait(&p_full[w], (uint32_t)(t >> 1) & 1u, abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t vp = vb_smem_u32(v_s + slot * Cfg::kSlotV);
+            const uint32_t d = tmem + kAtO + (uint32_t)(w * 128);
+#pragma unroll
+            for (int ks = 0; ks < kAtKeys / 16; ks++) {
+                const uint64_t hi = at_desc_mn(vp + ks * 2048), lo = at_desc_mn(vp + DV * kAtBlock + ks * 2048);
+                const uint32_t ph = tmem + (uint32_t)(w * kAtKeys + (ks >> 1) * 32 + (ks & 1) * 8);
+                at_mma_ts(d, ph, hi, idesc_o, (t >> 1 | ks) != 0 ? 1u : 0u);
+                at_mma_ts(d, ph, lo, idesc_o, 1u);
+                at_mma_ts(d, ph + 16, hi, idesc_o, 1u);
+            }
+            umma_commit(&v_empty[slot]);
+            umma_commit(&o_done[w]);
+            /* takes the columns of P once the products above have read them: MMAs of one thread run in order */
+            if (t + 2 < n_tiles) ok = scores(t + 2);
+        }
+        if (!ok) give_up();
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 12) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kAtTmemCols) : "memory");
+    }
+}
+
+template <int DK, int DV, class SRC>
+int launch_attn_tc(const AtArgs &a, const SRC &src, cudaStream_t st) {
+    using Cfg = AtCfg<DK, DV>;
+    static bool attr = false;
+    if (!attr) {
+        if (cudaFuncSetAttribute(vb_attn_tc_kernel<DK, DV, SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem) != cudaSuccess) {
+            cudaGetLastError();
+            return -1;
+        }
+        attr = true;
+    }
+    const int tiles = (int)(((long long)a.M * (a.heads / a.kv_heads) + kAtRows - 1) / kAtRows);
+    return launch_pdl(vb_attn_tc_kernel<DK, DV, SRC>, dim3(a.kv_heads, tiles), dim3(kAtThreads), (size_t)Cfg::kSmem, st, a, src) == cudaSuccess
+               ? 0
+               : -1;
+}
+
+} // namespace vb
+
+#endif

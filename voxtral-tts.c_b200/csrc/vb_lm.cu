@@ -796,6 +796,7 @@ int vb200_lm::latent_wide(const Layer &l, const LmMixer &m, const LmLatent &a, c
     t.heads = t.kv_heads = m.heads; t.dim = m.dim + m.rot_dim; t.vdim = m.vdim;
     t.window = m.mask.window; t.scale = (float)m.scale; t.rot = m.rope.dims;
     t.ring = s.ring;
+    t.status = status;
     t.out = a.out;
     LmWide w = {};
     w.kv = wide; w.plane = (size_t)rp * l.mix.ukv.N; w.ld = l.mix.ukv.N; w.v0 = m.heads * m.dim; w.first = first;
@@ -901,7 +902,7 @@ int vb200_lm::mixer(const Layer &l, const LmLayer &spec, const RunState &s, int 
         a.ring = s.ring;
         a.k = {slabs + s.a, slab}; a.v = {slabs + s.b, slab};
         a.split = !f32() && lm_attn_mma_ok(m.dim, m.vdim);
-        a.qkv = in; a.q = q; a.scratch = scratch; a.tickets = tickets;
+        a.qkv = in; a.q = q; a.scratch = scratch; a.tickets = tickets; a.status = status;
         a.out = sink(l.mix.acts, M);
         if (M == 1 && lm_attn_step_ok(a)) {
             LM_DO(lm_attn_step(a, st));

@@ -8,13 +8,13 @@
  *   lm_attn_generic  fp32 pipes: any sizes, short portions and the 32-bit mode (keys split over CTAs,
  *                    last arrival merges)
  *   lm_attn_step     one token, preparation included
- *   lm_attn_mma      prompts: mma.sync on hi + lo BF16 halves of q, k, v and the weights; the cache keeps
- *                    k and v as such halves
+ *   lm_attn_mma      prompts: tensor cores on hi + lo BF16 halves of q, k, v and the weights (vb_attn_tc.cuh); the
+ *                    cache keeps k and v as such halves
  *
  * Keys are visited in two stretches, the kept first tokens and the window; a stretch that is out
  * of reach of all of a CTA's rows is never loaded.
  */
-#include "vb_lm_attn.cuh"
+#include "vb_attn_tc.cuh"
 #include "vb_tc.cuh"
 
 namespace vb {
@@ -472,254 +472,136 @@ int launch_attn_step(const LmAttn &a, int splits, int lanes_h, cudaStream_t st) 
     return ok(launch_pdl(lm_attn_step_kernel<ND, NV, KP, SPLIT>, dim3(splits, a.kv_heads), dim3(kSaThreads), smem, st, a, lanes_h));
 }
 
-/* ------------------------------------------------------------------ prompts on the warp-level tensor cores */
-constexpr int kMaThreads = 256, kMaWarps = 8, kMaKeys = 32;
+/* ------------------------------------------------------------------ prompts on the tensor cores (vb_attn_tc.cuh) */
+/* Rows of a value tile beyond its keys: their weights are zero, and so must they be. */
+template <int BLOCKS>
+VB_DEVINL void clear_keys(unsigned char *slot, int lw, int lane, int n) {
+    for (int key = n > lw * 16 ? n : lw * 16; key < lw * 16 + 16; key++)
+        for (int f = lane; f < 2 * BLOCKS * 8; f += 32) *reinterpret_cast<uint4 *>(slot + (f >> 3) * kAtBlock + at_off(key, f)) = make_uint4(0u, 0u, 0u, 0u);
+}
 
-/* Requests 32 keys of one KV head: the high and low halves of the cache rows, 16 bytes per copy,
- * straight into the swizzled tiles. What lies beyond the head's size in a tile is not touched. */
-template <int STEPS>
-VB_DEVINL void request_tile(unsigned char *hi_t, const float *cache, int ld, int col0, int size, int j0, int n, const LmRing &ring) {
-    const int per = size / 8;                           /* chunks of a plane */
-    for (int i = threadIdx.x; i < n * 2 * per; i += kMaThreads) {
-        const int key = i / (2 * per), f = i % (2 * per), plane = f >= per ? 1 : 0, chunk = f - plane * per;
-        const uint16_t *src = reinterpret_cast<const uint16_t *>(cache + (size_t)lm_ring_row(ring, j0 + key) * ld + col0) + f * 8;
-        lm_cp16(hi_t + plane * (kMaKeys * STEPS * 32) + tile_off<STEPS>(key, chunk), src);
+/* Keys and values from a cache of split rows. */
+struct AtCache {
+    static constexpr bool kAsync = true;
+    const LmDyn *dyn;
+    const float *q;
+    LmState k, v;
+    LmRing ring;
+    LmSink out;
+    int heads, kv_heads, dim, vdim;
+    const float *kc, *vc;
+    VB_DEVINL void start() { kc = lm_state(k, dyn); vc = lm_state(v, dyn); }
+    VB_DEVINL int pos0() const { return dyn->pos; }
+    VB_DEVINL void q8(int row, int head, int d, float (&e)[8]) const {
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+        if (d < dim) {
+            const float4 *p = reinterpret_cast<const float4 *>(q + ((size_t)row * heads + head) * dim + d);
+            x = p[0];
+            y = p[1];
+        }
+        e[0] = x.x; e[1] = x.y; e[2] = x.z; e[3] = x.w; e[4] = y.x; e[5] = y.y; e[6] = y.z; e[7] = y.w;
     }
-}
-/* The same out of keys and values that were read out of a latent: a head's own columns from the written-out
- * rows, then `shared` columns (the key part all heads have in common) from the latent's cache row. */
-template <int STEPS>
-VB_DEVINL void request_wide(unsigned char *hi_t, const LmWide &w, int col0, int size, int shared, int j0, int n, const LmRing &ring) {
-    const int own = size / 8, per = own + shared / 8, row = w.rank + w.rot_dim;
-    for (int i = threadIdx.x; i < n * 2 * per; i += kMaThreads) {
-        const int key = i / (2 * per), f = i % (2 * per), plane = f >= per ? 1 : 0, chunk = f - plane * per;
-        const uint16_t *src;
-        if (chunk < own) src = w.kv + plane * w.plane + (size_t)(j0 + key - w.first) * w.ld + col0 + chunk * 8;
-        else src = reinterpret_cast<const uint16_t *>(w.cache + (size_t)lm_ring_row(ring, j0 + key) * row) + plane * row + w.rank + (chunk - own) * 8;
-        lm_cp16(hi_t + plane * (kMaKeys * STEPS * 32) + tile_off<STEPS>(key, chunk), src);
+    template <int BLOCKS>
+    VB_DEVINL void rows(const float *cache, int size, unsigned char *slot, int g, int lw, int lane, int j0, int n) const {
+        const int key = lw * 16 + (lane & 15);
+        const int own = lm_ring_row(ring, j0 + (key < n ? key : n - 1));
+        const int ld = kv_heads * size, per = size / 8;
+        int at[16];
+#pragma unroll
+        for (int x = 0; x < 16; x++) at[x] = __shfl_sync(0xffffffffu, own, x);
+#pragma unroll 1
+        for (int f = lane; f < 2 * per; f += 32) {
+            const int plane = f >= per ? 1 : 0, chunk = f - plane * per;
+            unsigned char *block = slot + (plane * BLOCKS + (chunk >> 3)) * kAtBlock;
+            const uint16_t *col = reinterpret_cast<const uint16_t *>(cache + g * size) + f * 8;
+#pragma unroll
+            for (int x = 0; x < 16; x++)
+                if (lw * 16 + x < n) lm_cp16(block + at_off(lw * 16 + x, chunk), col + (size_t)at[x] * ld * 2);
+        }
     }
-}
+    template <int BLOCKS>
+    VB_DEVINL void keys(const AtArgs &, unsigned char *slot, int g, int lw, int lane, int j0, int n) const {
+        rows<BLOCKS>(kc, dim, slot, g, lw, lane, j0, n);
+    }
+    template <int BLOCKS>
+    VB_DEVINL void values(const AtArgs &, unsigned char *slot, int g, int lw, int lane, int j0, int n) const {
+        rows<BLOCKS>(vc, vdim, slot, g, lw, lane, j0, n);
+        clear_keys<BLOCKS>(slot, lw, lane, n);
+    }
+    VB_DEVINL float gate(int, int) const { return 1.0f; }
+    VB_DEVINL void put4(int row, int c, const float (&e)[4]) const { lm_put4(out, row, c, e); }
+};
 
-struct LmNotWide {};
-template <bool WIDE> struct LmWideSel { using type = LmNotWide; };
-template <> struct LmWideSel<true> { using type = LmWide; };
-
-/* cap * tanh(x / cap), the hyperbolic tangent through one exponential (absolute error about 1e-7 of cap) */
-VB_DEVINL float soft_cap(float x, float cap, float two_over_cap) {
-    return cap - 2.0f * cap * __fdividef(1.0f, 1.0f + __expf(x * two_over_cap));
-}
-
-/* WIDE: every head has keys and values of its own, read out of a latent (LmWide).
- * A CTA serves one KV head; each of its eight warps owns 16 query rows of one query head of the
- * group (consecutive (row block, head) tiles), so that the staged keys are shared by up to eight
- * warps. Every product a.b is taken as a_hi.b_hi + a_hi.b_lo + a_lo.b_hi, accumulated in fp32;
- * scores, softcap, weights and the running maximum are fp32. DK, DV: 16-wide steps of the key
- * and value sizes (padded with zeros). */
-template <int DK, int DV, bool WIDE>
-__global__ void __launch_bounds__(kMaThreads) lm_attn_mma_kernel(const LmAttn a, const typename LmWideSel<WIDE>::type wide, int M) {
-    extern __shared__ __align__(128) unsigned char ma_tiles[];
-    /* two buffers of K high, K low, V high, V low */
-    constexpr int kTileK = kMaKeys * DK * 32, kTileV = kMaKeys * DV * 32, kBuf = 2 * (kTileK + kTileV);
-    pdl_launch_dependents();
-    for (int i = threadIdx.x; i < 2 * kBuf / 16; i += kMaThreads) reinterpret_cast<uint4 *>(ma_tiles)[i] = make_uint4(0u, 0u, 0u, 0u);
-    pdl_wait();
-    __syncthreads();
-    const int group = a.heads / a.kv_heads, g = blockIdx.y;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
-    const int n_tiles_q = (M + 15) / 16 * group;
-    /* the latest rows see the most keys: they go first */
-    const int T0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * kMaWarps, T1 = T0 + kMaWarps < n_tiles_q ? T0 + kMaWarps : n_tiles_q;
-    const int T = T0 + warp;
-    const bool active = T < T1;
-    const int r0 = active ? T / group * 16 : 0, h = g * group + (active ? T % group : 0);
-    const int pos0 = a.dyn->pos;
-    const int rowA = r0 + gq, rowB = rowA + 8;
-    const bool validA = active && rowA < M, validB = active && rowB < M;
-    const int iA = pos0 + rowA, iB = pos0 + rowB;
-    const int last_row = T1 > T0 ? ((T1 - 1) / group * 16 + 15 < M - 1 ? (T1 - 1) / group * 16 + 15 : M - 1) : 0;
-    const KeyTiles kt = key_tiles<kMaKeys>(pos0 + T0 / group * 16, pos0 + last_row, a.window, a.keep);
-    const int w_imin = pos0 + r0, w_imax = pos0 + (r0 + 15 < M - 1 ? r0 + 15 : M - 1);
-    const float *Kc = nullptr, *Vc = nullptr;
-    if constexpr (!WIDE) { Kc = lm_state(a.k, a.dyn); Vc = lm_state(a.v, a.dyn); }
-    const int ldk = a.kv_heads * a.dim, ldv = a.kv_heads * a.vdim;
-    typename LmWideSel<WIDE>::type lw = wide;
-    if constexpr (WIDE) lw.cache += (size_t)a.dyn->slot * lw.slab;
-
-    /* Q as A fragments: (row A, k 2t..), (row B, k 2t..), (row A, k 8 + 2t..), (row B, k 8 + 2t..) */
-    uint32_t qh[DK][4], ql[DK][4];
+/* Every head has keys and values of its own, read out of a latent (LmWide): a head's own columns of the written-out
+ * rows, then the key part that all heads share from the latent's cache row. */
+struct AtWide {
+    static constexpr bool kAsync = true;
+    const LmDyn *dyn;
+    LmWide w;
+    LmRing ring;
+    LmSink out;
+    int heads, dim, vdim, rot;
+    VB_DEVINL void start() { w.cache += (size_t)dyn->slot * w.slab; }
+    VB_DEVINL int pos0() const { return dyn->pos; }
+    VB_DEVINL void q8(int row, int head, int d, float (&e)[8]) const {
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+        if (d < dim) {
+            x = lm_sum4(w.q, row, head * dim + d);
+            y = lm_sum4(w.q, row, head * dim + d + 4);
+        }
+        e[0] = x.x; e[1] = x.y; e[2] = x.z; e[3] = x.w; e[4] = y.x; e[5] = y.y; e[6] = y.z; e[7] = y.w;
+        const int half = rot / 2, i0 = (d - (dim - w.rot_dim)) / 2;
+        if (d >= dim - w.rot_dim && d < dim) {
 #pragma unroll
-    for (int ks = 0; ks < DK; ks++)
-#pragma unroll
-        for (int hf = 0; hf < 2; hf++)
-#pragma unroll
-            for (int rr = 0; rr < 2; rr++) {
-                const int d = ks * 16 + hf * 8 + 2 * tq;
-                const bool v = rr ? validB : validA;
-                float q0 = 0.0f, q1 = 0.0f;
-                if constexpr (WIDE) {
-                    if (v && d < a.dim) {          /* dim is a multiple of 8: d and d + 1 are a rotated pair or neither is */
-                        const int row = rr ? rowB : rowA, i = (d - (a.dim - wide.rot_dim)) / 2, half = a.rot / 2;
-                        const float2 u = lm_sum2(wide.q, row, h * a.dim + d);
-                        q0 = u.x; q1 = u.y;
-                        if (d >= a.dim - wide.rot_dim && i < half) {
-                            const float c = wide.cs[(size_t)row * a.rot + i], s = wide.cs[(size_t)row * a.rot + half + i];
-                            q0 = u.x * c - u.y * s;
-                            q1 = u.y * c + u.x * s;
-                        }
-                    }
-                } else {
-                    const float *q = a.q + (size_t)(rr ? rowB : rowA) * a.heads * a.dim + (size_t)h * a.dim + d;
-                    if (v && d < a.dim) q0 = q[0];
-                    if (v && d + 1 < a.dim) q1 = q[1];
+            for (int i = 0; i < 4; i++) {
+                if (i0 + i < half) {
+                    const float c = w.cs[(size_t)row * rot + i0 + i], s = w.cs[(size_t)row * rot + half + i0 + i];
+                    const float u = e[2 * i], t = e[2 * i + 1];
+                    e[2 * i] = u * c - t * s;
+                    e[2 * i + 1] = t * c + u * s;
                 }
-                uint32_t h0, l0, h1, l1;
-                hilo(q0, h0, l0);
-                hilo(q1, h1, l1);
-                qh[ks][hf * 2 + rr] = h0 | (h1 << 16);
-                ql[ks][hf * 2 + rr] = l0 | (l1 << 16);
-            }
-    float o[2 * DV][4];
-#pragma unroll
-    for (int i = 0; i < 2 * DV; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
-    float mA = -INFINITY, mB = -INFINITY, lA = 0.0f, lB = 0.0f;
-    const uint32_t smem0 = vb_smem_u32(ma_tiles);
-    const int mat = lane >> 3, mr = lane & 7;
-    const float two_over_cap = a.softcap > 0.0f ? 2.0f / a.softcap : 0.0f;
-    auto request = [&](int t) {
-        int j0, n;
-        key_tile<kMaKeys>(kt, t, &j0, &n);
-        unsigned char *b = ma_tiles + (t & 1) * kBuf;
-        if constexpr (WIDE) {
-            request_wide<DK>(b, lw, g * (a.dim - lw.rot_dim), a.dim - lw.rot_dim, lw.rot_dim, j0, n, a.ring);
-            request_wide<DV>(b + 2 * kTileK, lw, lw.v0 + g * a.vdim, a.vdim, 0, j0, n, a.ring);
-        } else {
-            request_tile<DK>(b, Kc, ldk, g * a.dim, a.dim, j0, n, a.ring);
-            request_tile<DV>(b + 2 * kTileK, Vc, ldv, g * a.vdim, a.vdim, j0, n, a.ring);
-        }
-        lm_cp_commit();
-    };
-    if (kt.n_tiles > 0) request(0);
-
-    for (int t = 0; t < kt.n_tiles; t++) {
-        int j0, n;
-        key_tile<kMaKeys>(kt, t, &j0, &n);
-        lm_cp_wait_all();
-        __syncthreads();                               /* this buffer is complete, the other one is free */
-        if (t + 1 < kt.n_tiles) request(t + 1);
-        const uint32_t sKh = smem0 + (uint32_t)((t & 1) * kBuf), sKl = sKh + kTileK, sVh = sKl + kTileK, sVl = sVh + kTileV;
-        /* nothing of this tile for this warp's rows: later than all of them, or behind every window and not kept */
-        if (!active || j0 > w_imax || (a.window > 0 && w_imin - (j0 + n - 1) >= a.window && j0 >= a.keep)) continue;
-
-        float s[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.0f;
-#pragma unroll
-        for (int ks = 0; ks < DK; ks++) {
-#pragma unroll
-            for (int kp = 0; kp < 2; kp++) {           /* 16 keys each */
-                const uint32_t off = tile_off<DK>(kp * 16 + (mat >> 1) * 8 + mr, ks * 2 + (mat & 1));
-                uint32_t bh[4], bl[4];
-                ldsm(bh, sKh + off);
-                ldsm(bl, sKl + off);
-                mma_bf16(s[kp * 2], qh[ks], bh[0], bh[1]);
-                mma_bf16(s[kp * 2 + 1], qh[ks], bh[2], bh[3]);
-                mma_bf16(s[kp * 2], qh[ks], bl[0], bl[1]);
-                mma_bf16(s[kp * 2 + 1], qh[ks], bl[2], bl[3]);
-                mma_bf16(s[kp * 2], ql[ks], bh[0], bh[1]);
-                mma_bf16(s[kp * 2 + 1], ql[ks], bh[2], bh[3]);
-            }
-        }
-        float tA = -INFINITY, tB = -INFINITY;
-#pragma unroll
-        for (int nt = 0; nt < 4; nt++)
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const int key = nt * 8 + 2 * tq + (c & 1);
-                float v = s[nt][c] * a.scale;
-                if (a.softcap > 0.0f) v = soft_cap(v, a.softcap, two_over_cap);
-                if (key >= n || !key_seen(c < 2 ? iA : iB, j0 + key, a.window, a.keep)) v = -INFINITY;
-                s[nt][c] = v;
-                if (c < 2) tA = fmaxf(tA, v); else tB = fmaxf(tB, v);
-            }
-        tA = fmaxf(tA, __shfl_xor_sync(0xffffffffu, tA, 1));
-        tA = fmaxf(tA, __shfl_xor_sync(0xffffffffu, tA, 2));
-        tB = fmaxf(tB, __shfl_xor_sync(0xffffffffu, tB, 1));
-        tB = fmaxf(tB, __shfl_xor_sync(0xffffffffu, tB, 2));
-        /* a row that has seen no key yet keeps a finite reference, so that every weight below is exp(-inf) = 0 */
-        const float nA = fmaxf(mA, tA), nB = fmaxf(mB, tB);
-        const float fA = nA > -INFINITY ? nA : 0.0f, fB = nB > -INFINITY ? nB : 0.0f;
-        const float cA = expf(mA - fA), cB = expf(mB - fB);
-        mA = nA; mB = nB;
-        float sumA = 0.0f, sumB = 0.0f;
-        uint32_t ph[2][4], pl[2][4];
-#pragma unroll
-        for (int nt = 0; nt < 4; nt++) {
-            const float p0 = expf(s[nt][0] - fA), p1 = expf(s[nt][1] - fA), p2 = expf(s[nt][2] - fB), p3 = expf(s[nt][3] - fB);
-            sumA += p0 + p1;
-            sumB += p2 + p3;
-            uint32_t h0, l0, h1, l1;
-            hilo(p0, h0, l0); hilo(p1, h1, l1);
-            ph[nt >> 1][(nt & 1) * 2] = h0 | (h1 << 16);
-            pl[nt >> 1][(nt & 1) * 2] = l0 | (l1 << 16);
-            hilo(p2, h0, l0); hilo(p3, h1, l1);
-            ph[nt >> 1][(nt & 1) * 2 + 1] = h0 | (h1 << 16);
-            pl[nt >> 1][(nt & 1) * 2 + 1] = l0 | (l1 << 16);
-        }
-        lA = lA * cA + sumA;
-        lB = lB * cB + sumB;
-#pragma unroll
-        for (int i = 0; i < 2 * DV; i++) { o[i][0] *= cA; o[i][1] *= cA; o[i][2] *= cB; o[i][3] *= cB; }
-#pragma unroll
-        for (int dp = 0; dp < DV; dp++) {
-#pragma unroll
-            for (int kp = 0; kp < 2; kp++) {
-                const uint32_t off = tile_off<DV>(kp * 16 + (mat & 1) * 8 + mr, dp * 2 + (mat >> 1));
-                uint32_t vh[4], vl[4];
-                ldsm_t(vh, sVh + off);
-                ldsm_t(vl, sVl + off);
-                mma_bf16(o[2 * dp], ph[kp], vh[0], vh[1]);
-                mma_bf16(o[2 * dp + 1], ph[kp], vh[2], vh[3]);
-                mma_bf16(o[2 * dp], ph[kp], vl[0], vl[1]);
-                mma_bf16(o[2 * dp + 1], ph[kp], vl[2], vl[3]);
-                mma_bf16(o[2 * dp], pl[kp], vh[0], vh[1]);
-                mma_bf16(o[2 * dp + 1], pl[kp], vh[2], vh[3]);
             }
         }
     }
-    lA += __shfl_xor_sync(0xffffffffu, lA, 1);
-    lA += __shfl_xor_sync(0xffffffffu, lA, 2);
-    lB += __shfl_xor_sync(0xffffffffu, lB, 1);
-    lB += __shfl_xor_sync(0xffffffffu, lB, 2);
-    float rA = 1.0f / lA, rB = 1.0f / lB;
-    if constexpr (WIDE) {
-        if (validA) rA *= wide.gate[(size_t)rowA * a.heads + h];
-        if (validB) rB *= wide.gate[(size_t)rowB * a.heads + h];
-    }
+    template <int BLOCKS>
+    VB_DEVINL void keys(const AtArgs &, unsigned char *slot, int g, int lw, int lane, int j0, int n) const {
+        const int own = (dim - w.rot_dim) / 8, per = dim / 8, row = w.rank + w.rot_dim;
+        const int first = j0 - w.first + lw * 16;
+        const int key = lw * 16 + (lane & 15);
+        const int mine = lm_ring_row(ring, j0 + (key < n ? key : n - 1));
+        int at[16];
 #pragma unroll
-    for (int nt = 0; nt < 2 * DV; nt++)
+        for (int x = 0; x < 16; x++) at[x] = __shfl_sync(0xffffffffu, mine, x);
+#pragma unroll 1
+        for (int f = lane; f < 2 * per; f += 32) {
+            const int plane = f >= per ? 1 : 0, chunk = f - plane * per;
+            unsigned char *block = slot + (plane * BLOCKS + (chunk >> 3)) * kAtBlock;
+            const uint16_t *p = chunk < own ? w.kv + plane * w.plane + (size_t)first * w.ld + g * own * 8 + chunk * 8
+                                            : reinterpret_cast<const uint16_t *>(w.cache) + plane * row + w.rank + (chunk - own) * 8;
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const int d = nt * 8 + 2 * tq + u;
-            if (d >= a.vdim) continue;
-            if (validA) lm_put(a.out, rowA, h * a.vdim + d, o[nt][u] * rA);
-            if (validB) lm_put(a.out, rowB, h * a.vdim + d, o[nt][2 + u] * rB);
+            for (int x = 0; x < 16; x++)
+                if (lw * 16 + x < n) lm_cp16(block + at_off(lw * 16 + x, chunk), p + (chunk < own ? (size_t)x * w.ld : (size_t)at[x] * row * 2));
         }
-}
+    }
+    template <int BLOCKS>
+    VB_DEVINL void values(const AtArgs &, unsigned char *slot, int g, int lw, int lane, int j0, int n) const {
+        const int per = vdim / 8, first = j0 - w.first + lw * 16;
+#pragma unroll 1
+        for (int f = lane; f < 2 * per; f += 32) {
+            const int plane = f >= per ? 1 : 0, chunk = f - plane * per;
+            unsigned char *block = slot + (plane * BLOCKS + (chunk >> 3)) * kAtBlock;
+            const uint16_t *p = w.kv + plane * w.plane + (size_t)first * w.ld + w.v0 + g * vdim + chunk * 8;
+#pragma unroll
+            for (int x = 0; x < 16; x++)
+                if (lw * 16 + x < n) lm_cp16(block + at_off(lw * 16 + x, chunk), p + (size_t)x * w.ld);
+        }
+        clear_keys<BLOCKS>(slot, lw, lane, n);
+    }
+    VB_DEVINL float gate(int row, int head) const { return w.gate[(size_t)row * heads + head]; }
+    VB_DEVINL void put4(int row, int c, const float (&e)[4]) const { lm_put4(out, row, c, e); }
+};
 
-template <int DK, int DV, bool WIDE>
-int launch_mma(const LmAttn &a, const typename LmWideSel<WIDE>::type &wide, int M, cudaStream_t st) {
-    constexpr size_t smem = (size_t)2 * kMaKeys * 64 * (DK + DV);
-    static bool attr = false;
-    if (!attr) {
-        if (cudaFuncSetAttribute(lm_attn_mma_kernel<DK, DV, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-            cudaGetLastError();
-            return -1;
-        }
-        attr = true;
-    }
-    const int tiles = (M + 15) / 16 * (a.heads / a.kv_heads);
-    return ok(launch_pdl(lm_attn_mma_kernel<DK, DV, WIDE>, dim3((tiles + kMaWarps - 1) / kMaWarps, a.kv_heads), dim3(kMaThreads), smem, st, a, wide, M));
-}
+AtArgs at_args(const LmAttn &a, int M) { return {M, a.heads, a.kv_heads, a.dim, a.vdim, a.window, a.keep, a.scale, a.softcap, a.status}; }
 
 constexpr int kSplitBudget = 296;        /* two CTAs per SM */
 constexpr int kStepCtas = 148;           /* one-token kernel: one CTA per SM */
@@ -769,10 +651,12 @@ int lm_attn_generic(const LmAttn &a, int M, cudaStream_t st) {
 bool lm_attn_mma_ok(int dim, int vdim) { return dim <= 128 && vdim <= 128 && dim % 8 == 0 && vdim % 8 == 0; }
 
 int lm_attn_mma(const LmAttn &a, int M, cudaStream_t st) {
-    const bool k4 = a.dim <= 64, v4 = a.vdim <= 64;
-    const LmNotWide w;
-    if (k4) return v4 ? launch_mma<4, 4, false>(a, w, M, st) : launch_mma<4, 8, false>(a, w, M, st);
-    return v4 ? launch_mma<8, 4, false>(a, w, M, st) : launch_mma<8, 8, false>(a, w, M, st);
+    AtCache c = {};
+    c.dyn = a.dyn; c.q = a.q; c.k = a.k; c.v = a.v; c.ring = a.ring; c.out = a.out;
+    c.heads = a.heads; c.kv_heads = a.kv_heads; c.dim = a.dim; c.vdim = a.vdim;
+    const AtArgs t = at_args(a, M);
+    if (a.dim <= 64) return a.vdim <= 64 ? launch_attn_tc<1, 1>(t, c, st) : launch_attn_tc<1, 2>(t, c, st);
+    return a.vdim <= 64 ? launch_attn_tc<2, 1>(t, c, st) : launch_attn_tc<2, 2>(t, c, st);
 }
 
 bool lm_attn_wide_ok(int plain, int rot_dim, int vdim) {
@@ -780,10 +664,14 @@ bool lm_attn_wide_ok(int plain, int rot_dim, int vdim) {
 }
 
 int lm_attn_wide(const LmAttn &a, const LmWide &w, int M, cudaStream_t st) {
-    const bool v4 = a.vdim <= 64;
-    if (a.dim <= 64) return v4 ? launch_mma<4, 4, true>(a, w, M, st) : launch_mma<4, 8, true>(a, w, M, st);
-    if (a.dim <= 128) return v4 ? launch_mma<8, 4, true>(a, w, M, st) : launch_mma<8, 8, true>(a, w, M, st);
-    return v4 ? launch_mma<12, 4, true>(a, w, M, st) : launch_mma<12, 8, true>(a, w, M, st);
+    AtWide c = {};
+    c.dyn = a.dyn; c.w = w; c.ring = a.ring; c.out = a.out;
+    c.heads = a.heads; c.dim = a.dim; c.vdim = a.vdim; c.rot = a.rot;
+    const AtArgs t = at_args(a, M);
+    const bool v1 = a.vdim <= 64;
+    if (a.dim <= 64) return v1 ? launch_attn_tc<1, 1>(t, c, st) : launch_attn_tc<1, 2>(t, c, st);
+    if (a.dim <= 128) return v1 ? launch_attn_tc<2, 1>(t, c, st) : launch_attn_tc<2, 2>(t, c, st);
+    return v1 ? launch_attn_tc<3, 1>(t, c, st) : launch_attn_tc<3, 2>(t, c, st);
 }
 
 bool lm_attn_step_ok(const LmAttn &a) {

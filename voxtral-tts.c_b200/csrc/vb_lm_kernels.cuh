@@ -208,6 +208,7 @@ struct LmAttn {
     float *q;                    /* [M][heads * dim] normed and rotated */
     float *scratch;              /* key-split partials */
     unsigned *tickets;
+    int *status;                 /* set non-zero when a bounded wait runs out */
     LmSink out;
 };
 constexpr int kLmAttnSplits = 32;        /* key splits of one row's attention, at most */
@@ -219,7 +220,7 @@ int lm_attn_generic(const LmAttn &a, int M, cudaStream_t st);              /* fp
 bool lm_attn_step_ok(const LmAttn &a);
 int lm_attn_step(const LmAttn &a, cudaStream_t st);                        /* one token: norm, rotation, append, attention */
 bool lm_attn_mma_ok(int dim, int vdim);                                    /* sizes it runs at; needs split caches */
-int lm_attn_mma(const LmAttn &a, int M, cudaStream_t st);                  /* warp-level tensor cores, prompts */
+int lm_attn_mma(const LmAttn &a, int M, cudaStream_t st);                  /* tensor cores, prompts */
 
 /* Keys and values of every head, written out of a latent for a prompt's attention. */
 struct LmWide {

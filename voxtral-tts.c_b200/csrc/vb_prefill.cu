@@ -9,6 +9,7 @@
  * on the streaming engine, eight rows at a time. Also here: the prompt assembled on
  * the device from token ids and BF16 voice rows (voxtral_tts.c:230-272).
  */
+#include "vb_attn_tc.cuh"
 #include "vb_common.cuh"
 #include "vb_model.cuh"
 #include "vb_simple.cuh"
@@ -77,234 +78,56 @@ __global__ void pf_qkv_finish_kernel(float *qkv, const float *part, int n_part, 
     else *reinterpret_cast<float2 *>(v_rows + (size_t)m * KVD + (col - QD - KVD)) = v;
 }
 
-/* Causal attention of a block of prompt rows over the cache prefix (tts_causal_attention,
- * voxtral_tts_kernels.c:403-465) on the warp-level tensor cores; head_dim 128, four query heads
- * per KV head. A CTA owns one KV head and 16 query rows; warps w and w + 4 serve query head 4 g + w
- * on the first and on the second 16 keys of every 32-key tile (two partial softmax states merged at
- * the end), so the K and V rows are staged in shared memory once per KV head, 32 keys at a time, and
- * every SM sub-core has two warps' worth of independent MMAs to issue.
- *
- * fp32 accuracy from BF16 MMAs: every fp32 operand is split into hi + lo BF16 halves and a
- * product a.b is taken as a_hi.b_hi + a_hi.b_lo + a_lo.b_hi (the dropped lo.lo term is 2^-16 of
- * the product). Per 32-key tile a warp issues, with mma.sync.m16n8k16, for its 16 keys:
- *   S[16 x 16]  = Q[16 x 128] . K^T     2 key tiles x 8 k-steps x 3 products
- *   O[16 x 128] += P[16 x 16] . V      16 dim tiles x 1 k-step x 3 products
- * Q lives in registers as A fragments (scaled by 1/sqrt(128) before the split); K rows [key][dim]
- * are the "column-major" B operand of Q.K^T (ldmatrix), V rows [key][dim] the row-major B operand
- * of P.V (ldmatrix.trans); both sit in shared memory as BF16 with the 16-byte chunks of a row
- * XOR-swizzled by the key index. The running maximum / sum update is the usual one per tile;
- * S's accumulator fragments become P's A fragments without leaving registers. Row blocks are
- * issued heaviest (latest rows) first. */
-constexpr int kFaRows = 16, kFaKeys = 32, kFaThreads = 256;
-
-VB_DEVINL void fa_split(float v, uint32_t &hi, uint32_t &lo) {
-    uint16_t a, b, c;
-    vb_split3(v, a, b, c);
-    hi = a;
-    lo = b;
-}
-VB_DEVINL void fa_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-VB_DEVINL void fa_ldsm(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-VB_DEVINL void fa_ldsm_t(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-/* byte offset of 16-byte chunk `chunk` (0..15) of key row `key` in a [32][128] BF16 tile */
-VB_DEVINL uint32_t fa_off(int key, int chunk) { return (uint32_t)(key * 256 + (((chunk & 8) | ((chunk ^ key) & 7)) << 4)); }
-
-__global__ void __launch_bounds__(kFaThreads)
-pf_attention_kernel(float *out, const float *q, const float *kc, const float *vc, int M, int start_pos, int ldq,
-                    int ldkv, int ldo, float scale) {
-    __shared__ __align__(128) unsigned char tiles[4 * kFaKeys * 256];   /* K hi, K lo, V hi, V lo; reused by the final merge */
-    __shared__ float ml[4][32][4];                                      /* second half's (mA, mB, lA, lB) per head and lane */
-    unsigned char *Kh = tiles, *Kl = tiles + kFaKeys * 256, *Vh = tiles + 2 * kFaKeys * 256, *Vl = tiles + 3 * kFaKeys * 256;
-    pdl_launch_dependents();
-    pdl_wait();
-    const int g = blockIdx.y, r0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * kFaRows;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
-    const int hw = warp & 3, half = warp >> 2;   /* head of the group; which 16 keys of every 32-key tile */
-    const int h = g * 4 + hw;
-    const int rowA = r0 + gq, rowB = rowA + 8;
-    const bool validA = rowA < M, validB = rowB < M;
-    const int limA = validA ? start_pos + rowA : 0, limB = validB ? start_pos + rowB : 0;   /* last key a row sees */
-    const int rows_here = M - r0 < kFaRows ? M - r0 : kFaRows;
-    const int n_keys = start_pos + r0 + rows_here;
-
-    /* Q as A fragments: a0 (row A, k 2t..), a1 (row B, k 2t..), a2 (row A, k 8+2t..), a3 (row B, k 8+2t..) */
-    uint32_t qh[8][4], ql[8][4];
+/* Causal attention of prompt rows over the cache prefix (tts_causal_attention, voxtral_tts_kernels.c:403-465) on the
+ * tensor cores (vb_attn_tc.cuh): queries, and the cache's fp32 keys and values, which the loading warps split into BF16
+ * halves on the way to shared memory. */
+struct AtRows {
+    static constexpr bool kAsync = false;
+    const float *q, *kc, *vc;
+    float *out;
+    int ldq, ldkv, ldo, start_pos;
+    VB_DEVINL void start() {}
+    VB_DEVINL int pos0() const { return start_pos; }
+    VB_DEVINL void q8(int row, int head, int d, float (&e)[8]) const {
+        const float4 *p = reinterpret_cast<const float4 *>(q + (size_t)row * ldq + head * VB200_HEAD_DIM + d);
+        const float4 x = p[0], y = p[1];
+        e[0] = x.x; e[1] = x.y; e[2] = x.z; e[3] = x.w; e[4] = y.x; e[5] = y.y; e[6] = y.z; e[7] = y.w;
+    }
+    /* a lane's four columns of 16 rows, eight loads in flight; rows beyond the tile's keys are zeros */
+    VB_DEVINL void rows(const float *cache, unsigned char *slot, int g, int lw, int lane, int j0, int n) const {
+        unsigned char *block = slot + (lane >> 4) * kAtBlock;
+        const float *col = cache + (size_t)(j0 + lw * 16) * ldkv + g * VB200_HEAD_DIM + lane * 4;
 #pragma unroll
-    for (int ks = 0; ks < 8; ks++) {
+        for (int x0 = 0; x0 < 16; x0 += 8) {
+            float4 v[8];
 #pragma unroll
-        for (int half = 0; half < 2; half++) {
+            for (int x = 0; x < 8; x++)
+                v[x] = lw * 16 + x0 + x < n ? vb_ldcg4(col + (size_t)(x0 + x) * ldkv) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int rr = 0; rr < 2; rr++) {
-                const int row = rr ? rowB : rowA;
-                float2 v = make_float2(0.f, 0.f);
-                if (rr ? validB : validA)
-                    v = *reinterpret_cast<const float2 *>(q + (size_t)row * ldq + h * VB200_HEAD_DIM + ks * 16 + half * 8 + 2 * tq);
-                uint32_t h0, l0, h1, l1;
-                fa_split(v.x * scale, h0, l0);
-                fa_split(v.y * scale, h1, l1);
-                qh[ks][half * 2 + rr] = h0 | (h1 << 16);
-                ql[ks][half * 2 + rr] = l0 | (l1 << 16);
+            for (int x = 0; x < 8; x++) {
+                uint2 hi, lo;
+                at_split2(v[x].x, v[x].y, hi.x, lo.x);
+                at_split2(v[x].z, v[x].w, hi.y, lo.y);
+                unsigned char *at = block + at_off(lw * 16 + x0 + x, (lane & 15) >> 1) + (lane & 1) * 8;
+                *reinterpret_cast<uint2 *>(at) = hi;
+                *reinterpret_cast<uint2 *>(at + 2 * kAtBlock) = lo;
             }
         }
     }
-    float o[16][4];
-#pragma unroll
-    for (int i = 0; i < 16; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
-    float mA = -1e30f, mB = -1e30f, lA = 0.0f, lB = 0.0f;
-    const uint32_t sKh = vb_smem_u32(Kh), sKl = vb_smem_u32(Kl), sVh = vb_smem_u32(Vh), sVl = vb_smem_u32(Vl);
-    const int mat = lane >> 3, mr = lane & 7;
-
-    for (int k0 = 0; k0 < n_keys; k0 += kFaKeys) {
-        __syncthreads();
-        /* stage 32 keys of K and V: fp32 -> hi / lo BF16, 4 values (8 bytes) per piece */
-        for (int i = tid; i < kFaKeys * 32; i += kFaThreads) {
-            const int key = i >> 5, f = i & 31, kk = k0 + key;
-            float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-            if (kk < n_keys) {
-                a = __ldg(reinterpret_cast<const float4 *>(kc + (size_t)kk * ldkv + g * VB200_HEAD_DIM) + f);
-                b = __ldg(reinterpret_cast<const float4 *>(vc + (size_t)kk * ldkv + g * VB200_HEAD_DIM) + f);
-            }
-            const float ea[4] = {a.x, a.y, a.z, a.w}, eb[4] = {b.x, b.y, b.z, b.w};
-            uint32_t ah[4], al[4], bh[4], bl[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) { fa_split(ea[j], ah[j], al[j]); fa_split(eb[j], bh[j], bl[j]); }
-            const uint32_t off = fa_off(key, f >> 1) + (uint32_t)(f & 1) * 8u;
-            *reinterpret_cast<uint2 *>(Kh + off) = make_uint2(ah[0] | (ah[1] << 16), ah[2] | (ah[3] << 16));
-            *reinterpret_cast<uint2 *>(Kl + off) = make_uint2(al[0] | (al[1] << 16), al[2] | (al[3] << 16));
-            *reinterpret_cast<uint2 *>(Vh + off) = make_uint2(bh[0] | (bh[1] << 16), bh[2] | (bh[3] << 16));
-            *reinterpret_cast<uint2 *>(Vl + off) = make_uint2(bl[0] | (bl[1] << 16), bl[2] | (bl[3] << 16));
-        }
-        __syncthreads();
-
-        /* S = Q . K^T for this warp's 2 tiles of 8 keys */
-        float s[2][4];
-#pragma unroll
-        for (int i = 0; i < 2; i++) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.0f;
-#pragma unroll
-        for (int ks = 0; ks < 8; ks++) {
-            /* matrices: (keys half*16.., dims ks*16..), (same keys, dims +8), (keys +8, dims), (keys +8, dims +8) */
-            const uint32_t off = fa_off(half * 16 + (mat >> 1) * 8 + mr, ks * 2 + (mat & 1));
-            uint32_t bh[4], bl[4];
-            fa_ldsm(bh, sKh + off);
-            fa_ldsm(bl, sKl + off);
-            fa_mma(s[0], qh[ks], bh[0], bh[1]);
-            fa_mma(s[1], qh[ks], bh[2], bh[3]);
-            fa_mma(s[0], qh[ks], bl[0], bl[1]);
-            fa_mma(s[1], qh[ks], bl[2], bl[3]);
-            fa_mma(s[0], ql[ks], bh[0], bh[1]);
-            fa_mma(s[1], ql[ks], bh[2], bh[3]);
-        }
-        /* causal mask, running maximum and sum (rows A and B of this thread's quad) */
-        float tmA = -1e30f, tmB = -1e30f;
-#pragma unroll
-        for (int nt = 0; nt < 2; nt++) {
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const int key = k0 + half * 16 + nt * 8 + 2 * tq + (c & 1);
-                if (key > (c < 2 ? limA : limB)) s[nt][c] = -1e30f;
-            }
-            tmA = fmaxf(tmA, fmaxf(s[nt][0], s[nt][1]));
-            tmB = fmaxf(tmB, fmaxf(s[nt][2], s[nt][3]));
-        }
-        tmA = fmaxf(tmA, __shfl_xor_sync(0xffffffffu, tmA, 1));
-        tmA = fmaxf(tmA, __shfl_xor_sync(0xffffffffu, tmA, 2));
-        tmB = fmaxf(tmB, __shfl_xor_sync(0xffffffffu, tmB, 1));
-        tmB = fmaxf(tmB, __shfl_xor_sync(0xffffffffu, tmB, 2));
-        const float nA = fmaxf(mA, tmA), nB = fmaxf(mB, tmB);
-        const float cA = expf(mA - nA), cB = expf(mB - nB);
-        mA = nA; mB = nB;
-        float sumA = 0.0f, sumB = 0.0f;
-        uint32_t ph[4], pl[4];
-#pragma unroll
-        for (int nt = 0; nt < 2; nt++) {
-            float p[4];
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const int key = k0 + half * 16 + nt * 8 + 2 * tq + (c & 1);
-                p[c] = key > (c < 2 ? limA : limB) ? 0.0f : expf(s[nt][c] - (c < 2 ? nA : nB));
-            }
-            sumA += p[0] + p[1];
-            sumB += p[2] + p[3];
-            /* accumulator layout of key tile nt -> A fragment of the one k-step:
-             * first tile: a0 (row A), a1 (row B); second tile: a2 (row A), a3 (row B) */
-            uint32_t h0, l0, h1, l1;
-            fa_split(p[0], h0, l0); fa_split(p[1], h1, l1);
-            ph[nt * 2] = h0 | (h1 << 16);
-            pl[nt * 2] = l0 | (l1 << 16);
-            fa_split(p[2], h0, l0); fa_split(p[3], h1, l1);
-            ph[nt * 2 + 1] = h0 | (h1 << 16);
-            pl[nt * 2 + 1] = l0 | (l1 << 16);
-        }
-        lA = lA * cA + sumA;
-        lB = lB * cB + sumB;
-#pragma unroll
-        for (int i = 0; i < 16; i++) { o[i][0] *= cA; o[i][1] *= cA; o[i][2] *= cB; o[i][3] *= cB; }
-        /* O += P . V over this warp's 16 keys */
-#pragma unroll
-        for (int dp = 0; dp < 8; dp++) {
-            /* matrices: (keys half*16.., dims dp*16..), (keys +8, dims), (keys, dims +8), (keys +8, dims +8) */
-            const uint32_t off = fa_off(half * 16 + (mat & 1) * 8 + mr, dp * 2 + (mat >> 1));
-            uint32_t vh[4], vl[4];
-            fa_ldsm_t(vh, sVh + off);
-            fa_ldsm_t(vl, sVl + off);
-            fa_mma(o[2 * dp], ph, vh[0], vh[1]);
-            fa_mma(o[2 * dp + 1], ph, vh[2], vh[3]);
-            fa_mma(o[2 * dp], ph, vl[0], vl[1]);
-            fa_mma(o[2 * dp + 1], ph, vl[2], vl[3]);
-            fa_mma(o[2 * dp], pl, vh[0], vh[1]);
-            fa_mma(o[2 * dp + 1], pl, vh[2], vh[3]);
-        }
+    template <int BLOCKS>
+    VB_DEVINL void keys(const AtArgs &, unsigned char *slot, int g, int lw, int lane, int j0, int n) const {
+        rows(kc, slot, g, lw, lane, j0, n);
     }
-    lA += __shfl_xor_sync(0xffffffffu, lA, 1);
-    lA += __shfl_xor_sync(0xffffffffu, lA, 2);
-    lB += __shfl_xor_sync(0xffffffffu, lB, 1);
-    lB += __shfl_xor_sync(0xffffffffu, lB, 2);
-    /* merge the two key halves of every head: the second half hands its (max, sum, O) over through
-     * the tile memory, the first half combines them with the usual log-sum-exp weights */
-    __syncthreads();
-    float *xo = reinterpret_cast<float *>(tiles);                 /* [head][64 values][32 lanes] */
-    if (half == 1) {
-#pragma unroll
-        for (int i = 0; i < 16; i++)
-#pragma unroll
-            for (int c = 0; c < 4; c++) xo[(hw * 64 + i * 4 + c) * 32 + lane] = o[i][c];
-        ml[hw][lane][0] = mA; ml[hw][lane][1] = mB; ml[hw][lane][2] = lA; ml[hw][lane][3] = lB;
+    template <int BLOCKS>
+    VB_DEVINL void values(const AtArgs &, unsigned char *slot, int g, int lw, int lane, int j0, int n) const {
+        rows(vc, slot, g, lw, lane, j0, n);
     }
-    __syncthreads();
-    if (half == 1) return;
-    {
-        const float m2A = ml[hw][lane][0], m2B = ml[hw][lane][1], l2A = ml[hw][lane][2], l2B = ml[hw][lane][3];
-        const float MA = fmaxf(mA, m2A), MB = fmaxf(mB, m2B);
-        const float w1A = expf(mA - MA), w2A = l2A > 0.0f ? expf(m2A - MA) : 0.0f;
-        const float w1B = expf(mB - MB), w2B = l2B > 0.0f ? expf(m2B - MB) : 0.0f;
-        lA = lA * w1A + l2A * w2A;
-        lB = lB * w1B + l2B * w2B;
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            o[i][0] = o[i][0] * w1A + xo[(hw * 64 + i * 4 + 0) * 32 + lane] * w2A;
-            o[i][1] = o[i][1] * w1A + xo[(hw * 64 + i * 4 + 1) * 32 + lane] * w2A;
-            o[i][2] = o[i][2] * w1B + xo[(hw * 64 + i * 4 + 2) * 32 + lane] * w2B;
-            o[i][3] = o[i][3] * w1B + xo[(hw * 64 + i * 4 + 3) * 32 + lane] * w2B;
-        }
+    VB_DEVINL float gate(int, int) const { return 1.0f; }
+    VB_DEVINL void put4(int row, int c, const float (&e)[4]) const {
+        *reinterpret_cast<float4 *>(out + (size_t)row * ldo + c) = make_float4(e[0], e[1], e[2], e[3]);
     }
-    const float iA = lA > 0.0f ? 1.0f / lA : 0.0f, iB = lB > 0.0f ? 1.0f / lB : 0.0f;
-#pragma unroll
-    for (int nt = 0; nt < 16; nt++) {
-        const int d = nt * 8 + 2 * tq;
-        if (validA) *reinterpret_cast<float2 *>(out + (size_t)rowA * ldo + h * VB200_HEAD_DIM + d) = make_float2(o[nt][0] * iA, o[nt][1] * iA);
-        if (validB) *reinterpret_cast<float2 *>(out + (size_t)rowB * ldo + h * VB200_HEAD_DIM + d) = make_float2(o[nt][2] * iB, o[nt][3] * iB);
-    }
-}
+};
+static_assert(VB200_HEAD_DIM == 128, "a lane's four columns cover a head");
 
 /* ---- tensor-core prefill ---- */
 struct PrefillTc {
@@ -405,8 +228,9 @@ static int prefill_tc(float *x, float *qkv, float *attn, const float *cs, int M,
                        (size_t)rows * QKV, cs + (size_t)r0 * VB200_HEAD_DIM, ck, cv, rows);
         }
         const float *k0 = m.kv_k + (size_t)l * m.kv_max * KVD, *v0 = m.kv_v + (size_t)l * m.kv_max * KVD;
-        launch_pdl(pf_attention_kernel, dim3((M + kFaRows - 1) / kFaRows, VB200_KV_HEADS), dim3(kFaThreads), 0, st, attn,
-                   (const float *)qkv, k0, v0, M, start_pos, QKV, KVD, QD, scale);
+        const AtRows rows_of = {qkv, k0, v0, attn, QKV, KVD, QD, start_pos};
+        const AtArgs at = {M, VB200_HEADS, VB200_KV_HEADS, VB200_HEAD_DIM, VB200_HEAD_DIM, 0, 0, scale, 0.0f, &m.d_out->status};
+        if (launch_attn_tc<2, 2>(at, rows_of, st)) return -1;
         if (l == VB200_DEC_LAYERS - 1) break;   /* only the cache is kept (voxtral_tts_llm.c:281) */
         for (int r0 = 0; r0 < M; r0 += kPfRows) {
             const int rows = M - r0 < kPfRows ? M - r0 : kPfRows;
