@@ -14,7 +14,13 @@
  * the epilogue of a tile runs under the main loop of the next. R is chosen per launch (pick_rows): a smaller one that
  * fills the last wave beats 256 where the tile count falls badly on the pairs.
  *
- * Warps: 0-7 epilogue (TMEM -> shared memory -> whole 512-byte row segments), 8 TMA producer, 9 MMA issuer (of the even
+ * The tensor core's fp32 sums are cut off, not rounded, at every step, and the error grows with the chain: 1203 speech
+ * rows with K in one piece were 7.1e-5 off 64 bits, in 3 to 6 splits 4.6e-5, at the price of as many partial results.
+ * So TMEM sums up to 2048 columns at a time (alternating accumulators) and the epilogue warps add these up in
+ * registers, 64 values a thread, under the main loop. A 4001-token prompt: 60.6 ms and 7.3e-5 in one piece, 61.9 ms and
+ * 4.9e-5 so, 63.3 ms and 3.3e-5 with 1024 columns (and 66 to 69 ms where eight warps held 128 values and spilled).
+ *
+ * Warps: 0-15 epilogue (TMEM -> registers -> shared memory -> whole 512-byte row segments), 16 TMA producer, 17 MMA issuer (of the even
  * CTA, for both). Full barriers and the accumulator hand-back live in the even CTA; commits arrive in both. No
  * multicast loads. All waits are bounded.
  */
@@ -32,7 +38,8 @@ constexpr int kPrMaxRows = 256, kPrTerms = 2, kPrStages = 4, kPrChunk = 64;
 constexpr int kPrStageW = kTcTileN * kTcBlockK * 2, kPrStageX = kPrMaxRows / 2 * kTcBlockK * 2;
 constexpr int kPrStage = kPrStageW + kPrTerms * kPrStageX;
 constexpr int kPrStaging = kPrChunk * kTcTileN * 4;
-constexpr int kPrEpiWarps = 8, kPrEpi = 32 * kPrEpiWarps, kPrThreads = kPrEpi + 64;
+constexpr int kPrSegment = 32;       /* k-blocks that are summed in TMEM, at most, before the sums move on to registers */
+constexpr int kPrEpiWarps = 16, kPrEpi = 32 * kPrEpiWarps, kPrThreads = kPrEpi + 64;
 constexpr int kPrSmemBytes = kPrStages * kPrStage + kPrStaging + kPrMaxRows * 4 + 256 + 1024;
 static_assert(kPrSmemBytes <= 232448, "over the 227 KB a CTA may use");
 constexpr uint32_t kPrTmemCols = 512;
@@ -91,7 +98,7 @@ VB_DEVINL void pr_commit(uint64_t *bar) {
 
 /* One tile of a pair: its place, and the MMA width its rows need. */
 struct PrTile {
-    int sp, t0, w0, m0, Mb, n_mma, kb0, n_it;
+    int sp, t0, w0, m0, Mb, n_mma, kb0, n_it, seg;
     bool used;
 };
 template <bool GROUPED>
@@ -114,20 +121,9 @@ VB_DEVINL PrTile pr_tile(const RowsArgs &a, int i, int kblocks) {
     t.n_mma = (t.Mb + 31) & ~31;
     t.kb0 = (int)((long long)kblocks * t.sp / a.splits);
     t.n_it = (int)((long long)kblocks * (t.sp + 1) / a.splits) - t.kb0;
+    const int segments = (t.n_it + kPrSegment - 1) / kPrSegment;
+    t.seg = (t.n_it + segments - 1) / segments;
     return t;
-}
-
-VB_DEVINL void pr_tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]),
-          "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]),
-          "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
 VB_DEVINL uint32_t pr_pack(uint16_t a, uint16_t b) { return a | ((uint32_t)b << 16); }
@@ -230,7 +226,7 @@ vb_tc_pair_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kPrStages; i++) { vb_mbar_init(&full[i], 1); vb_mbar_init(&empty[i], 1); }
-        for (int i = 0; i < 2; i++) { vb_mbar_init(&done[i], 1); vb_mbar_init(&drained[i], 2); }
+        for (int i = 0; i < 2; i++) { vb_mbar_init(&done[i], 1); vb_mbar_init(&drained[i], 2 * kPrEpiWarps); }
         *abort_flag = 0;
         vb_mbar_init_fence();
     }
@@ -312,46 +308,48 @@ vb_tc_pair_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
         for (int i = cluster; i < n_tiles && ok; i += n_clusters) {
             const PrTile t = pr_tile<GROUPED>(a, i, kblocks);
             if (!t.used) continue;
-            const uint32_t acc = n & 1u, d = tmem + acc * kPrMaxRows;
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(t.n_mma >> 3) << 17) | ((uint32_t)(2 * kTcTileN >> 4) << 24);
-            if (!vb_mbar_wait(&drained[acc], ((n >> 1) & 1u) ^ 1u, abort_flag)) {
-                atomicCAS(a.status, 0, 15);
-                *(volatile int *)abort_flag = 1;
-                break;
-            }
-            tc_fence_after();
-            for (int it = 0; it < t.n_it; it++, k++) {
-                const uint32_t s = k % kPrStages, use = k / kPrStages;
-                if (!vb_mbar_wait(&full[s], use & 1u, abort_flag)) {
-                    atomicCAS(a.status, 0, 12);
+            for (int it = 0; it < t.n_it && ok; n++) {
+                const uint32_t acc = n & 1u, d = tmem + acc * kPrMaxRows;
+                const int end = min(t.n_it, it + t.seg);
+                if (!vb_mbar_wait(&drained[acc], ((n >> 1) & 1u) ^ 1u, abort_flag)) {
+                    atomicCAS(a.status, 0, 15);
                     *(volatile int *)abort_flag = 1;
                     ok = false;
                     break;
                 }
                 tc_fence_after();
-                const unsigned char *sa = stages + (size_t)s * kPrStage;
-                const uint64_t adesc = umma_desc_k_sw128(sa);
+                for (bool first = true; it < end; it++, k++, first = false) {
+                    const uint32_t s = k % kPrStages, use = k / kPrStages;
+                    if (!vb_mbar_wait(&full[s], use & 1u, abort_flag)) {
+                        atomicCAS(a.status, 0, 12);
+                        *(volatile int *)abort_flag = 1;
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const unsigned char *sa = stages + (size_t)s * kPrStage;
+                    const uint64_t adesc = umma_desc_k_sw128(sa);
 #pragma unroll
-                for (int j = 0; j < kPrTerms; j++) {
-                    const uint64_t bdesc = umma_desc_k_sw128(sa + kPrStageW + j * kPrStageX);
+                    for (int j = 0; j < kPrTerms; j++) {
+                        const uint64_t bdesc = umma_desc_k_sw128(sa + kPrStageW + j * kPrStageX);
 #pragma unroll
-                    for (int q = 0; q < kTcBlockK / 16; q++) pr_mma(d, adesc + 2 * q, bdesc + 2 * q, idesc, (it | j | q) != 0 ? 1u : 0u);
+                        for (int q = 0; q < kTcBlockK / 16; q++) pr_mma(d, adesc + 2 * q, bdesc + 2 * q, idesc, (!first || (j | q) != 0) ? 1u : 0u);
+                    }
+                    pr_commit(&empty[s]);
                 }
-                pr_commit(&empty[s]);
+                pr_commit(&done[acc]);
             }
-            pr_commit(&done[acc]);
-            n++;
         }
     } else if (warp < kPrEpiWarps) {
         /* ---- epilogue: accumulators -> shared memory -> global, 64 rows at a time ---- */
-        const int lq = warp & 3, half = warp >> 2;
+        const int lq = warp & 3, part = warp >> 2;
         const uint32_t drained_bar[2] = {pr_leader(&drained[0]), pr_leader(&drained[1])};
         uint32_t n = 0;
         pdl_wait();
         for (int i = cluster; i < n_tiles; i += n_clusters) {
             const PrTile t = pr_tile<GROUPED>(a, i, kblocks);
             if (!t.used) continue;
-            const uint32_t acc = n & 1u, d = tmem + acc * kPrMaxRows + ((uint32_t)(lq * 32) << 16);
             if (a.ssq) {
                 vb_named_bar(1, kPrEpi);             /* the last tile's scales are read */
                 for (int m = threadIdx.x; m < t.Mb; m += kPrEpi) {
@@ -361,31 +359,52 @@ vb_tc_pair_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
                 }
                 vb_named_bar(1, kPrEpi);
             }
-            if (!vb_mbar_wait(&done[acc], (n >> 1) & 1u, abort_flag)) {
-                atomicCAS(a.status, 0, 13);
-                *(volatile int *)abort_flag = 1;
-            }
-            tc_fence_after();
-            for (int c0 = 0; c0 < t.Mb; c0 += kPrChunk) {
-                const int c = c0 + half * 32;
-                if (c < t.Mb) {
-                    uint32_t r[32];
-                    pr_tmem_ld32(d + (uint32_t)c, r);
+            /* this thread's column of the weight tile, rows part * 16 .. of every 64 */
+            constexpr int kChunks = kPrMaxRows / kPrChunk;
+            float sum[kChunks][16];
+            for (int it = 0; it < t.n_it; it += t.seg, n++) {
+                const uint32_t acc = n & 1u, d = tmem + acc * kPrMaxRows + ((uint32_t)(lq * 32) << 16) + (uint32_t)(part * 16);
+                /* after a wait that ran out the others fail at once: no thread leaves the barriers alone */
+                if (!vb_mbar_wait(&done[acc], (n >> 1) & 1u, abort_flag)) {
+                    atomicCAS(a.status, 0, 13);
+                    *(volatile int *)abort_flag = 1;
+                }
+                __syncwarp();
+                tc_fence_after();
 #pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        float v = __uint_as_float(r[j]);
-                        if (a.ssq && c + j < t.Mb) v *= rscale[c + j];
-                        stg[(half * 32 + j) * kTcTileN + lq * 32 + lane] = v;
+                for (int q = 0; q < kChunks; q++) {
+                    if (q * kPrChunk + part * 16 < t.Mb) {
+                        uint32_t r[16];
+                        tmem_ld16(d + (uint32_t)(q * kPrChunk), r);
+                        if (it == 0) {
+#pragma unroll
+                            for (int j = 0; j < 16; j++) sum[q][j] = __uint_as_float(r[j]);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 16; j++) sum[q][j] += __uint_as_float(r[j]);
+                        }
                     }
                 }
-                if (c0 + kPrChunk >= t.Mb) tc_fence_before();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) pr_arrive(drained_bar[acc]);
+            }
+#pragma unroll 1
+            for (int q = 0; q * kPrChunk < t.Mb; q++) {
+                const int c0 = q * kPrChunk, c = c0 + part * 16;
+                if (c < t.Mb) {
+                    float *to = stg + part * 16 * kTcTileN + lq * 32 + lane;
+#pragma unroll
+                    for (int u = 0; u < kChunks; u++)
+                        if (u == q) {                       /* registers have no index */
+#pragma unroll
+                            for (int j = 0; j < 16; j++) to[j * kTcTileN] = a.ssq ? sum[u][j] * rscale[min(c + j, t.Mb - 1)] : sum[u][j];
+                        }
+                }
                 vb_named_bar(1, kPrEpi);
-                /* the accumulator is free as soon as the last of it is staged */
-                if (c0 + kPrChunk >= t.Mb && threadIdx.x == 0) pr_arrive(drained_bar[acc]);
                 pr_store(a, stg, t, t.t0 + (int)rank, c0, warp, lane);
                 vb_named_bar(1, kPrEpi);
             }
-            n++;      /* after a wait that ran out the others fail at once: no thread leaves the barriers alone */
         }
     }
 
