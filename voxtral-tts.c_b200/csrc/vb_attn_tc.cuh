@@ -79,6 +79,12 @@ VB_DEVINL void at_st32(uint32_t taddr, const uint32_t (&r)[32]) {
         ::VB_AT_R8(r, 0), VB_AT_R8(r, 8), VB_AT_R8(r, 16), VB_AT_R8(r, 24), "r"(taddr)
         : "memory");
 }
+VB_DEVINL void at_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+        ::VB_AT_R8(r, 0), VB_AT_R8(r, 8), "r"(taddr)
+        : "memory");
+}
 VB_DEVINL void at_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 VB_DEVINL void at_proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 VB_DEVINL float at_ex2(float x) {
@@ -188,30 +194,25 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const AtArgs 
         const bool valid = P < pairs;
         const int row = valid ? P / group : 0, head = g * group + (valid ? P - row * group : 0), i = pos0 + row;
         const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16, tS = tmem + lanes + (uint32_t)(w * kAtKeys), tO = tmem + lanes + kAtO + (uint32_t)(w * 128);
-        /* the query row: its high halves go to TMEM by the first warpgroup, its low ones by the second */
+        /* the query row, 32 columns in turn by the two warpgroups: halves to TMEM, low ones of large heads to shared memory */
 #pragma unroll 1
-        for (int kb = 0; kb < DK; kb++) {
-            uint32_t reg[32];
+        for (int u = w; u < 2 * DK; u += 2) {
+            uint32_t hi[16], lo[16];
 #pragma unroll
-            for (int c = 0; c < 8; c++) {
-                float e[8];
-                if (valid) src.q8(row, head, kb * 64 + c * 8, e);
-                else
+            for (int c = 0; c < 4; c++) {
+                float e[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                if (valid) src.q8(row, head, u * 32 + c * 8, e);
 #pragma unroll
-                    for (int j = 0; j < 8; j++) e[j] = 0.0f;
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    uint32_t hi, lo;
-                    at_split2(e[2 * j], e[2 * j + 1], hi, lo);
-                    reg[c * 4 + j] = w == 0 ? hi : lo;
-                }
+                for (int j = 0; j < 4; j++) at_split2(e[2 * j], e[2 * j + 1], hi[c * 4 + j], lo[c * 4 + j]);
             }
-            if (w == 0 || Cfg::kQlTmem) {
-                at_st32(tmem + lanes + kAtQ + (uint32_t)((w * DK + kb) * 32), reg);
+            at_st16(tmem + lanes + kAtQ + (uint32_t)(u * 16), hi);
+            if constexpr (Cfg::kQlTmem) {
+                at_st16(tmem + lanes + kAtQ + (uint32_t)(DK * 32 + u * 16), lo);
             } else {
 #pragma unroll
-                for (int c = 0; c < 8; c++)
-                    *reinterpret_cast<uint4 *>(ql_s + kb * kAtRows * 128 + at_off(r, c)) = make_uint4(reg[c * 4], reg[c * 4 + 1], reg[c * 4 + 2], reg[c * 4 + 3]);
+                for (int c = 0; c < 4; c++)
+                    *reinterpret_cast<uint4 *>(ql_s + (u >> 1) * kAtRows * 128 + at_off(r, (u & 1) * 4 + c)) =
+                        make_uint4(lo[c * 4], lo[c * 4 + 1], lo[c * 4 + 2], lo[c * 4 + 3]);
             }
         }
         at_st_wait();
@@ -294,9 +295,13 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const AtArgs 
             vb_mbar_arrive(&p_full[w]);
         }
         if (it > 0 && !at_warp_wait(&o_done[w], (uint32_t)(it - 1) & 1u, abort_flag)) give_up();
-        /* both halves of the keys, merged: each warpgroup writes half of the columns */
+        /* Both halves of the keys, merged, each warpgroup half of the columns; by way of shared memory, so that a warp
+         * writes the columns of a row side by side (from the TMEM layout, a thread per row, every store touches 32 rows). */
         vb_named_bar(1, kAtSoft);                                 /* every product is done: the rings are free */
         float2 *ml = reinterpret_cast<float2 *>(k_s);
+        float *rows = reinterpret_cast<float *>(k_s + 2 * kAtRows * 8);
+        constexpr int kLd = DV * 64 + 4;                          /* 16 bytes on: eight rows of a column hit all banks */
+        static_assert(2 * kAtRows * 8 + kAtRows * kLd * 4 <= Cfg::kSlots * (Cfg::kSlotK + Cfg::kSlotV), "results do not fit the rings");
         ml[w * kAtRows + r] = make_float2(ref, sum);
         tc_fence_before();
         vb_named_bar(1, kAtSoft);
@@ -308,24 +313,25 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const AtArgs 
         const float ra = fa * inv, rb = fb * inv;
 #pragma unroll 1
         for (int c = w * DV; c < w * DV + DV; c++) {
-            if (c * 32 >= a.vdim) break;
             uint32_t oa[32], ob[32];
             at_ld32(tmem + lanes + kAtO + (uint32_t)(c * 32), oa);
-            if (n_tiles > 1) {
-                at_ld32(tmem + lanes + kAtO + 128u + (uint32_t)(c * 32), ob);
+            if (n_tiles > 1) at_ld32(tmem + lanes + kAtO + 128u + (uint32_t)(c * 32), ob);
 #pragma unroll
-                for (int k = 0; k < 32; k++)
-                    oa[k] = __float_as_uint(__uint_as_float(oa[k]) * ra + __uint_as_float(ob[k]) * rb);
-            } else {
-#pragma unroll
-                for (int k = 0; k < 32; k++) oa[k] = __float_as_uint(__uint_as_float(oa[k]) * ra);
+            for (int k = 0; k < 32; k++) {
+                float v = __uint_as_float(oa[k]) * ra;
+                if (n_tiles > 1) v += __uint_as_float(ob[k]) * rb;
+                oa[k] = __float_as_uint(v);
             }
-            if (valid) {
 #pragma unroll
-                for (int k = 0; k < 32; k += 4) {
-                    const float v[4] = {__uint_as_float(oa[k]), __uint_as_float(oa[k + 1]), __uint_as_float(oa[k + 2]), __uint_as_float(oa[k + 3])};
-                    if (c * 32 + k < a.vdim) src.put4(row, head * a.vdim + c * 32 + k, v);
-                }
+            for (int k = 0; k < 32; k += 4) *reinterpret_cast<uint4 *>(rows + r * kLd + c * 32 + k) = make_uint4(oa[k], oa[k + 1], oa[k + 2], oa[k + 3]);
+        }
+        vb_named_bar(1, kAtSoft);
+        for (int x = warp; x < kAtRows && P0 + x < pairs; x += kAtSoft / 32) {
+            const int m = (P0 + x) / group, hd = g * group + P0 + x - m * group;
+            for (int c = lane * 4; c < a.vdim; c += 128) {
+                const float4 o = *reinterpret_cast<const float4 *>(rows + x * kLd + c);
+                const float v[4] = {o.x, o.y, o.z, o.w};
+                src.put4(m, hd * a.vdim + c, v);
             }
         }
     } else if (warp < 12) {
