@@ -3,9 +3,9 @@
  * (tts_llm_prefill, voxtral_tts_llm.c:277-373): all prompt rows go through the
  * 26 layers, K and V of every row land in the cache, hidden states are dropped.
  *
- * The linears run on the tensor-core GEMM (vb_tc.cu; fp32 rows as three BF16 terms) in
- * blocks of up to 256 rows; RoPE, the cache write and the causal attention use the
- * stand-alone kernels. When the tensor maps cannot be made the same layer loop runs
+ * The linears run on the tensor-core GEMMs (vb_tc.cu, vb_tc_rows.cu; fp32 rows as three or two BF16 terms) in
+ * blocks of rows, the causal attention on the tensor cores too (vb_attn_tc.cuh). When the tensor maps cannot be made
+ * the same layer loop runs
  * on the streaming engine, eight rows at a time. Also here: the prompt assembled on
  * the device from token ids and BF16 voice rows (voxtral_tts.c:230-272).
  */
@@ -84,8 +84,8 @@ __global__ void pf_qkv_finish_kernel(float *qkv, const float *part, int n_part, 
 struct AtRows {
     static constexpr bool kAsync = false;
     const float *q, *kc, *vc;
-    float *out;
-    int ldq, ldkv, ldo, start_pos;
+    LmSink out;                  /* the terms that the O projection reads */
+    int ldq, ldkv, start_pos;
     VB_DEVINL void start() {}
     VB_DEVINL int pos0() const { return start_pos; }
     VB_DEVINL void q8(int row, int head, int d, float (&e)[8]) const {
@@ -123,162 +123,191 @@ struct AtRows {
         rows(vc, slot, g, lw, lane, j0, n);
     }
     VB_DEVINL float gate(int, int) const { return 1.0f; }
-    VB_DEVINL void put4(int row, int c, const float (&e)[4]) const {
-        *reinterpret_cast<float4 *>(out + (size_t)row * ldo + c) = make_float4(e[0], e[1], e[2], e[3]);
-    }
+    VB_DEVINL void put4(int row, int c, const float (&e)[4]) const { lm_put4(out, row, c, e); }
 };
 static_assert(VB200_HEAD_DIM == 128, "a lane's four columns cover a head");
 
 /* ---- tensor-core prefill ---- */
+/* Rows of a prompt that go through a layer at once: 1203 rows took 33.4 ms in blocks of 256, 23.9 ms in one. */
+constexpr int kPfRows = 2048;
+
 struct PrefillTc {
     bool ready = false;
     /* the decoder's tile-contiguous matrices (shared with the frame graph), fetched per call */
     const TcWeight *wqkv = nullptr, *wo = nullptr, *w13 = nullptr, *w2 = nullptr;
+    /* buffers of a call, kept between calls and only ever grown (allocating and freeing them per call cost up to
+     * 10 ms of a 7.6 ms prefill): rows of the whole prompt, then of a block of it */
+    float *x = nullptr, *cs = nullptr;
+    float *qkv = nullptr, *part = nullptr, *ssq = nullptr;
     uint16_t *bD = nullptr, *bQ = nullptr, *bH = nullptr;
-    float *part = nullptr, *ssq = nullptr;
-    TcActs aD[3], aQ[3], aH[3];   /* for 16, 64 and 256 padded rows, over the same buffers */
-    /* row buffers of a prefill call, kept between calls and only ever grown (allocating and
-     * freeing them per call cost up to 10 ms of a 7.6 ms prefill) */
-    float *x = nullptr, *qkv = nullptr, *attn = nullptr, *h = nullptr, *cs = nullptr;
-    int cap_rows = 0;
+    /* without tensor maps: all rows */
+    float *attn = nullptr, *h = nullptr;
+    /* a prompt given as ids and voice rows */
+    int *ids = nullptr;
+    uint16_t *voice = nullptr;
+    size_t cap[12] = {};
 };
 static PrefillTc g_pf;
 
 /* Called when the device context goes away: everything here pointed into it. */
 void prefill_free_all() {
     PrefillTc &t = g_pf;
-    cudaFree(t.x); cudaFree(t.qkv); cudaFree(t.attn); cudaFree(t.h); cudaFree(t.cs);
+    for (void *p : {(void *)t.x, (void *)t.cs, (void *)t.qkv, (void *)t.part, (void *)t.ssq, (void *)t.bD, (void *)t.bQ, (void *)t.bH,
+                    (void *)t.attn, (void *)t.h, (void *)t.ids, (void *)t.voice})
+        cudaFree(p);
     t = PrefillTc();
 }
 
-static int prefill_rows(int M) {
+/* Buffer i of g_pf at least that large; what it held is lost when it grows. New memory is zero: rows of the padding are
+ * multiplied like any other, and have to be finite. */
+template <class T>
+static int pf_grow(int i, T **p, size_t bytes) {
     PrefillTc &t = g_pf;
-    if (M <= t.cap_rows) return 0;
-    cudaFree(t.x); cudaFree(t.qkv); cudaFree(t.attn); cudaFree(t.h); cudaFree(t.cs);
-    t.x = t.qkv = t.attn = t.h = t.cs = nullptr;
-    t.cap_rows = 0;
-    const int cap = (M + 255) / 256 * 256;
-    if (cudaMalloc((void **)&t.x, (size_t)cap * D * 4) != cudaSuccess || cudaMalloc((void **)&t.qkv, (size_t)cap * QKV * 4) != cudaSuccess ||
-        cudaMalloc((void **)&t.attn, (size_t)cap * QD * 4) != cudaSuccess || cudaMalloc((void **)&t.h, (size_t)cap * HID * 4) != cudaSuccess ||
-        cudaMalloc((void **)&t.cs, (size_t)cap * VB200_HEAD_DIM * 4) != cudaSuccess) {
+    if (bytes <= t.cap[i]) return 0;
+    cudaFree(*p);
+    *p = nullptr;
+    t.cap[i] = 0;
+    if (cudaMalloc((void **)p, bytes) != cudaSuccess) {
         cudaGetLastError();
-        cudaFree(t.x); cudaFree(t.qkv); cudaFree(t.attn); cudaFree(t.h); cudaFree(t.cs);
-        t.x = t.qkv = t.attn = t.h = t.cs = nullptr;
+        *p = nullptr;
         return -1;
     }
-    t.cap_rows = cap;
-    return 0;
+    t.cap[i] = bytes;
+    return cudaMemsetAsync(*p, 0, bytes, model().st) == cudaSuccess ? 0 : -1;
 }
-static const int kPfRows = 256;
 
-static int pf_slot(int rows_pad) { return rows_pad == 16 ? 0 : rows_pad == 64 ? 1 : 2; }
-
-/* The activation-term buffers and their tensor maps; called after the decoder upload. Failing here is not fatal: prefill() then uses the streaming kernel. */
-int prefill_tc_setup() {
-    Model &m = model();
-    PrefillTc &t = g_pf;
-    t.ready = false;
-    if (getenv("VB200_NO_TC") || tc_init()) return 0;
-    if (!t.bD) {
-        void *p[5] = {};
-        const size_t sz[5] = {tc_acts_bytes(kPfRows, D), tc_acts_bytes(kPfRows, QD), tc_acts_bytes(kPfRows, HID),
-                              sizeof(float) * (size_t)kTcMaxSplits * kPfRows * QKV, sizeof(float) * kPfRows * 16};
-        for (int i = 0; i < 5; i++) {
-            if (cudaMalloc(&p[i], sz[i]) != cudaSuccess) return 0;
-            m.allocs.push_back(p[i]);
-            cudaMemset(p[i], 0, sz[i]);
-        }
-        t.bD = (uint16_t *)p[0]; t.bQ = (uint16_t *)p[1]; t.bH = (uint16_t *)p[2];
-        t.part = (float *)p[3]; t.ssq = (float *)p[4];
+/* Padded rows of a block, and the K splits of its GEMMs. */
+struct PfBlock {
+    int rows, rp, s_qkv, s_wo, s_w2;
+};
+static PfBlock pf_block(int rows) {
+    const int n = model().sm_count;
+    PfBlock b = {rows, tc_rows_pad_any(rows), 0, 0, 0};
+    if (b.rp <= 256) {           /* short sums, as in a frame's GEMMs; a GEMM of 256 rows has tiles for a sixth of the SMs */
+        b.s_qkv = tc_pick_splits(QKV, D, n); b.s_wo = tc_pick_splits(D, QD, n); b.s_w2 = tc_pick_splits(D, HID, n);
+    } else {
+        b.s_qkv = tc_row_splits(QKV, D, rows, n); b.s_wo = tc_row_splits(D, QD, rows, n); b.s_w2 = tc_row_splits(D, HID, rows, n);
     }
-    const int pads[3] = {16, 64, 256};
-    for (int i = 0; i < 3; i++)
-        if (tc_acts(&t.aD[i], t.bD, pads[i], D) || tc_acts(&t.aQ[i], t.bQ, pads[i], QD) ||
-            tc_acts(&t.aH[i], t.bH, pads[i], HID))
-            return 0;
-    t.ready = true;
+    return b;
+}
+
+static int pf_tc_buffers(int M, int block) {
+    PrefillTc &t = g_pf;
+    /* the last block may be split more ways than a full one */
+    size_t part = 0, pad = 0, rows = 0;
+    for (int r : {M < block ? M : block, M % block}) {
+        if (r == 0) continue;
+        const PfBlock b = pf_block(r);
+        for (size_t n : {(size_t)b.s_qkv * r * QKV, (size_t)b.s_wo * r * D, (size_t)b.s_w2 * r * D}) part = n > part ? n : part;
+        pad = (size_t)b.rp > pad ? b.rp : pad;
+        rows = (size_t)r > rows ? r : rows;
+    }
+    return pf_grow(2, &t.qkv, rows * QKV * 4) || pf_grow(3, &t.part, part * 4) || pf_grow(4, &t.ssq, rows * tc_prepare_chunks(D) * 4) ||
+                   pf_grow(5, &t.bD, tc_acts_bytes((int)pad, D)) || pf_grow(6, &t.bQ, tc_acts_bytes((int)pad, QD)) ||
+                   pf_grow(7, &t.bH, tc_acts_bytes((int)pad, HID))
+               ? -1
+               : 0;
+}
+
+/* Failing here is not fatal: prefill() then uses the streaming kernel. */
+int prefill_tc_setup() {
+    g_pf.ready = !getenv("VB200_NO_TC") && !tc_init();
     return 0;
 }
 
-/* Prefill with the tcgen05 GEMM (vb_tc.cu): per layer and per block of up to 256 rows
- * gain+terms -> QKV -> RoPE -> cache rows; causal attention over the whole cache prefix;
- * terms -> O -> residual+gain+terms -> gate/up with SwiGLU -> down -> residual. */
-static int prefill_tc(float *x, float *qkv, float *attn, const float *cs, int M, int start_pos) {
+/* Prefill with the tcgen05 GEMM (vb_tc.cu, vb_tc_rows.cu), a block of rows and a layer at a time:
+ * gain+terms -> QKV -> RoPE -> cache rows -> causal attention over the cache so far, which leaves terms -> O ->
+ * residual+gain+terms -> gate/up with SwiGLU -> down -> residual+gain+terms. */
+static int prefill_tc(float *x, const float *cs, int M, int start_pos, int block) {
     Model &m = model();
     PrefillTc &t = g_pf;
     cudaStream_t st = m.st;
     const float scale = 1.0f / sqrtf((float)VB200_HEAD_DIM);
-    const int s_qkv = tc_pick_splits(QKV, D, m.sm_count), s_wo = tc_pick_splits(D, QD, m.sm_count),
-              s_w2 = tc_pick_splits(D, HID, m.sm_count);
     const int chunksD = tc_prepare_chunks(D);
-    for (int l = 0; l < VB200_DEC_LAYERS; l++) {
-        const LayerDev &L = m.dec[l];
-        for (int r0 = 0; r0 < M; r0 += kPfRows) {
-            const int rows = M - r0 < kPfRows ? M - r0 : kPfRows;
-            const int slot = pf_slot(tc_rows_pad(rows));
-            float *xr = x + (size_t)r0 * D, *qr = qkv + (size_t)r0 * QKV;
-            tc_prepare(t.aD[slot], xr, D, rows, nullptr, 0, 0, nullptr, nullptr, L.attn_norm, t.ssq, st);
+    /* the row blocks follow one another through all layers: a row sees nothing of later rows */
+    for (int r0 = 0; r0 < M; r0 += block) {
+        const int rows = M - r0 < block ? M - r0 : block;
+        const PfBlock b = pf_block(rows);
+        TcActs aD, aQ, aH;
+        if (tc_acts(&aD, t.bD, b.rp, D) || tc_acts(&aQ, t.bQ, b.rp, QD) || tc_acts(&aH, t.bH, b.rp, HID)) return -1;
+        const LmSink q_terms = {nullptr, t.bQ, b.rp, QD, b.rp < 256 ? kTcTerms : 2};
+        const size_t psD = (size_t)rows * D;
+        float *xr = x + (size_t)r0 * D;
+        for (int l = 0; l < VB200_DEC_LAYERS; l++) {
+            const LayerDev &L = m.dec[l];
+            if (l == 0) tc_prepare(aD, xr, D, rows, nullptr, 0, 0, nullptr, nullptr, L.attn_norm, t.ssq, st);
             TcGemm g;
             g.M = rows; g.status = &m.d_out->status; g.epi = TC_EPI_PARTIAL; g.out = t.part; g.ld_out = QKV;
-            g.splits = s_qkv; g.ssq = t.ssq; g.ssq_chunks = chunksD; g.eps = VB200_NORM_EPS;
-            if (tc_gemm(t.wqkv[l], t.aD[slot], g, st)) return -1;
-            float *ck = m.kv_k + ((size_t)l * m.kv_max + start_pos + r0) * KVD;
-            float *cv = m.kv_v + ((size_t)l * m.kv_max + start_pos + r0) * KVD;
-            launch_pdl(pf_qkv_finish_kernel, dim3(QKV / 2 / 256, rows), dim3(256), 0, st, qr, (const float *)t.part, s_qkv,
-                       (size_t)rows * QKV, cs + (size_t)r0 * VB200_HEAD_DIM, ck, cv, rows);
-        }
-        const float *k0 = m.kv_k + (size_t)l * m.kv_max * KVD, *v0 = m.kv_v + (size_t)l * m.kv_max * KVD;
-        const AtRows rows_of = {qkv, k0, v0, attn, QKV, KVD, QD, start_pos};
-        const AtArgs at = {M, VB200_HEADS, VB200_KV_HEADS, VB200_HEAD_DIM, VB200_HEAD_DIM, 0, 0, scale, 0.0f, &m.d_out->status};
-        if (launch_attn_tc<2, 2>(at, rows_of, st)) return -1;
-        if (l == VB200_DEC_LAYERS - 1) break;   /* only the cache is kept (voxtral_tts_llm.c:281) */
-        for (int r0 = 0; r0 < M; r0 += kPfRows) {
-            const int rows = M - r0 < kPfRows ? M - r0 : kPfRows;
-            const int rp = tc_rows_pad(rows), slot = pf_slot(rp);
-            float *xr = x + (size_t)r0 * D;
-            const size_t psD = (size_t)rows * D;
-            tc_prepare(t.aQ[slot], attn + (size_t)r0 * QD, QD, rows, nullptr, 0, 0, nullptr, nullptr, nullptr, nullptr, st);
-            TcGemm g;
-            g.M = rows; g.status = &m.d_out->status; g.epi = TC_EPI_PARTIAL; g.out = t.part; g.ld_out = D;
-            g.splits = s_wo;
-            if (tc_gemm(t.wo[l], t.aQ[slot], g, st)) return -1;
-            tc_prepare(t.aD[slot], nullptr, D, rows, t.part, s_wo, psD, xr, xr, L.ffn_norm, t.ssq, st);
-            g.epi = TC_EPI_SWIGLU_TERMS; g.out = nullptr; g.out_terms = t.bH; g.out_rows_pad = rp; g.splits = 1;
-            g.ld_out = HID; g.ssq = t.ssq; g.ssq_chunks = chunksD; g.eps = VB200_NORM_EPS;
-            if (tc_gemm(t.w13[l], t.aD[slot], g, st)) return -1;
-            g.epi = TC_EPI_PARTIAL; g.out = t.part; g.out_terms = nullptr; g.splits = s_w2; g.ld_out = D;
+            g.splits = b.s_qkv; g.ssq = t.ssq; g.ssq_chunks = chunksD; g.eps = VB200_NORM_EPS;
+            if (tc_gemm(t.wqkv[l], aD, g, st)) return -1;
+            float *k0 = m.kv_k + (size_t)l * m.kv_max * KVD, *v0 = m.kv_v + (size_t)l * m.kv_max * KVD;
+            launch_pdl(pf_qkv_finish_kernel, dim3(QKV / 2 / 256, rows), dim3(256), 0, st, t.qkv, (const float *)t.part, b.s_qkv,
+                       (size_t)rows * QKV, cs + (size_t)r0 * VB200_HEAD_DIM, k0 + (size_t)(start_pos + r0) * KVD,
+                       v0 + (size_t)(start_pos + r0) * KVD, rows);
+            if (l == VB200_DEC_LAYERS - 1) break;   /* only the cache is kept (voxtral_tts_llm.c:281) */
+            const AtRows rows_of = {t.qkv, k0, v0, q_terms, QKV, KVD, start_pos + r0};
+            const AtArgs at = {rows, VB200_HEADS, VB200_KV_HEADS, VB200_HEAD_DIM, VB200_HEAD_DIM, 0, 0, scale, 0.0f, &m.d_out->status};
+            if (launch_attn_tc<2, 2>(at, rows_of, st)) return -1;
+            g.splits = b.s_wo; g.ld_out = D; g.ssq = nullptr; g.ssq_chunks = 0;
+            if (tc_gemm(t.wo[l], aQ, g, st)) return -1;
+            tc_prepare(aD, nullptr, D, rows, t.part, b.s_wo, psD, xr, xr, L.ffn_norm, t.ssq, st);
+            g.epi = TC_EPI_SWIGLU_TERMS; g.out = nullptr; g.out_terms = t.bH; g.out_rows_pad = b.rp; g.splits = 1;
+            g.ld_out = HID; g.ssq = t.ssq; g.ssq_chunks = chunksD;
+            if (tc_gemm(t.w13[l], aD, g, st)) return -1;
+            g.epi = TC_EPI_PARTIAL; g.out = t.part; g.out_terms = nullptr; g.splits = b.s_w2; g.ld_out = D;
             g.ssq = nullptr; g.ssq_chunks = 0;
-            if (tc_gemm(t.w2[l], t.aH[slot], g, st)) return -1;
-            /* residual add (the terms it also writes are overwritten by the next layer's prepare) */
-            tc_prepare(t.aD[slot], nullptr, D, rows, t.part, s_w2, psD, xr, xr, nullptr, nullptr, st);
+            if (tc_gemm(t.w2[l], aH, g, st)) return -1;
+            /* residual add and the next layer's rows */
+            tc_prepare(aD, nullptr, D, rows, t.part, b.s_w2, psD, xr, xr, m.dec[l + 1].attn_norm, t.ssq, st);
         }
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
+/* Checks, and the buffers of all rows: g_pf.x for the embeddings, the rotation table. */
+static int prefill_begin(int M, int start_pos) {
+    Model &m = model();
+    if (start_pos < 0 || start_pos + M > m.kv_max) {
+        fprintf(stderr, "voxtral_b200: prefill of %d rows at %d exceeds the %d-row cache\n", M, start_pos, m.kv_max);
+        return -1;
+    }
+    PrefillTc &t = g_pf;
+    if (pf_grow(0, &t.x, (size_t)M * D * 4) || pf_grow(1, &t.cs, (size_t)M * VB200_HEAD_DIM * 4)) return -1;
+    rope_table(t.cs, start_pos, M, VB200_HEAD_DIM, VB200_ROPE_THETA, m.st);
+    return 0;
+}
+
+static int prefill_run(int M, int start_pos);
+
 int prefill(const float *embeds, int seq_len, int start_pos) {
     Model &m = model();
     if (!m.inited || !m.llm_ready) return -1;
     if (seq_len <= 0) return 0;
-    if (start_pos < 0 || start_pos + seq_len > m.kv_max) {
-        fprintf(stderr, "voxtral_b200: prefill of %d rows at %d exceeds the %d-row cache\n", seq_len, start_pos,
-                m.kv_max);
-        return -1;
-    }
-    const int M = seq_len;
-    if (prefill_rows(M)) return -1;
-    float *x = g_pf.x, *qkv = g_pf.qkv, *attn = g_pf.attn, *h = g_pf.h, *cs = g_pf.cs;
+    if (prefill_begin(seq_len, start_pos)) return -1;
+    if (cudaMemcpyAsync(g_pf.x, embeds, (size_t)seq_len * D * 4, cudaMemcpyDefault, m.st) != cudaSuccess) return -1;
+    return prefill_run(seq_len, start_pos);
+}
+
+/* The rows are in g_pf.x. */
+static int prefill_run(int M, int start_pos) {
+    Model &m = model();
+    PrefillTc &t = g_pf;
+    float *x = t.x, *cs = t.cs;
     int rc = 0;
     const float scale = 1.0f / sqrtf((float)VB200_HEAD_DIM);
-    if (!rc && cudaMemcpyAsync(x, embeds, (size_t)M * D * 4, cudaMemcpyDefault, m.st) != cudaSuccess) rc = -1;
-    if (!rc) rope_table(cs, start_pos, M, VB200_HEAD_DIM, VB200_ROPE_THETA, m.st);
 
-    if (!rc && g_pf.ready && batch_tiled_decoder(&g_pf.wqkv, &g_pf.wo, &g_pf.w13, &g_pf.w2) == 0) {
-        rc = prefill_tc(x, qkv, attn, cs, M, start_pos);
-        if (cudaStreamSynchronize(m.st) != cudaSuccess) rc = -1;
+    if (t.ready && batch_tiled_decoder(&t.wqkv, &t.wo, &t.w13, &t.w2) == 0) {
+        int block = kPfRows;
+        while (pf_tc_buffers(M, block)) {      /* little memory left: smaller blocks */
+            if (block == 256) return -1;
+            block /= 2;
+        }
+        rc = prefill_tc(x, cs, M, start_pos, block);
+        int status = 0;
+        if (cudaMemcpyAsync(&status, &m.d_out->status, sizeof(int), cudaMemcpyDeviceToHost, m.st) != cudaSuccess ||
+            cudaStreamSynchronize(m.st) != cudaSuccess)
+            return -1;
         if (!rc) {
-            int status = 0;
-            cudaMemcpy(&status, &m.d_out->status, sizeof(int), cudaMemcpyDeviceToHost);
             m.last_status = status;
             if (status) {
                 /* the word is sticky on the device (kernels only set it from 0): clear it so the
@@ -289,6 +318,8 @@ int prefill(const float *embeds, int seq_len, int start_pos) {
         }
         return rc;
     }
+    if (pf_grow(2, &t.qkv, (size_t)M * QKV * 4) || pf_grow(8, &t.attn, (size_t)M * QD * 4) || pf_grow(9, &t.h, (size_t)M * HID * 4)) return -1;
+    float *qkv = t.qkv, *attn = t.attn, *h = t.h;
     for (int l = 0; l < VB200_DEC_LAYERS && !rc; l++) {
         const LayerDev &L = m.dec[l];
         float *ck = m.kv_k + ((size_t)l * m.kv_max + start_pos) * KVD;
@@ -390,27 +421,17 @@ int prefill_prompt(const int *text_ids, int n_text, const uint16_t *voice_bf16, 
     }
     ids.push_back(35);
     ids.push_back(25);
-    int *d_ids = nullptr;
-    uint16_t *d_voice = nullptr;
-    float *d_rows = nullptr;
-    int rc = -1;
-    do {
-        if (cudaMalloc(&d_ids, sizeof(int) * n) != cudaSuccess || cudaMalloc(&d_rows, sizeof(float) * (size_t)n * D) != cudaSuccess)
-            break;
-        if (n_voice > 0 && cudaMalloc(&d_voice, (size_t)n_voice * D * 2) != cudaSuccess) break;
-        if (cudaMemcpyAsync(d_ids, ids.data(), sizeof(int) * n, cudaMemcpyHostToDevice, m.st) != cudaSuccess) break;
-        if (n_voice > 0 &&
-            cudaMemcpyAsync(d_voice, voice_bf16, (size_t)n_voice * D * 2, cudaMemcpyHostToDevice, m.st) != cudaSuccess)
-            break;
-        prompt_rows_kernel<<<dim3((D + 255) / 256, n), 256, 0, m.st>>>(d_rows, m.tok_emb, d_voice, d_ids, D);
-        if (cudaGetLastError() != cudaSuccess) break;
-        rc = prefill(d_rows, n, start_pos) == 0 ? n : -1;    /* synchronises the stream */
-    } while (0);
-    cudaStreamSynchronize(m.st);
-    cudaFree(d_ids); cudaFree(d_voice); cudaFree(d_rows);
-    cudaGetLastError();
-    return rc;
+    if (prefill_begin(n, start_pos)) return -1;
+    PrefillTc &t = g_pf;
+    if (pf_grow(10, &t.ids, sizeof(int) * n) || pf_grow(11, &t.voice, (size_t)n_voice * D * 2)) return -1;
+    if (cudaMemcpyAsync(t.ids, ids.data(), sizeof(int) * n, cudaMemcpyHostToDevice, m.st) != cudaSuccess) return -1;
+    if (n_voice > 0 && cudaMemcpyAsync(t.voice, voice_bf16, (size_t)n_voice * D * 2, cudaMemcpyHostToDevice, m.st) != cudaSuccess) {
+        cudaStreamSynchronize(m.st);
+        return -1;
+    }
+    prompt_rows_kernel<<<dim3((D + 255) / 256, n), 256, 0, m.st>>>(t.x, m.tok_emb, t.voice, t.ids, D);
+    if (cudaGetLastError() != cudaSuccess) return -1;
+    return prefill_run(n, start_pos) == 0 ? n : -1;      /* synchronises the stream */
 }
 
 } // namespace vb
-
