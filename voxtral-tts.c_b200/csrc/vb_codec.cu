@@ -19,13 +19,18 @@
  *   C[m][parity * 1024 + oc] = sum over 2 taps of X[m - tap][ic] * W[ic][oc][parity + 2 tap],
  * whose row-major result [T][2048] IS the upsampled sequence [2T][1024]. Their (weight-normed)
  * weights are genuine fp32: they are split into W = hi + lo BF16 matrices (16 mantissa bits,
- * relative error 4e-6) and the row-block GEMM runs once on each, on the gathered activation
- * terms, into split-K partial buffers that one reduction sums together with the bias.
+ * relative error 4e-6), stacked as one matrix of 2 N rows, and the kernel that reads the partial
+ * results adds the two halves and the bias.
+ *
+ * A stage's GEMMs take the tile of its own row count and split K until the SMs are busy (5 frames: the
+ * down projection had 8 CTAs); the partial results are summed by the kernel that reads them, so that no
+ * launch only adds. 97 launches were, 75 are: 5 frames 0.62 -> 0.37 ms, 611 frames level.
  */
 #include "vb_common.cuh"
 #include "vb_model.cuh"
 #include "vb_tc.cuh"
 
+#include <algorithm>
 #include <math.h>
 #include <stdio.h>
 #include <string.h>
@@ -39,7 +44,6 @@ constexpr int CD = 1024, CH = 4096, CQKV = 3 * CD, CHEADS = 8, CHD = 128;
 constexpr int CEMB = 292, CSEM = 256, CSEM_ROWS = 8192, CPATCH = 240, CLAYERS = 8, CSTAGES = 4;
 constexpr float CEPS = 1e-2f, CQK_EPS = 1e-6f;
 constexpr int CFSQ = 21, CSPECIAL = 2, CCODES = 37;
-constexpr int kConvSplits = 4;      /* K splits per half (hi / lo) of a convolution GEMM */
 
 struct CodecLayer {
     TcWeight wqkv, wo, w13, w2;
@@ -52,9 +56,9 @@ struct Codec {
     bool ready = false;
     std::vector<void *> allocs;          /* weights */
     float *sem = nullptr;
-    /* convolutions as GEMMs: hi / lo BF16 halves of W[N][Kpad], bias[N] */
+    /* convolutions as GEMMs: hi BF16 halves of W[N][Kpad], the lo halves below them, bias[N] */
     struct Conv {
-        TcWeight hi, lo;
+        TcWeight w;
         float *bias = nullptr;
         int N = 0, K = 0, Kpad = 0, Cin = 0, taps = 0, mode = 0, left_pad = 0;
     } in_conv, up_conv[3], out_conv;
@@ -62,13 +66,13 @@ struct Codec {
     float *d_slopes = nullptr;
     /* activations, sized for cap_rows = 8 * frames */
     std::vector<void *> act_allocs;
-    int cap_frames = 0, rows_pad = 0;
+    int cap_frames = 0;
     int *codes = nullptr;
-    float *emb = nullptr, *x = nullptr, *x2 = nullptr, *y = nullptr, *qkv = nullptr, *attn = nullptr, *ssq = nullptr;
+    float *x = nullptr, *qkv = nullptr, *ssq = nullptr;
     float *pcm = nullptr;
     uint16_t *tD = nullptr, *tH = nullptr, *tC = nullptr;
-    float *part = nullptr;
-    TcActs aD, aH, aIn, aUp, aOut;
+    float *part = nullptr;               /* split-K partials of one GEMM */
+    size_t part_cap = 0;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     float last_ms = 0.0f;
 };
@@ -129,66 +133,126 @@ __global__ void convt_w_kernel(float *dst, const float *src, int ic, int oc, int
 
 /* ---------------------------------------------------------------- decode kernels */
 
-/* emb[t][0..255] = semantic_embedding[code], emb[t][256 + i] = FSQ level -> [-1, 1]
- * (voxtral_tts_codec.c:276-300). grid = frames, 320 threads. */
-__global__ void codec_embed_kernel(float *emb, const int *codes, const float *sem) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const int t = blockIdx.x, d = threadIdx.x;
-    const int *fc = codes + t * CCODES;
-    if (d < CSEM) {
-        int s = fc[0] - CSPECIAL;
-        s = s < 0 ? 0 : (s >= CSEM_ROWS ? CSEM_ROWS - 1 : s);
-        emb[(size_t)t * CEMB + d] = sem[(size_t)s * CSEM + d];
-    } else if (d < CEMB) {
-        int a = fc[d - CSEM + 1] - CSPECIAL;
-        a = a < 0 ? 0 : (a >= CFSQ ? CFSQ - 1 : a);
-        emb[(size_t)t * CEMB + d] = (float)a * 2.0f / (float)(CFSQ - 1) - 1.0f;
-    }
+/* Four values as BF16 terms; `term` elements between the terms, three of them or two. */
+VB_DEVINL void put_terms(uint16_t *o, size_t term, int n_terms, const float (&e)[4]) {
+    uint16_t t[3][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) vb_split3(e[i], t[0][i], t[1][i], t[2][i]);
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+        if (j < n_terms)
+            *reinterpret_cast<uint2 *>(o + j * term) = make_uint2(t[j][0] | ((uint32_t)t[j][1] << 16), t[j][2] | ((uint32_t)t[j][3] << 16));
 }
 
-/* The A operand of a convolution GEMM: terms[m][tap * Cin + ic] = hi / lo BF16 of X[src(m, tap)][ic]
- * (columns from taps * Cin up to Kpad are zero).
- * MODE 0, causal convolution with the reference's reflect rule (voxtral_tts_kernels.c:246-262):
- *   src = m + tap - left_pad; src < 0 -> -src; src >= T -> 2T - 2 - src; outside [0, T) -> 0.
- * MODE 1, stride-2 transposed convolution, kernel 4 (voxtral_tts_kernels.c:272-327: no left
- *   trim, the last two raw outputs dropped): src = m - tap, zero when negative.
- * grid = (Kpad / 1024 rounded up, T), 256 threads x 4 columns. */
-__global__ void codec_gather_kernel(uint16_t *buf, int rows_pad, int Kpad, const float *X, int ldx, int T, int Cin,
-                                    int taps, int mode, int left_pad) {
+/* Where a kernel's values come from: the sum of n split-K partials [rows][ld], `stride` floats apart. A convolution's
+ * has its lo half's columns `lo` further on (0: none), and its rows of N columns are rows of 1024 to the reader. */
+struct Parts {
+    const float *p;
+    int n, ld, N, lo;
+    size_t stride;
+    const float *bias;
+};
+VB_DEVINL float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+VB_DEVINL float4 parts_sum4(const Parts &g, int m, int c) {
+    const int e = m * CD + c, row = g.N == CD ? m : e / g.N, col = g.N == CD ? c : e - row * g.N;
+    const float *q = g.p + (size_t)row * g.ld + col;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 t[kTcMaxSplits], u[kTcMaxSplits];
+#pragma unroll
+    for (int i = 0; i < kTcMaxSplits; i++) {
+        t[i] = i < g.n ? vb_ldcg4(q + (size_t)i * g.stride) : zero;
+        u[i] = i < g.n && g.lo ? vb_ldcg4(q + (size_t)i * g.stride + g.lo) : zero;
+    }
+    float4 v = g.bias ? *reinterpret_cast<const float4 *>(g.bias + col) : zero;
+#pragma unroll
+    for (int i = 0; i < kTcMaxSplits; i++)
+        if (i < g.n) v = add4(v, g.lo ? add4(t[i], u[i]) : t[i]);
+    return v;
+}
+
+/* The operand of the input convolution's GEMM, straight from the codes: terms[m][tap * 292 + ic] of row
+ * src(m, tap) of the embedding (voxtral_tts_codec.c:276-300: 256 columns of the semantic table, then the FSQ levels as
+ * [-1, 1]), with the convolution's reflect rule (voxtral_tts_kernels.c:246-262: src = m + tap - left_pad; src < 0 ->
+ * -src; outside [0, T) -> 0; at the right end nothing reaches beyond). Columns from taps * 292 on are zero.
+ * grid = (Kpad / 1024 rounded up, T), 256 threads x 4 columns (292 is a multiple of 4: one tap each). */
+__global__ void codec_input_kernel(uint16_t *buf, int rows_pad, int n_terms, int Kpad, const int *codes, const float *sem, int T, int taps,
+                                   int left_pad) {
     pdl_launch_dependents();
     pdl_wait();
     const int m = blockIdx.y, k = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (k >= Kpad) return;
-    float e[4];
+    float e[4] = {0.f, 0.f, 0.f, 0.f};
+    const int tap = k / CEMB, ic = k - tap * CEMB;
+    int src = m + tap - left_pad;
+    if (src < 0) src = -src;
+    if (tap < taps && src < T) {
+        const int *fc = codes + src * CCODES;
+        if (ic < CSEM) {
+            int s = fc[0] - CSPECIAL;
+            s = s < 0 ? 0 : (s >= CSEM_ROWS ? CSEM_ROWS - 1 : s);
+            const float4 v = __ldg(reinterpret_cast<const float4 *>(sem + (size_t)s * CSEM + ic));
+            e[0] = v.x; e[1] = v.y; e[2] = v.z; e[3] = v.w;
+        } else {
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int kk = k + i;
-        float v = 0.0f;
-        if (kk < taps * Cin) {
-            const int tap = kk / Cin, ic = kk - tap * Cin;
-            int src;
-            bool ok;
-            if (mode == 0) {
-                src = m + tap - left_pad;
-                if (src < 0) src = -src;
-                else if (src >= T) src = 2 * T - 2 - src;
-                ok = src >= 0 && src < T;
-            } else {
-                src = m - tap;
-                ok = src >= 0;
+            for (int i = 0; i < 4; i++) {
+                int a = fc[ic + i - CSEM + 1] - CSPECIAL;
+                a = a < 0 ? 0 : (a >= CFSQ ? CFSQ - 1 : a);
+                e[i] = (float)a * 2.0f / (float)(CFSQ - 1) - 1.0f;
             }
-            if (ok) v = X[(size_t)src * ldx + ic];
         }
-        e[i] = v;
     }
-    uint16_t t0[4], t1[4], t2[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) vb_split3(e[i], t0[i], t1[i], t2[i]);
-    const size_t o = (size_t)m * Kpad + k, term = (size_t)rows_pad * Kpad;
-    *reinterpret_cast<uint2 *>(buf + o) = make_uint2(t0[0] | ((uint32_t)t0[1] << 16), t0[2] | ((uint32_t)t0[3] << 16));
-    *reinterpret_cast<uint2 *>(buf + term + o) = make_uint2(t1[0] | ((uint32_t)t1[1] << 16), t1[2] | ((uint32_t)t1[3] << 16));
-    *reinterpret_cast<uint2 *>(buf + 2 * term + o) = make_uint2(t2[0] | ((uint32_t)t2[1] << 16), t2[2] | ((uint32_t)t2[3] << 16));
+    put_terms(buf + (size_t)m * Kpad + k, (size_t)rows_pad * Kpad, n_terms, e);
+}
+
+/* A stage's last feed-forward update, and the operand of the convolution after it: row s, v = x + parts * scale, goes to
+ * every place terms[m][tap * 1024 ..] of the rows m that read it.
+ * UP, the stride-2 transposed convolution of kernel 4 (voxtral_tts_kernels.c:272-327: no left trim, the last two raw
+ * outputs dropped): rows s and s + 1, taps 0 and 1; row 0 has nothing in tap 1.
+ * Otherwise the causal convolution with the reflect rule: row s + left_pad - tap, and, mirrored, left_pad - tap - s for
+ * s > 0 (the last stage's rows are more than its taps). grid = T, 256 threads x 4 columns. */
+template <bool UP>
+__global__ void codec_scatter_kernel(uint16_t *buf, int rows_pad, int n_terms, const float *x, const Parts g, const float *scale, int T,
+                                     int taps) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int s = blockIdx.x, c = threadIdx.x * 4, K = taps * CD, left = taps - 1;
+    const float4 y = parts_sum4(g, s, c);
+    float4 v = *reinterpret_cast<const float4 *>(x + (size_t)s * CD + c);
+    if (scale) {
+        const float4 f = __ldg(reinterpret_cast<const float4 *>(scale + c));
+        v.x += y.x * f.x; v.y += y.y * f.y; v.z += y.z * f.z; v.w += y.w * f.w;
+    } else {
+        v = add4(v, y);
+    }
+    const float e[4] = {v.x, v.y, v.z, v.w};
+    const size_t term = (size_t)rows_pad * K;
+    if constexpr (UP) {
+        put_terms(buf + (size_t)s * K + c, term, n_terms, e);
+        if (s + 1 < T) put_terms(buf + (size_t)(s + 1) * K + CD + c, term, n_terms, e);
+        if (s == 0) {
+            const float none[4] = {0.f, 0.f, 0.f, 0.f};
+            put_terms(buf + CD + c, term, n_terms, none);
+        }
+    } else {
+        for (int tap = 0; tap < taps; tap++) {
+            const int m = s + left - tap, mirror = left - tap - s;
+            if (m < T) put_terms(buf + (size_t)m * K + tap * CD + c, term, n_terms, e);
+            if (s > 0 && mirror >= 0) put_terms(buf + (size_t)mirror * K + tap * CD + c, term, n_terms, e);
+        }
+    }
+}
+
+/* The output convolution's samples: partials of both halves and the bias. */
+__global__ void codec_samples_kernel(float *pcm, const Parts g, int T) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= T * g.N / 4) return;
+    const int m = i * 4 / g.N, c = i * 4 - m * g.N;
+    const float *q = g.p + (size_t)m * g.ld + c;
+    float4 v = g.bias ? *reinterpret_cast<const float4 *>(g.bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int p = 0; p < g.n; p++) v = add4(v, add4(vb_ldcg4(q + (size_t)p * g.stride), vb_ldcg4(q + (size_t)p * g.stride + g.lo)));
+    *reinterpret_cast<float4 *>(pcm + (size_t)m * g.N + c) = v;
 }
 
 /* W[N][K] fp32 -> hi[N][Kpad], lo[N][Kpad] BF16 with W = hi + lo up to 2^-17 (hi truncated, lo the
@@ -212,112 +276,118 @@ __global__ void split_w_kernel(uint16_t *hi, uint16_t *lo, const float *W, int N
 }
 
 /* Rows -> BF16 terms for the next GEMM, with the residual update folded in:
- *   v = x[m][c] (+ y[m][c] * yscale[c], or + y[m][c] without a layer scale);  x_out[m][c] = v
- *   terms = v * gain (or v), ssq[m] = sum v^2 (the GEMM applies 1/sqrt(ssq/K + eps))
- * grid = (K / 1024, rows), 256 threads x 4 columns; `buf` may be null (residual update only). */
-__global__ void codec_prepare_kernel(uint16_t *buf, int rows_pad, int K, const float *x, const float *y,
-                                     const float *yscale, float *x_out, const float *gain, float *ssq) {
+ *   v = parts (x null), x + parts * scale, or x + parts;  x_out[m] = v;  terms = v * gain,  ssq[m] = sum v^2 (the GEMM
+ *   applies 1/sqrt(ssq/K + eps)).  grid = rows, 256 threads x 4 columns. */
+__global__ void codec_prepare_kernel(uint16_t *buf, int rows_pad, int n_terms, const float *x, const Parts g, const float *scale,
+                                     float *x_out, const float *gain, float *ssq) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float red[8];
-    const int m = blockIdx.y, c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    float ss = 0.0f;
-    if (c < K) {
-        float4 v = *reinterpret_cast<const float4 *>(x + (size_t)m * K + c);
-        if (y) {
-            const float4 u = *reinterpret_cast<const float4 *>(y + (size_t)m * K + c);
-            if (yscale) {
-                const float4 s = __ldg(reinterpret_cast<const float4 *>(yscale + c));
-                v.x += u.x * s.x; v.y += u.y * s.y; v.z += u.z * s.z; v.w += u.w * s.w;
-            } else {
-                v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
-            }
-        }
-        if (x_out) *reinterpret_cast<float4 *>(x_out + (size_t)m * K + c) = v;
-        ss = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-        if (buf) {
-            if (gain) {
-                const float4 g = __ldg(reinterpret_cast<const float4 *>(gain + c));
-                v.x *= g.x; v.y *= g.y; v.z *= g.z; v.w *= g.w;
-            }
-            const float e[4] = {v.x, v.y, v.z, v.w};
-            uint16_t t0[4], t1[4], t2[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) vb_split3(e[i], t0[i], t1[i], t2[i]);
-            const size_t o = (size_t)m * K + c, term = (size_t)rows_pad * K;
-            *reinterpret_cast<uint2 *>(buf + o) = make_uint2(t0[0] | ((uint32_t)t0[1] << 16), t0[2] | ((uint32_t)t0[3] << 16));
-            *reinterpret_cast<uint2 *>(buf + term + o) = make_uint2(t1[0] | ((uint32_t)t1[1] << 16), t1[2] | ((uint32_t)t1[3] << 16));
-            *reinterpret_cast<uint2 *>(buf + 2 * term + o) = make_uint2(t2[0] | ((uint32_t)t2[1] << 16), t2[2] | ((uint32_t)t2[3] << 16));
+    const int m = blockIdx.x, c = threadIdx.x * 4;
+    float4 v = parts_sum4(g, m, c);
+    if (x) {
+        const float4 r = *reinterpret_cast<const float4 *>(x + (size_t)m * CD + c);
+        if (scale) {
+            const float4 f = __ldg(reinterpret_cast<const float4 *>(scale + c));
+            v = make_float4(r.x + v.x * f.x, r.y + v.y * f.y, r.z + v.z * f.z, r.w + v.w * f.w);
+        } else {
+            v = add4(r, v);
         }
     }
-    if (ssq) {
-        ss = vb_warp_sum(ss);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            float t = 0.0f;
-            for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[w];
-            ssq[m * gridDim.x + blockIdx.x] = t;
-        }
-    }
-}
-
-/* QK norm in place: RMSNorm over the whole 1024-wide q row and k row (tts_qk_norm,
- * voxtral_tts_kernels.c:351-355). grid = (rows, 2), 256 threads. */
-__global__ void codec_qknorm_kernel(float *qkv, const float *qw, const float *kw, float eps) {
-    pdl_launch_dependents();
-    pdl_wait();
-    __shared__ float red[8];
-    const float *w = blockIdx.y == 0 ? qw : kw;
-    if (!w) return;
-    float *row = qkv + (size_t)blockIdx.x * CQKV + blockIdx.y * CD;
-    float4 v = *reinterpret_cast<float4 *>(row + threadIdx.x * 4);
+    *reinterpret_cast<float4 *>(x_out + (size_t)m * CD + c) = v;
     float ss = vb_warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w);
+    const float4 w = __ldg(reinterpret_cast<const float4 *>(gain + c));
+    const float e[4] = {v.x * w.x, v.y * w.y, v.z * w.z, v.w * w.w};
+    put_terms(buf + (size_t)m * CD + c, (size_t)rows_pad * CD, n_terms, e);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
     __syncthreads();
-    float t = 0.0f;
-    for (int i = 0; i < 8; i++) t += red[i];
-    const float inv = 1.0f / sqrtf(t / (float)CD + eps);
-    const float4 g = __ldg(reinterpret_cast<const float4 *>(w + threadIdx.x * 4));
-    v.x = v.x * inv * g.x; v.y = v.y * inv * g.y; v.z = v.z * inv * g.z; v.w = v.w * inv * g.w;
-    *reinterpret_cast<float4 *>(row + threadIdx.x * 4) = v;
+    if (threadIdx.x == 0) {
+        float t = 0.0f;
+        for (int i = 0; i < 8; i++) t += red[i];
+        ssq[m] = t;
+    }
 }
 
-/* ALiBi sliding-window causal attention (tts_alibi_attention, voxtral_tts_kernels.c:527-596): one
- * warp per (row, head), a lane owns 4 of the 128 dims, keys max(0, i - window + 1) .. i taken in
- * order with the reference's running-maximum update. */
-__global__ void codec_attention_kernel(float *out, const float *qkv, int rows, int window, float scale,
-                                       const float *slopes8) {
+/* Sums q, k, v out of the partials; QK norm: RMSNorm over the whole 1024-wide q row and k row (tts_qk_norm,
+ * voxtral_tts_kernels.c:351-355). A single partial is normed in place (qkv = part), its values left alone.
+ * grid = (rows, 3, or 2 in place), 256 threads. */
+__global__ void codec_qkv_kernel(float *qkv, const float *part, int n, size_t stride, const float *qw, const float *kw, float eps) {
     pdl_launch_dependents();
     pdl_wait();
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= rows * CHEADS) return;
-    const int i = warp / CHEADS, h = warp % CHEADS;
+    __shared__ float red[8];
+    const float *w = blockIdx.y == 0 ? qw : blockIdx.y == 1 ? kw : nullptr;
+    const size_t at = (size_t)blockIdx.x * CQKV + blockIdx.y * CD + threadIdx.x * 4;
+    float4 t[kTcMaxSplits];
+#pragma unroll
+    for (int i = 0; i < kTcMaxSplits; i++) t[i] = i < n ? vb_ldcg4(part + i * stride + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v = t[0];
+#pragma unroll
+    for (int i = 1; i < kTcMaxSplits; i++)
+        if (i < n) v = add4(v, t[i]);
+    if (w) {
+        const float ss = vb_warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+        __syncthreads();
+        float sum = 0.0f;
+        for (int i = 0; i < 8; i++) sum += red[i];
+        const float inv = 1.0f / sqrtf(sum / (float)CD + eps);
+        const float4 g = __ldg(reinterpret_cast<const float4 *>(w + threadIdx.x * 4));
+        v.x = v.x * inv * g.x; v.y = v.y * inv * g.y; v.z = v.z * inv * g.z; v.w = v.w * inv * g.w;
+    }
+    *reinterpret_cast<float4 *>(qkv + at) = v;
+}
+
+/* ALiBi sliding-window causal attention (tts_alibi_attention, voxtral_tts_kernels.c:527-596), its result as the terms
+ * that the O projection reads: one warp per (row, head), a lane owns 4 of the 128 dims, keys max(0, i - window + 1) .. i
+ * in order, four of them requested together. The eight warps of a CTA take eight rows of one head, which share most of
+ * their keys in L1. grid = (rows / 8 rounded up, heads). */
+__global__ void __launch_bounds__(256) codec_attention_kernel(uint16_t *buf, int rows_pad, int n_terms, const float *qkv, int rows, int window,
+                                                              float scale, const float *slopes8) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5), h = blockIdx.y, lane = threadIdx.x & 31;
+    if (i >= rows) return;
     const float slope = slopes8[h];
-    const float4 q = *reinterpret_cast<const float4 *>(qkv + (size_t)i * CQKV + h * CHD + lane * 4);
+    const float *col = qkv + h * CHD + lane * 4;
+    const float4 q = *reinterpret_cast<const float4 *>(col + (size_t)i * CQKV);
     int j0 = 0;
     if (window > 0 && i - window + 1 > 0) j0 = i - window + 1;
     float mx = -1e30f, den = 0.0f;
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int j = j0; j <= i; j++) {
-        const float4 k = *reinterpret_cast<const float4 *>(qkv + (size_t)j * CQKV + CD + h * CHD + lane * 4);
-        const float4 v = *reinterpret_cast<const float4 *>(qkv + (size_t)j * CQKV + 2 * CD + h * CHD + lane * 4);
-        float s = vb_warp_sum(q.x * k.x + q.y * k.y + q.z * k.z + q.w * k.w);
-        s = __shfl_sync(0xffffffffu, s, 0);
-        s = s * scale + slope * (float)(j - i);
-        if (s > mx) {
-            const float corr = expf(mx - s);
-            den = den * corr + 1.0f;
-            o.x = o.x * corr + v.x; o.y = o.y * corr + v.y; o.z = o.z * corr + v.z; o.w = o.w * corr + v.w;
-            mx = s;
-        } else {
-            const float w = expf(s - mx);
+    for (int jb = j0; jb <= i; jb += 4) {
+        float4 k[4], v[4];
+        float s[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const float *r = col + (size_t)(jb + u < i ? jb + u : i) * CQKV;
+            k[u] = *reinterpret_cast<const float4 *>(r + CD);
+            v[u] = *reinterpret_cast<const float4 *>(r + 2 * CD);
+            s[u] = q.x * k[u].x + q.y * k[u].y + q.z * k[u].z + q.w * k[u].w;
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+            for (int u = 0; u < 4; u++) s[u] += __shfl_xor_sync(0xffffffffu, s[u], off);
+        float top = mx;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            s[u] = jb + u <= i ? s[u] * scale + slope * (float)(jb + u - i) : -INFINITY;
+            top = fmaxf(top, s[u]);
+        }
+        const float corr = expf(mx - top);
+        mx = top;
+        den *= corr;
+        o.x *= corr; o.y *= corr; o.z *= corr; o.w *= corr;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const float w = expf(s[u] - top);
             den += w;
-            o.x += w * v.x; o.y += w * v.y; o.z += w * v.z; o.w += w * v.w;
+            o.x += w * v[u].x; o.y += w * v[u].y; o.z += w * v[u].z; o.w += w * v[u].w;
         }
     }
     const float inv = den > 0.0f ? 1.0f / den : 0.0f;
-    *reinterpret_cast<float4 *>(out + (size_t)i * CD + h * CHD + lane * 4) = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+    const float e[4] = {o.x * inv, o.y * inv, o.z * inv, o.w * inv};
+    put_terms(buf + (size_t)i * CD + h * CHD + lane * 4, (size_t)rows_pad * CD, n_terms, e);
 }
 
 /* ---------------------------------------------------------------- host side */
@@ -361,87 +431,113 @@ int up_matrix(TcWeight *tw, const float *const *parts, const int *part_rows, int
     return rc;
 }
 
+/* The tile that a stage of so many rows takes, and the terms its GEMMs read of the activations. */
+int pad_of(int rows) { return rows <= 64 ? tc_rows_pad_frame(rows) : tc_rows_pad_any(rows); }
+int terms_of(int rows_pad) { return rows_pad < 256 ? kTcTerms : 2; }
+int splits_for(int N, int K, int rows) {
+    return pad_of(rows) < 256 ? tc_pick_splits(N, K, model().sm_count) : tc_row_splits(N, K, rows, model().sm_count);
+}
+
+/* Floats of split-K partials that a block of so many frames needs. */
+size_t part_floats(int frames) {
+    const Codec &c = g_codec;
+    size_t n = 0;
+    auto take = [&](int N, int K, int rows) { n = std::max(n, (size_t)splits_for(N, K, rows) * rows * N); };
+    take(2 * c.in_conv.N, c.in_conv.Kpad, frames);
+    for (int s = 0, rows = frames; s < CSTAGES; s++, rows *= 2) {
+        take(CQKV, CD, rows);
+        take(CD, CD, rows);
+        take(CD, CH, rows);
+        const Codec::Conv &cv = s < CSTAGES - 1 ? c.up_conv[s] : c.out_conv;
+        take(2 * cv.N, cv.Kpad, rows);
+    }
+    return n;
+}
+
 int ensure_buffers(int frames) {
     Codec &c = g_codec;
+    const size_t part = part_floats(frames);
+    if (part > c.part_cap) {
+        cudaFree(c.part);
+        c.part = nullptr;
+        c.part_cap = 0;
+        if (cudaMalloc((void **)&c.part, sizeof(float) * part) != cudaSuccess) {
+            cudaGetLastError();
+            c.part = nullptr;
+            fprintf(stderr, "voxtral_b200: codec: cudaMalloc(%zu bytes) failed\n", sizeof(float) * part);
+            return -1;
+        }
+        c.part_cap = part;
+    }
     if (frames <= c.cap_frames) return 0;
     c_free(&c.act_allocs);
     c.cap_frames = 0;
     const int rows = 8 * frames;
-    const int rp = tc_rows_pad_any(rows);
-    if (!rp) return -1;
+    /* operands: laid out anew for every stage and convolution (rows that a stage has not written hold an earlier one's:
+     * finite, and their results are never stored) */
+    size_t tD = 0, tH = 0, tC = tc_acts_bytes(pad_of(frames), c.in_conv.Kpad);
+    for (int s = 0; s < CSTAGES; s++) {
+        const int pad = pad_of(frames << s);
+        if (!pad) return -1;
+        tD = std::max(tD, tc_acts_bytes(pad, CD));
+        tH = std::max(tH, tc_acts_bytes(pad, CH));
+        tC = std::max(tC, tc_acts_bytes(pad, s < CSTAGES - 1 ? c.up_conv[s].Kpad : c.out_conv.Kpad));
+    }
     int rc = 0;
     rc |= c_alloc((void **)&c.codes, sizeof(int) * (size_t)frames * CCODES, &c.act_allocs);
-    rc |= c_alloc((void **)&c.emb, sizeof(float) * (size_t)frames * CEMB, &c.act_allocs);
     rc |= c_alloc((void **)&c.x, sizeof(float) * (size_t)rows * CD, &c.act_allocs);
-    rc |= c_alloc((void **)&c.x2, sizeof(float) * (size_t)rows * CD, &c.act_allocs);
-    rc |= c_alloc((void **)&c.y, sizeof(float) * (size_t)rows * CD, &c.act_allocs);
     rc |= c_alloc((void **)&c.qkv, sizeof(float) * (size_t)rows * CQKV, &c.act_allocs);
-    rc |= c_alloc((void **)&c.attn, sizeof(float) * (size_t)rows * CD, &c.act_allocs);
-    rc |= c_alloc((void **)&c.ssq, sizeof(float) * (size_t)rows * 4, &c.act_allocs);
+    rc |= c_alloc((void **)&c.ssq, sizeof(float) * (size_t)rows, &c.act_allocs);
     rc |= c_alloc((void **)&c.pcm, sizeof(float) * (size_t)rows * CPATCH, &c.act_allocs);
-    rc |= c_alloc((void **)&c.tD, tc_acts_bytes(rp, CD), &c.act_allocs);
-    rc |= c_alloc((void **)&c.tH, tc_acts_bytes(rp, CH), &c.act_allocs);
-    /* convolution operands: one buffer, laid out per convolution (every term is rewritten by the
-     * gather before each use); split-K partials of the largest convolution GEMM */
-    const int rp_in = tc_rows_pad_any(frames), rp_up = tc_rows_pad_any(4 * frames);
-    size_t conv_bytes = tc_acts_bytes(rp, c.out_conv.Kpad);
-    if (tc_acts_bytes(rp_up, c.up_conv[0].Kpad) > conv_bytes) conv_bytes = tc_acts_bytes(rp_up, c.up_conv[0].Kpad);
-    if (tc_acts_bytes(rp_in, c.in_conv.Kpad) > conv_bytes) conv_bytes = tc_acts_bytes(rp_in, c.in_conv.Kpad);
-    rc |= c_alloc((void **)&c.tC, conv_bytes, &c.act_allocs);
-    rc |= c_alloc((void **)&c.part, sizeof(float) * (size_t)2 * kConvSplits * 4 * frames * 2 * CD, &c.act_allocs);
+    rc |= c_alloc((void **)&c.tD, tD, &c.act_allocs);
+    rc |= c_alloc((void **)&c.tH, tH, &c.act_allocs);
+    rc |= c_alloc((void **)&c.tC, tC, &c.act_allocs);
     if (rc) { c_free(&c.act_allocs); return -1; }
-    cudaMemset(c.tC, 0, conv_bytes);
-    if (tc_acts(&c.aIn, c.tC, rp_in, c.in_conv.Kpad) || tc_acts(&c.aUp, c.tC, rp_up, c.up_conv[0].Kpad) ||
-        tc_acts(&c.aOut, c.tC, rp, c.out_conv.Kpad)) {
-        c_free(&c.act_allocs);
-        return -1;
-    }
-    /* rows of the padding are multiplied like any other (their results are never stored):
-     * keep them finite */
-    cudaMemset(c.tD, 0, tc_acts_bytes(rp, CD));
-    cudaMemset(c.tH, 0, tc_acts_bytes(rp, CH));
-    if (tc_acts(&c.aD, c.tD, rp, CD) || tc_acts(&c.aH, c.tH, rp, CH)) { c_free(&c.act_allocs); return -1; }
-    c.rows_pad = rp;
+    /* rows of the padding are multiplied like any other (their results are never stored): keep them finite */
+    cudaMemsetAsync(c.tD, 0, tD, model().st);
+    cudaMemsetAsync(c.tH, 0, tH, model().st);
+    cudaMemsetAsync(c.tC, 0, tC, model().st);
     c.cap_frames = frames;
     return 0;
 }
 
-/* One GEMM on `rows` rows of the padded term buffers. The term buffers are laid out for
- * c.rows_pad rows whatever `rows` is, so the same tensor maps serve every stage. */
-int gemm(const TcWeight &w, const TcActs &a, int rows, int epi, float *out, int ld_out, const float *ssq, float eps,
-         uint16_t *out_terms, cudaStream_t st) {
+/* One GEMM into split-K partials. */
+int gemm_parts(const TcWeight &w, const TcActs &a, int rows, const float *ssq, Parts *out, cudaStream_t st) {
     TcGemm g;
-    g.M = rows; g.splits = 1; g.epi = epi; g.out = out; g.ld_out = ld_out;
-    g.ssq = ssq; g.ssq_chunks = ssq ? 1 : 0; g.eps = eps;
-    g.out_terms = out_terms; g.out_rows_pad = g_codec.rows_pad;
+    g.M = rows; g.splits = splits_for(w.N, w.K, rows); g.epi = TC_EPI_PARTIAL; g.out = g_codec.part; g.ld_out = w.N;
+    g.ssq = ssq; g.ssq_chunks = ssq ? 1 : 0; g.eps = CEPS;
     g.status = &model().d_out->status;
+    *out = {g.out, g.splits, w.N, w.N, 0, (size_t)rows * w.N, nullptr};
     return tc_gemm(w, a, g, st);
 }
 
-int layer_forward(const CodecLayer &L, int rows, const float *y_prev, const float *yscale_prev, cudaStream_t st) {
+/* x and aD hold the rows of the layer's attention norm; leaves x and the partials of the feed-forward, which the caller
+ * adds (times ffn_scale) to x. */
+int layer_forward(const CodecLayer &L, const TcActs &aD, const TcActs &aH, int rows, Parts *out, cudaStream_t st) {
     Codec &c = g_codec;
+    const int rp = aD.rows_pad, terms = terms_of(rp);
     const float scale = 1.0f / sqrtf((float)CHD);
-    /* x (+ the previous layer's FFN update) -> attention-norm terms */
-    launch_pdl(codec_prepare_kernel, dim3(1, rows), dim3(256), 0, st, c.tD, c.rows_pad, CD, c.x, y_prev, yscale_prev,
-                                                        y_prev ? c.x : nullptr, L.attn_norm, c.ssq);
-    if (gemm(L.wqkv, c.aD, rows, TC_EPI_STORE, c.qkv, CQKV, c.ssq, CEPS, nullptr, st)) return -1;
-    if (L.q_norm || L.k_norm) launch_pdl(codec_qknorm_kernel, dim3(rows, 2), dim3(256), 0, st, c.qkv, L.q_norm, L.k_norm, CQK_EPS);
-    launch_pdl(codec_attention_kernel, dim3((rows * CHEADS * 32 + 255) / 256), dim3(256), 0, st, c.attn, c.qkv, rows, L.window, scale,
-                                                                            c.d_slopes);
-    launch_pdl(codec_prepare_kernel, dim3(1, rows), dim3(256), 0, st, c.tD, c.rows_pad, CD, c.attn, nullptr, nullptr, nullptr, nullptr,
-                                                        nullptr);
-    if (gemm(L.wo, c.aD, rows, TC_EPI_STORE, c.y, CD, nullptr, 0.0f, nullptr, st)) return -1;
-    /* x += proj * attn_scale -> FFN-norm terms */
-    launch_pdl(codec_prepare_kernel, dim3(1, rows), dim3(256), 0, st, c.tD, c.rows_pad, CD, c.x, c.y, L.attn_scale, c.x, L.ffn_norm,
-                                                        c.ssq);
-    if (gemm(L.w13, c.aD, rows, TC_EPI_SWIGLU_TERMS, nullptr, CH, c.ssq, CEPS, c.tH, st)) return -1;
-    if (gemm(L.w2, c.aH, rows, TC_EPI_STORE, c.y, CD, nullptr, 0.0f, nullptr, st)) return -1;
-    return 0;   /* the caller folds x += y * ffn_scale into the next step */
+    Parts p;
+    if (gemm_parts(L.wqkv, aD, rows, c.ssq, &p, st)) return -1;
+    float *qkv = p.n == 1 ? c.part : c.qkv;
+    if (p.n > 1 || L.q_norm || L.k_norm)
+        launch_pdl(codec_qkv_kernel, dim3(rows, p.n == 1 ? 2 : 3), dim3(256), 0, st, qkv, p.p, p.n, p.stride, (const float *)L.q_norm,
+                   (const float *)L.k_norm, CQK_EPS);
+    launch_pdl(codec_attention_kernel, dim3((rows + 7) / 8, CHEADS), dim3(256), 0, st, c.tD, rp, terms, (const float *)qkv, rows, L.window, scale,
+               (const float *)c.d_slopes);
+    if (gemm_parts(L.wo, aD, rows, nullptr, &p, st)) return -1;
+    launch_pdl(codec_prepare_kernel, dim3(rows), dim3(256), 0, st, c.tD, rp, terms, (const float *)c.x, p, (const float *)L.attn_scale, c.x,
+               (const float *)L.ffn_norm, c.ssq);
+    TcGemm g;
+    g.M = rows; g.splits = 1; g.epi = TC_EPI_SWIGLU_TERMS; g.ld_out = CH; g.ssq = c.ssq; g.ssq_chunks = 1; g.eps = CEPS;
+    g.out_terms = c.tH; g.out_rows_pad = rp; g.status = &model().d_out->status;
+    if (tc_gemm(L.w13, aD, g, st)) return -1;
+    return gemm_parts(L.w2, aH, rows, nullptr, out, st);
 }
 
 /* One convolution made ready as a GEMM: weights reordered to [N][taps * Cin] (a transposed
  * convolution: both parities stacked, N = 2 * out_ch, 2 taps each), split into hi / lo BF16
- * matrices and tiled; bias (repeated per parity). */
+ * matrices one below the other, tiled; bias (repeated per parity). */
 int conv_setup(Codec::Conv *cv, const vb200_conv_t &w, float *stage, std::vector<void *> *owner, cudaStream_t st) {
     const bool tr = w.is_transpose != 0;
     const size_t n = (size_t)w.in_ch * w.out_ch * w.kernel;
@@ -453,22 +549,18 @@ int conv_setup(Codec::Conv *cv, const vb200_conv_t &w, float *stage, std::vector
     cv->mode = tr ? 1 : 0;
     cv->left_pad = tr ? 0 : w.kernel - w.stride;
     float *ordered = stage + n;                                  /* second half of the staging buffer */
-    uint16_t *hi = nullptr, *lo = nullptr, *thi = nullptr, *tlo = nullptr;
+    uint16_t *both = nullptr, *tiled = nullptr;
     const size_t nk = (size_t)cv->N * cv->Kpad;
     int rc = 0;
     if (!w.weight || cudaMemcpyAsync(stage, w.weight, n * 4, cudaMemcpyHostToDevice, st) != cudaSuccess) return -1;
     if (tr) convt_w_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(ordered, stage, w.in_ch, w.out_ch, w.kernel);
     else conv_w_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(ordered, stage, w.out_ch, w.in_ch, w.kernel);
-    if (cudaMalloc((void **)&hi, nk * 2) != cudaSuccess || cudaMalloc((void **)&lo, nk * 2) != cudaSuccess) rc = -1;
-    if (!rc) split_w_kernel<<<(unsigned)((nk + 255) / 256), 256, 0, st>>>(hi, lo, ordered, cv->N, cv->K, cv->Kpad);
-    if (!rc && (c_alloc((void **)&thi, tc_tiled_bytes(cv->N, cv->Kpad), owner) ||
-                c_alloc((void **)&tlo, tc_tiled_bytes(cv->N, cv->Kpad), owner)))
-        rc = -1;
-    if (!rc && (tc_weight_tiled(&cv->hi, hi, cv->N, cv->Kpad, thi, st) || tc_weight_tiled(&cv->lo, lo, cv->N, cv->Kpad, tlo, st)))
-        rc = -1;
+    if (cudaMalloc((void **)&both, nk * 4) != cudaSuccess) rc = -1;
+    if (!rc) split_w_kernel<<<(unsigned)((nk + 255) / 256), 256, 0, st>>>(both, both + nk, ordered, cv->N, cv->K, cv->Kpad);
+    if (!rc && c_alloc((void **)&tiled, tc_tiled_bytes(2 * cv->N, cv->Kpad), owner)) rc = -1;
+    if (!rc && tc_weight_tiled(&cv->w, both, 2 * cv->N, cv->Kpad, tiled, st)) rc = -1;
     if (cudaStreamSynchronize(st) != cudaSuccess) rc = -1;
-    cudaFree(hi);
-    cudaFree(lo);
+    cudaFree(both);
     if (!rc && w.bias) {
         if (c_alloc((void **)&cv->bias, sizeof(float) * cv->N, owner)) return -1;
         for (int p = 0; p < (tr ? 2 : 1) && !rc; p++)
@@ -478,24 +570,10 @@ int conv_setup(Codec::Conv *cv, const vb200_conv_t &w, float *stage, std::vector
     return rc;
 }
 
-/* Runs one convolution: gather -> GEMM on the hi and on the lo matrix (split-K partials) -> sum +
- * bias into out [T][N]. */
-int conv_run(const Codec::Conv &cv, const TcActs &acts, const float *X, int ldx, int T, float *out, cudaStream_t st) {
-    Codec &c = g_codec;
-    launch_pdl(codec_gather_kernel, dim3((cv.Kpad + 1023) / 1024, T), dim3(256), 0, st, acts.buf, acts.rows_pad, cv.Kpad, X, ldx, T, cv.Cin,
-                                                                          cv.taps, cv.mode, cv.left_pad);
-    const int pairs = ((cv.N + kTcTileN - 1) / kTcTileN + 1) / 2, blocks = (T + 127) / 128;
-    int splits = model().sm_count / (pairs * blocks);
-    if (splits > kConvSplits) splits = kConvSplits;
-    if (splits > cv.Kpad / kTcBlockK) splits = cv.Kpad / kTcBlockK;
-    if (splits < 1) splits = 1;
-    TcGemm g;
-    g.M = T; g.splits = splits; g.epi = TC_EPI_PARTIAL; g.ld_out = cv.N; g.status = &model().d_out->status;
-    g.out = c.part;
-    if (tc_gemm(cv.hi, acts, g, st)) return -1;
-    g.out = c.part + (size_t)splits * T * cv.N;
-    if (tc_gemm(cv.lo, acts, g, st)) return -1;
-    tc_reduce(out, c.part, 2 * splits, (size_t)T * cv.N, (size_t)T * cv.N, cv.bias, cv.N, st);
+/* One convolution's GEMM on its operand in tC; the reader adds the halves and the bias. */
+int conv_run(const Codec::Conv &cv, const TcActs &acts, int T, Parts *out, cudaStream_t st) {
+    if (gemm_parts(cv.w, acts, T, nullptr, out, st)) return -1;
+    out->N = cv.N; out->lo = cv.N; out->bias = cv.bias;
     return 0;
 }
 
@@ -505,6 +583,7 @@ void codec_free_all() {
     Codec &c = g_codec;
     c_free(&c.allocs);
     c_free(&c.act_allocs);
+    cudaFree(c.part);
     if (c.e0) cudaEventDestroy(c.e0);
     if (c.e1) cudaEventDestroy(c.e1);
     c = Codec();
@@ -603,28 +682,30 @@ static int decode_block(const int *codes, int n_frames, int skip, float *samples
     if (cudaMemcpyAsync(c.codes, codes, sizeof(int) * (size_t)n_frames * CCODES, cudaMemcpyHostToDevice, st) != cudaSuccess)
         return -1;
     cudaEventRecord(c.e0, st);
-    launch_pdl(codec_embed_kernel, dim3(n_frames), dim3(320), 0, st, c.emb, c.codes, c.sem);
-    int rows = n_frames;
-    if (conv_run(c.in_conv, c.aIn, c.emb, CEMB, rows, c.x, st)) return -1;
+    int rows = n_frames, rp = pad_of(rows);
+    TcActs acts, aD, aH;
+    Parts p;
+    launch_pdl(codec_input_kernel, dim3((c.in_conv.Kpad + 1023) / 1024, rows), dim3(256), 0, st, c.tC, rp, terms_of(rp), c.in_conv.Kpad,
+               (const int *)c.codes, (const float *)c.sem, rows, c.in_conv.taps, c.in_conv.left_pad);
+    if (tc_acts(&acts, c.tC, rp, c.in_conv.Kpad) || conv_run(c.in_conv, acts, rows, &p, st)) return -1;
     int l = 0;
     for (int stage = 0; stage < CSTAGES; stage++) {
-        const float *y_prev = nullptr, *sc_prev = nullptr;
+        rp = pad_of(rows);
+        if (tc_acts(&aD, c.tD, rp, CD) || tc_acts(&aH, c.tH, rp, CH)) return -1;
         for (int i = 0; i < 2; i++, l++) {
-            if (layer_forward(c.L[l], rows, y_prev, sc_prev, st)) return -1;
-            y_prev = c.y;
-            sc_prev = c.L[l].ffn_scale;
+            /* the convolution's rows, or the layer before's feed-forward update */
+            launch_pdl(codec_prepare_kernel, dim3(rows), dim3(256), 0, st, c.tD, rp, terms_of(rp), i ? (const float *)c.x : (const float *)nullptr, p,
+                       i ? (const float *)c.L[l - 1].ffn_scale : (const float *)nullptr, c.x, (const float *)c.L[l].attn_norm, c.ssq);
+            if (layer_forward(c.L[l], aD, aH, rows, &p, st)) return -1;
         }
-        /* the stage's last FFN update, no terms */
-        launch_pdl(codec_prepare_kernel, dim3(1, rows), dim3(256), 0, st, nullptr, c.rows_pad, CD, c.x, y_prev, sc_prev, c.x, nullptr,
-                                                            nullptr);
-        if (stage < CSTAGES - 1) {
-            /* [rows][2 x 1024] row-major = [2 rows][1024] */
-            if (conv_run(c.up_conv[stage], c.aUp, c.x, CD, rows, c.x2, st)) return -1;
-            float *t = c.x; c.x = c.x2; c.x2 = t;
-            rows *= 2;
-        }
+        const bool up = stage < CSTAGES - 1;
+        const Codec::Conv &cv = up ? c.up_conv[stage] : c.out_conv;
+        launch_pdl(up ? codec_scatter_kernel<true> : codec_scatter_kernel<false>, dim3(rows), dim3(256), 0, st, c.tC, rp, terms_of(rp),
+                   (const float *)c.x, p, (const float *)c.L[l - 1].ffn_scale, rows, cv.taps);
+        if (tc_acts(&acts, c.tC, rp, cv.Kpad) || conv_run(cv, acts, rows, &p, st)) return -1;
+        if (up) rows *= 2;      /* [rows][2 x 1024] row-major = [2 rows][1024] */
     }
-    if (conv_run(c.out_conv, c.aOut, c.x, CD, rows, c.pcm, st)) return -1;
+    launch_pdl(codec_samples_kernel, dim3((rows * CPATCH / 4 + 255) / 256), dim3(256), 0, st, c.pcm, p, rows);
     cudaEventRecord(c.e1, st);
     int status = 0;
     if (cudaMemcpyAsync(samples_out, c.pcm + (size_t)skip * 8 * CPATCH, sizeof(float) * total, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
