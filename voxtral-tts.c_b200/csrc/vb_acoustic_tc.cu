@@ -4,10 +4,9 @@
  * tts_acoustic_forward (voxtral_tts_acoustic.c:268-373): semantic head + argmax, then 7
  * Euler steps; both guidance branches of a step run together as six token rows
  * (voxtral_tts_acoustic.c:198-212, :345-348), so every layer matrix is streamed once per
- * step by the tcgen05 GEMM (vb_tc.cu). Around the GEMMs sit small kernels: token
- * build + Euler update, 3-token attention, split-K reduction + residual + RMSNorm +
- * BF16 term split ("prepare"), velocity head, FSQ. The sequence (about 200 launches) is
- * captured once as a CUDA graph and replayed per frame.
+ * step by the tcgen05 GEMM (vb_tc.cu), whose out- and down projections also finish the sublayer (TcJoin). Between the
+ * GEMMs sit small kernels: token build + Euler update, 3-token attention, velocity head, FSQ. The sequence (127
+ * launches) is captured once as a CUDA graph and replayed per frame.
  */
 #include "vb_acoustic_tc.cuh"
 #include "vb_common.cuh"
@@ -27,7 +26,7 @@ struct AcTc {
     bool ready = false;
     TcWeight wqkv[VB200_AC_LAYERS], wo[VB200_AC_LAYERS], w13[VB200_AC_LAYERS], w2[VB200_AC_LAYERS];
     uint16_t *tiled[VB200_AC_LAYERS][4] = {};   /* tile-contiguous weight copies */
-    int s_qkv = 1, s_wo = 1, s_w2 = 1;
+    int s_qkv = 1;
     AcBuffers one;              /* the single-utterance buffers */
 };
 static AcTc g_ac;
@@ -159,12 +158,12 @@ __global__ void ac_attention_kernel(uint16_t *terms, const float *part, int n_pa
     *reinterpret_cast<uint2 *>(terms + 2 * term + off) = make_uint2(t2[0] | ((uint32_t)t2[1] << 16), t2[2] | ((uint32_t)t2[3] << 16));
 }
 
-/* Last residual add, final RMSNorm of token 0 of each branch (rows 0 and 3) and the 36-wide
+/* Final RMSNorm of token 0 of each branch (rows 0 and 3) and the 36-wide
  * velocity head (voxtral_tts_acoustic.c:255-261). grid = (9, 2 * utterances): blockIdx.y =
  * 2 * utterance + branch, four of the 36 outputs per CTA (every CTA re-derives the normalised
  * row; it is 12 KB). */
-__global__ void ac_velocity_kernel(float *vel, const float *X6, const float *part, int n_part, const float *gain,
-                                   float eps, const uint16_t *Wout, int ROWS, int vel_stride) {
+__global__ void ac_velocity_kernel(float *vel, const float *X6, const float *gain, float eps, const uint16_t *Wout,
+                                   int vel_stride) {
     __shared__ float xn[VB200_DIM];
     __shared__ float red[32];
     pdl_launch_dependents();
@@ -180,27 +179,17 @@ __global__ void ac_velocity_kernel(float *vel, const float *X6, const float *par
     }
     pdl_wait();
     const int row = blockIdx.y * 3;
-    const size_t ps = (size_t)ROWS * D;
     float ss = 0.0f;
-    /* 512 threads x 6 columns; the 6 x (n_part + 1) loads of a thread are issued together */
+    /* 512 threads x 6 columns; the loads of a thread are issued together */
     {
         constexpr int kCols = VB200_DIM / 512;
-        float pv[kCols][kTcMaxSplits], xv[kCols];
+        float xv[kCols];
+#pragma unroll
+        for (int i = 0; i < kCols; i++) xv[i] = __ldcg(X6 + (size_t)row * D + threadIdx.x + i * 512);
 #pragma unroll
         for (int i = 0; i < kCols; i++) {
-            const int c = threadIdx.x + i * 512;
-            xv[i] = __ldcg(X6 + (size_t)row * D + c);
-#pragma unroll
-            for (int p = 0; p < kTcMaxSplits; p++) pv[i][p] = p < n_part ? __ldcg(part + p * ps + (size_t)row * D + c) : 0.0f;
-        }
-#pragma unroll
-        for (int i = 0; i < kCols; i++) {
-            float s = 0.0f;
-#pragma unroll
-            for (int p = 0; p < kTcMaxSplits; p++) s += pv[i][p];     /* split order; unused splits add 0 */
-            const float v = xv[i] + s;
-            xn[threadIdx.x + i * 512] = v;
-            ss += v * v;
+            xn[threadIdx.x + i * 512] = xv[i];
+            ss += xv[i] * xv[i];
         }
     }
     ss = vb_warp_sum(ss);
@@ -283,7 +272,7 @@ int acoustic_buffers_alloc(AcBuffers *b, int B, std::vector<void *> *owner) {
     if (alloc_zero((void **)&b->bD, tc_acts_bytes(rp, D), owner) || alloc_zero((void **)&b->bQ, tc_acts_bytes(rp, QD), owner) ||
         alloc_zero((void **)&b->bH, tc_acts_bytes(rp, HID), owner) ||
         alloc_zero((void **)&b->part, sizeof(float) * kTcMaxSplits * rows * QKV, owner) ||
-        alloc_zero((void **)&b->ssq, sizeof(float) * rows * 16, owner))
+        alloc_zero((void **)&b->ssq, sizeof(float) * rows * (D / kTcTileN), owner))
         return -1;
     if (!b->X6 && alloc_zero((void **)&b->X6, sizeof(float) * rows * D, owner)) return -1;
     if (tc_acts(&b->aD, b->bD, rp, D) || tc_acts(&b->aQ, b->bQ, rp, QD) || tc_acts(&b->aH, b->bH, rp, HID)) return -1;
@@ -331,8 +320,6 @@ int acoustic_tc_setup() {
     o.dyn = &m.d_in->dyn;
     o.status = &m.d_out->status;
     t.s_qkv = tc_pick_splits(QKV, D, m.sm_count);
-    t.s_wo = tc_pick_splits(D, QD, m.sm_count);
-    t.s_w2 = tc_pick_splits(D, HID, m.sm_count);
     t.ready = true;
     return 0;
 }
@@ -350,38 +337,39 @@ int acoustic_tc_enqueue_on(const AcBuffers &b, const float *noise_all, int *code
     const float scale = 1.0f / sqrtf((float)VB200_HEAD_DIM);
     const int steps = VB200_FLOW_STEPS - 1;
     const int ROWS = b.rows;
-    const size_t psD = (size_t)ROWS * D;
-    const int chunksD = tc_prepare_chunks(D);
-    TcGemm g;
-    g.M = ROWS; g.status = b.status;
     for (int s = 0; s < steps; s++) {
         launch_pdl(ac_tokens_kernel, dim3((D + 127) / 128, b.B), dim3(128), 0, st, b.X6, b.lat, (const float *)b.vel,
                    (const uint16_t *)m.ac_input_proj, (const float *)m.ttok, (const float *)b.ltok, s,
                    VB200_CFG_ALPHA, s > 0 ? m.dt[s - 1] : 0.0f, noise_all, (const VbDyn *)b.dyn, b.sd);
         for (int l = 0; l < VB200_AC_LAYERS; l++) {
             const LayerDev &L = m.ac[l];
-            /* attention half: (reduce + residual +) gain -> QKV -> attention -> O */
+            /* attention half: QKV -> attention -> O, which leaves the new rows and the next norm's operand */
             if (l == 0) tc_prepare(b.aD, b.X6, D, ROWS, nullptr, 0, 0, nullptr, nullptr, L.attn_norm, b.ssq, st);
-            else tc_prepare(b.aD, nullptr, D, ROWS, b.part, t.s_w2, psD, b.X6, b.X6, L.attn_norm, b.ssq, st);
-            g.epi = TC_EPI_PARTIAL; g.out = b.part; g.out_terms = nullptr;
-            g.splits = t.s_qkv; g.ld_out = QKV; g.ssq = b.ssq; g.ssq_chunks = chunksD; g.eps = VB200_NORM_EPS;
+            TcGemm g;
+            g.M = ROWS; g.status = b.status;
+            g.epi = TC_EPI_PARTIAL; g.out = b.part;
+            g.splits = t.s_qkv; g.ld_out = QKV; g.ssq = b.ssq; g.ssq_chunks = l == 0 ? tc_prepare_chunks(D) : D / kTcTileN;
+            g.eps = VB200_NORM_EPS;
             if (tc_gemm(t.wqkv[l], b.aD, g, st)) return -1;
             launch_pdl(ac_attention_kernel, dim3((ROWS * VB200_HEADS * 32 + 255) / 256), dim3(256), 0, st, b.bQ,
                        (const float *)b.part, t.s_qkv, scale, ROWS, b.rows_pad);
-            g.splits = t.s_wo; g.ld_out = D; g.ssq = nullptr; g.ssq_chunks = 0;
+            g = TcGemm();
+            g.M = ROWS; g.status = b.status;
+            g.join = {b.X6, b.X6, L.ffn_norm, b.bD, b.rows_pad, b.ssq, nullptr};
             if (tc_gemm(t.wo[l], b.aQ, g, st)) return -1;
-            /* FFN half: reduce + residual + gain -> gate/up with SwiGLU (terms out) -> down */
-            tc_prepare(b.aD, nullptr, D, ROWS, b.part, t.s_wo, psD, b.X6, b.X6, L.ffn_norm, b.ssq, st);
-            g.epi = TC_EPI_SWIGLU_TERMS; g.out = nullptr; g.out_terms = b.bH; g.out_rows_pad = b.rows_pad;
-            g.splits = 1; g.ld_out = HID; g.ssq = b.ssq; g.ssq_chunks = chunksD;
+            /* FFN half: gate/up with SwiGLU (terms out) -> down */
+            g = TcGemm();
+            g.M = ROWS; g.status = b.status;
+            g.epi = TC_EPI_SWIGLU_TERMS; g.out_terms = b.bH; g.out_rows_pad = b.rows_pad;
+            g.ld_out = HID; g.ssq = b.ssq; g.ssq_chunks = D / kTcTileN; g.eps = VB200_NORM_EPS;
             if (tc_gemm(t.w13[l], b.aD, g, st)) return -1;
-            g.epi = TC_EPI_PARTIAL; g.out = b.part; g.out_terms = nullptr;
-            g.splits = t.s_w2; g.ld_out = D; g.ssq = nullptr; g.ssq_chunks = 0;
+            g = TcGemm();
+            g.M = ROWS; g.status = b.status;
+            g.join = {b.X6, b.X6, l + 1 < VB200_AC_LAYERS ? m.ac[l + 1].attn_norm : nullptr, b.bD, b.rows_pad, b.ssq, nullptr};
             if (tc_gemm(t.w2[l], b.aH, g, st)) return -1;
         }
-        launch_pdl(ac_velocity_kernel, dim3(9, 2 * b.B), dim3(512), 0, st, b.vel, (const float *)b.X6,
-                   (const float *)b.part, t.s_w2, (const float *)m.ac_norm, VB200_NORM_EPS, (const uint16_t *)m.ac_out,
-                   ROWS, b.sd.vel);
+        launch_pdl(ac_velocity_kernel, dim3(9, 2 * b.B), dim3(512), 0, st, b.vel, (const float *)b.X6, (const float *)m.ac_norm,
+                   VB200_NORM_EPS, (const uint16_t *)m.ac_out, b.sd.vel);
     }
     launch_pdl(ac_fsq_kernel, dim3(b.B), dim3(64), 0, st, b.codes, b.lat, (const float *)b.vel, steps,
                VB200_FSQ_LEVELS, VB200_CFG_ALPHA, m.dt[steps - 1], codes_all, b.dyn, frame_cap,

@@ -12,7 +12,8 @@
  *
  * One frame is a fixed sequence of launches (captured as a CUDA graph):
  *   embed (from the previous frame's codes)
- *   26 x [prepare, QKV GEMM, decode attention, O GEMM, prepare, gate/up GEMM, down GEMM]
+ *   prepare, 26 x [QKV GEMM, decode attention, O GEMM, gate/up GEMM, down GEMM]; the O and the down GEMM finish their
+ *   sublayers (TcJoin), under tensor parallelism a "prepare" after each does
  *   final norm, semantic-head GEMM + argmax, llm_proj GEMM
  *   7 Euler steps + FSQ (vb_acoustic_tc.cu), which also advances every utterance.
  *
@@ -958,7 +959,7 @@ static int ctx_open(Batch &t, bool single, int n_utt, int kv_max, int max_frames
         t.part_wo = (float *)(g_tp.arena + g_tp.ll.part[TP_WO]);
         t.part_w2 = (float *)(g_tp.arena + g_tp.ll.part[TP_W2]);
     }
-    rc |= bt_alloc((void **)&t.ssq, sizeof(float) * 16 * 16, &t.allocs);
+    rc |= bt_alloc((void **)&t.ssq, sizeof(float) * 16 * (D / kTcTileN), &t.allocs);
     rc |= bt_alloc((void **)&t.logit_part, sizeof(float) * kTcMaxSplits * B * NSEM, &t.allocs);
     rc |= bt_alloc((void **)&t.attn_scratch,
                    sizeof(float) * (size_t)B * VB200_KV_HEADS * kBtKeySplits * kGroup * (kHD + 2), &t.allocs);
@@ -1000,10 +1001,11 @@ static int enqueue_decoder(Batch &t) {
     cudaStream_t st = m.st;
     const int B = t.B;
     const float scale = 1.0f / sqrtf((float)kHD);
-    const int chunksD = tc_prepare_chunks(D);
     const size_t psD = (size_t)B * D, psQ = (size_t)B * QKV;
     /* Tensor parallelism: this rank's tile slice of each layer GEMM, split-K chosen for the slice. */
     const bool tp = t.tp;
+    /* who leaves a row's sums of squares: "prepare", or the GEMM before (TcJoin) */
+    const int chunksD = tp ? tc_prepare_chunks(D) : D / kTcTileN;
     int q0 = 0, qn = 0, o0 = 0, on = 0, h0 = 0, hn = 0;
     int s_qkv = w.s_qkv, s_wo = w.s_wo, s_w2 = w.s_w2;
     if (tp) {
@@ -1028,12 +1030,12 @@ static int enqueue_decoder(Batch &t) {
          * FFN half of every layer, as the parity tests read them (voxtral_tts_llm.c:245,263) */
         float *const tap_base = (t.single && m.tap_on) ? m.tap : nullptr;
         if (l == 0) tc_prepare(t.aD, t.X, D, B, nullptr, 0, 0, nullptr, nullptr, L.attn_norm, t.ssq, st);
-        else tc_prepare(t.aD, nullptr, D, B, t.part_w2, s_w2, psD, t.X, t.X, L.attn_norm, t.ssq, st,
+        else if (tp) tc_prepare(t.aD, nullptr, D, B, t.part_w2, s_w2, psD, t.X, t.X, L.attn_norm, t.ssq, st,
                         tp_wait_for(0, TP_W2, NL, l, t.status), tap_base ? tap_base + (size_t)(2 * l - 1) * D : nullptr);
         TcGemm g;
         g.M = B; g.status = t.status; g.eps = VB200_NORM_EPS;
         g.epi = TC_EPI_PARTIAL; g.out = t.part_qkv; g.splits = s_qkv; g.ld_out = QKV;
-        g.ssq = t.ssq; g.ssq_chunks = chunksD;
+        g.ssq = t.ssq; g.ssq_chunks = l == 0 ? tc_prepare_chunks(D) : chunksD;
         if (tp) { g.tile0 = q0; g.n_tiles = qn; g.push = tp_push(0, TP_QKV, NL, l + 1); }
         if (tc_gemm(w.wqkv[l], t.aD, g, st)) return -1;
         if (tp)
@@ -1053,8 +1055,9 @@ static int enqueue_decoder(Batch &t) {
         g.M = B; g.status = t.status; g.eps = VB200_NORM_EPS;
         g.epi = TC_EPI_PARTIAL; g.out = t.part_wo; g.splits = s_wo; g.ld_out = D;
         if (tp) { g.tile0 = o0; g.n_tiles = on; g.push = tp_push(0, TP_WO, NL, l + 1); }
+        else g.join = {t.X, t.X, L.ffn_norm, t.bD, 16, t.ssq, tap_base ? tap_base + (size_t)(2 * l) * D : nullptr};
         if (tc_gemm(w.wo[l], t.aQ, g, st)) return -1;
-        tc_prepare(t.aD, nullptr, D, B, t.part_wo, s_wo, psD, t.X, t.X, L.ffn_norm, t.ssq, st,
+        if (tp) tc_prepare(t.aD, nullptr, D, B, t.part_wo, s_wo, psD, t.X, t.X, L.ffn_norm, t.ssq, st,
                    tp_wait_for(0, TP_WO, NL, l + 1, t.status), tap_base ? tap_base + (size_t)(2 * l) * D : nullptr);
         g = TcGemm();
         g.M = B; g.status = t.status; g.eps = VB200_NORM_EPS;
@@ -1068,6 +1071,9 @@ static int enqueue_decoder(Batch &t) {
         if (tp) {
             g.tile0 = o0; g.n_tiles = on; g.push = tp_push(0, TP_W2, NL, l + 1);
             g.wait = tp_wait_for(0, TP_W13, NL, l + 1, t.status);     /* the SwiGLU terms come from every rank */
+        } else {
+            g.join = {t.X, t.X, l + 1 < NL ? m.dec[l + 1].attn_norm : nullptr, t.bD, 16, t.ssq,
+                      tap_base && l + 1 < NL ? tap_base + (size_t)(2 * l + 1) * D : nullptr};
         }
         if (tc_gemm(w.w2[l], t.aH, g, st)) return -1;
     }
@@ -1078,7 +1084,7 @@ static int enqueue_decoder(Batch &t) {
                    tp_wait_for(0, TP_W2, VB200_DEC_LAYERS, VB200_DEC_LAYERS, t.status));
     else
         launch_pdl(bt_final_kernel<false>, dim3(B), dim3(1024), 0, st, t.hidden, t.bD, 16, (const float *)t.X,
-                   (const float *)t.part_w2, s_w2, psD, (const float *)m.dec_norm, VB200_NORM_EPS, last_tap, TcNoWait());
+                   (const float *)nullptr, 0, (size_t)0, (const float *)m.dec_norm, VB200_NORM_EPS, last_tap, TcNoWait());
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -1252,7 +1258,7 @@ int batch_hidden(float *out) {
     return cudaMemcpy(out, t.hidden, sizeof(float) * t.B * D, cudaMemcpyDeviceToHost) == cudaSuccess ? 0 : -1;
 }
 
-int batch_launches_per_frame() { return 1 + VB200_DEC_LAYERS * 7 + 5 + (VB200_FLOW_STEPS - 1) * (2 + VB200_AC_LAYERS * 7) + 1; }
+int batch_launches_per_frame() { return 2 + VB200_DEC_LAYERS * 5 + 5 + (VB200_FLOW_STEPS - 1) * (3 + VB200_AC_LAYERS * 5) + 1; }
 
 /* The decoder's 104 layer GEMMs (QKV, O, gate/up, down x 26 layers: every decoder weight byte
  * once) launched back to back on the stream, `iters` times, between two events: the GEMM
@@ -1265,23 +1271,21 @@ int gemm_sweep(int which, int iters, float *ms_out, double *bytes_per_sweep, int
     Batch &t = which == 0 ? g_one : g_bt;
     if (!t.open || iters < 1 || bt_weights()) return -1;
     const BtWeights &w = g_w;
-    const int chunksD = tc_prepare_chunks(D);
-    TcGemm g;
-    g.M = t.B; g.status = t.status; g.eps = VB200_NORM_EPS;
+    const int chunksD = D / kTcTileN;
     cudaEventRecord(t.e0, m.st);
     for (int it = 0; it < iters; it++) {
         for (int l = 0; l < VB200_DEC_LAYERS; l++) {
+            TcGemm g, j;
+            g.M = j.M = t.B; g.status = j.status = t.status; g.eps = VB200_NORM_EPS;
+            j.join = {t.X, t.part, m.dec[l].ffn_norm, t.bD, 16, t.ssq, nullptr};      /* the rows stay as they are */
             g.epi = TC_EPI_PARTIAL; g.out = t.part; g.out_terms = nullptr;
             g.splits = w.s_qkv; g.ld_out = QKV; g.ssq = t.ssq; g.ssq_chunks = chunksD;
             if (tc_gemm(w.wqkv[l], t.aD, g, m.st)) return -1;
-            g.splits = w.s_wo; g.ld_out = D; g.ssq = nullptr; g.ssq_chunks = 0;
-            if (tc_gemm(w.wo[l], t.aQ, g, m.st)) return -1;
+            if (tc_gemm(w.wo[l], t.aQ, j, m.st)) return -1;
             g.epi = TC_EPI_SWIGLU_TERMS; g.out = nullptr; g.out_terms = t.bH; g.out_rows_pad = 16;
             g.splits = 1; g.ld_out = HID; g.ssq = t.ssq; g.ssq_chunks = chunksD;
             if (tc_gemm(w.w13[l], t.aD, g, m.st)) return -1;
-            g.epi = TC_EPI_PARTIAL; g.out = t.part; g.out_terms = nullptr;
-            g.splits = w.s_w2; g.ld_out = D; g.ssq = nullptr; g.ssq_chunks = 0;
-            if (tc_gemm(w.w2[l], t.aH, g, m.st)) return -1;
+            if (tc_gemm(w.w2[l], t.aH, j, m.st)) return -1;
         }
     }
     cudaEventRecord(t.e1, m.st);

@@ -202,14 +202,37 @@ struct TcTpArgs {
     TcWait wait;             /* the activation terms may be exchanged data */
 };
 struct TcNoTpArgs {};
-template <bool TP> struct TcTpSel { using type = TcNoTpArgs; };
-template <> struct TcTpSel<true> { using type = TcTpArgs; };
+/* TC_JOIN: see TcJoin. The kernel that added up the partial results of these GEMMs before ("prepare") was a launch of its
+ * own, 2 of 7 in a layer: a frame had 350 launches, 264 now; 2.86 -> 2.81 ms. */
+enum TcMode { TC_PLAIN = 0, TC_TP = 1, TC_JOIN = 2 };
+template <int MODE> struct TcTpSel { using type = TcNoTpArgs; };
+template <> struct TcTpSel<TC_TP> { using type = TcTpArgs; };
+template <> struct TcTpSel<TC_JOIN> { using type = TcJoin; };
 
-template <int NB, int ST, bool TP>
+VB_DEVINL uint32_t tc_cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+VB_DEVINL void tc_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+/* Four floats at the same place of CTA `rank`'s shared memory. */
+VB_DEVINL float4 tc_peer4(const float *p, uint32_t rank) {
+    uint32_t at;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(vb_smem_u32(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+    return v;
+}
+
+template <int NB, int ST, int MODE>
 __global__ void __launch_bounds__(kTcThreads, 1)
 vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-                  const TcKernelArgs ka, const typename TcTpSel<TP>::type tp) {
+                  const TcKernelArgs ka, const typename TcTpSel<MODE>::type tp) {
     using Cfg = TcCfg<NB, ST>;
+    constexpr bool TP = MODE == TC_TP;
     /* the tensor maps are fetched while the first reads of the parameter block are on their way */
     if (threadIdx.x == 128) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&mapA) : "memory");
@@ -269,6 +292,7 @@ vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
     tc_fence_after();
     const uint32_t tmem = *(volatile uint32_t *)tmem_slot;
 
+    float4 join_x = make_float4(0.f, 0.f, 0.f, 0.f), join_gain = join_x;   /* TC_JOIN: requested under the main loop */
     if (warp == 4 && lane == 0) {
         /* ---- TMA producer ----
          * The weights of the first ring-full are already on their way (above). Now the kernel
@@ -346,12 +370,17 @@ vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
          * 1/sqrt(mean(x^2)+eps) is applied to the accumulators (voxtral_tts_kernels.c:333-349). */
         pdl_wait();
         if (ka.ssq) {
-            for (int m = threadIdx.x; m < M; m += 128) {
-                float t = 0.0f;
-                for (int c = 0; c < ka.ssq_chunks; c++) t += __ldcg(ka.ssq + m * ka.ssq_chunks + c);
-                rscale[m] = 1.0f / sqrtf(t / (float)K + ka.eps);
+#pragma unroll 4
+            for (int m = warp; m < M; m += 4) {
+                const float t = vb_warp_sum(lane < ka.ssq_chunks ? __ldcg(ka.ssq + m * ka.ssq_chunks + lane) : 0.0f);
+                if (lane == 0) rscale[m] = 1.0f / sqrtf(t / (float)K + ka.eps);
             }
             vb_named_bar(1, 128);
+        }
+        if constexpr (MODE == TC_JOIN) {
+            const int m = (int)tc_cluster_rank() + kTcJoinSplits * warp;
+            if (m < M) join_x = vb_ldcg4(tp.x + (size_t)m * N + tile * kTcTileN + lane * 4);
+            if (tp.gain) join_gain = __ldg(reinterpret_cast<const float4 *>(tp.gain + tile * kTcTileN + lane * 4));
         }
         bool ok = vb_mbar_wait(accum, 0u, abort_flag);
         if (!ok) {
@@ -386,7 +415,7 @@ vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
                     if (m < M) stg[m * kTcTileN + warp * 32 + lane] = v;
                 }
             }
-            {
+            if constexpr (MODE != TC_JOIN) {
                 vb_named_bar(1, 128);
                 const int n = tile * kTcTileN + lane * 4;             /* this lane's four output columns */
                 for (int m = warp; m < M; m += 4) {
@@ -479,6 +508,40 @@ vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
 
     tc_fence_before();
     __syncthreads();
+    if constexpr (MODE == TC_JOIN) {
+        tc_cluster_sync();                    /* all partial results are staged */
+        const float *stg = (const float *)stages;
+        const int rank = (int)tc_cluster_rank(), n = tile * kTcTileN + lane * 4;
+        if (warp < 4) {
+            for (int m = rank + kTcJoinSplits * warp; m < M; m += kTcJoinSplits * 4) {
+                if (m >= kTcJoinSplits * 4) join_x = vb_ldcg4(tp.x + (size_t)m * N + n);
+                float4 q[kTcJoinSplits];
+#pragma unroll
+                for (int u = 0; u < kTcJoinSplits; u++) q[u] = tc_peer4(stg + m * kTcTileN + lane * 4, (uint32_t)u);
+                float4 v = q[0];
+#pragma unroll
+                for (int u = 1; u < kTcJoinSplits; u++) { v.x += q[u].x; v.y += q[u].y; v.z += q[u].z; v.w += q[u].w; }
+                v.x = join_x.x + v.x; v.y = join_x.y + v.y; v.z = join_x.z + v.z; v.w = join_x.w + v.w;
+                *reinterpret_cast<float4 *>(tp.x_out + (size_t)m * N + n) = v;
+                if (tp.tap) *reinterpret_cast<float4 *>(tp.tap + (size_t)m * N + n) = v;
+                if (tp.gain) {
+                    const float e[4] = {v.x * join_gain.x, v.y * join_gain.y, v.z * join_gain.z, v.w * join_gain.w};
+                    uint16_t t[3][4];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) vb_split3(e[i], t[0][i], t[1][i], t[2][i]);
+                    uint16_t *o = tp.terms + (size_t)m * N + n;
+#pragma unroll
+                    for (int j = 0; j < 3; j++)
+                        *reinterpret_cast<uint2 *>(o + (size_t)j * tp.rows_pad * N) =
+                            make_uint2(t[j][0] | ((uint32_t)t[j][1] << 16), t[j][2] | ((uint32_t)t[j][3] << 16));
+                    const float ss = vb_warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w);
+                    if (lane == 0) tp.ssq[m * (N / kTcTileN) + tile] = ss;
+                }
+            }
+        }
+        __syncwarp();
+        tc_cluster_sync();                    /* nobody reads this CTA's shared memory any more */
+    }
     /* abort path: let copies already in flight land before the shared memory goes away */
     if (warp == 4 && lane == 0 && *(volatile int *)abort_flag) {
         /* the last load issued into stage s was iteration `it` with it % kStages == s: wait for
@@ -498,13 +561,31 @@ vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
     }
 }
 
-template <int NB, int ST, bool TP>
-static int launch_tc_tp(const TcWeight &w, const TcActs &a, const TcKernelArgs &ka, const TcTpArgs &tpa,
+/* launch_pdl with clusters of so many CTAs (0: none). */
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_pdl_cluster(void (*kernel)(KArgs...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+    if (cluster == 0) return launch_pdl(kernel, grid, block, smem, st, args...);
+    static const bool no_pdl = getenv("VB200_NO_PDL") != nullptr;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = no_pdl ? 1 : 2;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+template <int NB, int ST, int MODE>
+static int launch_tc_tp(const TcWeight &w, const TcActs &a, const TcKernelArgs &ka, const typename TcTpSel<MODE>::type &arg,
                         cudaStream_t st) {
     using Cfg = TcCfg<NB, ST>;
     static bool attr = false;
     if (!attr) {
-        if (cudaFuncSetAttribute(vb_tc_gemm_kernel<NB, ST, TP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (cudaFuncSetAttribute(vb_tc_gemm_kernel<NB, ST, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  Cfg::kSmemBytes) != cudaSuccess) {
             cudaGetLastError();
             return -1;
@@ -512,22 +593,37 @@ static int launch_tc_tp(const TcWeight &w, const TcActs &a, const TcKernelArgs &
         attr = true;
     }
     const int tiles = ka.n_tiles_launch;
-    typename TcTpSel<TP>::type arg;
-    if constexpr (TP) arg = tpa;
-    return launch_pdl(vb_tc_gemm_kernel<NB, ST, TP>, dim3(tiles * ka.splits), dim3(kTcThreads), (size_t)Cfg::kSmemBytes, st,
-                      w.map, a.map, ka, arg) == cudaSuccess
+    return launch_pdl_cluster(vb_tc_gemm_kernel<NB, ST, MODE>, MODE == TC_JOIN ? kTcJoinSplits : 0, dim3(tiles * ka.splits), dim3(kTcThreads),
+                              (size_t)Cfg::kSmemBytes, st, w.map, a.map, ka, arg) == cudaSuccess
                ? 0
                : -1;
 }
 
 template <int NB, int ST>
 static int launch_tc(const TcWeight &w, const TcActs &a, const TcKernelArgs &ka, const TcTpArgs &tpa, cudaStream_t st) {
-    if (tpa.push.n_dst > 0 || tpa.wait.n > 0) return launch_tc_tp<NB, ST, true>(w, a, ka, tpa, st);
-    return launch_tc_tp<NB, ST, false>(w, a, ka, tpa, st);
+    if (tpa.push.n_dst > 0 || tpa.wait.n > 0) return launch_tc_tp<NB, ST, TC_TP>(w, a, ka, tpa, st);
+    return launch_tc_tp<NB, ST, TC_PLAIN>(w, a, ka, TcNoTpArgs(), st);
+}
+
+static int tc_gemm_join(const TcWeight &w, const TcActs &a, const TcGemm &g, cudaStream_t st) {
+    const TcJoin &j = g.join;
+    if (w.N % kTcTileN || w.K / kTcBlockK < kTcJoinSplits || !j.x_out || (j.gain && (!j.terms || !j.ssq || j.rows_pad < g.M))) return -1;
+    if (g.n_tiles || g.push.n_dst || g.wait.n || g.ssq || g.bias) return -1;
+    TcKernelArgs ka = {};
+    ka.a_tiled = w.tiled ? 1 : 0;
+    ka.N = w.N; ka.K = w.K; ka.M = g.M; ka.rows_pad = a.rows_pad; ka.splits = kTcJoinSplits; ka.status = g.status;
+    ka.n_tiles_launch = w.N / kTcTileN;
+    switch (a.rows_pad) {
+    case 16: return launch_tc_tp<16, 6, TC_JOIN>(w, a, ka, j, st);
+    case 48: return launch_tc_tp<48, 6, TC_JOIN>(w, a, ka, j, st);
+    case 64: return launch_tc_tp<64, 5, TC_JOIN>(w, a, ka, j, st);
+    default: return -1;
+    }
 }
 
 int tc_gemm(const TcWeight &w, const TcActs &a, const TcGemm &g, cudaStream_t st) {
     if (!w.ok || !a.ok || w.K != a.K || g.M < 1 || g.M > a.rows_pad) return -1;
+    if (g.join.x) return tc_gemm_join(w, a, g, st);
     if (g.splits < 1 || g.splits > kTcMaxSplits || g.splits > w.K / kTcBlockK) return -1;
     if (g.epi != TC_EPI_PARTIAL && g.splits != 1) return -1;
     if ((g.epi == TC_EPI_SWIGLU || g.epi == TC_EPI_SWIGLU_TERMS) && (w.N & 1)) return -1;

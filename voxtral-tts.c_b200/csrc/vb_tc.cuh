@@ -88,6 +88,22 @@ struct TcNoWait {};
 template <bool TP> struct TcWaitSel { using type = TcNoWait; };
 template <> struct TcWaitSel<true> { using type = TcWait; };
 
+/* A GEMM that ends a sublayer (out-projection, down projection): K is split over the CTAs of a cluster, which add their
+ * partial results up through distributed shared memory and finish the sublayer - the new residual rows, and the next
+ * norm's operand: terms of row * gain, and a sum of squares per row and 128 columns (the RMSNorm scalar is applied by
+ * the GEMM that reads them). */
+struct TcJoin {
+    const float *x = nullptr;         /* residual rows [M][N]; null: not such a GEMM */
+    float *x_out = nullptr;           /* the new ones (may be x) */
+    const float *gain = nullptr;      /* null: no next norm */
+    uint16_t *terms = nullptr;        /* [3][rows_pad][N] */
+    int rows_pad = 0;
+    float *ssq = nullptr;             /* [M][N / 128] */
+    float *tap = nullptr;             /* optional copy of the new rows */
+};
+/* 24 tiles of 3072 columns: clusters of six find room for 22 at once; one utterance, 212 frames: 596 ms with four or five */
+constexpr int kTcJoinSplits = 4;
+
 /* One GEMM launch. */
 struct TcGemm {
     int M = 0, splits = 1, epi = TC_EPI_STORE;
@@ -105,6 +121,7 @@ struct TcGemm {
     int tile0 = 0, n_tiles = 0;       /* output tiles [tile0, tile0 + n_tiles) of the weight matrix; 0 = all */
     TcPush push;
     TcWait wait;                      /* the activation terms (and ssq) are exchanged data */
+    TcJoin join;                      /* up to 64 rows, N a multiple of 128; epi, splits and out are not used */
 };
 
 int tc_init();                                     /* resolves cuTensorMapEncodeTiled; 0 when usable */
