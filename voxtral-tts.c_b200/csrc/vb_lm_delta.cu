@@ -454,7 +454,34 @@ __global__ void __launch_bounds__(kGtThreads) lm_delta_gate_kernel(const LmDelta
     pdl_wait();
     const int m = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nv = a.heads * a.vdim, ch = 2 * a.kv_heads * a.dim + nv;
-    for (int h = warp; h < a.heads; h += kGtThreads / 32) {
+    /* a lane has four columns of every 128 (scalar loads and 2-byte stores: 45 us per 2048 rows of 24 x 128, 37 us so) */
+    const bool by4 = ((a.vdim | ch) & 3) == 0 && a.vdim <= 256;
+    for (int h = warp; h < a.heads && by4; h += kGtThreads / 32) {
+        const float *o = a.o + (size_t)m * nv + h * a.vdim;
+        float4 v[2], z[2];
+        float s = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int d = i * 128 + lane * 4;
+            v[i] = z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (d < a.vdim) {
+                v[i] = vb_ldcg4(o + d);
+                z[i] = lm_sum4(a.in, m, ch + h * a.vdim + d);
+            }
+            s += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+        }
+        const float r = 1.0f / sqrtf(vb_warp_sum(s) / (float)a.vdim + a.eps);
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int d = i * 128 + lane * 4;
+            if (d >= a.vdim) continue;
+            const float4 g = __ldg(reinterpret_cast<const float4 *>(a.norm + d));
+            const float e[4] = {v[i].x * r * g.x * silu(z[i].x), v[i].y * r * g.y * silu(z[i].y), v[i].z * r * g.z * silu(z[i].z),
+                                v[i].w * r * g.w * silu(z[i].w)};
+            lm_put4(a.out, m, h * a.vdim + d, e);
+        }
+    }
+    for (int h = warp; h < a.heads && !by4; h += kGtThreads / 32) {
         const float *o = a.o + (size_t)m * nv + h * a.vdim;
         float s = 0.0f;
         for (int d = lane; d < a.vdim; d += 32) s += o[d] * o[d];

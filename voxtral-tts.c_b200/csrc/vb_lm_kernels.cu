@@ -19,27 +19,64 @@ VB_DEVINL float cta_sum(float v, float *red) {
     return vb_warp_sum(lane < warps ? red[lane] : 0.0f);
 }
 
+/* Takes the mean off the CTA's N values a thread and returns the sum of their squares after that, with one barrier: every
+ * thread's own mean and squared deviations, put together pairwise (equal counts: the means' mean, and n / 2 times the
+ * square of their difference on top). Every thread has to have N values. */
+template <int N>
+VB_DEVINL float cta_centre(float (&x)[N], float2 *red) {
+    const int lane = threadIdx.x & 31, warps = (int)blockDim.x >> 5;
+    float mean = 0.0f, ss = 0.0f, n = (float)N;
+#pragma unroll
+    for (int i = 0; i < N; i++) mean += x[i];
+    mean *= 1.0f / N;
+#pragma unroll
+    for (int i = 0; i < N; i++) ss += (x[i] - mean) * (x[i] - mean);
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1, n += n) {
+        const float m2 = __shfl_xor_sync(0xffffffffu, mean, off), d = m2 - mean;
+        ss = ss + __shfl_xor_sync(0xffffffffu, ss, off) + d * d * (0.5f * n);
+        mean = 0.5f * (mean + m2);
+    }
+    if (lane == 0) red[threadIdx.x >> 5] = make_float2(mean, ss);
+    __syncthreads();
+    const float2 w = lane < warps ? red[lane] : make_float2(0.0f, 0.0f);
+    mean = vb_warp_sum(w.x) / (float)warps;
+    const float d = lane < warps ? w.x - mean : 0.0f;
+    ss = vb_warp_sum(w.y + n * d * d);
+#pragma unroll
+    for (int i = 0; i < N; i++) x[i] -= mean;
+    return ss;
+}
+
 /* One row of the residual stream per CTA, held in registers: the sublayer's output (split-K
  * partials) is normalised or taken as it is, added to the stream, and the new row is normalised for
- * the next sublayer. Variances are means of squared deviations. A thread owns NV groups of VEC columns. */
-template <int VEC, int NV>
-__global__ void __launch_bounds__(1024) lm_residual_kernel(const LmResidual a) {
+ * the next sublayer. Variances are means of squared deviations. A thread owns NV groups of VEC columns. MANY: 256 threads,
+ * five rows on an SM, gains read where they are used. */
+template <int VEC, int NV, bool MANY>
+__global__ void __launch_bounds__(MANY ? 256 : 1024, MANY ? 5 : 1) lm_residual_kernel(const LmResidual a) {
     __shared__ float red[4][32];
+    __shared__ float2 red2[2][32];
     constexpr int N = VEC * NV;
     pdl_launch_dependents();
     const int m = blockIdx.x, tid = threadIdx.x, W = a.width;
+    const bool centre = !a.rms && W == (int)blockDim.x * N;      /* no thread without columns: one barrier instead of two */
     const float inv_w = 1.0f / (float)W;
     auto col = [&](int i) { return (tid + i * (int)blockDim.x) * VEC; };
     /* the gains depend on nothing that runs before */
     float gp[N], gn[N];
+    auto gains = [&](bool post) {
+        float *g = post ? gp : gn;
+        const float *src = post ? a.post_gain : a.next_gain;
+        const bool on = post ? a.join == LM_JOIN_NORMED : a.next == LM_NEXT_NORM;
 #pragma unroll
-    for (int i = 0; i < NV; i++)
+        for (int i = 0; i < NV; i++)
 #pragma unroll
-        for (int j = 0; j < VEC; j++) {
-            const int c = col(i) + j;
-            gp[i * VEC + j] = a.join == LM_JOIN_NORMED && c < W ? __ldg(a.post_gain + c) : 0.0f;
-            gn[i * VEC + j] = a.next == LM_NEXT_NORM && c < W ? __ldg(a.next_gain + c) : 0.0f;
-        }
+            for (int j = 0; j < VEC; j++) {
+                const int c = col(i) + j;
+                g[i * VEC + j] = on && c < W ? __ldg(src + c) : 0.0f;
+            }
+    };
+    if (!MANY) { gains(true); gains(false); }
     pdl_wait();
     const int src = a.row_of ? a.row_of[m] : m;
     float x[N];
@@ -88,16 +125,22 @@ __global__ void __launch_bounds__(1024) lm_residual_kernel(const LmResidual a) {
             for (int i = 0; i < N; i++) x[i] = r[i] + x[i];
         } else if (add) {
             float s = 0.0f;
+            if (centre) {
+                s = cta_centre<N>(x, red2[0]);
+            } else {
 #pragma unroll
-            for (int i = 0; i < N; i++) s += x[i];
-            const float mean = a.rms ? 0.0f : cta_sum(s, red[0]) * inv_w;
-            s = 0.0f;
+                for (int i = 0; i < N; i++) s += x[i];
+                const float mean = a.rms ? 0.0f : cta_sum(s, red[0]) * inv_w;
+                s = 0.0f;
 #pragma unroll
-            for (int i = 0; i < N; i++) {
-                x[i] = col(i / VEC) < W ? x[i] - mean : 0.0f;
-                s += x[i] * x[i];
+                for (int i = 0; i < N; i++) {
+                    x[i] = col(i / VEC) < W ? x[i] - mean : 0.0f;
+                    s += x[i] * x[i];
+                }
+                s = cta_sum(s, red[1]);
             }
-            const float rstd = 1.0f / sqrtf(cta_sum(s, red[1]) * inv_w + a.eps);
+            const float rstd = 1.0f / sqrtf(s * inv_w + a.eps);
+            if (MANY) gains(true);
 #pragma unroll
             for (int i = 0; i < N; i++) x[i] = r[i] + x[i] * rstd * gp[i];      /* zero beyond the row */
         }
@@ -125,16 +168,22 @@ __global__ void __launch_bounds__(1024) lm_residual_kernel(const LmResidual a) {
     };
     if (a.next == LM_NEXT_NORM) {
         float s = 0.0f;
+        if (centre) {
+            s = cta_centre<N>(x, red2[1]);
+        } else {
 #pragma unroll
-        for (int i = 0; i < N; i++) s += x[i];
-        const float mean = a.rms ? 0.0f : cta_sum(s, red[2]) * inv_w;
-        s = 0.0f;
+            for (int i = 0; i < N; i++) s += x[i];
+            const float mean = a.rms ? 0.0f : cta_sum(s, red[2]) * inv_w;
+            s = 0.0f;
 #pragma unroll
-        for (int i = 0; i < N; i++) {
-            x[i] = col(i / VEC) < W ? x[i] - mean : 0.0f;
-            s += x[i] * x[i];
+            for (int i = 0; i < N; i++) {
+                x[i] = col(i / VEC) < W ? x[i] - mean : 0.0f;
+                s += x[i] * x[i];
+            }
+            s = cta_sum(s, red[3]);
         }
-        const float rstd = 1.0f / sqrtf(cta_sum(s, red[3]) * inv_w + a.eps);
+        const float rstd = 1.0f / sqrtf(s * inv_w + a.eps);
+        if (MANY) gains(false);
 #pragma unroll
         for (int i = 0; i < N; i++) x[i] = x[i] * rstd * gn[i];
 #pragma unroll
@@ -219,16 +268,25 @@ int lm_residual(const LmResidual &a, int M, cudaStream_t st) {
     if (M <= 0) return 0;
     const bool v4 = (a.width & 3) == 0;
     const int groups = v4 ? a.width / 4 : a.width;
-    const int threads = groups >= 1024 ? 1024 : (groups + 31) / 32 * 32, nv = (groups + threads - 1) / threads;
+    /* Few rows: all of a row's columns at once. More rows than fit the chip at a CTA per row and half an SM: 256 threads,
+     * so that more rows are on their way per SM and a row's four sums cross eight warps instead of 24 (2048 rows of 3072
+     * columns: 52 us before, 27 us now). */
+    const bool many = M > 296 && v4 && groups > 256 && groups <= 1024;
+    const int threads = many ? 256 : groups >= 1024 ? 1024 : (groups + 31) / 32 * 32, nv = (groups + threads - 1) / threads;
     const dim3 g(M), b(threads);
+    if (many) {
+        if (nv <= 2) return ok(launch_pdl(lm_residual_kernel<4, 2, true>, g, b, 0, st, a));
+        if (nv <= 3) return ok(launch_pdl(lm_residual_kernel<4, 3, true>, g, b, 0, st, a));
+        return ok(launch_pdl(lm_residual_kernel<4, 4, true>, g, b, 0, st, a));
+    }
     if (v4) {
-        if (nv <= 1) return ok(launch_pdl(lm_residual_kernel<4, 1>, g, b, 0, st, a));
-        if (nv <= 2) return ok(launch_pdl(lm_residual_kernel<4, 2>, g, b, 0, st, a));
-        if (nv <= 4) return ok(launch_pdl(lm_residual_kernel<4, 4>, g, b, 0, st, a));
+        if (nv <= 1) return ok(launch_pdl(lm_residual_kernel<4, 1, false>, g, b, 0, st, a));
+        if (nv <= 2) return ok(launch_pdl(lm_residual_kernel<4, 2, false>, g, b, 0, st, a));
+        if (nv <= 4) return ok(launch_pdl(lm_residual_kernel<4, 4, false>, g, b, 0, st, a));
     } else {
-        if (nv <= 1) return ok(launch_pdl(lm_residual_kernel<1, 1>, g, b, 0, st, a));
-        if (nv <= 4) return ok(launch_pdl(lm_residual_kernel<1, 4>, g, b, 0, st, a));
-        if (nv <= 16) return ok(launch_pdl(lm_residual_kernel<1, 16>, g, b, 0, st, a));
+        if (nv <= 1) return ok(launch_pdl(lm_residual_kernel<1, 1, false>, g, b, 0, st, a));
+        if (nv <= 4) return ok(launch_pdl(lm_residual_kernel<1, 4, false>, g, b, 0, st, a));
+        if (nv <= 16) return ok(launch_pdl(lm_residual_kernel<1, 16, false>, g, b, 0, st, a));
     }
     return -1;
 }
