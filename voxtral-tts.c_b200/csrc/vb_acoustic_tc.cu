@@ -26,6 +26,7 @@ struct AcTc {
     bool ready = false;
     TcWeight wqkv[VB200_AC_LAYERS], wo[VB200_AC_LAYERS], w13[VB200_AC_LAYERS], w2[VB200_AC_LAYERS];
     uint16_t *tiled[VB200_AC_LAYERS][4] = {};   /* tile-contiguous weight copies */
+    TcWeight wtime;             /* time_proj */
     int s_qkv = 1;
     AcBuffers one;              /* the single-utterance buffers */
 };
@@ -87,6 +88,29 @@ __global__ void ac_tokens_kernel(float *X6, float *lat, const float *vel, const 
     X6[4 * D + n] = tt;
     X6[2 * D + n] = ltok[n];
     X6[5 * D + n] = 0.0f;
+}
+
+/* The three input rows of a single velocity call (voxtral_tts_acoustic.c:198-212): input_proj(x), and the split-K partials
+ * [n_part][2][3072] of time_proj on row 1 and of llm_proj on row 0 of (hidden, time embedding). */
+__global__ void ac_rows_kernel(float *X, const float *x, const uint16_t *Wip, const float *time_part, const float *llm_part, int n_part) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= D) return;
+    const uint16_t *wr = Wip + (size_t)n * A;
+    float acc = 0.0f;
+    for (int k = 0; k < A; k++) acc = __fadd_rn(acc, __fmul_rn(__uint_as_float((uint32_t)wr[k] << 16), __ldcg(x + k)));
+    float a[kTcMaxSplits], b[kTcMaxSplits], ta = 0.0f, tb = 0.0f;
+#pragma unroll
+    for (int p = 0; p < kTcMaxSplits; p++) {
+        a[p] = p < n_part ? __ldcg(time_part + ((size_t)p * 2 + 1) * D + n) : 0.0f;
+        b[p] = p < n_part ? __ldcg(llm_part + (size_t)p * 2 * D + n) : 0.0f;
+    }
+#pragma unroll
+    for (int p = 0; p < kTcMaxSplits; p++) { ta += a[p]; tb += b[p]; }
+    X[n] = acc;
+    X[D + n] = ta;
+    X[2 * D + n] = tb;
 }
 
 /* Unmasked attention inside each 3-token sequence (tts_bidirectional_attention,
@@ -319,12 +343,49 @@ int acoustic_tc_setup() {
     o.codes = m.d_out->codes;
     o.dyn = &m.d_in->dyn;
     o.status = &m.d_out->status;
+    if (tc_weight(&t.wtime, m.ac_time_proj, D, D)) return -1;
     t.s_qkv = tc_pick_splits(QKV, D, m.sm_count);
     t.ready = true;
     return 0;
 }
 
 bool acoustic_tc_ready() { return g_ac.ready; }
+
+/* The layers on the rows in X6, whose terms are not made yet. */
+static int enqueue_layers(const AcBuffers &b, int ROWS) {
+    Model &m = model();
+    AcTc &t = g_ac;
+    cudaStream_t st = m.st;
+    const float scale = 1.0f / sqrtf((float)VB200_HEAD_DIM);
+    for (int l = 0; l < VB200_AC_LAYERS; l++) {
+        const LayerDev &L = m.ac[l];
+        /* attention half: QKV -> attention -> O, which leaves the new rows and the next norm's operand */
+        if (l == 0) tc_prepare(b.aD, b.X6, D, ROWS, nullptr, 0, 0, nullptr, nullptr, L.attn_norm, b.ssq, st);
+        TcGemm g;
+        g.M = ROWS; g.status = b.status;
+        g.epi = TC_EPI_PARTIAL; g.out = b.part;
+        g.splits = t.s_qkv; g.ld_out = QKV; g.ssq = b.ssq; g.ssq_chunks = l == 0 ? tc_prepare_chunks(D) : D / kTcTileN;
+        g.eps = VB200_NORM_EPS;
+        if (tc_gemm(t.wqkv[l], b.aD, g, st)) return -1;
+        launch_pdl(ac_attention_kernel, dim3((ROWS * VB200_HEADS * 32 + 255) / 256), dim3(256), 0, st, b.bQ,
+                   (const float *)b.part, t.s_qkv, scale, ROWS, b.rows_pad);
+        g = TcGemm();
+        g.M = ROWS; g.status = b.status;
+        g.join = {b.X6, b.X6, L.ffn_norm, b.bD, b.rows_pad, b.ssq, nullptr};
+        if (tc_gemm(t.wo[l], b.aQ, g, st)) return -1;
+        /* FFN half: gate/up with SwiGLU (terms out) -> down */
+        g = TcGemm();
+        g.M = ROWS; g.status = b.status;
+        g.epi = TC_EPI_SWIGLU_TERMS; g.out_terms = b.bH; g.out_rows_pad = b.rows_pad;
+        g.ld_out = HID; g.ssq = b.ssq; g.ssq_chunks = D / kTcTileN; g.eps = VB200_NORM_EPS;
+        if (tc_gemm(t.w13[l], b.aD, g, st)) return -1;
+        g = TcGemm();
+        g.M = ROWS; g.status = b.status;
+        g.join = {b.X6, b.X6, l + 1 < VB200_AC_LAYERS ? m.ac[l + 1].attn_norm : nullptr, b.bD, b.rows_pad, b.ssq, nullptr};
+        if (tc_gemm(t.w2[l], b.aH, g, st)) return -1;
+    }
+    return 0;
+}
 
 /* Enqueues the 7 Euler steps + FSQ on the library's stream. The semantic head, llm token
  * and argmax have already run; the llm token rows are in b.ltok. */
@@ -334,40 +395,13 @@ int acoustic_tc_enqueue_on(const AcBuffers &b, const float *noise_all, int *code
     AcTc &t = g_ac;
     if (!t.ready) return -1;
     cudaStream_t st = m.st;
-    const float scale = 1.0f / sqrtf((float)VB200_HEAD_DIM);
     const int steps = VB200_FLOW_STEPS - 1;
     const int ROWS = b.rows;
     for (int s = 0; s < steps; s++) {
         launch_pdl(ac_tokens_kernel, dim3((D + 127) / 128, b.B), dim3(128), 0, st, b.X6, b.lat, (const float *)b.vel,
                    (const uint16_t *)m.ac_input_proj, (const float *)m.ttok, (const float *)b.ltok, s,
                    VB200_CFG_ALPHA, s > 0 ? m.dt[s - 1] : 0.0f, noise_all, (const VbDyn *)b.dyn, b.sd);
-        for (int l = 0; l < VB200_AC_LAYERS; l++) {
-            const LayerDev &L = m.ac[l];
-            /* attention half: QKV -> attention -> O, which leaves the new rows and the next norm's operand */
-            if (l == 0) tc_prepare(b.aD, b.X6, D, ROWS, nullptr, 0, 0, nullptr, nullptr, L.attn_norm, b.ssq, st);
-            TcGemm g;
-            g.M = ROWS; g.status = b.status;
-            g.epi = TC_EPI_PARTIAL; g.out = b.part;
-            g.splits = t.s_qkv; g.ld_out = QKV; g.ssq = b.ssq; g.ssq_chunks = l == 0 ? tc_prepare_chunks(D) : D / kTcTileN;
-            g.eps = VB200_NORM_EPS;
-            if (tc_gemm(t.wqkv[l], b.aD, g, st)) return -1;
-            launch_pdl(ac_attention_kernel, dim3((ROWS * VB200_HEADS * 32 + 255) / 256), dim3(256), 0, st, b.bQ,
-                       (const float *)b.part, t.s_qkv, scale, ROWS, b.rows_pad);
-            g = TcGemm();
-            g.M = ROWS; g.status = b.status;
-            g.join = {b.X6, b.X6, L.ffn_norm, b.bD, b.rows_pad, b.ssq, nullptr};
-            if (tc_gemm(t.wo[l], b.aQ, g, st)) return -1;
-            /* FFN half: gate/up with SwiGLU (terms out) -> down */
-            g = TcGemm();
-            g.M = ROWS; g.status = b.status;
-            g.epi = TC_EPI_SWIGLU_TERMS; g.out_terms = b.bH; g.out_rows_pad = b.rows_pad;
-            g.ld_out = HID; g.ssq = b.ssq; g.ssq_chunks = D / kTcTileN; g.eps = VB200_NORM_EPS;
-            if (tc_gemm(t.w13[l], b.aD, g, st)) return -1;
-            g = TcGemm();
-            g.M = ROWS; g.status = b.status;
-            g.join = {b.X6, b.X6, l + 1 < VB200_AC_LAYERS ? m.ac[l + 1].attn_norm : nullptr, b.bD, b.rows_pad, b.ssq, nullptr};
-            if (tc_gemm(t.w2[l], b.aH, g, st)) return -1;
-        }
+        if (enqueue_layers(b, ROWS)) return -1;
         launch_pdl(ac_velocity_kernel, dim3(9, 2 * b.B), dim3(512), 0, st, b.vel, (const float *)b.X6, (const float *)m.ac_norm,
                    VB200_NORM_EPS, (const uint16_t *)m.ac_out, b.sd.vel);
     }
@@ -393,11 +427,13 @@ struct GraphSlot {
     cudaGraphExec_t exec = nullptr;
 };
 static GraphSlot g_slots[2];
+static GraphSlot g_velocity;
+static const uint16_t *g_velocity_llm = nullptr;      /* the llm_proj in its launches */
 
 void acoustic_tc_drop_graphs() {
-    for (GraphSlot &s : g_slots) {
-        if (s.exec) cudaGraphExecDestroy(s.exec);
-        s = GraphSlot();
+    for (GraphSlot *s : {&g_slots[0], &g_slots[1], &g_velocity}) {
+        if (s->exec) cudaGraphExecDestroy(s->exec);
+        *s = GraphSlot();
     }
 }
 
@@ -407,26 +443,19 @@ void acoustic_tc_free_all() {
     g_ac = AcTc();
 }
 
-int acoustic_tc_enqueue(const float *noise_all, int *codes_all, int frame_cap, bool advance, bool ignore_end) {
+/* What is captured or run directly for a slot: `enqueue`. */
+template <class F>
+static int run_slot(GraphSlot &s, const F &enqueue) {
     Model &m = model();
-    if (getenv("VB200_NO_GRAPH")) return enqueue_direct(noise_all, codes_all, frame_cap, advance, ignore_end);
-    GraphSlot &s = g_slots[advance ? 1 : 0];
-    const bool same = s.used && s.noise_all == noise_all && s.codes_all == codes_all && s.cap == frame_cap &&
-                      s.advance == advance && s.ignore_end == ignore_end;
-    if (!same) {
-        if (s.exec) cudaGraphExecDestroy(s.exec);
-        s = GraphSlot();
-        s.noise_all = noise_all; s.codes_all = codes_all; s.cap = frame_cap;
-        s.advance = advance; s.ignore_end = ignore_end; s.used = true;
-    }
+    if (getenv("VB200_NO_GRAPH")) return enqueue();
     if (s.exec) return cudaGraphLaunch(s.exec, m.st) == cudaSuccess ? 0 : -1;
-    if (s.calls++ == 0) return enqueue_direct(noise_all, codes_all, frame_cap, advance, ignore_end);
+    if (s.calls++ == 0) return enqueue();
     cudaGraph_t graph = nullptr;
     if (cudaStreamBeginCapture(m.st, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
         cudaGetLastError();
-        return enqueue_direct(noise_all, codes_all, frame_cap, advance, ignore_end);
+        return enqueue();
     }
-    const int rc = enqueue_direct(noise_all, codes_all, frame_cap, advance, ignore_end);
+    const int rc = enqueue();
     const cudaError_t ee = cudaStreamEndCapture(m.st, &graph);
     if (rc || ee != cudaSuccess || !graph) {
         if (graph) cudaGraphDestroy(graph);
@@ -441,6 +470,54 @@ int acoustic_tc_enqueue(const float *noise_all, int *codes_all, int frame_cap, b
         return -1;
     }
     return cudaGraphLaunch(s.exec, m.st) == cudaSuccess ? 0 : -1;
+}
+
+/* One velocity call on what lies in d_in (latent 0, hidden state, time embedding): 21 launches, against the streaming
+ * GEMV kernel's one of 0.25 ms; 0.17 ms. 1: not on this path. */
+static int enqueue_velocity(const TcWeight *llm) {
+    Model &m = model();
+    AcTc &t = g_ac;
+    const AcBuffers &b = t.one;
+    cudaStream_t st = m.st;
+    static_assert(offsetof(DevIn, temb) - offsetof(DevIn, hidden_in) == sizeof(float) * VB200_DIM, "two rows");
+    tc_prepare(b.aD, m.d_in->hidden_in, D, 2, nullptr, 0, 0, nullptr, nullptr, nullptr, nullptr, st);
+    const int s = tc_pick_splits(D, D, m.sm_count);
+    float *const time_part = b.part, *const llm_part = b.part + (size_t)kTcMaxSplits * 2 * D;
+    TcGemm g;
+    g.M = 2; g.status = b.status; g.epi = TC_EPI_PARTIAL; g.splits = s; g.ld_out = D;
+    g.out = time_part;
+    if (tc_gemm(t.wtime, b.aD, g, st)) return -1;
+    g.out = llm_part;
+    if (tc_gemm(*llm, b.aD, g, st)) return -1;
+    launch_pdl(ac_rows_kernel, dim3((D + 127) / 128), dim3(128), 0, st, b.X6, (const float *)m.d_in->lat[0], (const uint16_t *)m.ac_input_proj,
+               (const float *)time_part, (const float *)llm_part, s);
+    if (enqueue_layers(b, 3)) return -1;
+    launch_pdl(ac_velocity_kernel, dim3(9, 1), dim3(512), 0, st, b.vel, (const float *)b.X6, (const float *)m.ac_norm, VB200_NORM_EPS,
+               (const uint16_t *)m.ac_out, b.sd.vel);
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+int acoustic_tc_velocity() {
+    const TcWeight *llm = batch_llm_proj();
+    if (!g_ac.ready || !g_ac.wtime.ok || !llm) return 1;
+    if (g_velocity_llm != llm->W) {        /* the decoder's weights were uploaded anew */
+        if (g_velocity.exec) cudaGraphExecDestroy(g_velocity.exec);
+        g_velocity = GraphSlot();
+        g_velocity_llm = llm->W;
+    }
+    return run_slot(g_velocity, [&] { return enqueue_velocity(llm); });
+}
+
+int acoustic_tc_enqueue(const float *noise_all, int *codes_all, int frame_cap, bool advance, bool ignore_end) {
+    GraphSlot &s = g_slots[advance ? 1 : 0];
+    const bool same = s.used && s.noise_all == noise_all && s.codes_all == codes_all && s.cap == frame_cap &&
+                      s.advance == advance && s.ignore_end == ignore_end;
+    if (!same) {
+        if (s.exec) cudaGraphExecDestroy(s.exec);
+        s = GraphSlot();
+        s.noise_all = noise_all; s.codes_all = codes_all; s.cap = frame_cap;
+        s.advance = advance; s.ignore_end = ignore_end; s.used = true;
+    }
+    return run_slot(s, [&] { return enqueue_direct(noise_all, codes_all, frame_cap, advance, ignore_end); });
 }
 
 } // namespace vb

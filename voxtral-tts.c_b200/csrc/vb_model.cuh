@@ -130,6 +130,7 @@ void prefill_free_all();
 int acoustic_tc_setup();
 bool acoustic_tc_ready();
 void acoustic_tc_free_all();
+int acoustic_tc_velocity();
 int acoustic_tc_enqueue(const float *noise_all, int *codes_all, int frame_cap, bool advance, bool ignore_end);
 
 /* several utterances in lock step (vb_batch.cu) */
@@ -158,6 +159,7 @@ void tp_close();
 void batch_close();
 void batch_invalidate();
 struct TcWeight;
+const TcWeight *batch_llm_proj();
 int batch_tiled_decoder(const TcWeight **wqkv, const TcWeight **wo, const TcWeight **w13, const TcWeight **w2);
 void batch_options_changed();
 void single_path_changed();
