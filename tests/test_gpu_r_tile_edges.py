@@ -39,6 +39,11 @@ PROMPT_ATTENTION = {
     "72_128": attention(heads=6, kv_heads=2, dim=72, vdim=128, window=64, keep=64, scale=0.12, ff=0),
     "24_72": attention(heads=5, kv_heads=1, dim=24, vdim=72, window=63, keep=1, ff=0),
     "8_64": attention(heads=3, kv_heads=3, dim=8, vdim=64, window=130, keep=70, rot=8, ff=0),
+    # whole columns of 64, so that tiles come by TMA, on rings that wrap inside a tile
+    "64_128_wraps": attention(heads=4, kv_heads=2, dim=64, vdim=128, window=100, keep=5, ff=0),
+    "128_64_wraps": attention(heads=6, kv_heads=2, dim=128, vdim=64, window=90, keep=0, scale=0.09, ff=0),
+    "latent_128_64_wraps": latent(heads=2, dim=64, rot_dim=64, vdim=64, kv_rank=72, window=100, scale=0.09, ff=0),
+    "latent_192_128_wraps": latent(heads=2, dim=128, rot_dim=64, vdim=128, kv_rank=64, window=77, scale=0.08, ff=0),
     "latent_192_128": latent(heads=2, dim=128, rot_dim=64, vdim=128, kv_rank=64, window=0, scale=0.08, ff=0),
     "latent_136_72": latent(heads=3, dim=72, rot_dim=64, vdim=72, window=65, scale=0.09, ff=0),
     "latent_176_16": latent(heads=2, dim=168, rot_dim=8, vdim=16, window=64, scale=0.08, ff=0),

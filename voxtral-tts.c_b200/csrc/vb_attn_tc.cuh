@@ -14,8 +14,7 @@
  * the other is in its softmax. An accumulator is rescaled only when a row's maximum has risen by more than 2^8: the
  * reference a row is taken against cancels in the quotient.
  *
- * Warps: 0-3, 4-7 softmax, 8-11 bring keys and values into two rings (K slots are free after S, V slots after O), 12
- * issues the MMAs. All waits are bounded.
+ * Warps: 0-3, 4-7 softmax, 8-11 bring keys and 12-13 values into two rings, 14 issues the MMAs. All waits are bounded.
  *
  * What bounds it: a 64-key tile of 128-wide heads costs the tensor pipe 8 x 3 x 32 + 4 x 3 x 64 = 1536 clocks and the
  * softmax about as much; the warp-level MMAs used before (mma.sync, 16 rows per warp) ran at 44 useful TFLOP/s.
@@ -29,9 +28,11 @@
 namespace vb {
 
 constexpr int kAtRows = 128, kAtKeys = 64;
-constexpr int kAtSoft = 256, kAtLoaders = 128, kAtThreads = kAtSoft + kAtLoaders + 32;
+constexpr int kAtSoft = 256, kAtLoadK = 128, kAtLoadV = 64, kAtThreads = kAtSoft + kAtLoadK + kAtLoadV + 32;
+constexpr int kAtMmaWarp = (kAtThreads - 32) / 32;
 constexpr int kAtBlock = kAtKeys * 128;            /* 64 keys x 64 columns */
 constexpr int kAtStatus = 52;
+constexpr int kAtStage = 12;                       /* words of a row in a softmax warp's staging of the queries: 8 columns, and 16 bytes on */
 constexpr uint32_t kAtTmemCols = 512, kAtO = 128, kAtQ = 384;
 
 /* What every use has in common. */
@@ -40,6 +41,11 @@ struct AtArgs {
     int window, keep;
     float scale, softcap;
     int *status;
+    int tma;                     /* the tensor maps are there: whole tiles of keys are brought in by TMA */
+};
+/* Keys (and a part that all heads share), values: 64 columns x 64 rows of a plane. */
+struct AtMaps {
+    CUtensorMap k, k2, v;
 };
 
 template <int DK, int DV>
@@ -48,7 +54,7 @@ struct AtCfg {
     static constexpr int kSlots = DK <= 2 ? 3 : 2;
     static constexpr int kSlotK = 2 * DK * kAtBlock, kSlotV = 2 * DV * kAtBlock;
     static constexpr int kQl = kQlTmem ? 0 : DK * kAtRows * 128;
-    static constexpr int kSmem = kQl + kSlots * (kSlotK + kSlotV) + 1024 + 256;
+    static constexpr int kSmem = kQl + kSlots * (kSlotK + kSlotV) + 1024 + 256 + 8 * 32 * kAtStage * 4;
     static_assert(kSmem <= 232448, "over the 227 KB a CTA may use");
     static_assert(kAtQ + (kQlTmem ? 2 : 1) * DK * 32 <= kAtTmemCols, "Q does not fit TMEM");
 };
@@ -92,20 +98,27 @@ VB_DEVINL float at_ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+VB_DEVINL float at_rcp(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
 /* vb_mbar_wait with one answer for the warp: no lane leaves the others alone in a warp-wide instruction */
 VB_DEVINL bool at_warp_wait(uint64_t *bar, uint32_t parity, volatile int *cta_abort) {
     return __all_sync(0xffffffffu, vb_mbar_wait(bar, parity, cta_abort));
+}
+VB_DEVINL void at_tma(void *dst, const CUtensorMap *map, int x, int y, int z, uint64_t *bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
+            vb_smem_u32(dst)),
+        "l"(map), "r"(vb_smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+        : "memory");
 }
 /* Two values as packed BF16 high halves and packed remainders. */
 VB_DEVINL void at_split2(float a, float b, uint32_t &hi, uint32_t &lo) {
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(b), "f"(a));
     const float ra = a - __uint_as_float(hi << 16), rb = b - __uint_as_float(hi & 0xffff0000u);
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(rb), "f"(ra));
-}
-
-/* cap * tanh(x / cap), the hyperbolic tangent through one exponential (absolute error about 1e-7 of cap) */
-VB_DEVINL float soft_cap(float x, float cap, float two_over_cap) {
-    return cap - 2.0f * cap * __fdividef(1.0f, 1.0f + __expf(x * two_over_cap));
 }
 
 /* Rows [key][64 dims] as the B operand of P . V, read along the dims (MN-major): groups of eight keys 1024 bytes apart,
@@ -126,14 +139,16 @@ VB_DEVINL uint32_t at_off(int row, int chunk) { return (uint32_t)(row * 128 + ((
 
 /* A use (SRC) says where things come from and go:
  *   kAsync                       keys and values are copied with cp.async (else: stored by the loading threads)
+ *   kTma                         ... whole tiles by TMA, where AtArgs says so: boxes(...) says whether tile (j0, n) is one,
+ *                                tma_keys(...) and tma_values(...) request it
  *   start()                      after the wait for the previous kernel: resolves what lies in device memory
  *   pos0()                       position of row 0
- *   q8(row, head, d, v)          eight query values (zeros beyond the head)
+ *   q4(row, head, d)             four query values (zeros beyond the head)
  *   keys(...) / values(...)      a loading warp's 16 keys of a tile, into blocks of 64 columns: high halves, then low ones
  *   gate(row, head)              factor of a result row
  *   put4(row, column, v)         four results */
 template <int DK, int DV, class SRC>
-__global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const AtArgs a, const SRC src_arg) {
+__global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const __grid_constant__ AtMaps maps, const AtArgs a, const SRC src_arg) {
     using Cfg = AtCfg<DK, DV>;
     extern __shared__ unsigned char at_smem_raw[];
     unsigned char *base = (unsigned char *)(((uintptr_t)at_smem_raw + 1023) & ~(uintptr_t)1023);
@@ -147,8 +162,8 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const AtArgs 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
         for (int i = 0; i < Cfg::kSlots; i++) {
-            vb_mbar_init(&k_full[i], kAtLoaders);
-            vb_mbar_init(&v_full[i], kAtLoaders);
+            vb_mbar_init(&k_full[i], kAtLoadK);
+            vb_mbar_init(&v_full[i], kAtLoadV);
             vb_mbar_init(&k_empty[i], 1);
             vb_mbar_init(&v_empty[i], 1);
         }
@@ -161,7 +176,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const AtArgs 
         *abort_flag = 0;
         vb_mbar_init_fence();
     }
-    if (warp == 12) {
+    if (warp == kAtMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(vb_smem_u32(tmem_slot)), "r"(kAtTmemCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -194,16 +209,44 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const AtArgs 
         const bool valid = P < pairs;
         const int row = valid ? P / group : 0, head = g * group + (valid ? P - row * group : 0), i = pos0 + row;
         const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16, tS = tmem + lanes + (uint32_t)(w * kAtKeys), tO = tmem + lanes + kAtO + (uint32_t)(w * 128);
-        /* the query row, 32 columns in turn by the two warpgroups: halves to TMEM, low ones of large heads to shared memory */
+        /* The query rows, 32 columns in turn by the two warpgroups: two lanes read 32 bytes of a row (a lane per row reads 32
+         * rows at once: 18 us for 128 x 192), which then move to the lane that owns the row; halves to TMEM, low ones of
+         * large heads to shared memory. */
+        uint32_t *stage = reinterpret_cast<uint32_t *>((unsigned char *)bars + 256) + warp * 32 * kAtStage;
+        int qrow[2], qhead[2];
+#pragma unroll
+        for (int i2 = 0; i2 < 2; i2++) {
+            const int x = P0 + (warp & 3) * 32 + (lane >> 1) + 16 * i2;
+            qrow[i2] = x < pairs ? x / group : -1;
+            qhead[i2] = g * group + (x < pairs ? x - qrow[i2] * group : 0);
+        }
 #pragma unroll 1
         for (int u = w; u < 2 * DK; u += 2) {
             uint32_t hi[16], lo[16];
+            float4 v[4][2];
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+#pragma unroll
+                for (int i2 = 0; i2 < 2; i2++)
+                    v[c][i2] = qrow[i2] >= 0 ? src.q4(qrow[i2], qhead[i2], u * 32 + c * 8 + (lane & 1) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int c = 0; c < 4; c++) {
-                float e[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                if (valid) src.q8(row, head, u * 32 + c * 8, e);
+                __syncwarp();
 #pragma unroll
-                for (int j = 0; j < 4; j++) at_split2(e[2 * j], e[2 * j + 1], hi[c * 4 + j], lo[c * 4 + j]);
+                for (int i2 = 0; i2 < 2; i2++) {
+                    float4 e = v[c][i2];
+                    if (a.scale <= 0.0f) {             /* the scores are multiplied by |scale| below, or by one */
+                        const float f = a.scale < 0.0f ? -1.0f : 0.0f;
+                        e = make_float4(e.x * f, e.y * f, e.z * f, e.w * f);
+                    }
+                    uint32_t *to = stage + ((lane >> 1) + 16 * i2) * kAtStage + (lane & 1) * 2;
+                    at_split2(e.x, e.y, to[0], to[4]);
+                    at_split2(e.z, e.w, to[1], to[5]);
+                }
+                __syncwarp();
+                const uint4 h4 = *reinterpret_cast<const uint4 *>(stage + lane * kAtStage), l4 = *reinterpret_cast<const uint4 *>(stage + lane * kAtStage + 4);
+                hi[c * 4] = h4.x; hi[c * 4 + 1] = h4.y; hi[c * 4 + 2] = h4.z; hi[c * 4 + 3] = h4.w;
+                lo[c * 4] = l4.x; lo[c * 4 + 1] = l4.y; lo[c * 4 + 2] = l4.z; lo[c * 4 + 3] = l4.w;
             }
             at_st16(tmem + lanes + kAtQ + (uint32_t)(u * 16), hi);
             if constexpr (Cfg::kQlTmem) {
@@ -220,8 +263,13 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const AtArgs 
         tc_fence_before();
         vb_mbar_arrive(q_full);
 
-        const float kLog2eHi = 1.44269502f, kLog2eLo = 1.92596303e-8f;
-        const float two_over_cap = a.softcap > 0.0f ? 2.0f / a.softcap : 0.0f;
+        /* Scores as powers of two: S times mul (to twice fp32's precision), or with a softcap
+         * cap * tanh(x / cap) = cap - 2 cap / (1 + e^(2 x / cap)), x = S * scale, in these units. */
+        const double log2e = 1.4426950408889634, dmul = a.softcap > 0.0f || a.scale == 0.0f ? 1.0 : fabs((double)a.scale) * log2e;
+        float mul = __double2float_rz(dmul);
+        if ((double)mul == dmul) mul = __uint_as_float(__float_as_uint(mul) - 1u);       /* mul_lo > 0: a masked -inf stays one */
+        const float mul_lo = (float)(dmul - (double)mul);
+        const float cap2 = (float)(a.softcap * log2e), cap_in = a.softcap > 0.0f ? (float)(2.0 * log2e * fabs((double)a.scale) / a.softcap) : 0.0f;
         float ref = -INFINITY, sum = 0.0f;      /* the row's reference (in powers of two), its sum of weights against it */
         int it = 0;
         for (int t = w; t < n_tiles; t += 2, it++) {
@@ -235,11 +283,11 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const AtArgs 
                 uint32_t reg[32];
                 at_ld32(tS + (uint32_t)(c * 32), reg);
 #pragma unroll
-                for (int k = 0; k < 32; k++) s[c * 32 + k] = __uint_as_float(reg[k]) * a.scale;
+                for (int k = 0; k < 32; k++) s[c * 32 + k] = __uint_as_float(reg[k]);
             }
             if (a.softcap > 0.0f) {
 #pragma unroll
-                for (int k = 0; k < kAtKeys; k++) s[k] = soft_cap(s[k], a.softcap, two_over_cap);
+                for (int k = 0; k < kAtKeys; k++) s[k] = fmaf(-2.0f * cap2, at_rcp(1.0f + at_ex2(s[k] * cap_in)), cap2);
             }
             const bool all_seen = n == kAtKeys && j0 + kAtKeys - 1 <= imin && (a.window <= 0 || imax - j0 < a.window || j0 + kAtKeys <= a.keep);
             if (!all_seen) {
@@ -252,7 +300,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const AtArgs 
             float top4[4] = {s[0], s[1], s[2], s[3]};
 #pragma unroll
             for (int k = 4; k < kAtKeys; k++) top4[k & 3] = fmaxf(top4[k & 3], s[k]);
-            const float top = fmaxf(fmaxf(top4[0], top4[1]), fmaxf(top4[2], top4[3])) * kLog2eHi;
+            const float top = fmaxf(fmaxf(top4[0], top4[1]), fmaxf(top4[2], top4[3])) * mul;
             const bool rise = top > ref + 8.0f;
             if (__any_sync(0xffffffffu, rise)) {
                 const float now = rise ? top : ref, f = rise ? at_ex2(ref - now) : 1.0f;     /* the first time: 0 */
@@ -282,7 +330,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const AtArgs 
 #pragma unroll
                     for (int u = 0; u < 2; u++) {
                         const float x = s[c * 32 + k + u];
-                        p[u] = at_ex2(fmaf(x, kLog2eLo, fmaf(x, kLog2eHi, -m)));
+                        p[u] = at_ex2(fmaf(x, mul_lo, fmaf(x, mul, -m)));
                         sum4[(k + u) & 3] += p[u];
                     }
                     at_split2(p[0], p[1], reg[k / 2], reg[16 + k / 2]);
@@ -334,75 +382,94 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const AtArgs 
                 src.put4(m, hd * a.vdim + c, v);
             }
         }
-    } else if (warp < 12) {
-        /* ---- keys and values: K0, K1, V0, K2, V1, ... as the MMAs take them ---- */
-        const int lw = warp - 8;
-        if (a.dim % 16) {          /* the last 16 columns of a product reach beyond the head: zeros there, for good */
+    } else if (warp < kAtMmaWarp) {
+        /* ---- four warps for the keys, two for the values: a slot of K is free after S, one of V only after the softmax,
+         * and a loader that took both in turn handed keys over no sooner than the values before them ---- */
+        const bool is_k = warp < 12;
+        const int lw = is_k ? warp - 8 : (warp - 12) * 2;      /* 16 keys each, values 32 */
+        uint64_t *full = is_k ? k_full : v_full, *empty = is_k ? k_empty : v_empty;
+        if (is_k && a.dim % 16) {          /* the last 16 columns of a product reach beyond the head: zeros there, for good */
             const int chunk = a.dim / 8;
-            for (int x = tid - kAtSoft; x < Cfg::kSlots * 2 * kAtKeys; x += kAtLoaders) {
+            for (int x = tid - kAtSoft; x < Cfg::kSlots * 2 * kAtKeys; x += kAtLoadK) {
                 const int key = x % kAtKeys, plane = x / kAtKeys;
                 *reinterpret_cast<uint4 *>(k_s + (plane * DK + (chunk >> 3)) * kAtBlock + at_off(key, chunk)) = make_uint4(0u, 0u, 0u, 0u);
             }
         }
-        int told = 0;              /* steps before this one are handed over */
+        int told = 0;              /* tiles before this one are handed over */
         auto hand_over = [&](int upto) {
             if (told >= upto) return;
             at_proxy_fence();
-            for (; told < upto; told++) {
-                if (told == 2 * n_tiles - 1) continue;
-                const bool is_k = told == 0 || (told & 1);
-                const int t = is_k ? (told + 1) / 2 : told / 2 - 1;
-                vb_mbar_arrive(is_k ? &k_full[t % Cfg::kSlots] : &v_full[t % Cfg::kSlots]);
-            }
+            for (; told < upto; told++) vb_mbar_arrive(&full[told % Cfg::kSlots]);
         };
-        for (int step = 0; step <= 2 * n_tiles; step++) {
-            if (step != 2 * n_tiles - 1) {
-                const bool is_k = step == 0 || (step & 1);
-                const int t = is_k ? (step + 1) / 2 : step / 2 - 1, slot = t % Cfg::kSlots;
-                uint64_t *empty = is_k ? &k_empty[slot] : &v_empty[slot];
-                const uint32_t parity = ((uint32_t)(t / Cfg::kSlots) & 1u) ^ 1u;
-                if (!__all_sync(0xffffffffu, vb_mbar_try_wait(empty, parity))) {
-                    if constexpr (SRC::kAsync) {         /* what waits for the slot may wait for what is on its way */
-                        lm_cp_wait_all();
-                        hand_over(step);
-                    }
-                    if (!at_warp_wait(empty, parity, abort_flag)) { give_up(); break; }
+        /* (Copied row by row, 16 bytes a lane, a tile of 192-wide keys takes a warp 4000 clocks of address arithmetic. That
+         * remains for tiles that end early, wrap around the ring, or have columns that are not whole boxes.) */
+        for (int t = 0; t < n_tiles; t++) {
+            const int slot = t % Cfg::kSlots;
+            const uint32_t parity = ((uint32_t)(t / Cfg::kSlots) & 1u) ^ 1u;
+            if (!__all_sync(0xffffffffu, vb_mbar_try_wait(&empty[slot], parity))) {
+                if constexpr (SRC::kAsync) {         /* what waits for the slot may wait for what is on its way */
+                    lm_cp_wait_all();
+                    hand_over(t);
                 }
-                int j0, n;
-                key_tile<kAtKeys>(kt, t, &j0, &n);
-                if (is_k) src.template keys<DK>(a, k_s + slot * Cfg::kSlotK, g, lw, lane, j0, n);
-                else src.template values<DV>(a, v_s + slot * Cfg::kSlotV, g, lw, lane, j0, n);
+                if (!at_warp_wait(&empty[slot], parity, abort_flag)) { give_up(); break; }
+            }
+            int j0, n;
+            key_tile<kAtKeys>(kt, t, &j0, &n);
+            if constexpr (SRC::kTma) {
+                if (a.tma && n == kAtKeys && src.boxes(j0)) {
+                    lm_cp_wait_all();
+                    hand_over(t);
+                    if (lw == 0 && lane == 0) {
+                        vb_mbar_arrive_expect_tx(&full[slot], is_k ? Cfg::kSlotK : Cfg::kSlotV);
+                        if (is_k) src.template tma_keys<DK>(a, maps, k_s + slot * Cfg::kSlotK, g, j0, &full[slot]);
+                        else src.template tma_values<DV>(a, maps, v_s + slot * Cfg::kSlotV, g, j0, &full[slot]);
+                    } else {
+                        vb_mbar_arrive(&full[slot]);
+                    }
+                    told = t + 1;
+                    continue;
+                }
+            }
+            if (is_k) {
+                src.template keys<DK>(a, k_s + slot * Cfg::kSlotK, g, lw, lane, j0, n);
+            } else {
+                src.template values<DV>(a, v_s + slot * Cfg::kSlotV, g, lw, lane, j0, n);
+                src.template values<DV>(a, v_s + slot * Cfg::kSlotV, g, lw + 1, lane, j0, n);
             }
             if constexpr (SRC::kAsync) {
                 lm_cp_commit();
-                asm volatile("cp.async.wait_group 2;" ::: "memory");
-                hand_over(step - 1);
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+                hand_over(t);
             } else {
-                hand_over(step + 1);
+                hand_over(t + 1);
             }
         }
         if constexpr (SRC::kAsync) lm_cp_wait_all();
-        if (!*(volatile int *)abort_flag) hand_over(2 * n_tiles + 1);
+        if (!*(volatile int *)abort_flag) hand_over(n_tiles);
     } else if (lane == 0) {
         /* ---- MMA issuer ---- */
         const int k_steps = (a.dim + 15) / 16;
         const uint32_t idesc_s = at_idesc(kAtKeys, false), idesc_o = at_idesc((a.vdim + 15) & ~15, true);
+        /* descriptors once: the one issuing thread has 32 to 64 clocks per MMA (addresses stay below 2^18, so sums carry
+         * into nothing else) */
+        const uint64_t k_desc = umma_desc_k_sw128(k_s), q_desc = umma_desc_k_sw128(ql_s), v_desc = at_desc_mn(vb_smem_u32(v_s));
         bool ok = vb_mbar_wait(q_full, 0u, abort_flag);
         tc_fence_after();
         auto scores = [&](int t) {
             const int slot = t % Cfg::kSlots;
             if (!vb_mbar_wait(&k_full[slot], (uint32_t)(t / Cfg::kSlots) & 1u, abort_flag)) return false;
             tc_fence_after();
-            const unsigned char *kp = k_s + slot * Cfg::kSlotK;
+            const uint64_t kd = k_desc + (uint64_t)(slot * (Cfg::kSlotK >> 4));
             const uint32_t d = tmem + (uint32_t)((t & 1) * kAtKeys);
-            for (int ks = 0; ks < k_steps; ks++) {
-                const uint64_t hi = umma_desc_k_sw128(kp + (ks >> 2) * kAtBlock) + 2 * (ks & 3);
-                const uint64_t lo = umma_desc_k_sw128(kp + (DK + (ks >> 2)) * kAtBlock) + 2 * (ks & 3);
+#pragma unroll
+            for (int ks = 0; ks < DK * 4; ks++) {
+                if (ks >= k_steps) break;
+                const uint64_t hi = kd + (uint64_t)((ks >> 2) * (kAtBlock >> 4) + 2 * (ks & 3)), lo = hi + DK * (kAtBlock >> 4);
                 const uint32_t qh = tmem + kAtQ + (uint32_t)(ks * 8);
                 at_mma_ts(d, qh, hi, idesc_s, ks != 0 ? 1u : 0u);
                 at_mma_ts(d, qh, lo, idesc_s, 1u);
                 if constexpr (Cfg::kQlTmem) at_mma_ts(d, qh + DK * 32, hi, idesc_s, 1u);
-                else umma_bf16(d, umma_desc_k_sw128(ql_s + (ks >> 2) * kAtRows * 128) + 2 * (ks & 3), hi, idesc_s, 1u);
+                else umma_bf16(d, q_desc + (uint64_t)((ks >> 2) * (kAtRows * 128 >> 4) + 2 * (ks & 3)), hi, idesc_s, 1u);
             }
             umma_commit(&k_empty[slot]);
             umma_commit(&s_full[t & 1]);
@@ -416,11 +483,11 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const AtArgs 
                  vb_mbar_wait(&p_full[w], (uint32_t)(t >> 1) & 1u, abort_flag);
             if (!ok) break;
             tc_fence_after();
-            const uint32_t vp = vb_smem_u32(v_s + slot * Cfg::kSlotV);
+            const uint64_t vd = v_desc + (uint64_t)(slot * (Cfg::kSlotV >> 4));
             const uint32_t d = tmem + kAtO + (uint32_t)(w * 128);
 #pragma unroll
             for (int ks = 0; ks < kAtKeys / 16; ks++) {
-                const uint64_t hi = at_desc_mn(vp + ks * 2048), lo = at_desc_mn(vp + DV * kAtBlock + ks * 2048);
+                const uint64_t hi = vd + (uint64_t)(ks * (2048 >> 4)), lo = hi + DV * (kAtBlock >> 4);
                 const uint32_t ph = tmem + (uint32_t)(w * kAtKeys + (ks >> 1) * 32 + (ks & 1) * 8);
                 at_mma_ts(d, ph, hi, idesc_o, (t >> 1 | ks) != 0 ? 1u : 0u);
                 at_mma_ts(d, ph, lo, idesc_o, 1u);
@@ -435,14 +502,14 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const AtArgs 
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 12) {
+    if (warp == kAtMmaWarp) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kAtTmemCols) : "memory");
     }
 }
 
 template <int DK, int DV, class SRC>
-int launch_attn_tc(const AtArgs &a, const SRC &src, cudaStream_t st) {
+int launch_attn_tc(const AtArgs &a, const SRC &src, cudaStream_t st, const AtMaps &maps = AtMaps()) {
     using Cfg = AtCfg<DK, DV>;
     static bool attr = false;
     if (!attr) {
@@ -453,7 +520,7 @@ int launch_attn_tc(const AtArgs &a, const SRC &src, cudaStream_t st) {
         attr = true;
     }
     const int tiles = (int)(((long long)a.M * (a.heads / a.kv_heads) + kAtRows - 1) / kAtRows);
-    return launch_pdl(vb_attn_tc_kernel<DK, DV, SRC>, dim3(a.kv_heads, tiles), dim3(kAtThreads), (size_t)Cfg::kSmem, st, a, src) == cudaSuccess
+    return launch_pdl(vb_attn_tc_kernel<DK, DV, SRC>, dim3(a.kv_heads, tiles), dim3(kAtThreads), (size_t)Cfg::kSmem, st, maps, a, src) == cudaSuccess
                ? 0
                : -1;
 }

@@ -796,6 +796,7 @@ int vb200_lm::latent_wide(const Layer &l, const LmMixer &m, const LmLatent &a, c
     t.heads = t.kv_heads = m.heads; t.dim = m.dim + m.rot_dim; t.vdim = m.vdim;
     t.window = m.mask.window; t.scale = (float)m.scale; t.rot = m.rope.dims;
     t.ring = s.ring;
+    t.slots = (int)seqs.size();
     t.status = status;
     t.out = a.out;
     LmWide w = {};
@@ -900,7 +901,7 @@ int vb200_lm::mixer(const Layer &l, const LmLayer &spec, const RunState &s, int 
         a.rot = m.rope.dims; a.freq = l.mix.freq; a.mag = l.mix.mag;
         a.q_gain = l.mix.q_gain; a.k_gain = l.mix.k_gain; a.eps = (float)cfg.eps;
         a.ring = s.ring;
-        a.k = {slabs + s.a, slab}; a.v = {slabs + s.b, slab};
+        a.k = {slabs + s.a, slab}; a.v = {slabs + s.b, slab}; a.slots = (int)seqs.size();
         a.split = !f32() && lm_attn_mma_ok(m.dim, m.vdim);
         a.qkv = in; a.q = q; a.scratch = scratch; a.tickets = tickets; a.status = status;
         a.out = sink(l.mix.acts, M);

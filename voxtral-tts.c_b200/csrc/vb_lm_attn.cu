@@ -482,7 +482,7 @@ VB_DEVINL void clear_keys(unsigned char *slot, int lw, int lane, int n) {
 
 /* Keys and values from a cache of split rows. */
 struct AtCache {
-    static constexpr bool kAsync = true;
+    static constexpr bool kAsync = true, kTma = true;
     const LmDyn *dyn;
     const float *q;
     LmState k, v;
@@ -492,14 +492,23 @@ struct AtCache {
     const float *kc, *vc;
     VB_DEVINL void start() { kc = lm_state(k, dyn); vc = lm_state(v, dyn); }
     VB_DEVINL int pos0() const { return dyn->pos; }
-    VB_DEVINL void q8(int row, int head, int d, float (&e)[8]) const {
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
-        if (d < dim) {
-            const float4 *p = reinterpret_cast<const float4 *>(q + ((size_t)row * heads + head) * dim + d);
-            x = p[0];
-            y = p[1];
-        }
-        e[0] = x.x; e[1] = x.y; e[2] = x.z; e[3] = x.w; e[4] = y.x; e[5] = y.y; e[6] = y.z; e[7] = y.w;
+    VB_DEVINL float4 q4(int row, int head, int d) const {
+        return d < dim ? vb_ldcg4(q + ((size_t)row * heads + head) * dim + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    VB_DEVINL bool boxes(int j0) const { return lm_ring_row(ring, j0 + kAtKeys - 1) - lm_ring_row(ring, j0) == kAtKeys - 1; }
+    template <int BLOCKS>
+    VB_DEVINL void box(const CUtensorMap *map, int size, unsigned char *slot, int g, int j0, uint64_t *bar) const {
+        const int row = lm_ring_row(ring, j0);
+#pragma unroll
+        for (int b = 0; b < 2 * BLOCKS; b++) at_tma(slot + b * kAtBlock, map, g * 2 * size + (b / BLOCKS) * size + (b % BLOCKS) * 64, row, dyn->slot, bar);
+    }
+    template <int BLOCKS>
+    VB_DEVINL void tma_keys(const AtArgs &, const AtMaps &m, unsigned char *slot, int g, int j0, uint64_t *bar) const {
+        box<BLOCKS>(&m.k, dim, slot, g, j0, bar);
+    }
+    template <int BLOCKS>
+    VB_DEVINL void tma_values(const AtArgs &, const AtMaps &m, unsigned char *slot, int g, int j0, uint64_t *bar) const {
+        box<BLOCKS>(&m.v, vdim, slot, g, j0, bar);
     }
     template <int BLOCKS>
     VB_DEVINL void rows(const float *cache, int size, unsigned char *slot, int g, int lw, int lane, int j0, int n) const {
@@ -535,7 +544,7 @@ struct AtCache {
 /* Every head has keys and values of its own, read out of a latent (LmWide): a head's own columns of the written-out
  * rows, then the key part that all heads share from the latent's cache row. */
 struct AtWide {
-    static constexpr bool kAsync = true;
+    static constexpr bool kAsync = true, kTma = true;
     const LmDyn *dyn;
     LmWide w;
     LmRing ring;
@@ -543,17 +552,14 @@ struct AtWide {
     int heads, dim, vdim, rot;
     VB_DEVINL void start() { w.cache += (size_t)dyn->slot * w.slab; }
     VB_DEVINL int pos0() const { return dyn->pos; }
-    VB_DEVINL void q8(int row, int head, int d, float (&e)[8]) const {
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
-        if (d < dim) {
-            x = lm_sum4(w.q, row, head * dim + d);
-            y = lm_sum4(w.q, row, head * dim + d + 4);
-        }
-        e[0] = x.x; e[1] = x.y; e[2] = x.z; e[3] = x.w; e[4] = y.x; e[5] = y.y; e[6] = y.z; e[7] = y.w;
+    VB_DEVINL float4 q4(int row, int head, int d) const {
+        if (d >= dim) return make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 x = lm_sum4(w.q, row, head * dim + d);
         const int half = rot / 2, i0 = (d - (dim - w.rot_dim)) / 2;
-        if (d >= dim - w.rot_dim && d < dim) {
+        float e[4] = {x.x, x.y, x.z, x.w};
+        if (d >= dim - w.rot_dim) {
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
+            for (int i = 0; i < 2; i++) {
                 if (i0 + i < half) {
                     const float c = w.cs[(size_t)row * rot + i0 + i], s = w.cs[(size_t)row * rot + half + i0 + i];
                     const float u = e[2 * i], t = e[2 * i + 1];
@@ -562,6 +568,23 @@ struct AtWide {
                 }
             }
         }
+        return make_float4(e[0], e[1], e[2], e[3]);
+    }
+    VB_DEVINL bool boxes(int j0) const { return lm_ring_row(ring, j0 + kAtKeys - 1) - lm_ring_row(ring, j0) == kAtKeys - 1; }
+    template <int BLOCKS>
+    VB_DEVINL void tma_keys(const AtArgs &, const AtMaps &m, unsigned char *slot, int g, int j0, uint64_t *bar) const {
+        const int own = (dim - w.rot_dim) / 64, row = w.rank + w.rot_dim;
+#pragma unroll
+        for (int b = 0; b < 2 * BLOCKS; b++) {
+            const int plane = b / BLOCKS, c = b % BLOCKS;
+            if (c < own) at_tma(slot + b * kAtBlock, &m.k, (g * own + c) * 64, j0 - w.first, plane, bar);
+            else at_tma(slot + b * kAtBlock, &m.k2, plane * row + w.rank + (c - own) * 64, lm_ring_row(ring, j0), dyn->slot, bar);
+        }
+    }
+    template <int BLOCKS>
+    VB_DEVINL void tma_values(const AtArgs &, const AtMaps &m, unsigned char *slot, int g, int j0, uint64_t *bar) const {
+#pragma unroll
+        for (int b = 0; b < 2 * BLOCKS; b++) at_tma(slot + b * kAtBlock, &m.v, w.v0 + g * vdim + (b % BLOCKS) * 64, j0 - w.first, b / BLOCKS, bar);
     }
     template <int BLOCKS>
     VB_DEVINL void keys(const AtArgs &, unsigned char *slot, int g, int lw, int lane, int j0, int n) const {
@@ -601,7 +624,7 @@ struct AtWide {
     VB_DEVINL void put4(int row, int c, const float (&e)[4]) const { lm_put4(out, row, c, e); }
 };
 
-AtArgs at_args(const LmAttn &a, int M) { return {M, a.heads, a.kv_heads, a.dim, a.vdim, a.window, a.keep, a.scale, a.softcap, a.status}; }
+AtArgs at_args(const LmAttn &a, int M) { return {M, a.heads, a.kv_heads, a.dim, a.vdim, a.window, a.keep, a.scale, a.softcap, a.status, 0}; }
 
 constexpr int kSplitBudget = 296;        /* two CTAs per SM */
 constexpr int kStepCtas = 148;           /* one-token kernel: one CTA per SM */
@@ -654,9 +677,15 @@ int lm_attn_mma(const LmAttn &a, int M, cudaStream_t st) {
     AtCache c = {};
     c.dyn = a.dyn; c.q = a.q; c.k = a.k; c.v = a.v; c.ring = a.ring; c.out = a.out;
     c.heads = a.heads; c.kv_heads = a.kv_heads; c.dim = a.dim; c.vdim = a.vdim;
-    const AtArgs t = at_args(a, M);
-    if (a.dim <= 64) return a.vdim <= 64 ? launch_attn_tc<1, 1>(t, c, st) : launch_attn_tc<1, 2>(t, c, st);
-    return a.vdim <= 64 ? launch_attn_tc<2, 1>(t, c, st) : launch_attn_tc<2, 2>(t, c, st);
+    AtArgs t = at_args(a, M);
+    AtMaps m = {};
+    if (a.dim % 64 == 0 && a.vdim % 64 == 0) {
+        const uint64_t rows = (uint64_t)a.ring.keep + a.ring.ring, ck = (uint64_t)2 * a.kv_heads * a.dim, cv = (uint64_t)2 * a.kv_heads * a.vdim;
+        t.tma = tc_map3(&m.k, a.k.base, a.slots, a.k.slab * 4, rows, ck * 2, ck, kAtKeys) == 0 &&
+                tc_map3(&m.v, a.v.base, a.slots, a.v.slab * 4, rows, cv * 2, cv, kAtKeys) == 0;
+    }
+    if (a.dim <= 64) return a.vdim <= 64 ? launch_attn_tc<1, 1>(t, c, st, m) : launch_attn_tc<1, 2>(t, c, st, m);
+    return a.vdim <= 64 ? launch_attn_tc<2, 1>(t, c, st, m) : launch_attn_tc<2, 2>(t, c, st, m);
 }
 
 bool lm_attn_wide_ok(int plain, int rot_dim, int vdim) {
@@ -667,11 +696,18 @@ int lm_attn_wide(const LmAttn &a, const LmWide &w, int M, cudaStream_t st) {
     AtWide c = {};
     c.dyn = a.dyn; c.w = w; c.ring = a.ring; c.out = a.out;
     c.heads = a.heads; c.dim = a.dim; c.vdim = a.vdim; c.rot = a.rot;
-    const AtArgs t = at_args(a, M);
+    AtArgs t = at_args(a, M);
+    AtMaps m = {};
+    if (a.dim % 64 == 0 && w.rot_dim % 64 == 0 && a.vdim % 64 == 0) {
+        const uint64_t row = (uint64_t)w.rank + w.rot_dim, rows = w.plane / w.ld;
+        t.tma = tc_map3(&m.k, w.kv, 2, w.plane * 2, rows, (uint64_t)w.ld * 2, w.ld, kAtKeys) == 0 &&
+                (w.rot_dim == 0 || tc_map3(&m.k2, w.cache, a.slots, w.slab * 4, (uint64_t)a.ring.keep + a.ring.ring, row * 4, row * 2, kAtKeys) == 0);
+        m.v = m.k;
+    }
     const bool v1 = a.vdim <= 64;
-    if (a.dim <= 64) return v1 ? launch_attn_tc<1, 1>(t, c, st) : launch_attn_tc<1, 2>(t, c, st);
-    if (a.dim <= 128) return v1 ? launch_attn_tc<2, 1>(t, c, st) : launch_attn_tc<2, 2>(t, c, st);
-    return v1 ? launch_attn_tc<3, 1>(t, c, st) : launch_attn_tc<3, 2>(t, c, st);
+    if (a.dim <= 64) return v1 ? launch_attn_tc<1, 1>(t, c, st, m) : launch_attn_tc<1, 2>(t, c, st, m);
+    if (a.dim <= 128) return v1 ? launch_attn_tc<2, 1>(t, c, st, m) : launch_attn_tc<2, 2>(t, c, st, m);
+    return v1 ? launch_attn_tc<3, 1>(t, c, st, m) : launch_attn_tc<3, 2>(t, c, st, m);
 }
 
 bool lm_attn_step_ok(const LmAttn &a) {

@@ -82,16 +82,14 @@ __global__ void pf_qkv_finish_kernel(float *qkv, const float *part, int n_part, 
  * tensor cores (vb_attn_tc.cuh): queries, and the cache's fp32 keys and values, which the loading warps split into BF16
  * halves on the way to shared memory. */
 struct AtRows {
-    static constexpr bool kAsync = false;
+    static constexpr bool kAsync = false, kTma = false;
     const float *q, *kc, *vc;
     LmSink out;                  /* the terms that the O projection reads */
     int ldq, ldkv, start_pos;
     VB_DEVINL void start() {}
     VB_DEVINL int pos0() const { return start_pos; }
-    VB_DEVINL void q8(int row, int head, int d, float (&e)[8]) const {
-        const float4 *p = reinterpret_cast<const float4 *>(q + (size_t)row * ldq + head * VB200_HEAD_DIM + d);
-        const float4 x = p[0], y = p[1];
-        e[0] = x.x; e[1] = x.y; e[2] = x.z; e[3] = x.w; e[4] = y.x; e[5] = y.y; e[6] = y.z; e[7] = y.w;
+    VB_DEVINL float4 q4(int row, int head, int d) const {
+        return vb_ldcg4(q + (size_t)row * ldq + head * VB200_HEAD_DIM + d);
     }
     /* a lane's four columns of 16 rows, eight loads in flight; rows beyond the tile's keys are zeros */
     VB_DEVINL void rows(const float *cache, unsigned char *slot, int g, int lw, int lane, int j0, int n) const {
@@ -246,7 +244,7 @@ static int prefill_tc(float *x, const float *cs, int M, int start_pos, int block
                        v0 + (size_t)(start_pos + r0) * KVD, rows);
             if (l == VB200_DEC_LAYERS - 1) break;   /* only the cache is kept (voxtral_tts_llm.c:281) */
             const AtRows rows_of = {t.qkv, k0, v0, q_terms, QKV, KVD, start_pos + r0};
-            const AtArgs at = {rows, VB200_HEADS, VB200_KV_HEADS, VB200_HEAD_DIM, VB200_HEAD_DIM, 0, 0, scale, 0.0f, &m.d_out->status};
+            const AtArgs at = {rows, VB200_HEADS, VB200_KV_HEADS, VB200_HEAD_DIM, VB200_HEAD_DIM, 0, 0, scale, 0.0f, &m.d_out->status, 0};
             if (launch_attn_tc<2, 2>(at, rows_of, st)) return -1;
             g.splits = b.s_wo; g.ld_out = D; g.ssq = nullptr; g.ssq_chunks = 0;
             if (tc_gemm(t.wo[l], aQ, g, st)) return -1;

@@ -68,6 +68,19 @@ int tc_map(CUtensorMap *m, const void *base, uint64_t rows, uint64_t cols, uint3
     return r == CUDA_SUCCESS ? 0 : -1;
 }
 
+int tc_map3(CUtensorMap *m, const void *base, uint64_t planes, uint64_t plane_bytes, uint64_t rows, uint64_t row_bytes, uint64_t cols, uint32_t box_rows) {
+    if (tc_init()) return -1;
+    if (((uintptr_t)base & 15) || row_bytes % 16 || plane_bytes % 16 || cols < kTcBlockK) return -1;
+    cuuint64_t gdim[3] = {cols, rows, planes};
+    cuuint64_t gstride[2] = {row_bytes, plane_bytes};
+    cuuint32_t box[3] = {(cuuint32_t)kTcBlockK, box_rows, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = g_encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void *)base, gdim, gstride, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : -1;
+}
+
 int tc_weight(TcWeight *w, const uint16_t *d_W, int N, int K) {
     w->ok = false;
     w->W = d_W; w->N = N; w->K = K; w->tiled = false;

@@ -152,6 +152,8 @@ int tc_gemm_rows(const TcWeight &w, const TcActs &acts, const TcGemm &g, cudaStr
 int tc_row_splits(int N, int K, int M, int n_sm);
 /* [rows, cols] BF16 row-major as a tensor map; box = 64 columns x box_rows rows, 128-byte swizzle. */
 int tc_map(CUtensorMap *m, const void *base, uint64_t rows, uint64_t cols, uint32_t box_rows);
+/* The same of `planes` such matrices, with row and plane pitches in bytes. */
+int tc_map3(CUtensorMap *m, const void *base, uint64_t planes, uint64_t plane_bytes, uint64_t rows, uint64_t row_bytes, uint64_t cols, uint32_t box_rows);
 
 /* Grouped GEMM: several weight matrices of equal size stacked in one TcWeight (each padded to whole
  * 128-row tiles), and rows sorted by matrix in blocks of 128. table[b] = {matrix or -1, first row, rows,
