@@ -138,13 +138,13 @@ VB_DEVINL uint32_t at_idesc(int n, bool mn_major) {
 VB_DEVINL uint32_t at_off(int row, int chunk) { return (uint32_t)(row * 128 + (((chunk ^ row) & 7) << 4)); }
 
 /* A use (SRC) says where things come from and go:
- *   kAsync                       keys and values are copied with cp.async (else: stored by the loading threads)
- *   kTma                         ... whole tiles by TMA, where AtArgs says so: boxes(...) says whether tile (j0, n) is one,
- *                                tma_keys(...) and tma_values(...) request it
+ *   tma_keys(...) / tma_values(...)   request a tile by TMA: where AtArgs says so and boxes(j0, n) does, or always (kBoxes:
+ *                                what lies beyond the last key is zeros)
  *   start()                      after the wait for the previous kernel: resolves what lies in device memory
  *   pos0()                       position of row 0
  *   q4(row, head, d)             four query values (zeros beyond the head)
- *   keys(...) / values(...)      a loading warp's 16 keys of a tile, into blocks of 64 columns: high halves, then low ones
+ *   keys(...) / values(...)      otherwise, with cp.async: a loading warp's 16 keys, into blocks of 64 columns, high halves
+ *                                first
  *   gate(row, head)              factor of a result row
  *   put4(row, column, v)         four results */
 template <int DK, int DV, class SRC>
@@ -407,44 +407,38 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const __grid_
             const int slot = t % Cfg::kSlots;
             const uint32_t parity = ((uint32_t)(t / Cfg::kSlots) & 1u) ^ 1u;
             if (!__all_sync(0xffffffffu, vb_mbar_try_wait(&empty[slot], parity))) {
-                if constexpr (SRC::kAsync) {         /* what waits for the slot may wait for what is on its way */
-                    lm_cp_wait_all();
-                    hand_over(t);
-                }
+                lm_cp_wait_all();                    /* what waits for the slot may wait for what is on its way */
+                hand_over(t);
                 if (!at_warp_wait(&empty[slot], parity, abort_flag)) { give_up(); break; }
             }
             int j0, n;
             key_tile<kAtKeys>(kt, t, &j0, &n);
-            if constexpr (SRC::kTma) {
-                if (a.tma && n == kAtKeys && src.boxes(j0)) {
-                    lm_cp_wait_all();
-                    hand_over(t);
-                    if (lw == 0 && lane == 0) {
-                        vb_mbar_arrive_expect_tx(&full[slot], is_k ? Cfg::kSlotK : Cfg::kSlotV);
-                        if (is_k) src.template tma_keys<DK>(a, maps, k_s + slot * Cfg::kSlotK, g, j0, &full[slot]);
-                        else src.template tma_values<DV>(a, maps, v_s + slot * Cfg::kSlotV, g, j0, &full[slot]);
-                    } else {
-                        vb_mbar_arrive(&full[slot]);
-                    }
-                    told = t + 1;
-                    continue;
+            if (SRC::kBoxes || (a.tma && src.boxes(j0, n))) {
+                lm_cp_wait_all();
+                hand_over(t);
+                if (lw == 0 && lane == 0) {
+                    vb_mbar_arrive_expect_tx(&full[slot], is_k ? Cfg::kSlotK : Cfg::kSlotV);
+                    if (is_k) src.template tma_keys<DK>(a, maps, k_s + slot * Cfg::kSlotK, g, j0, &full[slot]);
+                    else src.template tma_values<DV>(a, maps, v_s + slot * Cfg::kSlotV, g, j0, &full[slot]);
+                } else {
+                    vb_mbar_arrive(&full[slot]);
+                }
+                told = t + 1;
+                continue;
+            }
+            if constexpr (!SRC::kBoxes) {
+                if (is_k) {
+                    src.template keys<DK>(a, k_s + slot * Cfg::kSlotK, g, lw, lane, j0, n);
+                } else {
+                    src.template values<DV>(a, v_s + slot * Cfg::kSlotV, g, lw, lane, j0, n);
+                    src.template values<DV>(a, v_s + slot * Cfg::kSlotV, g, lw + 1, lane, j0, n);
                 }
             }
-            if (is_k) {
-                src.template keys<DK>(a, k_s + slot * Cfg::kSlotK, g, lw, lane, j0, n);
-            } else {
-                src.template values<DV>(a, v_s + slot * Cfg::kSlotV, g, lw, lane, j0, n);
-                src.template values<DV>(a, v_s + slot * Cfg::kSlotV, g, lw + 1, lane, j0, n);
-            }
-            if constexpr (SRC::kAsync) {
-                lm_cp_commit();
-                asm volatile("cp.async.wait_group 1;" ::: "memory");
-                hand_over(t);
-            } else {
-                hand_over(t + 1);
-            }
+            lm_cp_commit();
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            hand_over(t);
         }
-        if constexpr (SRC::kAsync) lm_cp_wait_all();
+        lm_cp_wait_all();
         if (!*(volatile int *)abort_flag) hand_over(n_tiles);
     } else if (lane == 0) {
         /* ---- MMA issuer ---- */

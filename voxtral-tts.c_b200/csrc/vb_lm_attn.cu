@@ -482,7 +482,7 @@ VB_DEVINL void clear_keys(unsigned char *slot, int lw, int lane, int n) {
 
 /* Keys and values from a cache of split rows. */
 struct AtCache {
-    static constexpr bool kAsync = true, kTma = true;
+    static constexpr bool kBoxes = false;
     const LmDyn *dyn;
     const float *q;
     LmState k, v;
@@ -495,7 +495,7 @@ struct AtCache {
     VB_DEVINL float4 q4(int row, int head, int d) const {
         return d < dim ? vb_ldcg4(q + ((size_t)row * heads + head) * dim + d) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    VB_DEVINL bool boxes(int j0) const { return lm_ring_row(ring, j0 + kAtKeys - 1) - lm_ring_row(ring, j0) == kAtKeys - 1; }
+    VB_DEVINL bool boxes(int j0, int n) const { return n == kAtKeys && lm_ring_row(ring, j0 + kAtKeys - 1) - lm_ring_row(ring, j0) == kAtKeys - 1; }
     template <int BLOCKS>
     VB_DEVINL void box(const CUtensorMap *map, int size, unsigned char *slot, int g, int j0, uint64_t *bar) const {
         const int row = lm_ring_row(ring, j0);
@@ -544,7 +544,7 @@ struct AtCache {
 /* Every head has keys and values of its own, read out of a latent (LmWide): a head's own columns of the written-out
  * rows, then the key part that all heads share from the latent's cache row. */
 struct AtWide {
-    static constexpr bool kAsync = true, kTma = true;
+    static constexpr bool kBoxes = false;
     const LmDyn *dyn;
     LmWide w;
     LmRing ring;
@@ -570,7 +570,7 @@ struct AtWide {
         }
         return make_float4(e[0], e[1], e[2], e[3]);
     }
-    VB_DEVINL bool boxes(int j0) const { return lm_ring_row(ring, j0 + kAtKeys - 1) - lm_ring_row(ring, j0) == kAtKeys - 1; }
+    VB_DEVINL bool boxes(int j0, int n) const { return n == kAtKeys && lm_ring_row(ring, j0 + kAtKeys - 1) - lm_ring_row(ring, j0) == kAtKeys - 1; }
     template <int BLOCKS>
     VB_DEVINL void tma_keys(const AtArgs &, const AtMaps &m, unsigned char *slot, int g, int j0, uint64_t *bar) const {
         const int own = (dim - w.rot_dim) / 64, row = w.rank + w.rot_dim;

@@ -50,17 +50,42 @@ static int run_row_blocks(VbOp proto, int M, int x_ld, int y_ld, bool res_is_y) 
 
 /* ---- glue kernels of the tensor-core prefill ---- */
 
+/* A layer's keys and values as BF16 halves, [row][KV head][128 high, 128 low]: what the attention reads. */
+struct PfSplit {
+    uint16_t *k, *v;
+};
+VB_DEVINL void pf_split(uint16_t *rows, size_t row, int col, float2 v) {
+    uint32_t hi, lo;
+    at_split2(v.x, v.y, hi, lo);
+    uint32_t *at = reinterpret_cast<uint32_t *>(rows + row * 2 * KVD + (col >> 7) * 256 + (col & 127));
+    at[0] = hi;
+    at[64] = lo;
+}
+/* The cache's earlier rows. One thread per pair of columns; grid = (KVD / 512, rows). */
+__global__ void pf_split_kernel(PfSplit to, const float *kc, const float *vc) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int col = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    const size_t row = blockIdx.y;
+    pf_split(to.k, row, col, __ldcg(reinterpret_cast<const float2 *>(kc + row * KVD + col)));
+    pf_split(to.v, row, col, __ldcg(reinterpret_cast<const float2 *>(vc + row * KVD + col)));
+}
+
 /* QKV of a row block: sums the split-K partials in fixed order, rotates the q and k heads
  * (interleaved pairs, voxtral_tts_kernels.c:616-634), leaves q in `qkv` for the attention
- * and writes k and v straight into the cache rows (voxtral_tts_llm.c:318-330). One thread per
- * pair of columns. */
+ * and writes k and v straight into the cache rows (voxtral_tts_llm.c:318-330) and, split, from row `at` on for the
+ * attention, whose tiles of 64 keys end in rows of zeros. One thread per pair of columns. */
 __global__ void pf_qkv_finish_kernel(float *qkv, const float *part, int n_part, size_t part_stride, const float *cs,
-                                     float *k_rows, float *v_rows, int rows) {
+                                     float *k_rows, float *v_rows, PfSplit split, int at, int rows) {
     pdl_launch_dependents();
     pdl_wait();
     const int m = blockIdx.y;
     const int col = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
-    if (col >= QKV || m >= rows) return;
+    if (col >= QKV) return;
+    if (m >= rows) {
+        if (col >= QD) pf_split(col < QD + KVD ? split.k : split.v, at + m, col < QD + KVD ? col - QD : col - QD - KVD, make_float2(0.0f, 0.0f));
+        return;
+    }
     float2 v = make_float2(0.0f, 0.0f);
     for (int p = 0; p < n_part; p++) {
         const float2 t = __ldcg(reinterpret_cast<const float2 *>(part + (size_t)p * part_stride + (size_t)m * QKV + col));
@@ -74,56 +99,45 @@ __global__ void pf_qkv_finish_kernel(float *qkv, const float *part, int n_part, 
         v.y = a * t.y + b * t.x;
     }
     if (col < QD) *reinterpret_cast<float2 *>(qkv + (size_t)m * QKV + col) = v;
-    else if (col < QD + KVD) *reinterpret_cast<float2 *>(k_rows + (size_t)m * KVD + (col - QD)) = v;
-    else *reinterpret_cast<float2 *>(v_rows + (size_t)m * KVD + (col - QD - KVD)) = v;
+    else if (col < QD + KVD) {
+        *reinterpret_cast<float2 *>(k_rows + (size_t)m * KVD + (col - QD)) = v;
+        pf_split(split.k, at + m, col - QD, v);
+    } else {
+        *reinterpret_cast<float2 *>(v_rows + (size_t)m * KVD + (col - QD - KVD)) = v;
+        pf_split(split.v, at + m, col - QD - KVD, v);
+    }
 }
 
 /* Causal attention of prompt rows over the cache prefix (tts_causal_attention, voxtral_tts_kernels.c:403-465) on the
- * tensor cores (vb_attn_tc.cuh): queries, and the cache's fp32 keys and values, which the loading warps split into BF16
- * halves on the way to shared memory. */
+ * tensor cores (vb_attn_tc.cuh). */
 struct AtRows {
-    static constexpr bool kAsync = false, kTma = false;
-    const float *q, *kc, *vc;
+    static constexpr bool kBoxes = true;
+    const float *q;
     LmSink out;                  /* the terms that the O projection reads */
-    int ldq, ldkv, start_pos;
+    int ldq, start_pos;
     VB_DEVINL void start() {}
     VB_DEVINL int pos0() const { return start_pos; }
     VB_DEVINL float4 q4(int row, int head, int d) const {
         return vb_ldcg4(q + (size_t)row * ldq + head * VB200_HEAD_DIM + d);
     }
-    /* a lane's four columns of 16 rows, eight loads in flight; rows beyond the tile's keys are zeros */
-    VB_DEVINL void rows(const float *cache, unsigned char *slot, int g, int lw, int lane, int j0, int n) const {
-        unsigned char *block = slot + (lane >> 4) * kAtBlock;
-        const float *col = cache + (size_t)(j0 + lw * 16) * ldkv + g * VB200_HEAD_DIM + lane * 4;
+    VB_DEVINL bool boxes(int, int) const { return true; }
+    template <int BLOCKS>
+    VB_DEVINL void box(const CUtensorMap *map, unsigned char *slot, int g, int j0, uint64_t *bar) const {
 #pragma unroll
-        for (int x0 = 0; x0 < 16; x0 += 8) {
-            float4 v[8];
-#pragma unroll
-            for (int x = 0; x < 8; x++)
-                v[x] = lw * 16 + x0 + x < n ? vb_ldcg4(col + (size_t)(x0 + x) * ldkv) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int x = 0; x < 8; x++) {
-                uint2 hi, lo;
-                at_split2(v[x].x, v[x].y, hi.x, lo.x);
-                at_split2(v[x].z, v[x].w, hi.y, lo.y);
-                unsigned char *at = block + at_off(lw * 16 + x0 + x, (lane & 15) >> 1) + (lane & 1) * 8;
-                *reinterpret_cast<uint2 *>(at) = hi;
-                *reinterpret_cast<uint2 *>(at + 2 * kAtBlock) = lo;
-            }
-        }
+        for (int b = 0; b < 2 * BLOCKS; b++) at_tma(slot + b * kAtBlock, map, (g * 2 * BLOCKS + b) * 64, j0, 0, bar);
     }
     template <int BLOCKS>
-    VB_DEVINL void keys(const AtArgs &, unsigned char *slot, int g, int lw, int lane, int j0, int n) const {
-        rows(kc, slot, g, lw, lane, j0, n);
+    VB_DEVINL void tma_keys(const AtArgs &, const AtMaps &m, unsigned char *slot, int g, int j0, uint64_t *bar) const {
+        box<BLOCKS>(&m.k, slot, g, j0, bar);
     }
     template <int BLOCKS>
-    VB_DEVINL void values(const AtArgs &, unsigned char *slot, int g, int lw, int lane, int j0, int n) const {
-        rows(vc, slot, g, lw, lane, j0, n);
+    VB_DEVINL void tma_values(const AtArgs &, const AtMaps &m, unsigned char *slot, int g, int j0, uint64_t *bar) const {
+        box<BLOCKS>(&m.v, slot, g, j0, bar);
     }
     VB_DEVINL float gate(int, int) const { return 1.0f; }
     VB_DEVINL void put4(int row, int c, const float (&e)[4]) const { lm_put4(out, row, c, e); }
 };
-static_assert(VB200_HEAD_DIM == 128, "a lane's four columns cover a head");
+static_assert(VB200_HEAD_DIM == 128, "two blocks of 64 columns");
 
 /* ---- tensor-core prefill ---- */
 /* Rows of a prompt that go through a layer at once: 1203 rows took 33.4 ms in blocks of 256, 23.9 ms in one. */
@@ -143,7 +157,8 @@ struct PrefillTc {
     /* a prompt given as ids and voice rows */
     int *ids = nullptr;
     uint16_t *voice = nullptr;
-    size_t cap[12] = {};
+    PfSplit split = {};          /* of one layer, whole tiles of 64 rows */
+    size_t cap[14] = {};
 };
 static PrefillTc g_pf;
 
@@ -151,7 +166,7 @@ static PrefillTc g_pf;
 void prefill_free_all() {
     PrefillTc &t = g_pf;
     for (void *p : {(void *)t.x, (void *)t.cs, (void *)t.qkv, (void *)t.part, (void *)t.ssq, (void *)t.bD, (void *)t.bQ, (void *)t.bH,
-                    (void *)t.attn, (void *)t.h, (void *)t.ids, (void *)t.voice})
+                    (void *)t.attn, (void *)t.h, (void *)t.ids, (void *)t.voice, (void *)t.split.k, (void *)t.split.v})
         cudaFree(p);
     t = PrefillTc();
 }
@@ -189,8 +204,10 @@ static PfBlock pf_block(int rows) {
     return b;
 }
 
-static int pf_tc_buffers(int M, int block) {
+static int pf_tc_buffers(int M, int start_pos, int block) {
     PrefillTc &t = g_pf;
+    const size_t keys = (size_t)(start_pos + M + kAtKeys - 1) / kAtKeys * kAtKeys;
+    if (pf_grow(12, &t.split.k, keys * 4 * KVD) || pf_grow(13, &t.split.v, keys * 4 * KVD)) return -1;
     /* the last block may be split more ways than a full one */
     size_t part = 0, pad = 0, rows = 0;
     for (int r : {M < block ? M : block, M % block}) {
@@ -228,6 +245,11 @@ static int prefill_tc(float *x, const float *cs, int M, int start_pos, int block
         const PfBlock b = pf_block(rows);
         TcActs aD, aQ, aH;
         if (tc_acts(&aD, t.bD, b.rp, D) || tc_acts(&aQ, t.bQ, b.rp, QD) || tc_acts(&aH, t.bH, b.rp, HID)) return -1;
+        const uint64_t keys = (uint64_t)(start_pos + r0 + rows + kAtKeys - 1) / kAtKeys * kAtKeys;
+        AtMaps maps = {};
+        if (tc_map3(&maps.k, t.split.k, 1, keys * 4 * KVD, keys, 4 * KVD, 2 * KVD, kAtKeys) ||
+            tc_map3(&maps.v, t.split.v, 1, keys * 4 * KVD, keys, 4 * KVD, 2 * KVD, kAtKeys))
+            return -1;
         const LmSink q_terms = {nullptr, t.bQ, b.rp, QD, b.rp < 256 ? kTcTerms : 2};
         const size_t psD = (size_t)rows * D;
         float *xr = x + (size_t)r0 * D;
@@ -239,13 +261,14 @@ static int prefill_tc(float *x, const float *cs, int M, int start_pos, int block
             g.splits = b.s_qkv; g.ssq = t.ssq; g.ssq_chunks = chunksD; g.eps = VB200_NORM_EPS;
             if (tc_gemm(t.wqkv[l], aD, g, st)) return -1;
             float *k0 = m.kv_k + (size_t)l * m.kv_max * KVD, *v0 = m.kv_v + (size_t)l * m.kv_max * KVD;
-            launch_pdl(pf_qkv_finish_kernel, dim3(QKV / 2 / 256, rows), dim3(256), 0, st, t.qkv, (const float *)t.part, b.s_qkv,
-                       (size_t)rows * QKV, cs + (size_t)r0 * VB200_HEAD_DIM, k0 + (size_t)(start_pos + r0) * KVD,
-                       v0 + (size_t)(start_pos + r0) * KVD, rows);
+            const int at = start_pos + r0, tail = (kAtKeys - (at + rows) % kAtKeys) % kAtKeys;
+            if (at > 0) launch_pdl(pf_split_kernel, dim3(KVD / 512, at), dim3(256), 0, st, t.split, (const float *)k0, (const float *)v0);
+            launch_pdl(pf_qkv_finish_kernel, dim3(QKV / 2 / 256, rows + tail), dim3(256), 0, st, t.qkv, (const float *)t.part, b.s_qkv,
+                       (size_t)rows * QKV, cs + (size_t)r0 * VB200_HEAD_DIM, k0 + (size_t)at * KVD, v0 + (size_t)at * KVD, t.split, at, rows);
             if (l == VB200_DEC_LAYERS - 1) break;   /* only the cache is kept (voxtral_tts_llm.c:281) */
-            const AtRows rows_of = {t.qkv, k0, v0, q_terms, QKV, KVD, start_pos + r0};
-            const AtArgs at = {rows, VB200_HEADS, VB200_KV_HEADS, VB200_HEAD_DIM, VB200_HEAD_DIM, 0, 0, scale, 0.0f, &m.d_out->status, 0};
-            if (launch_attn_tc<2, 2>(at, rows_of, st)) return -1;
+            const AtRows rows_of = {t.qkv, q_terms, QKV, at};
+            const AtArgs args = {rows, VB200_HEADS, VB200_KV_HEADS, VB200_HEAD_DIM, VB200_HEAD_DIM, 0, 0, scale, 0.0f, &m.d_out->status, 1};
+            if (launch_attn_tc<2, 2>(args, rows_of, st, maps)) return -1;
             g.splits = b.s_wo; g.ld_out = D; g.ssq = nullptr; g.ssq_chunks = 0;
             if (tc_gemm(t.wo[l], aQ, g, st)) return -1;
             tc_prepare(aD, nullptr, D, rows, t.part, b.s_wo, psD, xr, xr, L.ffn_norm, t.ssq, st);
@@ -296,7 +319,7 @@ static int prefill_run(int M, int start_pos) {
 
     if (t.ready && batch_tiled_decoder(&t.wqkv, &t.wo, &t.w13, &t.w2) == 0) {
         int block = kPfRows;
-        while (pf_tc_buffers(M, block)) {      /* little memory left: smaller blocks */
+        while (pf_tc_buffers(M, start_pos, block)) {      /* little memory left: smaller blocks */
             if (block == 256) return -1;
             block /= 2;
         }
