@@ -27,7 +27,7 @@ struct AcTc {
     TcWeight wqkv[VB200_AC_LAYERS], wo[VB200_AC_LAYERS], w13[VB200_AC_LAYERS], w2[VB200_AC_LAYERS];
     uint16_t *tiled[VB200_AC_LAYERS][4] = {};   /* tile-contiguous weight copies */
     TcWeight wtime;             /* time_proj */
-    int s_qkv = 1;
+    int s_qkv = 1, s_wo = 1, s_w2 = 1;
     AcBuffers one;              /* the single-utterance buffers */
 };
 static AcTc g_ac;
@@ -182,12 +182,12 @@ __global__ void ac_attention_kernel(uint16_t *terms, const float *part, int n_pa
     *reinterpret_cast<uint2 *>(terms + 2 * term + off) = make_uint2(t2[0] | ((uint32_t)t2[1] << 16), t2[2] | ((uint32_t)t2[3] << 16));
 }
 
-/* Final RMSNorm of token 0 of each branch (rows 0 and 3) and the 36-wide
+/* Last residual add where it is due (n_part > 0), final RMSNorm of token 0 of each branch (rows 0 and 3) and the 36-wide
  * velocity head (voxtral_tts_acoustic.c:255-261). grid = (9, 2 * utterances): blockIdx.y =
  * 2 * utterance + branch, four of the 36 outputs per CTA (every CTA re-derives the normalised
  * row; it is 12 KB). */
-__global__ void ac_velocity_kernel(float *vel, const float *X6, const float *gain, float eps, const uint16_t *Wout,
-                                   int vel_stride) {
+__global__ void ac_velocity_kernel(float *vel, const float *X6, const float *part, int n_part, const float *gain,
+                                   float eps, const uint16_t *Wout, int ROWS, int vel_stride) {
     __shared__ float xn[VB200_DIM];
     __shared__ float red[32];
     pdl_launch_dependents();
@@ -203,17 +203,27 @@ __global__ void ac_velocity_kernel(float *vel, const float *X6, const float *gai
     }
     pdl_wait();
     const int row = blockIdx.y * 3;
+    const size_t ps = (size_t)ROWS * D;
     float ss = 0.0f;
-    /* 512 threads x 6 columns; the loads of a thread are issued together */
+    /* 512 threads x 6 columns; the 6 x (n_part + 1) loads of a thread are issued together */
     {
         constexpr int kCols = VB200_DIM / 512;
-        float xv[kCols];
-#pragma unroll
-        for (int i = 0; i < kCols; i++) xv[i] = __ldcg(X6 + (size_t)row * D + threadIdx.x + i * 512);
+        float pv[kCols][kTcMaxSplits], xv[kCols];
 #pragma unroll
         for (int i = 0; i < kCols; i++) {
-            xn[threadIdx.x + i * 512] = xv[i];
-            ss += xv[i] * xv[i];
+            const int c = threadIdx.x + i * 512;
+            xv[i] = __ldcg(X6 + (size_t)row * D + c);
+#pragma unroll
+            for (int p = 0; p < kTcMaxSplits; p++) pv[i][p] = p < n_part ? __ldcg(part + p * ps + (size_t)row * D + c) : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < kCols; i++) {
+            float s = 0.0f;
+#pragma unroll
+            for (int p = 0; p < kTcMaxSplits; p++) s += pv[i][p];     /* split order; unused splits add 0 */
+            const float v = xv[i] + s;
+            xn[threadIdx.x + i * 512] = v;
+            ss += v * v;
         }
     }
     ss = vb_warp_sum(ss);
@@ -345,43 +355,57 @@ int acoustic_tc_setup() {
     o.status = &m.d_out->status;
     if (tc_weight(&t.wtime, m.ac_time_proj, D, D)) return -1;
     t.s_qkv = tc_pick_splits(QKV, D, m.sm_count);
+    t.s_wo = tc_pick_splits(D, QD, m.sm_count);
+    t.s_w2 = tc_pick_splits(D, HID, m.sm_count);
     t.ready = true;
     return 0;
 }
 
 bool acoustic_tc_ready() { return g_ac.ready; }
 
+/* Up to 16 rows the O and down projections finish their sublayers (TcJoin); 18 to 48, of three to eight utterances, leave
+ * partial results for a "prepare" and the velocity head: three rows a warp out of four CTAs' shared memory cost more than
+ * the launch (eight utterances, 24 frames: 118.4 ms joined, 113.8 ms so). */
+static bool joined(int rows) { return rows <= 16; }
+
 /* The layers on the rows in X6, whose terms are not made yet. */
 static int enqueue_layers(const AcBuffers &b, int ROWS) {
+    const bool join = joined(ROWS);
+    const int chunks = join ? D / kTcTileN : tc_prepare_chunks(D);
+    const size_t psD = (size_t)ROWS * D;
     Model &m = model();
     AcTc &t = g_ac;
     cudaStream_t st = m.st;
     const float scale = 1.0f / sqrtf((float)VB200_HEAD_DIM);
     for (int l = 0; l < VB200_AC_LAYERS; l++) {
         const LayerDev &L = m.ac[l];
-        /* attention half: QKV -> attention -> O, which leaves the new rows and the next norm's operand */
+        /* attention half: QKV -> attention -> O */
         if (l == 0) tc_prepare(b.aD, b.X6, D, ROWS, nullptr, 0, 0, nullptr, nullptr, L.attn_norm, b.ssq, st);
+        else if (!join) tc_prepare(b.aD, nullptr, D, ROWS, b.part, t.s_w2, psD, b.X6, b.X6, L.attn_norm, b.ssq, st);
         TcGemm g;
         g.M = ROWS; g.status = b.status;
         g.epi = TC_EPI_PARTIAL; g.out = b.part;
-        g.splits = t.s_qkv; g.ld_out = QKV; g.ssq = b.ssq; g.ssq_chunks = l == 0 ? tc_prepare_chunks(D) : D / kTcTileN;
+        g.splits = t.s_qkv; g.ld_out = QKV; g.ssq = b.ssq; g.ssq_chunks = l == 0 ? tc_prepare_chunks(D) : chunks;
         g.eps = VB200_NORM_EPS;
         if (tc_gemm(t.wqkv[l], b.aD, g, st)) return -1;
         launch_pdl(ac_attention_kernel, dim3((ROWS * VB200_HEADS * 32 + 255) / 256), dim3(256), 0, st, b.bQ,
                    (const float *)b.part, t.s_qkv, scale, ROWS, b.rows_pad);
         g = TcGemm();
         g.M = ROWS; g.status = b.status;
-        g.join = {b.X6, b.X6, L.ffn_norm, b.bD, b.rows_pad, b.ssq, nullptr};
+        g.epi = TC_EPI_PARTIAL; g.out = b.part; g.splits = t.s_wo; g.ld_out = D;
+        if (join) g.join = {b.X6, b.X6, L.ffn_norm, b.bD, b.rows_pad, b.ssq, nullptr};
         if (tc_gemm(t.wo[l], b.aQ, g, st)) return -1;
+        if (!join) tc_prepare(b.aD, nullptr, D, ROWS, b.part, t.s_wo, psD, b.X6, b.X6, L.ffn_norm, b.ssq, st);
         /* FFN half: gate/up with SwiGLU (terms out) -> down */
         g = TcGemm();
         g.M = ROWS; g.status = b.status;
         g.epi = TC_EPI_SWIGLU_TERMS; g.out_terms = b.bH; g.out_rows_pad = b.rows_pad;
-        g.ld_out = HID; g.ssq = b.ssq; g.ssq_chunks = D / kTcTileN; g.eps = VB200_NORM_EPS;
+        g.ld_out = HID; g.ssq = b.ssq; g.ssq_chunks = chunks; g.eps = VB200_NORM_EPS;
         if (tc_gemm(t.w13[l], b.aD, g, st)) return -1;
         g = TcGemm();
         g.M = ROWS; g.status = b.status;
-        g.join = {b.X6, b.X6, l + 1 < VB200_AC_LAYERS ? m.ac[l + 1].attn_norm : nullptr, b.bD, b.rows_pad, b.ssq, nullptr};
+        g.epi = TC_EPI_PARTIAL; g.out = b.part; g.splits = t.s_w2; g.ld_out = D;
+        if (join) g.join = {b.X6, b.X6, l + 1 < VB200_AC_LAYERS ? m.ac[l + 1].attn_norm : nullptr, b.bD, b.rows_pad, b.ssq, nullptr};
         if (tc_gemm(t.w2[l], b.aH, g, st)) return -1;
     }
     return 0;
@@ -402,8 +426,8 @@ int acoustic_tc_enqueue_on(const AcBuffers &b, const float *noise_all, int *code
                    (const uint16_t *)m.ac_input_proj, (const float *)m.ttok, (const float *)b.ltok, s,
                    VB200_CFG_ALPHA, s > 0 ? m.dt[s - 1] : 0.0f, noise_all, (const VbDyn *)b.dyn, b.sd);
         if (enqueue_layers(b, ROWS)) return -1;
-        launch_pdl(ac_velocity_kernel, dim3(9, 2 * b.B), dim3(512), 0, st, b.vel, (const float *)b.X6, (const float *)m.ac_norm,
-                   VB200_NORM_EPS, (const uint16_t *)m.ac_out, b.sd.vel);
+        launch_pdl(ac_velocity_kernel, dim3(9, 2 * b.B), dim3(512), 0, st, b.vel, (const float *)b.X6, (const float *)b.part,
+                   joined(ROWS) ? 0 : t.s_w2, (const float *)m.ac_norm, VB200_NORM_EPS, (const uint16_t *)m.ac_out, ROWS, b.sd.vel);
     }
     launch_pdl(ac_fsq_kernel, dim3(b.B), dim3(64), 0, st, b.codes, b.lat, (const float *)b.vel, steps,
                VB200_FSQ_LEVELS, VB200_CFG_ALPHA, m.dt[steps - 1], codes_all, b.dyn, frame_cap,
@@ -492,8 +516,8 @@ static int enqueue_velocity(const TcWeight *llm) {
     launch_pdl(ac_rows_kernel, dim3((D + 127) / 128), dim3(128), 0, st, b.X6, (const float *)m.d_in->lat[0], (const uint16_t *)m.ac_input_proj,
                (const float *)time_part, (const float *)llm_part, s);
     if (enqueue_layers(b, 3)) return -1;
-    launch_pdl(ac_velocity_kernel, dim3(9, 1), dim3(512), 0, st, b.vel, (const float *)b.X6, (const float *)m.ac_norm, VB200_NORM_EPS,
-               (const uint16_t *)m.ac_out, b.sd.vel);
+    launch_pdl(ac_velocity_kernel, dim3(9, 1), dim3(512), 0, st, b.vel, (const float *)b.X6, (const float *)nullptr, 0, (const float *)m.ac_norm,
+               VB200_NORM_EPS, (const uint16_t *)m.ac_out, 3, b.sd.vel);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 int acoustic_tc_velocity() {

@@ -1261,7 +1261,10 @@ int batch_hidden(float *out) {
     return cudaMemcpy(out, t.hidden, sizeof(float) * t.B * D, cudaMemcpyDeviceToHost) == cudaSuccess ? 0 : -1;
 }
 
-int batch_launches_per_frame() { return 2 + VB200_DEC_LAYERS * 5 + 5 + (VB200_FLOW_STEPS - 1) * (3 + VB200_AC_LAYERS * 5) + 1; }
+int batch_launches_per_frame() {
+    const int prepares = g_bt.open && 6 * g_bt.B > 16 ? 2 * VB200_AC_LAYERS : 1;      /* per Euler step; else its GEMMs do it */
+    return 2 + VB200_DEC_LAYERS * 5 + 5 + (VB200_FLOW_STEPS - 1) * (2 + prepares + VB200_AC_LAYERS * 5) + 1;
+}
 
 /* The decoder's 104 layer GEMMs (QKV, O, gate/up, down x 26 layers: every decoder weight byte
  * once) launched back to back on the stream, `iters` times, between two events: the GEMM
