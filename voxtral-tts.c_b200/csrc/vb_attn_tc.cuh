@@ -16,8 +16,10 @@
  *
  * Warps: 0-3, 4-7 softmax, 8-11 bring keys and 12-13 values into two rings, 14 issues the MMAs. All waits are bounded.
  *
- * What bounds it: a 64-key tile of 128-wide heads costs the tensor pipe 8 x 3 x 32 + 4 x 3 x 64 = 1536 clocks and the
- * softmax about as much; the warp-level MMAs used before (mma.sync, 16 rows per warp) ran at 44 useful TFLOP/s.
+ * What bounds it, by a timeline on the device: the S products, 24 MMAs of 64 columns a tile at 77 clocks (36 of 65 for
+ * heads of 192), which is what MMAs of 128 columns take too, then P . V, 12 at 60; 3300 and 4000 clocks a tile. 2048 rows,
+ * window 1024, 32 heads: 128 on 8 KV heads 588 us on warp-level MMAs (mma.sync, 16 rows a warp, 44 useful TFLOP/s), 201 with
+ * tiles copied 16 bytes a lane, 164 now; 192 + 128 each with its own 830, 282, 225 us.
  */
 #ifndef VB_ATTN_TC_CUH
 #define VB_ATTN_TC_CUH

@@ -11,8 +11,8 @@
  *         -> causal conv 1024 -> 240, kernel 7 -> [8T, 240] = the waveform
  *
  * Rows stay row-major [time, channel] throughout (the reference transposes to channel-first
- * around every convolution). The transformer linears run on the tensor-core row-block GEMM
- * (vb_tc.cu) with BF16 weights - exact, because the checkpoint's BF16 values were only widened to
+ * around every convolution). The transformer linears run on the tensor-core GEMMs
+ * (vb_tc.cu, vb_tc_rows.cu) with BF16 weights - exact, because the checkpoint's BF16 values were only widened to
  * fp32 by the loader - and the activations as hi + lo BF16 terms. A convolution is a GEMM too,
  *   C[t][oc] = bias[oc] + sum over taps and input channels of X[src(t, tap)][ic] * W[oc][tap][ic],
  * and a stride-2 transposed convolution is one with both output parities as columns,

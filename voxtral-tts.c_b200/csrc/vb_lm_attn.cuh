@@ -108,13 +108,6 @@ VB_DEVINL void ldsm_t(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
-/* Byte offset of the 16-byte chunk `chunk` of key row `key` in a [keys][16 * STEPS] BF16 tile; chunks are
- * XOR-swizzled by the key so that eight rows of one chunk column hit eight different banks. */
-template <int STEPS>
-VB_DEVINL uint32_t tile_off(int key, int chunk) {
-    return (uint32_t)(key * STEPS * 32 + (((chunk & ~7) | ((chunk ^ key) & 7)) << 4));
-}
-
 VB_DEVINL void lm_cp16(void *smem_dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(vb_smem_u32(smem_dst)), "l"(src) : "memory");
 }
