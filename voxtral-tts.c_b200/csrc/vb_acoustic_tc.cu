@@ -26,7 +26,7 @@ struct AcTc {
     bool ready = false;
     TcWeight wqkv[VB200_AC_LAYERS], wo[VB200_AC_LAYERS], w13[VB200_AC_LAYERS], w2[VB200_AC_LAYERS];
     uint16_t *tiled[VB200_AC_LAYERS][4] = {};   /* tile-contiguous weight copies */
-    TcWeight wtime;             /* time_proj */
+    TcWeight wtime, wllm;       /* time_proj and llm_proj of a single velocity call, row-major as uploaded */
     int s_qkv = 1, s_wo = 1, s_w2 = 1;
     AcBuffers one;              /* the single-utterance buffers */
 };
@@ -353,7 +353,7 @@ int acoustic_tc_setup() {
     o.codes = m.d_out->codes;
     o.dyn = &m.d_in->dyn;
     o.status = &m.d_out->status;
-    if (tc_weight(&t.wtime, m.ac_time_proj, D, D)) return -1;
+    if (tc_weight(&t.wtime, m.ac_time_proj, D, D) || tc_weight(&t.wllm, m.ac_llm_proj, D, D)) return -1;
     t.s_qkv = tc_pick_splits(QKV, D, m.sm_count);
     t.s_wo = tc_pick_splits(D, QD, m.sm_count);
     t.s_w2 = tc_pick_splits(D, HID, m.sm_count);
@@ -452,7 +452,6 @@ struct GraphSlot {
 };
 static GraphSlot g_slots[2];
 static GraphSlot g_velocity;
-static const uint16_t *g_velocity_llm = nullptr;      /* the llm_proj in its launches */
 
 void acoustic_tc_drop_graphs() {
     for (GraphSlot *s : {&g_slots[0], &g_slots[1], &g_velocity}) {
@@ -497,8 +496,8 @@ static int run_slot(GraphSlot &s, const F &enqueue) {
 }
 
 /* One velocity call on what lies in d_in (latent 0, hidden state, time embedding): 21 launches, against the streaming
- * GEMV kernel's one of 0.25 ms; 0.17 ms. 1: not on this path. */
-static int enqueue_velocity(const TcWeight *llm) {
+ * GEMV kernel's one of 0.25 ms; 0.17 ms. */
+static int enqueue_velocity() {
     Model &m = model();
     AcTc &t = g_ac;
     const AcBuffers &b = t.one;
@@ -512,7 +511,7 @@ static int enqueue_velocity(const TcWeight *llm) {
     g.out = time_part;
     if (tc_gemm(t.wtime, b.aD, g, st)) return -1;
     g.out = llm_part;
-    if (tc_gemm(*llm, b.aD, g, st)) return -1;
+    if (tc_gemm(t.wllm, b.aD, g, st)) return -1;
     launch_pdl(ac_rows_kernel, dim3((D + 127) / 128), dim3(128), 0, st, b.X6, (const float *)m.d_in->lat[0], (const uint16_t *)m.ac_input_proj,
                (const float *)time_part, (const float *)llm_part, s);
     if (enqueue_layers(b, 3)) return -1;
@@ -520,16 +519,9 @@ static int enqueue_velocity(const TcWeight *llm) {
                VB200_NORM_EPS, (const uint16_t *)m.ac_out, 3, b.sd.vel);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
-int acoustic_tc_velocity() {
-    const TcWeight *llm = batch_llm_proj();
-    if (!g_ac.ready || !g_ac.wtime.ok || !llm) return 1;
-    if (g_velocity_llm != llm->W) {        /* the decoder's weights were uploaded anew */
-        if (g_velocity.exec) cudaGraphExecDestroy(g_velocity.exec);
-        g_velocity = GraphSlot();
-        g_velocity_llm = llm->W;
-    }
-    return run_slot(g_velocity, [&] { return enqueue_velocity(llm); });
-}
+/* 1: not on this path. It reads what the acoustic upload left and nothing of the decoder: llm_proj out of the frame's
+ * tile-contiguous matrices cost a program without a prefill those of the whole decoder, 6 GB, at its first call. */
+int acoustic_tc_velocity() { return g_ac.ready ? run_slot(g_velocity, enqueue_velocity) : 1; }
 
 int acoustic_tc_enqueue(const float *noise_all, int *codes_all, int frame_cap, bool advance, bool ignore_end) {
     GraphSlot &s = g_slots[advance ? 1 : 0];

@@ -616,9 +616,6 @@ static int bt_weights() {
     return 0;
 }
 
-/* The tile-contiguous llm_proj, or null. */
-const TcWeight *batch_llm_proj() { return model().ac_ready && model().llm_ready && bt_weights() == 0 ? &g_w.wllm : nullptr; }
-
 /* The decoder's tile-contiguous matrices for the prefill: [26] each, in layer order. */
 int batch_tiled_decoder(const TcWeight **wqkv, const TcWeight **wo, const TcWeight **w13, const TcWeight **w2) {
     if (!model().llm_ready || bt_weights()) return -1;

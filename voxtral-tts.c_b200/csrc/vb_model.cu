@@ -707,8 +707,8 @@ int predict_velocity(float *out_v, const float *x_t, const float *hidden, float 
         m.h_in->temb[D / 2 + k] = sinf(ang);
     }
     VB_CHECK(cudaMemcpyAsync(m.d_in, m.h_in, sizeof(DevIn), cudaMemcpyHostToDevice, m.st));
-    /* the launches of an Euler step on three rows; the streaming kernel serves when that path is off, when there are no
-     * decoder weights, and while launches are timed one by one */
+    /* the launches of an Euler step on three rows; the streaming kernel serves when that path is off, and while launches
+     * are timed one by one */
     const int rc = m.timing ? 1 : acoustic_tc_velocity();
     if (rc < 0 || (rc > 0 && run_program(m.p_pv))) return -1;
     if (finish(sizeof(DevOut))) return -1;

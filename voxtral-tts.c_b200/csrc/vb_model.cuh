@@ -159,7 +159,6 @@ void tp_close();
 void batch_close();
 void batch_invalidate();
 struct TcWeight;
-const TcWeight *batch_llm_proj();
 int batch_tiled_decoder(const TcWeight **wqkv, const TcWeight **wo, const TcWeight **w13, const TcWeight **w2);
 void batch_options_changed();
 void single_path_changed();
