@@ -37,6 +37,31 @@ def velocity():
     assert np.array_equal(calls(), alone)                                 # the same launches on the same weights
 
 
+def take(eng, leave):
+    """All of the device's memory but `leave` bytes."""
+    p = eng.L.tts_cuda_alloc(free_bytes() - leave)
+    assert p and free_bytes() < leave + 64 * MB
+    return p
+
+
+def copies():
+    """A prefill that finds no room for the decoder's tile-contiguous copies does without, and keeps none of them."""
+    eng = pkg.Engine(kv_cache_max=64)
+    eng.upload(pkg.SynthModel(seed=77, acoustic=False, audio_table=False, dec_layers=1), decoder=True, acoustic=False)
+    x = pkg.synth_f32((9, 3072), 5, "mem.rows", 0.0, 0.5)
+    full = take(eng, 2048 * MB)
+    before, rows = free_bytes(), []
+    for _ in range(2):
+        eng.prefill(x, 0)
+        assert before - free_bytes() < 64 * MB, (before, free_bytes())
+        rows.append(np.stack([eng.kv_read(l, 0, 9) for l in (0, 25)]))
+    assert np.array_equal(*rows)
+    eng.L.tts_cuda_free_ptr(full)
+    eng.prefill(x, 0)
+    got = np.stack([eng.kv_read(l, 0, 9) for l in (0, 25)])
+    assert np.linalg.norm(got - rows[0]) < 1e-4 * np.linalg.norm(got)     # sums in other orders
+
+
 if __name__ == "__main__":
-    {"velocity": velocity}[sys.argv[1]]()
+    {"velocity": velocity, "copies": copies}[sys.argv[1]]()
     print("OK")

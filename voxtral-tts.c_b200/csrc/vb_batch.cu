@@ -584,14 +584,9 @@ static void drop_graphs(Batch &t) {
     }
 }
 
-/* Tile-contiguous copies of the decoder's matrices and of the two heads, made once per
- * weight upload. */
-static int bt_weights() {
+static int bt_make_weights() {
     Model &m = model();
     BtWeights &w = g_w;
-    if (w.ready) return 0;
-    if (tc_init()) return -1;
-    bt_free(&w.allocs);
     auto tiled = [&](TcWeight *tw, const uint16_t *src, int N, int K) -> int {
         void *dst = nullptr;
         if (bt_alloc(&dst, tc_tiled_bytes(N, K), &w.allocs)) return -1;
@@ -612,8 +607,19 @@ static int bt_weights() {
     w.s_w2 = tc_pick_splits(D, HID, m.sm_count);
     w.s_sem = tc_pick_splits(NSEM, D, m.sm_count);
     w.s_llm = tc_pick_splits(D, D, m.sm_count);
-    w.ready = true;
     return 0;
+}
+
+/* Tile-contiguous copies of the decoder's matrices and of the two heads, made once per weight upload. All of them or
+ * none: what there was room for goes back, so that a call which does without them leaves the device as it found it. */
+static int bt_weights() {
+    BtWeights &w = g_w;
+    if (w.ready) return 0;
+    if (tc_init()) return -1;
+    bt_free(&w.allocs);
+    w.ready = bt_make_weights() == 0;
+    if (!w.ready) bt_free(&w.allocs);
+    return w.ready ? 0 : -1;
 }
 
 /* The decoder's tile-contiguous matrices for the prefill: [26] each, in layer order. */
