@@ -62,6 +62,26 @@ def copies():
     assert np.linalg.norm(got - rows[0]) < 1e-4 * np.linalg.norm(got)     # sums in other orders
 
 
+def far():
+    """Prompt rows behind more cache rows than a grid's y axis has places, against the decoder step row by row. The earlier
+    rows that count are a few on both sides: keys large enough that the zeros between them have no weight. Scores of up
+    to 20 as two-term products (2^-16 of a product's size) set the limit."""
+    first, n = 65537, 3
+    eng = pkg.Engine(kv_cache_max=first + 63)
+    eng.upload(pkg.SynthModel(seed=77, acoustic=False, audio_table=False, dec_layers=2), decoder=True, acoustic=False)
+    for at in (0, first - 100):
+        for l in range(26):
+            eng.kv_write(l, at, pkg.synth_f32((100, 1024), 100 * l + 1, f"far.k{at}", 0.0, 5.0), pkg.synth_f32((100, 1024), 100 * l + 2, f"far.v{at}"))
+    x = pkg.synth_f32((n, 3072), 5, "far.rows", 0.0, 0.5)
+    eng.prefill(x, first)
+    got = [eng.kv_read(l, first, n) for l in (0, 1, 25)]
+    for i in range(n):
+        eng.llm_forward(x[i], first + i)
+    for l, (k, v) in zip((0, 1, 25), got):
+        k2, v2 = eng.kv_read(l, first, n)
+        assert np.linalg.norm(k - k2) < 1e-3 * np.linalg.norm(k2) and np.linalg.norm(v - v2) < 1e-3 * np.linalg.norm(v2), l
+
+
 if __name__ == "__main__":
-    {"velocity": velocity, "copies": copies}[sys.argv[1]]()
+    {"velocity": velocity, "copies": copies, "far": far}[sys.argv[1]]()
     print("OK")

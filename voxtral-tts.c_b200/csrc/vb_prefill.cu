@@ -61,12 +61,13 @@ VB_DEVINL void pf_split(uint16_t *rows, size_t row, int col, float2 v) {
     at[0] = hi;
     at[64] = lo;
 }
-/* The cache's earlier rows. One thread per pair of columns; grid = (KVD / 512, rows). */
+/* The cache's earlier rows. One thread per pair of columns; grid = (rows, KVD / 512): a cache has more rows than a grid's
+ * y axis (65535). */
 __global__ void pf_split_kernel(PfSplit to, const float *kc, const float *vc) {
     pdl_launch_dependents();
     pdl_wait();
-    const int col = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
-    const size_t row = blockIdx.y;
+    const int col = 2 * (blockIdx.y * blockDim.x + threadIdx.x);
+    const size_t row = blockIdx.x;
     pf_split(to.k, row, col, __ldcg(reinterpret_cast<const float2 *>(kc + row * KVD + col)));
     pf_split(to.v, row, col, __ldcg(reinterpret_cast<const float2 *>(vc + row * KVD + col)));
 }
@@ -262,9 +263,12 @@ static int prefill_tc(float *x, const float *cs, int M, int start_pos, int block
             if (tc_gemm(t.wqkv[l], aD, g, st)) return -1;
             float *k0 = m.kv_k + (size_t)l * m.kv_max * KVD, *v0 = m.kv_v + (size_t)l * m.kv_max * KVD;
             const int at = start_pos + r0, tail = (kAtKeys - (at + rows) % kAtKeys) % kAtKeys;
-            if (at > 0) launch_pdl(pf_split_kernel, dim3(KVD / 512, at), dim3(256), 0, st, t.split, (const float *)k0, (const float *)v0);
-            launch_pdl(pf_qkv_finish_kernel, dim3(QKV / 2 / 256, rows + tail), dim3(256), 0, st, t.qkv, (const float *)t.part, b.s_qkv,
-                       (size_t)rows * QKV, cs + (size_t)r0 * VB200_HEAD_DIM, k0 + (size_t)at * KVD, v0 + (size_t)at * KVD, t.split, at, rows);
+            if (at > 0 && launch_pdl(pf_split_kernel, dim3(at, KVD / 512), dim3(256), 0, st, t.split, (const float *)k0, (const float *)v0) != cudaSuccess)
+                return -1;
+            if (launch_pdl(pf_qkv_finish_kernel, dim3(QKV / 2 / 256, rows + tail), dim3(256), 0, st, t.qkv, (const float *)t.part, b.s_qkv,
+                           (size_t)rows * QKV, cs + (size_t)r0 * VB200_HEAD_DIM, k0 + (size_t)at * KVD, v0 + (size_t)at * KVD, t.split, at,
+                           rows) != cudaSuccess)
+                return -1;
             if (l == VB200_DEC_LAYERS - 1) break;   /* only the cache is kept (voxtral_tts_llm.c:281) */
             const AtRows rows_of = {t.qkv, q_terms, QKV, at};
             const AtArgs args = {rows, VB200_HEADS, VB200_KV_HEADS, VB200_HEAD_DIM, VB200_HEAD_DIM, 0, 0, scale, 0.0f, &m.d_out->status, 1};
