@@ -82,6 +82,32 @@ def far():
         assert np.linalg.norm(k - k2) < 1e-3 * np.linalg.norm(k2) and np.linalg.norm(v - v2) < 1e-3 * np.linalg.norm(v2), l
 
 
+def short():
+    """A prompt with less and less memory left: smaller blocks of rows, then the streaming kernel; the same cache rows, up to
+    the order of sums and 16-bit halves, as with room for all."""
+    n, small = 600, 200
+    eng = pkg.Engine(kv_cache_max=640)
+    eng.upload(pkg.SynthModel(seed=77, acoustic=False, audio_table=False, dec_layers=2), decoder=True, acoustic=False)
+    x = pkg.synth_f32((n, 3072), 5, "short.rows", 0.0, 0.5)
+
+    def rows(m):
+        eng.kv_write(25, 0, np.zeros((n, 1024), np.float32), np.zeros((n, 1024), np.float32))
+        eng.prefill(x[:m], 0)
+        return np.concatenate(eng.kv_read(25, 0, m), axis=1)
+
+    eng.prefill(x[:5], 0)                             # the decoder's copies are made
+    full, got = take(eng, 200 * MB), []
+    for leave, m in ((30, small), (60, small), (100, n), (130, n), (200, n)):
+        eng.L.tts_cuda_free_ptr(full)
+        full = take(eng, leave * MB)
+        got.append((leave, rows(m)))
+    eng.L.tts_cuda_free_ptr(full)
+    want = rows(n)
+    for leave, g in got:
+        w = want[:len(g)]
+        assert np.linalg.norm(g - w) < 1e-4 * np.linalg.norm(w), (leave, len(g))
+
+
 if __name__ == "__main__":
-    {"velocity": velocity, "copies": copies, "far": far}[sys.argv[1]]()
+    {"velocity": velocity, "copies": copies, "far": far, "short": short}[sys.argv[1]]()
     print("OK")

@@ -4,9 +4,8 @@
  * 26 layers, K and V of every row land in the cache, hidden states are dropped.
  *
  * The linears run on the tensor-core GEMMs (vb_tc.cu, vb_tc_rows.cu; fp32 rows as three or two BF16 terms) in
- * blocks of rows, the causal attention on the tensor cores too (vb_attn_tc.cuh). When the tensor maps cannot be made
- * the same layer loop runs
- * on the streaming engine, eight rows at a time. Also here: the prompt assembled on
+ * blocks of rows, the causal attention on the tensor cores too (vb_attn_tc.cuh). When the tensor maps cannot be made or
+ * there is no memory for a block's operands, the same layer loop runs on the streaming engine, eight rows at a time. Also here: the prompt assembled on
  * the device from token ids and BF16 voice rows (voxtral_tts.c:230-272).
  */
 #include "vb_attn_tc.cuh"
@@ -190,6 +189,16 @@ static int pf_grow(int i, T **p, size_t bytes) {
     return cudaMemsetAsync(*p, 0, bytes, model().st) == cudaSuccess ? 0 : -1;
 }
 
+/* What a block of rows needs beside the rows themselves goes back. */
+static void pf_release_block() {
+    PrefillTc &t = g_pf;
+    cudaFree(t.qkv); cudaFree(t.part); cudaFree(t.ssq); cudaFree(t.bD); cudaFree(t.bQ); cudaFree(t.bH); cudaFree(t.split.k); cudaFree(t.split.v);
+    t.qkv = t.part = t.ssq = nullptr;
+    t.bD = t.bQ = t.bH = nullptr;
+    t.split = PfSplit();
+    for (int i : {2, 3, 4, 5, 6, 7, 12, 13}) t.cap[i] = 0;
+}
+
 /* Padded rows of a block, and the K splits of its GEMMs. */
 struct PfBlock {
     int rows, rp, s_qkv, s_wo, s_w2;
@@ -223,6 +232,16 @@ static int pf_tc_buffers(int M, int start_pos, int block) {
                    pf_grow(7, &t.bH, tc_acts_bytes((int)pad, HID))
                ? -1
                : 0;
+}
+
+/* Rows that go through a layer at once, with buffers for them: fewer where little memory is left; 0: the streaming
+ * kernel, which takes a third of what a block of 256 rows takes here. */
+static int pf_fit(int M, int start_pos) {
+    for (int block = kPfRows; block >= 256; block /= 2) {
+        if (pf_tc_buffers(M, start_pos, block) == 0) return block;
+        pf_release_block();
+    }
+    return 0;
 }
 
 /* Failing here is not fatal: prefill() then uses the streaming kernel. */
@@ -321,12 +340,8 @@ static int prefill_run(int M, int start_pos) {
     int rc = 0;
     const float scale = 1.0f / sqrtf((float)VB200_HEAD_DIM);
 
-    if (t.ready && batch_tiled_decoder(&t.wqkv, &t.wo, &t.w13, &t.w2) == 0) {
-        int block = kPfRows;
-        while (pf_tc_buffers(M, start_pos, block)) {      /* little memory left: smaller blocks */
-            if (block == 256) return -1;
-            block /= 2;
-        }
+    const int block = t.ready && batch_tiled_decoder(&t.wqkv, &t.wo, &t.w13, &t.w2) == 0 ? pf_fit(M, start_pos) : 0;
+    if (block > 0) {
         rc = prefill_tc(x, cs, M, start_pos, block);
         int status = 0;
         if (cudaMemcpyAsync(&status, &m.d_out->status, sizeof(int), cudaMemcpyDeviceToHost, m.st) != cudaSuccess ||
