@@ -108,6 +108,29 @@ def short():
         assert np.linalg.norm(g - w) < 1e-4 * np.linalg.norm(w), (leave, len(g))
 
 
+def blocks():
+    """A prompt of more rows than go through a layer at once: the same bits as those blocks in calls of their own, and up to
+    the order of sums the rows of calls cut elsewhere."""
+    eng = pkg.Engine(kv_cache_max=4500)
+    eng.upload(pkg.SynthModel(seed=77, acoustic=False, audio_table=False, dec_layers=2), decoder=True, acoustic=False)
+    for n, calls in ((2300, (2048, 252)), (2048 + 40, (2048, 40)), (2048 + 256 + 9, (2048, 256, 9)), (4400, (2048, 2048, 304 - 48, 48))):
+        x = pkg.synth_f32((n, 3072), 5, "blocks.rows", 0.0, 0.5)
+
+        def rows(sizes):
+            at = 0
+            for m in sizes:
+                eng.prefill(x[at:at + m], at)
+                at += m
+            assert at == n
+            return np.stack([np.concatenate(eng.kv_read(l, 0, n), axis=1) for l in (0, 1, 25)])
+
+        whole = rows((n,))
+        assert np.array_equal(rows(calls), whole), calls
+        other = rows((700, n - 700))
+        for l in range(3):
+            assert np.linalg.norm(other[l] - whole[l]) < 1e-4 * np.linalg.norm(whole[l]), (n, l)
+
+
 if __name__ == "__main__":
-    {"velocity": velocity, "copies": copies, "far": far, "short": short}[sys.argv[1]]()
+    {"velocity": velocity, "copies": copies, "far": far, "short": short, "blocks": blocks}[sys.argv[1]]()
     print("OK")

@@ -78,3 +78,17 @@ def test_prefill_attention_tiles(pkg, engine, synth_model, first, rows):
     for (k1, v1), l in zip(whole, (0, 1, 25)):
         k2, v2 = engine.kv_read(l, 0, first + rows)
         assert np.linalg.norm(k2 - k1) < 1e-4 * np.linalg.norm(k1) and np.linalg.norm(v2 - v1) < 1e-4 * np.linalg.norm(v1), l
+
+
+@pytest.mark.parametrize("rows", [257, 300, 320])
+def test_prefill_last_rows_keep_three_terms(pkg, engine, synth_model, rows):
+    """Up to 64 rows behind a multiple of 256 are multiplied with all the bits that 64 rows alone are: the same bits come
+    out as from a call of their own."""
+    x = pkg.synth_f32((rows, 3072), 52, "last.rows", 0.0, 0.5)
+    engine.prefill(x, 0)
+    whole = [engine.kv_read(l, 0, rows) for l in (0, 1, 25)]
+    engine.prefill(x[:256], 0)
+    engine.prefill(x[256:], 256)
+    for (k1, v1), l in zip(whole, (0, 1, 25)):
+        k2, v2 = engine.kv_read(l, 0, rows)
+        assert np.array_equal(k2, k1) and np.array_equal(v2, v1), l

@@ -214,14 +214,23 @@ static PfBlock pf_block(int rows) {
     return b;
 }
 
+/* Rows of the next block when so many are left: all of them, but 1 to 64 behind a multiple of 256 go alone, for up to 64 rows
+ * are multiplied as three terms (24 bits) and more as two (16). 300 rows take 6.7 ms for it, 5.0 as one block of two
+ * terms; 1300 rows 18.3 and 16.4. */
+static int pf_next_rows(int left, int block) {
+    if (left > block) return block;
+    const int tail = left % 256;
+    return left > 256 && tail >= 1 && tail <= 64 ? left - tail : left;
+}
+
 static int pf_tc_buffers(int M, int start_pos, int block) {
     PrefillTc &t = g_pf;
     const size_t keys = (size_t)(start_pos + M + kAtKeys - 1) / kAtKeys * kAtKeys;
     if (pf_grow(12, &t.split.k, keys * 4 * KVD) || pf_grow(13, &t.split.v, keys * 4 * KVD)) return -1;
-    /* the last block may be split more ways than a full one */
+    /* a last block may be split more ways than a full one */
     size_t part = 0, pad = 0, rows = 0;
-    for (int r : {M < block ? M : block, M % block}) {
-        if (r == 0) continue;
+    for (int left = M, r; left > 0; left -= r) {
+        r = pf_next_rows(left, block);
         const PfBlock b = pf_block(r);
         for (size_t n : {(size_t)b.s_qkv * r * QKV, (size_t)b.s_wo * r * D, (size_t)b.s_w2 * r * D}) part = n > part ? n : part;
         pad = (size_t)b.rp > pad ? b.rp : pad;
@@ -260,8 +269,8 @@ static int prefill_tc(float *x, const float *cs, int M, int start_pos, int block
     const float scale = 1.0f / sqrtf((float)VB200_HEAD_DIM);
     const int chunksD = tc_prepare_chunks(D);
     /* the row blocks follow one another through all layers: a row sees nothing of later rows */
-    for (int r0 = 0; r0 < M; r0 += block) {
-        const int rows = M - r0 < block ? M - r0 : block;
+    for (int r0 = 0, rows; r0 < M; r0 += rows) {
+        rows = pf_next_rows(M - r0, block);
         const PfBlock b = pf_block(rows);
         TcActs aD, aQ, aH;
         if (tc_acts(&aD, t.bD, b.rp, D) || tc_acts(&aQ, t.bQ, b.rp, QD) || tc_acts(&aH, t.bH, b.rp, HID)) return -1;
