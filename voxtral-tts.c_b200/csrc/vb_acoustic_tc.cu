@@ -439,7 +439,7 @@ static int enqueue_direct(const float *noise_all, int *codes_all, int frame_cap,
     return acoustic_tc_enqueue_on(g_ac.one, noise_all, codes_all, frame_cap, advance, ignore_end);
 }
 
-/* The ~200 launches of a frame are captured once per argument set as a CUDA graph and
+/* The 127 launches of a frame are captured once per argument set as a CUDA graph and
  * replayed; the first call with a new argument set runs directly (it also sets the
  * kernels' shared-memory attributes, which must not happen inside a capture). */
 struct GraphSlot {

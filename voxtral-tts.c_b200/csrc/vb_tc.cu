@@ -1,26 +1,25 @@
 /*
- * vb_tc.cu - tcgen05 / TMEM / TMA skinny GEMM (sm_100a) for M >= 2 activation rows:
- * the acoustic transformer's CFG-batched passes (M = 6) and the prompt prefill.
+ * vb_tc.cu - tcgen05 / TMEM / TMA skinny GEMM (sm_100a) for up to 64 activation rows: the frame's decoder step and
+ * acoustic passes, short prompts, the language models' steps. (More rows: vb_tc_rows.cu.)
  *
  *   y[M,N] = x[M,K] . W[N,K]^T, BF16 W, fp32 x and y (tts_linear_nobias_bf16 with
  *   seq_len > 1, voxtral_tts_kernels.c:187-198, which the reference runs as
  *   weight expansion + SGEMM).
  *
- * Swap-AB: a 128-row weight tile is the UMMA A operand (K-major, 128-byte swizzle,
- * brought in by 2-D TMA), the activation rows are the narrow B operand (UMMA N =
- * 16 / 64 / 256), the fp32 accumulator tile [128 x N] sits in TMEM. The kernel is
- * HBM-bound (every weight byte is read once); tensor work is a few percent.
+ * Swap-AB: a 128-row weight tile is the UMMA A operand (K-major, 128-byte swizzle, brought in by 2-D TMA), the
+ * activation rows are the narrow B operand (tiles of 16, 48 or 64 rows, their three terms side by side: UMMA N = 48,
+ * 144, 192), the fp32 accumulator tile [128 x N] sits in TMEM. The kernel is HBM-bound (every weight byte is read once);
+ * tensor work is a few percent.
  *
- * fp32 fidelity: the reference multiplies fp32 activations by exactly expanded
- * BF16 weights. Each activation is split into three BF16 terms, x = hi + lo + lo2
- * (8 + 8 + 8 mantissa bits), and the three MMAs accumulate into the same TMEM
- * tile; BF16 x BF16 products are exact in fp32, so only the summation order
- * differs from the reference.
+ * fp32 fidelity: the reference multiplies fp32 activations by exactly expanded BF16 weights. Each activation is split
+ * into three BF16 terms, x = hi + lo + lo2 (8 + 8 + 8 mantissa bits), whose products with the weights are summed apart in
+ * TMEM and added up by the epilogue; BF16 x BF16 products are exact in fp32, so only the summation differs from the
+ * reference.
  *
- * Warp roles: warps 0-3 epilogue (TMEM lanes 32w..32w+31 -> registers -> global),
- * warp 4 lane 0 TMA producer, warp 5 lane 0 MMA issuer. No cluster, no multicast.
- * All waits are bounded; on expiry a status word is set, every role falls through,
- * and the TMEM columns are released before the CTA exits.
+ * Warp roles: warps 0-3 epilogue (TMEM lanes 32w..32w+31 -> registers -> global), warp 4 lane 0 TMA producer, warp 5
+ * lane 0 MMA issuer. The GEMMs that end a sublayer (TcJoin) run in clusters of kTcJoinSplits CTAs, the others without;
+ * no multicast. All waits are bounded; on expiry a status word is set, every role falls through, and the TMEM columns
+ * are released before the CTA exits.
  */
 #include "vb_tc.cuh"
 #include "vb_common.cuh"
@@ -175,14 +174,13 @@ struct TcCfg {
     static constexpr int kStageA = kTcTileN * kTcBlockK * 2;        /* 16 KB */
     static constexpr int kTermB = NB * kTcBlockK * 2;               /* one BF16 term of the activations */
     static constexpr int kStage = kStageA + kTcTerms * kTermB;
-    static constexpr int kStages = ST;   /* NB=16: several CTAs fit one SM, so the next GEMMs of the stream fetch their first weight tiles under the tail of the running one */
-    /* The three BF16 terms of the activations lie one after another in a stage, so for
-     * NB <= 64 they form ONE B operand of 3*NB rows: a single MMA per 16-wide K step writes the
-     * three partial products to separate TMEM column groups (summed in the epilogue) instead of
-     * three narrow MMAs - the narrow ones are issue-latency bound, not throughput bound. */
-    static constexpr bool kFusedTerms = (kTcTerms * NB) <= 256;
-    static constexpr int kMmaN = kFusedTerms ? kTcTerms * NB : NB;
-    static constexpr int kAccCols = kFusedTerms ? kTcTerms * NB : NB;
+    static constexpr int kStages = ST;   /* one CTA per SM: rings small enough for two cost more than the overlap gave (212 frames: 611 ms and more for 594) */
+    /* The three BF16 terms of the activations lie one after another in a stage, so that they
+     * form ONE B operand of 3*NB rows: a single MMA per 16-wide K step writes the three partial
+     * products to separate TMEM column groups (summed in the epilogue) instead of three narrow
+     * MMAs - the narrow ones are issue-latency bound, not throughput bound. */
+    static constexpr int kAccCols = kTcTerms * NB;
+    static_assert(kAccCols <= 256, "wider than an MMA");
     static constexpr int kTmemCols = kAccCols <= 32 ? 32 : kAccCols <= 64 ? 64 : kAccCols <= 128 ? 128 : 256;
     static constexpr int kSmemBytes = kStages * kStage + 1024 /* alignment slack */ + 256 /* barriers */ + 4 * NB;
     static_assert(kSmemBytes <= 232448, "over the 227 KB a CTA may use");
@@ -204,7 +202,6 @@ struct TcKernelArgs {
     int *status;
     int tile0;               /* first output tile of this launch */
     int n_tiles_launch;      /* tiles this launch covers (host side: the grid) */
-    int act_n0, out_terms_ld, out_col0;   /* row-block kernel: TC_EPI_TERMS, TC_EPI_RELU2_TERMS */
 };
 
 /* Tensor parallelism is a separate instantiation of every kernel that takes part in it, with
@@ -345,7 +342,7 @@ vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
         }
     } else if (warp == 5 && lane == 0) {
         /* ---- MMA issuer ---- */
-        const uint32_t idesc = umma_idesc_bf16(Cfg::kMmaN);
+        const uint32_t idesc = umma_idesc_bf16(Cfg::kAccCols);
         bool ok = true;
         for (int it = 0; it < n_it && ok; it++) {
             const int s = it % Cfg::kStages, use = it / Cfg::kStages;
@@ -359,20 +356,10 @@ vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
             const unsigned char *sa = stages + (size_t)s * Cfg::kStage;
             const uint64_t adesc = umma_desc_k_sw128(sa);
             /* 16 BF16 = 32 bytes further along K inside the swizzled row: +2 in 16-byte units */
-            if (Cfg::kFusedTerms) {
-                const uint64_t bdesc = umma_desc_k_sw128(sa + Cfg::kStageA);
+            const uint64_t bdesc = umma_desc_k_sw128(sa + Cfg::kStageA);
 #pragma unroll
-                for (int k = 0; k < kTcBlockK / 16; k++)
-                    umma_bf16(tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (it | k) != 0 ? 1u : 0u);
-            } else {
-#pragma unroll
-                for (int j = 0; j < kTcTerms; j++) {
-                    const uint64_t bdesc = umma_desc_k_sw128(sa + Cfg::kStageA + j * Cfg::kTermB);
-#pragma unroll
-                    for (int k = 0; k < kTcBlockK / 16; k++)
-                        umma_bf16(tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (it | j | k) != 0 ? 1u : 0u);
-                }
-            }
+            for (int k = 0; k < kTcBlockK / 16; k++)
+                umma_bf16(tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (it | k) != 0 ? 1u : 0u);
             umma_commit(&empty[s]);   /* stage reusable once these MMAs have read it */
         }
         umma_commit(accum);           /* accumulator complete (arrives at once when nothing was issued) */
@@ -391,7 +378,7 @@ vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
             vb_named_bar(1, 128);
         }
         if constexpr (MODE == TC_JOIN) {
-            const int m = (int)tc_cluster_rank() + kTcJoinSplits * warp;
+            const int m = (int)tc_cluster_rank() + kTcJoinSplits * warp;      /* up to 16 rows: one a warp */
             if (m < M) join_x = vb_ldcg4(tp.x + (size_t)m * N + tile * kTcTileN + lane * 4);
             if (tp.gain) join_gain = __ldg(reinterpret_cast<const float4 *>(tp.gain + tile * kTcTileN + lane * 4));
         }
@@ -411,15 +398,13 @@ vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
             for (int c0 = 0; c0 < NB && c0 < M; c0 += 16) {
                 uint32_t r[16];
                 tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r);
-                if (Cfg::kFusedTerms) {
-                    /* column groups NB and 2*NB hold the lo and lo2 products: add them in */
-                    uint32_t r1[16], r2[16];
-                    tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(NB + c0), r1);
-                    tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(2 * NB + c0), r2);
+                /* column groups NB and 2*NB hold the lo and lo2 products: add them in */
+                uint32_t r1[16], r2[16];
+                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(NB + c0), r1);
+                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(2 * NB + c0), r2);
 #pragma unroll
-                    for (int i = 0; i < 16; i++)
-                        r[i] = __float_as_uint((__uint_as_float(r[i]) + __uint_as_float(r1[i])) + __uint_as_float(r2[i]));
-                }
+                for (int i = 0; i < 16; i++)
+                    r[i] = __float_as_uint((__uint_as_float(r[i]) + __uint_as_float(r1[i])) + __uint_as_float(r2[i]));
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
                     const int m = c0 + i;
@@ -525,31 +510,29 @@ vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
         tc_cluster_sync();                    /* all partial results are staged */
         const float *stg = (const float *)stages;
         const int rank = (int)tc_cluster_rank(), n = tile * kTcTileN + lane * 4;
-        if (warp < 4) {
-            for (int m = rank + kTcJoinSplits * warp; m < M; m += kTcJoinSplits * 4) {
-                if (m >= kTcJoinSplits * 4) join_x = vb_ldcg4(tp.x + (size_t)m * N + n);
-                float4 q[kTcJoinSplits];
+        const int m = rank + kTcJoinSplits * warp;
+        if (warp < 4 && m < M) {
+            float4 q[kTcJoinSplits];
 #pragma unroll
-                for (int u = 0; u < kTcJoinSplits; u++) q[u] = tc_peer4(stg + m * kTcTileN + lane * 4, (uint32_t)u);
-                float4 v = q[0];
+            for (int u = 0; u < kTcJoinSplits; u++) q[u] = tc_peer4(stg + m * kTcTileN + lane * 4, (uint32_t)u);
+            float4 v = q[0];
 #pragma unroll
-                for (int u = 1; u < kTcJoinSplits; u++) { v.x += q[u].x; v.y += q[u].y; v.z += q[u].z; v.w += q[u].w; }
-                v.x = join_x.x + v.x; v.y = join_x.y + v.y; v.z = join_x.z + v.z; v.w = join_x.w + v.w;
-                *reinterpret_cast<float4 *>(tp.x_out + (size_t)m * N + n) = v;
-                if (tp.tap) *reinterpret_cast<float4 *>(tp.tap + (size_t)m * N + n) = v;
-                if (tp.gain) {
-                    const float e[4] = {v.x * join_gain.x, v.y * join_gain.y, v.z * join_gain.z, v.w * join_gain.w};
-                    uint16_t t[3][4];
+            for (int u = 1; u < kTcJoinSplits; u++) { v.x += q[u].x; v.y += q[u].y; v.z += q[u].z; v.w += q[u].w; }
+            v.x = join_x.x + v.x; v.y = join_x.y + v.y; v.z = join_x.z + v.z; v.w = join_x.w + v.w;
+            *reinterpret_cast<float4 *>(tp.x_out + (size_t)m * N + n) = v;
+            if (tp.tap) *reinterpret_cast<float4 *>(tp.tap + (size_t)m * N + n) = v;
+            if (tp.gain) {
+                const float e[4] = {v.x * join_gain.x, v.y * join_gain.y, v.z * join_gain.z, v.w * join_gain.w};
+                uint16_t t[3][4];
 #pragma unroll
-                    for (int i = 0; i < 4; i++) vb_split3(e[i], t[0][i], t[1][i], t[2][i]);
-                    uint16_t *o = tp.terms + (size_t)m * N + n;
+                for (int i = 0; i < 4; i++) vb_split3(e[i], t[0][i], t[1][i], t[2][i]);
+                uint16_t *o = tp.terms + (size_t)m * N + n;
 #pragma unroll
-                    for (int j = 0; j < 3; j++)
-                        *reinterpret_cast<uint2 *>(o + (size_t)j * tp.rows_pad * N) =
-                            make_uint2(t[j][0] | ((uint32_t)t[j][1] << 16), t[j][2] | ((uint32_t)t[j][3] << 16));
-                    const float ss = vb_warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w);
-                    if (lane == 0) tp.ssq[m * (N / kTcTileN) + tile] = ss;
-                }
+                for (int j = 0; j < 3; j++)
+                    *reinterpret_cast<uint2 *>(o + (size_t)j * tp.rows_pad * N) =
+                        make_uint2(t[j][0] | ((uint32_t)t[j][1] << 16), t[j][2] | ((uint32_t)t[j][3] << 16));
+                const float ss = vb_warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w);
+                if (lane == 0) tp.ssq[m * (N / kTcTileN) + tile] = ss;
             }
         }
         __syncwarp();
@@ -620,18 +603,13 @@ static int launch_tc(const TcWeight &w, const TcActs &a, const TcKernelArgs &ka,
 
 static int tc_gemm_join(const TcWeight &w, const TcActs &a, const TcGemm &g, cudaStream_t st) {
     const TcJoin &j = g.join;
-    if (w.N % kTcTileN || w.K / kTcBlockK < kTcJoinSplits || !j.x_out || (j.gain && (!j.terms || !j.ssq || j.rows_pad < g.M))) return -1;
+    if (a.rows_pad != 16 || w.N % kTcTileN || w.K / kTcBlockK < kTcJoinSplits || !j.x_out || (j.gain && (!j.terms || !j.ssq || j.rows_pad < g.M))) return -1;
     if (g.n_tiles || g.push.n_dst || g.wait.n || g.ssq || g.bias) return -1;
     TcKernelArgs ka = {};
     ka.a_tiled = w.tiled ? 1 : 0;
     ka.N = w.N; ka.K = w.K; ka.M = g.M; ka.rows_pad = a.rows_pad; ka.splits = kTcJoinSplits; ka.status = g.status;
     ka.n_tiles_launch = w.N / kTcTileN;
-    switch (a.rows_pad) {
-    case 16: return launch_tc_tp<16, 6, TC_JOIN>(w, a, ka, j, st);
-    case 48: return launch_tc_tp<48, 6, TC_JOIN>(w, a, ka, j, st);
-    case 64: return launch_tc_tp<64, 5, TC_JOIN>(w, a, ka, j, st);
-    default: return -1;
-    }
+    return launch_tc_tp<16, 6, TC_JOIN>(w, a, ka, j, st);
 }
 
 int tc_gemm(const TcWeight &w, const TcActs &a, const TcGemm &g, cudaStream_t st) {
@@ -642,8 +620,10 @@ int tc_gemm(const TcWeight &w, const TcActs &a, const TcGemm &g, cudaStream_t st
     if ((g.epi == TC_EPI_SWIGLU || g.epi == TC_EPI_SWIGLU_TERMS) && (w.N & 1)) return -1;
     if (g.epi == TC_EPI_SWIGLU_TERMS && (!g.out_terms || g.out_rows_pad < g.M)) return -1;
     if ((g.epi == TC_EPI_TERMS || g.epi == TC_EPI_RELU2_TERMS) && a.rows_pad < 256) return -1;
-    /* sliced or exchanged launches (tensor parallelism) do not occur beyond 64 rows */
-    if (a.rows_pad >= 256 && g.n_tiles == 0 && g.push.n_dst == 0 && g.wait.n == 0) return tc_gemm_rows(w, a, g, st);
+    if (a.rows_pad >= 256) {
+        /* sliced or exchanged launches (tensor parallelism) do not occur beyond 64 rows */
+        return g.n_tiles || g.push.n_dst || g.wait.n ? -1 : tc_gemm_rows(w, a, g, st);
+    }
     TcKernelArgs ka;
     ka.a_tiled = w.tiled ? 1 : 0;
     ka.N = w.N; ka.K = w.K; ka.M = g.M; ka.rows_pad = a.rows_pad; ka.ld_out = g.ld_out; ka.splits = g.splits;
@@ -664,7 +644,6 @@ int tc_gemm(const TcWeight &w, const TcActs &a, const TcGemm &g, cudaStream_t st
     case 16: return launch_tc<16, 6>(w, a, ka, tpa, st);
     case 48: return launch_tc<48, 6>(w, a, ka, tpa, st);   /* 8 utterances' acoustic rows: 34 KB stages, six of them */
     case 64: return launch_tc<64, 5>(w, a, ka, tpa, st);
-    case 256: return launch_tc<256, 2>(w, a, ka, tpa, st);
     default: return -1;
     }
 }

@@ -47,7 +47,7 @@ struct TcWeight {
     bool tiled;          /* W points at the tile-contiguous copy (tc_weight_tiled) */
 };
 
-/* Activation rows split into BF16 terms: [terms][rows_pad][K], rows_pad = 16, 64 or 256. */
+/* Activation rows split into BF16 terms: [terms][rows_pad][K], rows_pad = 16, 48, 64, 256 or a larger multiple of 128. */
 struct TcActs {
     CUtensorMap map;        /* rows_pad <= 256 */
     uint16_t *buf;
@@ -121,7 +121,7 @@ struct TcGemm {
     int tile0 = 0, n_tiles = 0;       /* output tiles [tile0, tile0 + n_tiles) of the weight matrix; 0 = all */
     TcPush push;
     TcWait wait;                      /* the activation terms (and ssq) are exchanged data */
-    TcJoin join;                      /* up to 64 rows, N a multiple of 128; epi, splits and out are not used */
+    TcJoin join;                      /* up to 16 rows, N a multiple of 128; epi, splits and out are not used */
 };
 
 int tc_init();                                     /* resolves cuTensorMapEncodeTiled; 0 when usable */
