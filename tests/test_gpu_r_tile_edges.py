@@ -92,3 +92,60 @@ def test_prefill_last_rows_keep_three_terms(pkg, engine, synth_model, rows):
     for (k1, v1), l in zip(whole, (0, 1, 25)):
         k2, v2 = engine.kv_read(l, 0, rows)
         assert np.array_equal(k2, k1) and np.array_equal(v2, v1), l
+
+
+@pytest.mark.parametrize("rows", [2, 8, 9, 16, 17, 48, 64])
+@pytest.mark.parametrize("K,N", [(64, 200), (576, 128), (1088, 9600), (3072, 9600)])
+def test_skinny_gemm_sums_stay_short(pkg, engine, rows, K, N):
+    """Products of one sign: the worst case for sums that are cut off at every step. Up to 16 rows TMEM adds one half of K
+    and then the other, 16 columns a step: every cut at most 2^-23 of a sum that is half its final size on the average,
+    and the two are added with a rounding, as are the terms. (9600 columns leave no K splits.)"""
+    x = np.abs(pkg.synth_f32((rows, K), 53, "sum.x", 0.0, 1.0))
+    W = pkg.synth_bf16((N, K), 54, "sum.W") & 0x7FFF
+    dx, dW, dy = pkg.DeviceBuffer(x), pkg.DeviceBuffer(W), pkg.DeviceBuffer(nbytes=rows * N * 4)
+    engine.L.tts_cuda_linear_bf16(dy.ptr, dx.ptr, None, rows, K, N, dW.ptr)
+    got = dy.get((rows, N))
+    want = x.astype(np.float64) @ (W.astype(np.uint32) << 16).view(np.float32).astype(np.float64).T
+    off = np.abs(got / want - 1.0).max()
+    for d in (dx, dW, dy):
+        d.free()
+    steps = 4 * ((K // 64 + 1) // 2 if rows <= 16 else K // 64)
+    assert off < steps / 2 * 2.0 ** -23 + 4 * 2.0 ** -24, off
+
+
+def _velocity64(t, x, hidden, time):
+    """predict_velocity (voxtral_tts_acoustic.c:182-262) in 64 bits: three tokens, three layers, the head of the first."""
+    p = "acoustic_transformer"
+
+    def mul(a, name):
+        return a @ (t[f"{name}.weight"].astype(np.uint32) << 16).view(np.float32).T.astype(np.float64)
+
+    def rms(a, name):
+        return a / np.sqrt((a * a).mean(-1, keepdims=True) + 1e-5) * t[f"{name}.weight"].astype(np.float64)
+    angle = (np.float32(time) * t[f"{p}.time_embedding.inv_freq"]).astype(np.float32)
+    temb = np.concatenate([np.cos(angle), np.sin(angle)]).astype(np.float64)
+    y = np.stack([mul(x.astype(np.float64), f"{p}.input_projection"), mul(temb, f"{p}.time_projection"),
+                  mul(hidden.astype(np.float64), f"{p}.llm_projection")])
+    for l in range(3):
+        n = f"{p}.layers.{l}"
+        h = rms(y, f"{n}.attention_norm")
+        q, k, v = (mul(h, f"{n}.attention.w{c}") for c in "qkv")
+        q, k, v = q.reshape(3, 8, 4, 128), k.reshape(3, 8, 128), v.reshape(3, 8, 128)
+        s = np.exp(np.einsum("igrd,jgd->grij", q, k) * 128 ** -0.5)
+        o = np.einsum("grij,jgd->igrd", s / s.sum(-1, keepdims=True), v).reshape(3, 4096)
+        y = y + mul(o, f"{n}.attention.wo")
+        h = rms(y, f"{n}.ffn_norm")
+        g = mul(h, f"{n}.feed_forward.w1")
+        y = y + mul(g / (1.0 + np.exp(-g)) * mul(h, f"{n}.feed_forward.w3"), f"{n}.feed_forward.w2")
+    return mul(rms(y[:1], f"{p}.norm"), f"{p}.acoustic_codebook_output")[0]
+
+
+@pytest.mark.parametrize("seed,time", [(3, 0.0), (4, 0.5), (5, 6.0 / 7.0)])
+def test_velocity_against_64_bits(pkg, engine, synth_model, seed, time):
+    """The longest sums in TMEM are 768 columns, 48 steps, each cut at most 2^-23 of a sum that is half its final size on the
+    average; fourteen GEMMs follow one another. Products of random signs leave about an eighth of that (with all of K in
+    one sum it was 7e-6 to 1e-5)."""
+    x, hidden = pkg.synth_f32(36, seed, "v64.x"), pkg.synth_f32(3072, seed, "v64.h")
+    want = _velocity64(synth_model.t, x, hidden, time)
+    off = np.linalg.norm(engine.predict_velocity(x, hidden, time) - want) / np.linalg.norm(want)
+    assert off < 14 * 24 * 2.0 ** -23 / 8, off

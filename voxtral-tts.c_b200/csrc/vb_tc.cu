@@ -169,7 +169,7 @@ int tc_pick_splits(int N, int K, int n_sm) {
 }
 
 /* ---------------------------------------------------------------- the kernel */
-template <int NB, int ST>
+template <int NB, int ST, int ACCS>
 struct TcCfg {
     static constexpr int kStageA = kTcTileN * kTcBlockK * 2;        /* 16 KB */
     static constexpr int kTermB = NB * kTcBlockK * 2;               /* one BF16 term of the activations */
@@ -181,7 +181,13 @@ struct TcCfg {
      * MMAs - the narrow ones are issue-latency bound, not throughput bound. */
     static constexpr int kAccCols = kTcTerms * NB;
     static_assert(kAccCols <= 256, "wider than an MMA");
-    static constexpr int kTmemCols = kAccCols <= 32 ? 32 : kAccCols <= 64 ? 64 : kAccCols <= 128 ? 128 : 256;
+    /* The tensor core cuts its fp32 sums off at every step, so that their error grows with the chain: a CTA's share of K
+     * goes into ACCS accumulators, one after another, whose sums the epilogue adds. One utterance, 40 frames: 2.714 ms a
+     * frame with one accumulator (and 16 columns read for every row count), 2.709 with two, whose hidden states are 2.0e-5
+     * for 2.4e-5 off 64 bits; segments of 512 to 1024 columns that the epilogue fetches under the main loop, with a commit
+     * for each, 2.74 to 2.78. A velocity call: 8.7e-6 with one, 4.4e-6 with two, 2.2e-6 with four. */
+    static constexpr int kTmemCols = ACCS * kAccCols <= 128 ? 128 : 256;
+    static_assert(ACCS * kAccCols <= kTmemCols, "accumulators over TMEM");
     static constexpr int kSmemBytes = kStages * kStage + 1024 /* alignment slack */ + 256 /* barriers */ + 4 * NB;
     static_assert(kSmemBytes <= 232448, "over the 227 KB a CTA may use");
 };
@@ -237,11 +243,35 @@ VB_DEVINL float4 tc_peer4(const float *p, uint32_t rank) {
     return v;
 }
 
-template <int NB, int ST, int MODE>
+/* Rows [c0, c0 + COLS) of this lane's output column, out of TMEM to their places in shared memory: the column groups NB and
+ * 2 * NB on hold the lo and lo2 products, each accumulator a part of K. */
+template <int NB, int COLS, int ACCS>
+VB_DEVINL void tc_stage_rows(float *to, uint32_t t, int c0, int M, int n_it, int seg, const float *rscale) {
+    float v[COLS];
+    t += (uint32_t)c0;
+#pragma unroll
+    for (int a = 0; a < ACCS; a++, t += kTcTerms * NB) {
+        if (a > 0 && n_it <= a * seg) break;
+        uint32_t r[3][COLS];
+        tmem_ld_x3<COLS>(t, t + NB, t + 2 * NB, r);
+#pragma unroll
+        for (int i = 0; i < COLS; i++) {
+            const float u = (__uint_as_float(r[0][i]) + __uint_as_float(r[1][i])) + __uint_as_float(r[2][i]);
+            v[i] = a == 0 ? u : v[i] + u;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < COLS; i++) {
+        const int m = c0 + i;
+        if (m < M) to[m * kTcTileN] = rscale ? v[i] * rscale[m] : v[i];
+    }
+}
+
+template <int NB, int ST, int MODE, int ACCS>
 __global__ void __launch_bounds__(kTcThreads, 1)
 vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                   const TcKernelArgs ka, const typename TcTpSel<MODE>::type tp) {
-    using Cfg = TcCfg<NB, ST>;
+    using Cfg = TcCfg<NB, ST, ACCS>;
     constexpr bool TP = MODE == TC_TP;
     /* the tensor maps are fetched while the first reads of the parameter block are on their way */
     if (threadIdx.x == 128) {
@@ -272,6 +302,7 @@ vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
     const int kblocks = K / kTcBlockK;
     const int kb0 = (int)((long long)kblocks * sp / splits), kb1 = (int)((long long)kblocks * (sp + 1) / splits);
     const int n_it = kb1 - kb0;
+    const int seg = (n_it + ACCS - 1) / ACCS;      /* k-blocks of an accumulator */
 
     int first = 0;   /* producer thread only: stages of the first ring-full */
     if (warp == 4 && lane == 0) {
@@ -344,6 +375,8 @@ vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
         /* ---- MMA issuer ---- */
         const uint32_t idesc = umma_idesc_bf16(Cfg::kAccCols);
         bool ok = true;
+        uint32_t d = tmem, more = 0;
+        int end = seg;
         for (int it = 0; it < n_it && ok; it++) {
             const int s = it % Cfg::kStages, use = it / Cfg::kStages;
             if (!vb_mbar_wait(&full[s], use & 1u, abort_flag)) {
@@ -357,9 +390,9 @@ vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
             const uint64_t adesc = umma_desc_k_sw128(sa);
             /* 16 BF16 = 32 bytes further along K inside the swizzled row: +2 in 16-byte units */
             const uint64_t bdesc = umma_desc_k_sw128(sa + Cfg::kStageA);
+            if (ACCS > 1 && it == end) { d += Cfg::kAccCols; end += seg; more = 0; }
 #pragma unroll
-            for (int k = 0; k < kTcBlockK / 16; k++)
-                umma_bf16(tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (it | k) != 0 ? 1u : 0u);
+            for (int k = 0; k < kTcBlockK / 16; k++, more = 1) umma_bf16(d, adesc + 2 * k, bdesc + 2 * k, idesc, more);
             umma_commit(&empty[s]);   /* stage reusable once these MMAs have read it */
         }
         umma_commit(accum);           /* accumulator complete (arrives at once when nothing was issued) */
@@ -394,24 +427,13 @@ vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
          * measured at ~90 ns per store and 1.5 us per launch even with a single row. */
         float *stg = (float *)stages;                              /* [M][128 output columns] */
         if (ok && n_it > 0) {
+            const uint32_t t0 = tmem + ((uint32_t)(warp * 32) << 16);
+            const float *const rs = ka.ssq ? rscale : nullptr;
+            if (NB <= 16 && M <= 8) {          /* half as many columns to read: 0.04 us a launch */
+                tc_stage_rows<NB, 8, ACCS>(stg + warp * 32 + lane, t0, 0, M, n_it, seg, rs);
+            } else {
 #pragma unroll 1
-            for (int c0 = 0; c0 < NB && c0 < M; c0 += 16) {
-                uint32_t r[16];
-                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r);
-                /* column groups NB and 2*NB hold the lo and lo2 products: add them in */
-                uint32_t r1[16], r2[16];
-                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(NB + c0), r1);
-                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(2 * NB + c0), r2);
-#pragma unroll
-                for (int i = 0; i < 16; i++)
-                    r[i] = __float_as_uint((__uint_as_float(r[i]) + __uint_as_float(r1[i])) + __uint_as_float(r2[i]));
-#pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    const int m = c0 + i;
-                    float v = __uint_as_float(r[i]);
-                    if (ka.ssq && m < M) v *= rscale[m];
-                    if (m < M) stg[m * kTcTileN + warp * 32 + lane] = v;
-                }
+                for (int c0 = 0; c0 < NB && c0 < M; c0 += 16) tc_stage_rows<NB, 16, ACCS>(stg + warp * 32 + lane, t0, c0, M, n_it, seg, rs);
             }
             if constexpr (MODE != TC_JOIN) {
                 vb_named_bar(1, 128);
@@ -575,13 +597,13 @@ static cudaError_t launch_pdl_cluster(void (*kernel)(KArgs...), int cluster, dim
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-template <int NB, int ST, int MODE>
+template <int NB, int ST, int MODE, int ACCS>
 static int launch_tc_tp(const TcWeight &w, const TcActs &a, const TcKernelArgs &ka, const typename TcTpSel<MODE>::type &arg,
                         cudaStream_t st) {
-    using Cfg = TcCfg<NB, ST>;
+    using Cfg = TcCfg<NB, ST, ACCS>;
     static bool attr = false;
     if (!attr) {
-        if (cudaFuncSetAttribute(vb_tc_gemm_kernel<NB, ST, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (cudaFuncSetAttribute(vb_tc_gemm_kernel<NB, ST, MODE, ACCS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  Cfg::kSmemBytes) != cudaSuccess) {
             cudaGetLastError();
             return -1;
@@ -589,16 +611,16 @@ static int launch_tc_tp(const TcWeight &w, const TcActs &a, const TcKernelArgs &
         attr = true;
     }
     const int tiles = ka.n_tiles_launch;
-    return launch_pdl_cluster(vb_tc_gemm_kernel<NB, ST, MODE>, MODE == TC_JOIN ? kTcJoinSplits : 0, dim3(tiles * ka.splits), dim3(kTcThreads),
+    return launch_pdl_cluster(vb_tc_gemm_kernel<NB, ST, MODE, ACCS>, MODE == TC_JOIN ? kTcJoinSplits : 0, dim3(tiles * ka.splits), dim3(kTcThreads),
                               (size_t)Cfg::kSmemBytes, st, w.map, a.map, ka, arg) == cudaSuccess
                ? 0
                : -1;
 }
 
-template <int NB, int ST>
+template <int NB, int ST, int ACCS>
 static int launch_tc(const TcWeight &w, const TcActs &a, const TcKernelArgs &ka, const TcTpArgs &tpa, cudaStream_t st) {
-    if (tpa.push.n_dst > 0 || tpa.wait.n > 0) return launch_tc_tp<NB, ST, TC_TP>(w, a, ka, tpa, st);
-    return launch_tc_tp<NB, ST, TC_PLAIN>(w, a, ka, TcNoTpArgs(), st);
+    if (tpa.push.n_dst > 0 || tpa.wait.n > 0) return launch_tc_tp<NB, ST, TC_TP, ACCS>(w, a, ka, tpa, st);
+    return launch_tc_tp<NB, ST, TC_PLAIN, ACCS>(w, a, ka, TcNoTpArgs(), st);
 }
 
 static int tc_gemm_join(const TcWeight &w, const TcActs &a, const TcGemm &g, cudaStream_t st) {
@@ -609,7 +631,7 @@ static int tc_gemm_join(const TcWeight &w, const TcActs &a, const TcGemm &g, cud
     ka.a_tiled = w.tiled ? 1 : 0;
     ka.N = w.N; ka.K = w.K; ka.M = g.M; ka.rows_pad = a.rows_pad; ka.splits = kTcJoinSplits; ka.status = g.status;
     ka.n_tiles_launch = w.N / kTcTileN;
-    return launch_tc_tp<16, 6, TC_JOIN>(w, a, ka, j, st);
+    return g.exact ? launch_tc_tp<16, 6, TC_JOIN, 4>(w, a, ka, j, st) : launch_tc_tp<16, 6, TC_JOIN, 2>(w, a, ka, j, st);
 }
 
 int tc_gemm(const TcWeight &w, const TcActs &a, const TcGemm &g, cudaStream_t st) {
@@ -617,6 +639,7 @@ int tc_gemm(const TcWeight &w, const TcActs &a, const TcGemm &g, cudaStream_t st
     if (g.join.x) return tc_gemm_join(w, a, g, st);
     if (g.splits < 1 || g.splits > kTcMaxSplits || g.splits > w.K / kTcBlockK) return -1;
     if (g.epi != TC_EPI_PARTIAL && g.splits != 1) return -1;
+    if (g.exact && (g.push.n_dst || g.wait.n)) return -1;
     if ((g.epi == TC_EPI_SWIGLU || g.epi == TC_EPI_SWIGLU_TERMS) && (w.N & 1)) return -1;
     if (g.epi == TC_EPI_SWIGLU_TERMS && (!g.out_terms || g.out_rows_pad < g.M)) return -1;
     if ((g.epi == TC_EPI_TERMS || g.epi == TC_EPI_RELU2_TERMS) && a.rows_pad < 256) return -1;
@@ -641,9 +664,9 @@ int tc_gemm(const TcWeight &w, const TcActs &a, const TcGemm &g, cudaStream_t st
     tpa.wait = g.wait;
     tpa.wait.status = g.status;
     switch (a.rows_pad) {
-    case 16: return launch_tc<16, 6>(w, a, ka, tpa, st);
-    case 48: return launch_tc<48, 6>(w, a, ka, tpa, st);   /* 8 utterances' acoustic rows: 34 KB stages, six of them */
-    case 64: return launch_tc<64, 5>(w, a, ka, tpa, st);
+    case 16: return g.exact ? launch_tc_tp<16, 6, TC_PLAIN, 4>(w, a, ka, TcNoTpArgs(), st) : launch_tc<16, 6, 2>(w, a, ka, tpa, st);
+    case 48: return launch_tc<48, 6, 1>(w, a, ka, tpa, st);   /* 8 utterances' acoustic rows: 34 KB stages, six of them */
+    case 64: return launch_tc<64, 5, 1>(w, a, ka, tpa, st);
     default: return -1;
     }
 }

@@ -63,6 +63,32 @@ VB_DEVINL void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+/* COLS (8 or 16) columns at each of three places, with one wait for all */
+#define VB_TM8(x) "=r"((x)[0]), "=r"((x)[1]), "=r"((x)[2]), "=r"((x)[3]), "=r"((x)[4]), "=r"((x)[5]), "=r"((x)[6]), "=r"((x)[7])
+template <int COLS>
+VB_DEVINL void tmem_ld_x3(uint32_t a, uint32_t b, uint32_t c, uint32_t (&r)[3][COLS]) {
+    static_assert(COLS == 8 || COLS == 16, "");
+    if constexpr (COLS == 8)
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%24];\n\t"
+            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%25];\n\t"
+            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16, %17, %18, %19, %20, %21, %22, %23}, [%26];\n\t"
+            "tcgen05.wait::ld.sync.aligned;"
+            : VB_TM8(r[0]), VB_TM8(r[1]), VB_TM8(r[2])
+            : "r"(a), "r"(b), "r"(c)
+            : "memory");
+    else
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%48];\n\t"
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%49];\n\t"
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47}, [%50];\n\t"
+            "tcgen05.wait::ld.sync.aligned;"
+            : VB_TM8(r[0]), VB_TM8(&r[0][8]), VB_TM8(r[1]), VB_TM8(&r[1][8]), VB_TM8(r[2]), VB_TM8(&r[2][8])
+            : "r"(a), "r"(b), "r"(c)
+            : "memory");
+}
+#undef VB_TM8
+
 /* Tensor-parallel consumer wait (one thread): every source rank has published this visit of
  * the buffer. Bounded; false (and a status code) when it runs out. */
 VB_DEVINL bool tp_wait(const TcWait &w) {
