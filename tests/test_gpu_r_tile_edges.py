@@ -149,3 +149,61 @@ def test_velocity_against_64_bits(pkg, engine, synth_model, seed, time):
     want = _velocity64(synth_model.t, x, hidden, time)
     off = np.linalg.norm(engine.predict_velocity(x, hidden, time) - want) / np.linalg.norm(want)
     assert off < 14 * 24 * 2.0 ** -23 / 8, off
+
+
+def test_prompt_attention_maxima_that_rise_late(pkg, tmp_path):
+    """Rows whose largest score rises by more than 2^8 in a later tile of the same half, where the sums so far are scaled down.
+    |q||k| of 98 in two terms is off by 98 * 2^-17 in a score: the limit is two of these."""
+    c = Case(pkg, tmp_path, config([attention(heads=4, kv_heads=2, dim=64, vdim=64, window=0, rot=0, scale=0.6, softcap=0, ff=0)]), seed=9)
+    toks = tokens(c.cfg, 420, 9)
+    w, eps = c.w, c.cfg["norm"]["eps"]
+    h = plain.layer_norm(w["embed"][np.array(toks)], w["l0.norm1"], eps)
+    q = plain.rms_norm(h @ w["l0.mix.q"].T, w["l0.mix.q.norm"], eps)[:, :64]
+    k = plain.rms_norm(h @ w["l0.mix.k"].T, w["l0.mix.k.norm"], eps)[:, :64]
+    top = (q[384:] @ k[:384].T * 0.6 / np.log(2.0)).reshape(-1, 3, 2, 64).max(3)      # [row, tile of a half, half]
+    assert (top[:, 1:] > top[:, :1] + 8.0).any(2).any(1).sum() > 10
+    want = plain.forward(w, c.cfg, toks)[0]
+    with c.open("bfloat16") as lm:
+        assert error(lm.step(lm.open(), toks, range(420)), want) < 2 * 98 * 2.0 ** -17
+
+
+@pytest.mark.parametrize("scale,cap", [(-0.2, 0), (-0.2, 15.0), (0.0, 0), (0.0, 15.0)])
+def test_prompt_attention_scales(pkg, tmp_path, scale, cap):
+    """A negative scale turns the order of the keys around, with a scale of zero all weigh the same."""
+    c = Case(pkg, tmp_path, config([attention(dim=64, vdim=64, window=90, scale=scale, softcap=cap, ff=0)]), seed=10)
+    toks = tokens(c.cfg, 200, 10)
+    want = plain.forward(c.w, c.cfg, toks)[0]
+    with c.open("bfloat16") as lm:
+        assert error(feed(lm, lm.open(), toks, [199, 1]), want) < LIMIT["bfloat16"]
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_rows_that_are_not_finite_stay_behind_their_tile(pkg, tmp_path, bad):
+    """A token whose row is not finite spoils the rows that see it, and those before it in its tile of 64 keys at most
+    (weights of zero times a value that is not finite)."""
+    c = Case(pkg, tmp_path, config([attention(heads=4, kv_heads=4, dim=64, vdim=64, window=0, ff=72), attention(heads=4, kv_heads=2, dim=24, vdim=40)]),
+             seed=11)
+    toks = np.array(tokens(c.cfg, 400, 11))
+    toks[toks == 5] = 6
+    with c.open("bfloat16") as lm:
+        clean = lm.step(lm.open(), toks.tolist(), range(400))
+    c.w["embed"][5] = bad
+    c.rewrite()
+    toks[300] = 5
+    with c.open("bfloat16") as lm:
+        got = lm.step(lm.open(), toks.tolist(), range(400))
+    assert np.array_equal(got[:256], clean[:256]) and not np.isfinite(got[300]).any()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("width,rows", [(2048, 40), (2048, 300), (3072, 297), (4096, 300), (1100, 300), (1028, 297), (1024, 300)])
+def test_centred_norms_by_width(pkg, tmp_path, dtype, width, rows):
+    """Widths that give every thread of the residual kernel equal columns (one barrier a norm) and others, each up to 296
+    rows and in the smaller CTAs beyond; rows whose mean is eight times their spread. The limits are those of the types."""
+    c = Case(pkg, tmp_path, config([attention(ff=40)], width=width, vocab=101), seed=width + rows)
+    c.w["embed"] += 8.0
+    c.rewrite()
+    toks = tokens(c.cfg, rows, 12)
+    want = plain.forward(c.w, c.cfg, toks)[0]
+    with c.open(dtype) as lm:
+        assert error(lm.step(lm.open(), toks, range(rows)), want) < LIMIT[dtype]
