@@ -151,6 +151,16 @@ def test_velocity_against_64_bits(pkg, engine, synth_model, seed, time):
     assert off < 14 * 24 * 2.0 ** -23 / 8, off
 
 
+@pytest.mark.parametrize("cap", [30.0, 1000.0, 1e5])
+def test_prompt_softcap(pkg, tmp_path, cap):
+    """Scores far below the cap keep their digits. The limit is the two-term products'."""
+    c = Case(pkg, tmp_path, config([attention(dim=64, vdim=64, window=0, softcap=cap, ff=0)]), seed=8)
+    toks = tokens(c.cfg, 300, 8)
+    want = plain.forward(c.w, c.cfg, toks)[0]
+    with c.open("bfloat16") as lm:
+        assert error(feed(lm, lm.open(), toks, [299, 1]), want) < LIMIT["bfloat16"]
+
+
 def test_prompt_attention_maxima_that_rise_late(pkg, tmp_path):
     """Rows whose largest score rises by more than 2^8 in a later tile of the same half, where the sums so far are scaled down.
     |q||k| of 98 in two terms is off by 98 * 2^-17 in a score: the limit is two of these."""
