@@ -107,6 +107,7 @@ constexpr int kTcJoinSplits = 4;
 /* One GEMM launch. */
 struct TcGemm {
     int M = 0, splits = 1, epi = TC_EPI_STORE;
+    int segment = 32;                 /* 65 rows and more: k-blocks that are summed in TMEM, at most, before registers take over */
     bool exact = false;               /* up to 16 rows: four accumulators in place of two (see TcCfg) */
     float *out = nullptr;
     int ld_out = 0;

@@ -18,7 +18,8 @@
  * rows with K in one piece were 7.1e-5 off 64 bits, in 3 to 6 splits 4.6e-5, at the price of as many partial results.
  * So TMEM sums up to 2048 columns at a time (alternating accumulators) and the epilogue warps add these up in
  * registers, 64 values a thread, under the main loop. A 4001-token prompt: 60.6 ms and 7.3e-5 in one piece, 61.9 ms and
- * 4.9e-5 so, 63.3 ms and 3.3e-5 with 1024 columns (and 66 to 69 ms where eight warps held 128 values and spilled).
+ * 4.9e-5 so, 63.3 ms and 3.3e-5 with 1024 columns (and 66 to 69 ms where eight warps held 128 values and spilled). The
+ * codec, whose K splits are fewer than before this kernel, takes 1024 (TcGemm::segment).
  *
  * Warps: 0-15 epilogue (TMEM -> registers -> shared memory -> whole 512-byte row segments), 16 TMA producer, 17 MMA issuer (of the even
  * CTA, for both). Full barriers and the accumulator hand-back live in the even CTA; commits arrive in both. No
@@ -38,7 +39,6 @@ constexpr int kPrMaxRows = 256, kPrTerms = 2, kPrStages = 4, kPrChunk = 64;
 constexpr int kPrStageW = kTcTileN * kTcBlockK * 2, kPrStageX = kPrMaxRows / 2 * kTcBlockK * 2;
 constexpr int kPrStage = kPrStageW + kPrTerms * kPrStageX;
 constexpr int kPrStaging = kPrChunk * kTcTileN * 4;
-constexpr int kPrSegment = 32;       /* k-blocks that are summed in TMEM, at most, before the sums move on to registers */
 constexpr int kPrEpiWarps = 16, kPrEpi = 32 * kPrEpiWarps, kPrThreads = kPrEpi + 64;
 constexpr int kPrSmemBytes = kPrStages * kPrStage + kPrStaging + kPrMaxRows * 4 + 256 + 1024;
 static_assert(kPrSmemBytes <= 232448, "over the 227 KB a CTA may use");
@@ -52,7 +52,7 @@ struct RowsArgs {
     int *status;
     float eps;
     int N, K, M, R, rows_pad, ld_out, splits, epi, ssq_chunks, a_tiled, out_rows_pad, act_n0, out_terms_ld, out_col0;
-    int row_blocks, pairs, group_tiles;
+    int row_blocks, pairs, group_tiles, segment;
 };
 
 VB_DEVINL uint32_t pr_rank() {
@@ -121,7 +121,7 @@ VB_DEVINL PrTile pr_tile(const RowsArgs &a, int i, int kblocks) {
     t.n_mma = (t.Mb + 31) & ~31;
     t.kb0 = (int)((long long)kblocks * t.sp / a.splits);
     t.n_it = (int)((long long)kblocks * (t.sp + 1) / a.splits) - t.kb0;
-    const int segments = (t.n_it + kPrSegment - 1) / kPrSegment;
+    const int segments = (t.n_it + a.segment - 1) / a.segment;
     t.seg = (t.n_it + segments - 1) / segments;
     return t;
 }
@@ -474,7 +474,7 @@ RowsArgs rows_args(const TcWeight &w, const TcActs &a, const TcGemm &g) {
     ra.out = g.out; ra.out_terms = g.out_terms; ra.bias = g.bias; ra.ssq = g.ssq; ra.status = g.status; ra.eps = g.eps;
     ra.K = w.K; ra.rows_pad = a.rows_pad; ra.ld_out = g.ld_out; ra.splits = g.splits; ra.epi = g.epi; ra.ssq_chunks = g.ssq_chunks;
     ra.a_tiled = w.tiled ? 1 : 0; ra.out_rows_pad = g.out_rows_pad; ra.act_n0 = g.act_n0; ra.out_terms_ld = g.out_terms_ld;
-    ra.out_col0 = g.out_col0;
+    ra.out_col0 = g.out_col0; ra.segment = g.segment > 0 ? g.segment : 1;
     return ra;
 }
 
