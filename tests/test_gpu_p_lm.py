@@ -123,6 +123,14 @@ def test_portions(mixed, dtype, sizes):
         assert error(feed(lm, s, mixed.toks, sizes), mixed.want) < LIMIT[dtype]
 
 
+@pytest.mark.parametrize("rows", [32, 33, 64, 65, 96, 97, 128, 129, 256, 257, 385])
+def test_32_bit_rows(mixed, rows):
+    """Portions on both sides of the change from streamed weights to the row-block GEMM, and of its tiles."""
+    with mixed.open("float32") as lm:
+        s = lm.open()
+        assert error(lm.step(s, mixed.toks[:rows], range(rows)), mixed.want[:rows]) < LIMIT["float32"]
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("block", [1, 5, 24, 70, 130])
 def test_blocks_and_ring_wraps(mixed, dtype, block):

@@ -9,7 +9,7 @@
  *   GEMM of every projection that reads the norm, mixer kernels [, experts], GEMM of the two
  *   out-projections side by side, residual + norm
  * with the GEMMs of vb_tc.cu (split-K partials, summed by the consumer) and, in the 32-bit mode,
- * a plain fp32 GEMM in their place. One-token steps are captured once as a CUDA graph and
+ * those of vb_lm_gemm32.cu in their place. One-token steps are captured once as a CUDA graph and
  * replayed for every position and slot.
  */
 #include "../../include/voxtral_b200_lm.h"
@@ -148,6 +148,8 @@ struct vb200_lm {
     float *x = nullptr, *part_in = nullptr, *part_out = nullptr, *part_head = nullptr, *logits = nullptr;
     float *q = nullptr, *k = nullptr, *v = nullptr, *o = nullptr, *beta = nullptr, *decays = nullptr, *gram = nullptr;
     float *scratch = nullptr, *tap = nullptr;
+    uint16_t *terms = nullptr;           /* 32-bit mode: rows of the GEMM at hand as terms, up to terms_k columns */
+    int terms_k = 0;
     unsigned *tickets = nullptr;
     int *status = nullptr, *log = nullptr, *zero = nullptr;
     /* latent attention */
@@ -370,6 +372,8 @@ int vb200_lm::linear(const Source &s, const std::vector<Piece> &pieces, int N, i
         allocs.push_back(rows);
         l->W = rows;
         weight_bytes += elems * 2;
+        if (!rc && tc_weight(&l->tc, rows, l->N, l->Kp)) rc = fail("tensor map of a weight matrix could not be made");
+        terms_k = std::max(terms_k, l->Kp);
     }
     return rc;
 }
@@ -656,6 +660,7 @@ int vb200_lm::make_buffers() {
         alloc(&gram, (B + kLmDeltaRows) / kLmDeltaGroup * gn * 2 * kLmDeltaGroup * kLmDeltaGroup) || alloc(&scratch, scr) || alloc(&tickets, (size_t)tick, true) ||
         alloc(&status, 4, true) || alloc(&log, kLogCap, true) || alloc(&zero, 4, true) || alloc(&d_in, 4 + 2 * B, true))
         return -1;
+    if (f32() && alloc(&terms, (size_t)kTcTerms * lm_gemm_f32_rows_pad(std::max(block, kHeadRows)) * terms_k, true)) return -1;
     for (int i = 0; i < 2; i++) {
         LM_CUDA(cudaHostAlloc(&h_in[i], sizeof(int) * (4 + 2 * B), cudaHostAllocDefault));
         LM_CUDA(cudaEventCreateWithFlags(&in_free[i], cudaEventDisableTiming));
@@ -742,6 +747,7 @@ int vb200_lm::gemm(const Linear &l, Acts *in, int M, float *part, Acts *swiglu_o
         const int ld = l.swiglu ? swiglu_out->Kp : l.N;
         const int splits = splits_of(l, M);
         if (out) *out = {part, splits, l.N, (size_t)M * l.N};
+        if (M > kLmF32FewRows) return lm_gemm_f32_many(y, ld, in->rows, in->Kp, l.tc, terms, M, l.swiglu, st, splits, status);
         return lm_gemm_f32(y, ld, in->rows, in->Kp, l.W, l.Kp, M, l.N, l.K, l.swiglu ? LM_ACT_SWIGLU : LM_ACT_NONE, st, splits);
     }
     TcActs *a = map_of(in, M);

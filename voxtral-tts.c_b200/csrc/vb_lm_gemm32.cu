@@ -1,10 +1,13 @@
 /*
- * vb_lm_gemm32.cu - the GEMM of the language models' 32-bit mode: fp32 rows times BF16 weights, every product and
- * sum on the fp32 pipes.
+ * vb_lm_gemm32.cu - the GEMMs of the language models' 32-bit mode: fp32 rows times BF16 weights, no product rounded,
+ * sums as exact as the fp32 pipes make them.
  *
- * Two kernels. Up to kSkinnyM rows the weights are the traffic: a warp streams whole weight rows and keeps one sum
- * per row and lane. Above, the fp32 pipes are the bound: a register-tiled kernel on packed pairs. Both split K over
- * CTAs when a matrix alone does not fill the chip; the partial sums are added by the kernel that reads them.
+ * Up to kLmF32FewRows rows the weights are the traffic: a warp streams whole weight rows and keeps one fp32 sum per
+ * row and lane. Above, the arithmetic is the bound, and the tensor cores do it: a row is the sum of three BF16 terms (24 bits),
+ * a term's products with BF16 weights are exact, and the row-block GEMM adds them up in short stretches (kManySegment).
+ * 390 x 11264 x 2048: 569 us in register tiles on the fp32 pipes, 32 TFLOP/s of their 74. Experts' rows, sorted by
+ * matrix, still run in such tiles. All split K over CTAs when a matrix alone does not fill the chip; the partial sums are
+ * added by the kernel that reads them.
  */
 #include "vb_lm_kernels.cuh"
 
@@ -40,7 +43,7 @@ VB_DEVINL float2 f2_get(f2 v) {
 
 VB_DEVINL float act_of(float v, int act) { return act == LM_ACT_RELU2 ? fmaxf(v, 0.0f) * fmaxf(v, 0.0f) : v; }
 
-/* ---------------------------------------------------------------- many rows */
+/* ---------------------------------------------------------------- rows sorted by matrix */
 /* 64 x 128 results per CTA, 8 x 8 per thread, 16 columns of K per step, double-buffered. A warp's step is 32 packed
  * multiply-adds on 6 wavefronts of shared memory, so the fp32 pipes are the bound. Three CTAs fit an SM.
  * The sum over K is taken in two levels of 32 columns, so that its rounding error grows with the step length and the
@@ -167,8 +170,6 @@ lm_gemm_f32_tile_kernel(float *y, int ld_out, size_t part_stride, const float *x
  * over the warp at the end. Bound by the weight stream (and, at eight rows, by shared memory: two 16-byte reads of
  * x serve R rows of weights). 5 x 22528 x 2048: 314 us in 64-row tiles. */
 constexpr int kSkWarps = 8, kSkRows = 8, kSkCols = 512;
-constexpr int kSkinnyM = 32;     /* 64-row tiles do the work of 64 rows: at 32 rows four passes over the weights (L2) still cost less */
-
 template <int R>
 __global__ void __launch_bounds__(32 * kSkWarps)
 lm_gemm_f32_rows_kernel(float *y, int ld_out, size_t part_stride, const float *x, int ldx, const uint16_t *W, int ldw, int M, int N,
@@ -250,17 +251,48 @@ lm_gemm_f32_rows_kernel(float *y, int ld_out, size_t part_stride, const float *x
     }
 }
 
+/* ---------------------------------------------------------------- rows as terms */
+/* fp32 rows -> three BF16 terms [3][rows_pad][ld], whose sum is the row to 24 bits. What BF16 cannot hold stays what the
+ * fp32 pipes would have multiplied: infinities and NaN are their own first term, a finite value that rounds to
+ * infinity is cut off. */
+__global__ void __launch_bounds__(256) lm_split_rows_kernel(uint16_t *terms, int rows_pad, int ld, const float *x, int n4) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= n4) return;
+    const float4 v = __ldcg(reinterpret_cast<const float4 *>(x) + i);
+    const float e[4] = {v.x, v.y, v.z, v.w};
+    uint16_t t[3][4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        vb_split3(e[j], t[0][j], t[1][j], t[2][j]);
+        if ((t[0][j] & 0x7f80u) == 0x7f80u) {
+            const uint32_t u = __float_as_uint(e[j]);
+            if ((u & 0x7f800000u) == 0x7f800000u) {
+                t[1][j] = t[2][j] = 0;
+            } else {
+                uint16_t last;
+                t[0][j] = (uint16_t)(u >> 16);
+                vb_split3(e[j] - __uint_as_float(u & 0xffff0000u), t[1][j], t[2][j], last);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        *(reinterpret_cast<uint2 *>(terms + (size_t)k * rows_pad * ld) + i) =
+            make_uint2(t[k][0] | ((uint32_t)t[k][1] << 16), t[k][2] | ((uint32_t)t[k][3] << 16));
+}
+
 /* Weight rows per warp: four halve the reads of x per weight; two where four would leave SMs without a CTA. */
 int skinny_rows(int N) { return N >= 148 * kSkWarps * 4 ? 4 : 2; }
 
 } // namespace
 
-/* K splits: enough CTAs for three (tiles) or two (few rows) per SM, no split shorter than 512 columns. */
+/* K splits: enough CTAs for two per SM, no split shorter than 512 columns. Many rows: what suits the row-block GEMM. */
 int lm_gemm_f32_splits(int M, int N, int K, int n_sm) {
-    const int ctas = M <= kSkinnyM ? ((N + kSkWarps * skinny_rows(N) - 1) / (kSkWarps * skinny_rows(N))) * ((M + kSkRows - 1) / kSkRows)
-                                   : ((N + kFgN - 1) / kFgN) * ((M + kFgM - 1) / kFgM);
-    const int want = M <= kSkinnyM ? 2 * n_sm : 3 * n_sm;
-    return std::max(1, std::min({want / ctas, K / 512, 4}));
+    if (M > kLmF32FewRows) return tc_row_splits(N, (K + kTcBlockK - 1) / kTcBlockK * kTcBlockK, M, n_sm, kTcTerms);
+    const int rows = kSkWarps * skinny_rows(N), ctas = ((N + rows - 1) / rows) * ((M + kSkRows - 1) / kSkRows);
+    return std::max(1, std::min({2 * n_sm / ctas, K / 512, 4}));
 }
 
 int lm_gemm_f32(float *y, int ld_out, const float *x, int ldx, const uint16_t *W, int ldw, int M, int N, int K, LmAct act,
@@ -269,7 +301,8 @@ int lm_gemm_f32(float *y, int ld_out, const float *x, int ldx, const uint16_t *W
     if (M < 1 || N < 1 || (ldx & 3) || (ldw & 31) || (K + 31) / 32 * 32 > std::min(ldx, ldw) || splits < 1 || (splits > 1 && act != LM_ACT_NONE)) return -1;
     const size_t stride = (size_t)M * ld_out;
     cudaError_t e;
-    if (M <= kSkinnyM && !table) {
+    if (!table) {
+        if (M > kLmF32FewRows) return -1;
         const int r = skinny_rows(N), cols = (K + 31) / 32 * 32;
         const dim3 g((N + kSkWarps * r - 1) / (kSkWarps * r), (M + kSkRows - 1) / kSkRows, splits);
         e = launch_pdl(r == 4 ? lm_gemm_f32_rows_kernel<4> : lm_gemm_f32_rows_kernel<2>, g, dim3(32 * kSkWarps), 0, st, y, ld_out, stride, x,
@@ -280,6 +313,28 @@ int lm_gemm_f32(float *y, int ld_out, const float *x, int ldx, const uint16_t *W
                        table, group_rows);
     }
     return e == cudaSuccess ? 0 : -1;
+}
+
+/* k-blocks that TMEM sums before registers add them up. A 24-run model of width 2048, seven prompts of 40 to 390 rows,
+ * logits off 64 bits on average: 4.2e-6 on the fp32 pipes, 3.3e-6 with one or two k-blocks, 4.2e-6 with four, 6.7e-6
+ * with eight; 390 rows take 13.9, 12.1, 11.5 and 11.3 ms (37.8 on the fp32 pipes). */
+constexpr int kManySegment = 2;
+
+int lm_gemm_f32_many(float *y, int ld_out, const float *x, int ldx, const TcWeight &w, uint16_t *terms, int M, bool swiglu, cudaStream_t st,
+                     int splits, int *status) {
+    TcActs a;
+    if (ldx != w.K || tc_acts_blocks(&a, terms, lm_gemm_f32_rows_pad(M), w.K)) return -1;
+    const int n4 = (int)((size_t)M * ldx / 4);
+    if (launch_pdl(lm_split_rows_kernel, dim3((n4 + 255) / 256), dim3(256), 0, st, terms, a.rows_pad, ldx, x, n4) != cudaSuccess) return -1;
+    TcGemm g;
+    g.M = M;
+    g.terms = kTcTerms;
+    g.segment = kManySegment;
+    g.status = status;
+    g.out = y; g.ld_out = ld_out;
+    g.epi = swiglu ? TC_EPI_SWIGLU : TC_EPI_PARTIAL;
+    g.splits = splits;
+    return tc_gemm(w, a, g, st);
 }
 
 } // namespace vb

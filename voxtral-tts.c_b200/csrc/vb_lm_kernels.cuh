@@ -175,15 +175,22 @@ int lm_pack_rows(uint16_t *dst, int Kp, int row0, int step, int col0, const uint
 int lm_widen(float *dst, const uint16_t *src, int n, cudaStream_t st);
 int lm_fill_random(uint16_t *dst, size_t n, uint32_t seed, float mean, float scale, cudaStream_t st);
 
-/* ---- fp32 GEMM on the fp32 pipes (vb_lm_gemm32.cu) ----
+/* ---- GEMMs of the 32-bit mode (vb_lm_gemm32.cu) ----
  * y[M][ld_out] = x[M][ldx] . W[N][ldw]^T, BF16 W; columns of x and W from K up to the next multiple of 32 are zero.
  * LM_ACT_SWIGLU: rows of W interleaved (gate, up), y[M][N / 2] = silu(gate) * up. splits > 1 (LM_ACT_NONE): that many
  * partial results, M * ld_out floats apart. With a table of row blocks (as for tc_gemm_grouped, M = 128 times
- * their number) a block uses the matrix that starts at row matrix * group_rows of W. */
+ * their number) a block uses the matrix that starts at row matrix * group_rows of W.
+ * lm_gemm_f32: up to kLmF32FewRows rows, or a table. lm_gemm_f32_many: the rows above, as three terms (`terms`: room for
+ * 3 * lm_gemm_f32_rows_pad(M) rows) through the row-block GEMM. */
 enum LmAct { LM_ACT_NONE = 0, LM_ACT_SWIGLU = 1, LM_ACT_RELU2 = 2 };
+constexpr int kLmF32FewRows = 32;
+inline int lm_gemm_f32_rows_pad(int M) { return M <= 256 ? 256 : (M + 127) / 128 * 128; }
 int lm_gemm_f32_splits(int M, int N, int K, int n_sm);
 int lm_gemm_f32(float *y, int ld_out, const float *x, int ldx, const uint16_t *W, int ldw, int M, int N, int K, LmAct act,
                 cudaStream_t st, int splits = 1, const int4 *table = nullptr, int group_rows = 0);
+struct TcWeight;
+int lm_gemm_f32_many(float *y, int ld_out, const float *x, int ldx, const TcWeight &w, uint16_t *terms, int M, bool swiglu, cudaStream_t st,
+                     int splits, int *status);
 
 /* Largest logit of row 0 (first one on a tie) becomes the next token: tokens[0], log[dyn->logged++];
  * the sequence moves on by the `rows` positions just run. */

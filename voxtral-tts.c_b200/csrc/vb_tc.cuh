@@ -108,6 +108,7 @@ constexpr int kTcJoinSplits = 4;
 struct TcGemm {
     int M = 0, splits = 1, epi = TC_EPI_STORE;
     int segment = 32;                 /* 65 rows and more: k-blocks that are summed in TMEM, at most, before registers take over */
+    int terms = 2;                    /* the same: terms of the rows that are multiplied, 2 or 3 */
     bool exact = false;               /* up to 16 rows: four accumulators in place of two (see TcCfg) */
     float *out = nullptr;
     int ld_out = 0;
@@ -148,10 +149,10 @@ void tc_prepare(const TcActs &acts, const float *x, int ldx, int M, const float 
                 cudaStream_t st, const TcWait &wait = TcWait(), float *tap = nullptr);
 
 int tc_gemm(const TcWeight &w, const TcActs &acts, const TcGemm &g, cudaStream_t st);
-/* rows_pad >= 256 (vb_tc_rows.cu; two terms of the activations are read): what tc_gemm calls for them, and the K splits
- * that suit M rows. */
+/* Many rows (vb_tc_rows.cu; two or three terms of the activations are read): what tc_gemm calls from rows_pad = 256 on, and
+ * the K splits that suit M rows. */
 int tc_gemm_rows(const TcWeight &w, const TcActs &acts, const TcGemm &g, cudaStream_t st);
-int tc_row_splits(int N, int K, int M, int n_sm);
+int tc_row_splits(int N, int K, int M, int n_sm, int terms = 2);
 /* [rows, cols] BF16 row-major as a tensor map; box = 64 columns x box_rows rows, 128-byte swizzle. */
 int tc_map(CUtensorMap *m, const void *base, uint64_t rows, uint64_t cols, uint32_t box_rows);
 /* The same of `planes` such matrices, with row and plane pitches in bytes. */

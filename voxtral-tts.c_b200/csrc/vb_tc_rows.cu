@@ -1,7 +1,8 @@
 /*
  * vb_tc_rows.cu - the tensor-core GEMM for many activation rows (65 and more): prompts, the codec, mixtures of experts.
  *
- *   y[M,N] = x[M,K] . W[N,K]^T, BF16 W, x as hi + lo BF16 terms (16 mantissa bits: 4e-6 relative), fp32 sums
+ *   y[M,N] = x[M,K] . W[N,K]^T, BF16 W, x as hi + lo BF16 terms (16 mantissa bits: 4e-6 relative) or, for the language
+ *   models' 32-bit mode, as three (24 bits), fp32 sums
  *
  * A pair of CTAs (one cluster, tcgen05 cta_group::2) owns 256 weight rows x R activation rows: each CTA brings in its
  * own 128 weight rows and half of the activation rows, and every MMA (256 x R x 16) reads both halves. What bounds a
@@ -21,6 +22,10 @@
  * 4.9e-5 so, 63.3 ms and 3.3e-5 with 1024 columns (and 66 to 69 ms where eight warps held 128 values and spilled). The
  * codec, whose K splits are fewer than before this kernel, takes 1024 (TcGemm::segment).
  *
+ * Three terms: R <= 128, and the two low terms have a sum of their own, so that the high one is cut off a third as often; the
+ * stages keep 40 KB (a k-block costs 512 + 3 R clocks of shared memory, 6 R of the tensor pipe). The epilogue adds a
+ * segment up within the time of its main loop down to a single k-block (vb_lm_gemm32.cu has the figures).
+ *
  * Warps: 0-15 epilogue (TMEM -> registers -> shared memory -> whole 512-byte row segments), 16 TMA producer, 17 MMA issuer (of the even
  * CTA, for both). Full barriers and the accumulator hand-back live in the even CTA; commits arrive in both. No
  * multicast loads. All waits are bounded.
@@ -35,14 +40,17 @@ namespace vb {
 
 namespace {
 
-constexpr int kPrMaxRows = 256, kPrTerms = 2, kPrStages = 4, kPrChunk = 64;
-constexpr int kPrStageW = kTcTileN * kTcBlockK * 2, kPrStageX = kPrMaxRows / 2 * kTcBlockK * 2;
-constexpr int kPrStage = kPrStageW + kPrTerms * kPrStageX;
+constexpr int kPrStages = 4, kPrChunk = 64, kPrAcc = 256;      /* kPrAcc: TMEM columns of an accumulator */
+constexpr int kPrStageW = kTcTileN * kTcBlockK * 2;
 constexpr int kPrStaging = kPrChunk * kTcTileN * 4;
 constexpr int kPrEpiWarps = 16, kPrEpi = 32 * kPrEpiWarps, kPrThreads = kPrEpi + 64;
-constexpr int kPrSmemBytes = kPrStages * kPrStage + kPrStaging + kPrMaxRows * 4 + 256 + 1024;
-static_assert(kPrSmemBytes <= 232448, "over the 227 KB a CTA may use");
 constexpr uint32_t kPrTmemCols = 512;
+template <int TERMS> struct PrCfg {
+    static constexpr int max_rows = TERMS == 3 ? 128 : 256;
+    static constexpr int stage_x = max_rows / 2 * kTcBlockK * 2, stage = kPrStageW + TERMS * stage_x;
+    static constexpr int smem = kPrStages * stage + kPrStaging + max_rows * 4 + 256 + 1024;
+    static_assert(smem <= 232448, "over the 227 KB a CTA may use");
+};
 
 struct RowsArgs {
     float *out;
@@ -129,6 +137,7 @@ VB_DEVINL PrTile pr_tile(const RowsArgs &a, int i, int kblocks) {
 VB_DEVINL uint32_t pr_pack(uint16_t a, uint16_t b) { return a | ((uint32_t)b << 16); }
 
 /* Rows [c0, c0 + 64) of a tile's results, staged as [row][128 columns], to where they belong; `t` is this CTA's weight tile. */
+template <int TERMS>
 VB_DEVINL void pr_store(const RowsArgs &a, const float *stg, const PrTile &tl, int t, int c0, int warp, int lane) {
     const int n = t * kTcTileN + lane * 4, end = min(tl.Mb, c0 + kPrChunk);
     if (a.epi == TC_EPI_SWIGLU || a.epi == TC_EPI_SWIGLU_TERMS) {
@@ -149,7 +158,7 @@ VB_DEVINL void pr_store(const RowsArgs &a, const float *stg, const PrTile &tl, i
                 vb_split3(r0, p[0], p[1], p[2]);
                 vb_split3(r1, q[0], q[1], q[2]);
 #pragma unroll
-                for (int j = 0; j < kPrTerms; j++) {
+                for (int j = 0; j < TERMS; j++) {
                     uint16_t *o = a.out_terms + ((size_t)j * a.out_rows_pad + m) * ko + col;
                     if (both && (ko & 1) == 0) {
                         *(uint32_t *)o = pr_pack(p[j], q[j]);
@@ -175,7 +184,7 @@ VB_DEVINL void pr_store(const RowsArgs &a, const float *stg, const PrTile &tl, i
                 vb_split3(e[i], q[0][i], q[1][i], q[2][i]);
             }
 #pragma unroll
-            for (int j = 0; j < kPrTerms; j++) {
+            for (int j = 0; j < TERMS; j++) {
                 uint16_t *o = a.out_terms + ((size_t)j * a.out_rows_pad + tl.m0 + mb) * a.out_terms_ld + col;
                 if (n + 3 < a.N) {
                     *(uint2 *)o = make_uint2(pr_pack(q[j][0], q[j][1]), pr_pack(q[j][2], q[j][3]));
@@ -202,16 +211,17 @@ VB_DEVINL void pr_store(const RowsArgs &a, const float *stg, const PrTile &tl, i
     }
 }
 
-template <bool GROUPED>
+template <bool GROUPED, int TERMS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPrThreads, 1)
 vb_tc_pair_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const RowsArgs a) {
     pdl_launch_dependents();
     extern __shared__ unsigned char pr_smem_raw[];
     unsigned char *base = (unsigned char *)(((uintptr_t)pr_smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char *stages = base;
-    float *stg = (float *)(base + kPrStages * kPrStage);
+    using C = PrCfg<TERMS>;
+    float *stg = (float *)(base + kPrStages * C::stage);
     float *rscale = (float *)((unsigned char *)stg + kPrStaging);
-    uint64_t *full = (uint64_t *)(rscale + kPrMaxRows);
+    uint64_t *full = (uint64_t *)(rscale + C::max_rows);
     uint64_t *empty = full + kPrStages;
     uint64_t *done = empty + kPrStages;      /* accumulator finished, [2] */
     uint64_t *drained = done + 2;            /* accumulator read by both CTAs, [2] */
@@ -243,22 +253,22 @@ vb_tc_pair_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
 
     if (warp == kPrEpiWarps && lane == 0) {
         /* ---- TMA producer of this CTA; the bytes of both count on the even CTA's barriers ---- */
-        const uint32_t x_bytes = (uint32_t)(a.R / 2) * kTcBlockK * 2, tx = 2u * (kPrStageW + kPrTerms * x_bytes);
+        const uint32_t x_bytes = (uint32_t)(a.R / 2) * kTcBlockK * 2, tx = 2u * (kPrStageW + TERMS * x_bytes);
         uint32_t full_bar[kPrStages];
 #pragma unroll
         for (int s = 0; s < kPrStages; s++) full_bar[s] = pr_leader(&full[s]);
         auto load_w = [&](const PrTile &t, int it, uint32_t s) {
-            unsigned char *sa = stages + (size_t)s * kPrStage;
+            unsigned char *sa = stages + (size_t)s * C::stage;
             const int tile = t.w0 + (int)rank;      /* beyond the last tile: zeros */
             if (a.a_tiled) pr_load(sa, &mapA, 0, (tile * kblocks + t.kb0 + it) * kTcTileN, full_bar[s]);
             else pr_load(sa, &mapA, (t.kb0 + it) * kTcBlockK, tile * kTcTileN, full_bar[s]);
         };
         auto load_x = [&](const PrTile &t, int it, uint32_t s) {
-            unsigned char *sx = stages + (size_t)s * kPrStage + kPrStageW;
+            unsigned char *sx = stages + (size_t)s * C::stage + kPrStageW;
             const int row = t.m0 + (int)rank * (t.n_mma >> 1);
 #pragma unroll
-            for (int j = 0; j < kPrTerms; j++)
-                pr_load(sx + j * kPrStageX, &mapB, (t.kb0 + it) * kTcBlockK, j * a.rows_pad + row, full_bar[s]);
+            for (int j = 0; j < TERMS; j++)
+                pr_load(sx + j * C::stage_x, &mapB, (t.kb0 + it) * kTcBlockK, j * a.rows_pad + row, full_bar[s]);
         };
         bool ok = true, first = true;
         if constexpr (GROUPED) pdl_wait();          /* the table is made by an earlier kernel */
@@ -310,7 +320,7 @@ vb_tc_pair_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
             if (!t.used) continue;
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(t.n_mma >> 3) << 17) | ((uint32_t)(2 * kTcTileN >> 4) << 24);
             for (int it = 0; it < t.n_it && ok; n++) {
-                const uint32_t acc = n & 1u, d = tmem + acc * kPrMaxRows;
+                const uint32_t acc = n & 1u, d = tmem + acc * kPrAcc;
                 const int end = min(t.n_it, it + t.seg);
                 if (!vb_mbar_wait(&drained[acc], ((n >> 1) & 1u) ^ 1u, abort_flag)) {
                     atomicCAS(a.status, 0, 15);
@@ -328,13 +338,17 @@ vb_tc_pair_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
                         break;
                     }
                     tc_fence_after();
-                    const unsigned char *sa = stages + (size_t)s * kPrStage;
+                    const unsigned char *sa = stages + (size_t)s * C::stage;
                     const uint64_t adesc = umma_desc_k_sw128(sa);
 #pragma unroll
-                    for (int j = 0; j < kPrTerms; j++) {
-                        const uint64_t bdesc = umma_desc_k_sw128(sa + kPrStageW + j * kPrStageX);
+                    for (int j = 0; j < TERMS; j++) {
+                        const uint64_t bdesc = umma_desc_k_sw128(sa + kPrStageW + j * C::stage_x);
 #pragma unroll
-                        for (int q = 0; q < kTcBlockK / 16; q++) pr_mma(d, adesc + 2 * q, bdesc + 2 * q, idesc, (!first || (j | q) != 0) ? 1u : 0u);
+                        for (int q = 0; q < kTcBlockK / 16; q++) {
+                            /* three terms: the second and third have sums of their own */
+                            const bool low = TERMS == 3 && j > 0;
+                            pr_mma(low ? d + kPrAcc / 2 : d, adesc + 2 * q, bdesc + 2 * q, idesc, (!first || q > 0 || j > (low ? 1 : 0)) ? 1u : 0u);
+                        }
                     }
                     pr_commit(&empty[s]);
                 }
@@ -360,10 +374,10 @@ vb_tc_pair_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
                 vb_named_bar(1, kPrEpi);
             }
             /* this thread's column of the weight tile, rows part * 16 .. of every 64 */
-            constexpr int kChunks = kPrMaxRows / kPrChunk;
+            constexpr int kChunks = C::max_rows / kPrChunk;
             float sum[kChunks][16];
             for (int it = 0; it < t.n_it; it += t.seg, n++) {
-                const uint32_t acc = n & 1u, d = tmem + acc * kPrMaxRows + ((uint32_t)(lq * 32) << 16) + (uint32_t)(part * 16);
+                const uint32_t acc = n & 1u, d = tmem + acc * kPrAcc + ((uint32_t)(lq * 32) << 16) + (uint32_t)(part * 16);
                 /* after a wait that ran out the others fail at once: no thread leaves the barriers alone */
                 if (!vb_mbar_wait(&done[acc], (n >> 1) & 1u, abort_flag)) {
                     atomicCAS(a.status, 0, 13);
@@ -376,6 +390,12 @@ vb_tc_pair_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
                     if (q * kPrChunk + part * 16 < t.Mb) {
                         uint32_t r[16];
                         tmem_ld16(d + (uint32_t)(q * kPrChunk), r);
+                        if constexpr (TERMS == 3) {
+                            uint32_t low[16];
+                            tmem_ld16(d + (uint32_t)(kPrAcc / 2 + q * kPrChunk), low);
+#pragma unroll
+                            for (int j = 0; j < 16; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(low[j]));
+                        }
                         if (it == 0) {
 #pragma unroll
                             for (int j = 0; j < 16; j++) sum[q][j] = __uint_as_float(r[j]);
@@ -402,7 +422,7 @@ vb_tc_pair_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
                         }
                 }
                 vb_named_bar(1, kPrEpi);
-                pr_store(a, stg, t, t.t0 + (int)rank, c0, warp, lane);
+                pr_store<TERMS>(a, stg, t, t.t0 + (int)rank, c0, warp, lane);
                 vb_named_bar(1, kPrEpi);
             }
         }
@@ -434,37 +454,38 @@ int sm_pairs() {
 }
 
 /* Clocks of a launch with tiles of R rows, as the note at the top counts them: a k-block costs the larger of the tensor
- * pipe's 4 R and shared memory's 384 + 2 R clocks; the epilogue of the last tile is not hidden. */
-long long launch_cost(int M, int pairs, int k_iters, int splits, int clusters, int R) {
+ * pipe's 2 R a term and shared memory's (16 + 8 R / 64 KB read and as many written per term, and 16 KB of weights); the
+ * epilogue of the last tile is not hidden. */
+long long launch_cost(int M, int pairs, int k_iters, int splits, int clusters, int R, int terms) {
     const long long tiles = (long long)pairs * ((M + R - 1) / R) * splits;
-    return (tiles + clusters - 1) / clusters * (k_iters * (long long)(std::max(4 * R, 384 + 2 * R) + 24) + 200) + 24 * R;
+    return (tiles + clusters - 1) / clusters * (k_iters * (long long)(std::max(2 * terms * R, 128 * (1 + terms) + terms * R) + 24) + 200) + 24 * R;
 }
-int pick_rows(int M, int pairs, int k_iters, int splits, int clusters) {
+int pick_rows(int M, int pairs, int k_iters, int splits, int clusters, int terms) {
     int best = 0;
     long long cost = 0;
-    for (int R = kPrMaxRows; R >= 64; R -= 32) {
+    for (int R = terms == 3 ? PrCfg<3>::max_rows : PrCfg<2>::max_rows; R >= 64; R -= 32) {
         if (R > 64 && R >= M + 32) continue;
-        const long long c = launch_cost(M, pairs, k_iters, splits, clusters, R);
+        const long long c = launch_cost(M, pairs, k_iters, splits, clusters, R, terms);
         if (!best || c < cost) { best = R; cost = c; }
     }
     return best;
 }
 
-template <bool GROUPED>
+template <bool GROUPED, int TERMS>
 int launch_pair(const TcWeight &w, const TcActs &a, RowsArgs &ra, int clusters, cudaStream_t st) {
     static bool attr = false;
     if (!attr) {
-        if (cudaFuncSetAttribute(vb_tc_pair_kernel<GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrSmemBytes) != cudaSuccess) {
+        if (cudaFuncSetAttribute(vb_tc_pair_kernel<GROUPED, TERMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, PrCfg<TERMS>::smem) != cudaSuccess) {
             cudaGetLastError();
             return -1;
         }
         attr = true;
     }
     CUtensorMap map;
-    if (tc_map(&map, a.buf, (uint64_t)kPrTerms * a.rows_pad, (uint64_t)a.K, (uint32_t)ra.R / 2)) return -1;
+    if (tc_map(&map, a.buf, (uint64_t)TERMS * a.rows_pad, (uint64_t)a.K, (uint32_t)ra.R / 2)) return -1;
     const long long tiles = (long long)ra.pairs * ra.row_blocks * ra.splits;
-    return launch_pdl(vb_tc_pair_kernel<GROUPED>, dim3(2 * (unsigned)std::min<long long>(tiles, clusters)), dim3(kPrThreads),
-                      (size_t)kPrSmemBytes, st, w.map, map, ra) == cudaSuccess
+    return launch_pdl(vb_tc_pair_kernel<GROUPED, TERMS>, dim3(2 * (unsigned)std::min<long long>(tiles, clusters)), dim3(kPrThreads),
+                      (size_t)PrCfg<TERMS>::smem, st, w.map, map, ra) == cudaSuccess
                ? 0
                : -1;
 }
@@ -484,14 +505,14 @@ bool terms_epilogue_ok(const TcGemm &g) {
 
 } // namespace
 
-int tc_row_splits(int N, int K, int M, int n_sm) {
+int tc_row_splits(int N, int K, int M, int n_sm, int terms) {
     const int pairs = ((N + kTcTileN - 1) / kTcTileN + 1) / 2, clusters = n_sm / 2, kblocks = K / kTcBlockK;
     int best = 1;
     long long cost = 0;
     for (int s = 1; s <= std::min(kTcMaxSplits, kblocks); s++) {
         const int it = (kblocks + s - 1) / s;
         /* a further partial result is M rows of N written and read again: about 4 values per clock and pair */
-        const long long c = launch_cost(M, pairs, it, s, clusters, pick_rows(M, pairs, it, s, clusters)) +
+        const long long c = launch_cost(M, pairs, it, s, clusters, pick_rows(M, pairs, it, s, clusters, terms), terms) +
                             (long long)s * M * N / (4LL * clusters);
         if (s == 1 || c < cost) { best = s; cost = c; }
     }
@@ -507,15 +528,15 @@ int tc_gemm_rows(const TcWeight &w, const TcActs &a, const TcGemm &g, cudaStream
     RowsArgs ra = rows_args(w, a, g);
     ra.N = w.N; ra.M = g.M;
     ra.pairs = ((w.N + kTcTileN - 1) / kTcTileN + 1) / 2;
-    ra.R = pick_rows(g.M, ra.pairs, (w.K / kTcBlockK + g.splits - 1) / g.splits, g.splits, clusters);
+    ra.R = pick_rows(g.M, ra.pairs, (w.K / kTcBlockK + g.splits - 1) / g.splits, g.splits, clusters, g.terms);
     ra.row_blocks = (g.M + ra.R - 1) / ra.R;
-    return launch_pair<false>(w, a, ra, clusters, st);
+    return g.terms == 3 ? launch_pair<false, 3>(w, a, ra, clusters, st) : launch_pair<false, 2>(w, a, ra, clusters, st);
 }
 
 int tc_gemm_grouped(const TcWeight &w, const TcActs &a, const TcGemm &g, int n, const int4 *table, int n_blocks, cudaStream_t st) {
     constexpr int kRows = 128;
     const int tiles = (n + kTcTileN - 1) / kTcTileN;
-    if (!w.ok || !w.tiled || !a.ok || w.K != a.K || n < 1 || n_blocks < 1 || !table || g.splits != 1) return -1;
+    if (!w.ok || !w.tiled || !a.ok || w.K != a.K || n < 1 || n_blocks < 1 || !table || g.splits != 1 || g.terms != 2) return -1;
     if (w.N % (tiles * kTcTileN) || (size_t)n_blocks * kRows > (size_t)a.rows_pad || g.act_n0 != 0) return -1;
     if (g.epi == TC_EPI_TERMS || g.epi == TC_EPI_RELU2_TERMS) {
         if (!terms_epilogue_ok(g) || g.out_rows_pad < n_blocks * kRows) return -1;
@@ -531,7 +552,7 @@ int tc_gemm_grouped(const TcWeight &w, const TcActs &a, const TcGemm &g, int n, 
     ra.row_blocks = n_blocks;
     ra.pairs = (tiles + 1) / 2;
     ra.table = table; ra.group_tiles = tiles;
-    return launch_pair<true>(w, a, ra, clusters, st);
+    return launch_pair<true, 2>(w, a, ra, clusters, st);
 }
 
 } // namespace vb
