@@ -17,6 +17,8 @@
 #include "vb_attn_tc.cuh"
 #include "vb_tc.cuh"
 
+#include <algorithm>
+
 namespace vb {
 
 namespace {
@@ -101,27 +103,91 @@ __global__ void __launch_bounds__(kPrepThreads) lm_attn_prepare_kernel(const LmA
     }
 }
 
-/* ------------------------------------------------------------------ generic kernel */
-constexpr int kGaThreads = 256, kGaKeys = 32, kGaPairs = kLmAttnPairs;
+/* ------------------------------------------------------------------ any sizes, fp32 pipes */
+/* PAIRS (row, query head) pairs of a KV head per CTA, 64 keys at a time; a thread holds PAIRS / 16 pairs x 4 keys of the
+ * scores, then the same pairs x 4 * NV columns of the result, as packed fp32 pairs, so that a 16-byte read of shared
+ * memory serves 4 to 16 multiply-adds. (Scores by dot products of a lane each, results a column a time through shared
+ * memory: 390 rows of 16 heads of 128 took 405 us a layer, five rows at 400 keys 70 us.) 64 pairs for prompts, two
+ * CTAs an SM at heads of 128; 16 for a few rows, where the keys are split over CTAs and tiles of 64 pairs would be
+ * mostly empty. The last split to arrive merges in split order. */
+constexpr int kGaThreads = 256, kGaKeys = 64, kGaManyPairs = 64;
 
-inline size_t ga_smem(int dim, int vdim) {
-    return sizeof(float) * ((size_t)kGaPairs * dim + (size_t)kGaKeys * (dim + 1) + (size_t)kGaKeys * vdim +
-                            (size_t)kGaPairs * vdim + kGaPairs * (kGaKeys + 1) + 4 * kGaPairs + kLmAttnSplits * kGaPairs);
+typedef unsigned long long f2;   /* two packed floats */
+VB_DEVINL f2 f2_fma(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+VB_DEVINL f2 f2_mul(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+VB_DEVINL f2 f2_two(float v) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+    return r;
+}
+VB_DEVINL float2 f2_get(f2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
 }
 
-/* grid = (tiles of 16 (row, head) pairs, KV heads, key splits) */
+/* rows of a multiple of four floats; an odd number of 16-byte pieces, so that eight rows' pieces lie in different banks */
+inline __host__ __device__ int ga_ld(int n) { const int v = (n + 3) / 4 + 1; return 4 * (v | 1); }
+inline __host__ __device__ int ga_stride(int vdim) { return (vdim + 3) / 4 * 4 + 4; }   /* a pair's partial result: columns, maximum, sum */
+constexpr int kGaLdP = kGaKeys + 4;
+inline size_t ga_smem(int pairs, int dim, int vdim) {
+    return sizeof(float) * ((size_t)pairs * ga_ld(dim) + std::max(kGaKeys * ga_ld(dim), pairs * kGaLdP) + (size_t)kGaKeys * ((vdim + 3) / 4 * 4));
+}
+
+/* n rows of `size` floats or halves into shared memory, rows up to kGaKeys and columns up to a multiple of four as zeros; a warp takes
+ * every eighth row. True where a value is not finite. */
+template <bool SPLIT, typename Row>
+VB_DEVINL bool ga_load(float *to, int ld, int size, int n, const Row &row, int warp, int lane) {
+    const int pieces = (size + 3) / 4;
+    bool odd = false;
+    for (int c = lane; c < pieces; c += 32) {
+        float4 v[kGaKeys / 8];
+#pragma unroll
+        for (int i = 0; i < kGaKeys / 8; i++) {
+            const int j = warp + 8 * i;
+            v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (j >= n) continue;
+            const float *head = row(j);
+            if ((size & 3) == 0) {
+                v[i] = kv_get4<SPLIT>(head, size, 4 * c);
+            } else {
+                v[i].x = kv_get(head, size, 4 * c, SPLIT);
+                if (4 * c + 1 < size) v[i].y = kv_get(head, size, 4 * c + 1, SPLIT);
+                if (4 * c + 2 < size) v[i].z = kv_get(head, size, 4 * c + 2, SPLIT);
+                if (4 * c + 3 < size) v[i].w = kv_get(head, size, 4 * c + 3, SPLIT);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < kGaKeys / 8; i++) {
+            *(float4 *)(to + (size_t)(warp + 8 * i) * ld + 4 * c) = v[i];
+            odd |= !(fabsf(v[i].x) < INFINITY && fabsf(v[i].y) < INFINITY && fabsf(v[i].z) < INFINITY && fabsf(v[i].w) < INFINITY);
+        }
+    }
+    return odd;
+}
+
+/* grid = (tiles of pairs, KV heads, key splits) */
+template <int PAIRS, int NV, bool SPLIT>
 __global__ void __launch_bounds__(kGaThreads) lm_attn_generic_kernel(const LmAttn a, int M) {
-    extern __shared__ float ga[];
+    constexpr int TP = PAIRS / 16, TK = kGaKeys / 16;
+    extern __shared__ __align__(16) float ga[];
+    __shared__ float wgt[kLmAttnSplits][PAIRS], total[PAIRS];
     __shared__ int last_flag;
     pdl_launch_dependents();
     pdl_wait();
-    const int dim = a.dim, vdim = a.vdim, group = a.heads / a.kv_heads;
-    float *Q = ga, *K = Q + kGaPairs * dim, *V = K + kGaKeys * (dim + 1), *O = V + kGaKeys * vdim;
-    float *S = O + kGaPairs * vdim, *mx = S + kGaPairs * (kGaKeys + 1), *den = mx + kGaPairs, *cor = den + kGaPairs,
-          *wgt = cor + 2 * kGaPairs;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int g = blockIdx.y, p0 = blockIdx.x * kGaPairs;
-    const int np = M * group - p0 < kGaPairs ? M * group - p0 : kGaPairs;
+    const int dim = a.dim, vdim = a.vdim, group = a.heads / a.kv_heads, ld = ga_ld(dim), ldv = (vdim + 3) / 4 * 4;
+    float *Q = ga, *K = Q + PAIRS * ld, *P = K, *V = K + (kGaKeys * ld > PAIRS * kGaLdP ? kGaKeys * ld : PAIRS * kGaLdP);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, tx = tid & 15, ty = tid >> 4;
+    const int g = blockIdx.y, p0 = blockIdx.x * PAIRS;
+    const int np = M * group - p0 < PAIRS ? M * group - p0 : PAIRS;
     const int pos0 = a.dyn->pos;
     const KeyTiles kt = key_tiles<kGaKeys>(pos0 + p0 / group, pos0 + (p0 + np - 1) / group, a.window, a.keep);
     const int S_eff = (int)gridDim.z < kt.n_tiles ? (int)gridDim.z : kt.n_tiles;
@@ -129,80 +195,110 @@ __global__ void __launch_bounds__(kGaThreads) lm_attn_generic_kernel(const LmAtt
     if (sp >= S_eff) return;
     const int t0 = (int)((long long)kt.n_tiles * sp / S_eff), t1 = (int)((long long)kt.n_tiles * (sp + 1) / S_eff);
     const float *Kc = lm_state(a.k, a.dyn), *Vc = lm_state(a.v, a.dyn);
-    const int ldk = a.kv_heads * dim, ldv = a.kv_heads * vdim;
 
-    for (int i = tid; i < np * dim; i += kGaThreads) {
-        const int p = p0 + i / dim, d = i % dim;
-        Q[i] = a.q[(size_t)(p / group) * a.heads * dim + (size_t)(g * group + p % group) * dim + d];
+    for (int p = warp; p < PAIRS; p += kGaThreads / 32) {
+        const float *q = a.q + (size_t)((p0 + p) / group) * a.heads * dim + (size_t)(g * group + (p0 + p) % group) * dim;
+        for (int d = lane; d < (dim + 3) / 4 * 4; d += 32) Q[p * ld + d] = p < np && d < dim ? __ldcg(q + d) : 0.0f;
     }
-    for (int i = tid; i < np * vdim; i += kGaThreads) O[i] = 0.0f;
-    if (tid < kGaPairs) { mx[tid] = -INFINITY; den[tid] = 0.0f; }
+    float mx[TP], den[TP];
+    f2 o[TP][2 * NV];
+    int at[TP];                                  /* positions of this thread's rows */
+#pragma unroll
+    for (int i = 0; i < TP; i++) {
+        mx[i] = -INFINITY;
+        den[i] = 0.0f;
+        at[i] = pos0 + (p0 + ty * TP + i) / group;
+#pragma unroll
+        for (int c = 0; c < 2 * NV; c++) o[i][c] = 0ull;
+    }
 
     for (int t = t0; t < t1; t++) {
         int j0, n;
         key_tile<kGaKeys>(kt, t, &j0, &n);
-        __syncthreads();
-        for (int i = tid; i < n * dim; i += kGaThreads) {
-            const int j = i / dim, d = i % dim;
-            K[j * (dim + 1) + d] = kv_get(Kc + (size_t)lm_ring_row(a.ring, j0 + j) * ldk + g * dim, dim, d, a.split);
-        }
-        for (int i = tid; i < n * vdim; i += kGaThreads) {
-            const int j = i / vdim, d = i % vdim;
-            V[i] = kv_get(Vc + (size_t)lm_ring_row(a.ring, j0 + j) * ldv + g * vdim, vdim, d, a.split);
-        }
-        __syncthreads();
-        for (int p = warp; p < np; p += kGaThreads / 32) {
-            const int i = pos0 + (p0 + p) / group;
-            float s = -INFINITY;
-            if (lane < n && key_seen(i, j0 + lane, a.window, a.keep)) {
-                const float *q = Q + p * dim, *k = K + lane * (dim + 1);
-                float e0 = 0.0f, e1 = 0.0f, e2 = 0.0f, e3 = 0.0f;
-                int d = 0;
-                for (; d + 3 < dim; d += 4) {
-                    e0 = fmaf(q[d], k[d], e0);
-                    e1 = fmaf(q[d + 1], k[d + 1], e1);
-                    e2 = fmaf(q[d + 2], k[d + 2], e2);
-                    e3 = fmaf(q[d + 3], k[d + 3], e3);
-                }
-                for (; d < dim; d++) e0 = fmaf(q[d], k[d], e0);
-                s = ((e0 + e1) + (e2 + e3)) * a.scale;
-                if (a.softcap > 0.0f) s = a.softcap * tanhf(s / a.softcap);
-            }
-            float top = s;
+        __syncthreads();                         /* the last tile is read */
+        ga_load<SPLIT>(K, ld, dim, n, [&](int j) { return Kc + ((size_t)lm_ring_row(a.ring, j0 + j) * a.kv_heads + g) * dim; }, warp, lane);
+        const bool odd = ga_load<SPLIT>(V, ldv, vdim, n, [&](int j) { return Vc + ((size_t)lm_ring_row(a.ring, j0 + j) * a.kv_heads + g) * vdim; }, warp, lane);
+        const bool any_odd = __syncthreads_or(odd);
+        f2 acc[TP][TK] = {};
+#pragma unroll 4
+        for (int d = 0; d < dim; d += 4) {
+            ulonglong2 q[TP], k[TK];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-            const float old = mx[p], now = fmaxf(old, top);
-            const float w = s > -INFINITY ? expf(s - now) : 0.0f;
-            const float sum = vb_warp_sum(w);
-            S[p * (kGaKeys + 1) + lane] = w;
-            __syncwarp();
-            if (lane == 0) {
-                const float c = old > -INFINITY ? expf(old - now) : 0.0f;
-                cor[p] = c;
-                mx[p] = now;
-                den[p] = den[p] * c + sum;
-            }
+            for (int i = 0; i < TP; i++) q[i] = *(const ulonglong2 *)(Q + (ty * TP + i) * ld + d);
+#pragma unroll
+            for (int j = 0; j < TK; j++) k[j] = *(const ulonglong2 *)(K + (tx + 16 * j) * ld + d);
+#pragma unroll
+            for (int i = 0; i < TP; i++)
+#pragma unroll
+                for (int j = 0; j < TK; j++) acc[i][j] = f2_fma(q[i].y, k[j].y, f2_fma(q[i].x, k[j].x, acc[i][j]));
         }
-        __syncthreads();
-        for (int i = tid; i < np * vdim; i += kGaThreads) {
-            const int p = i / vdim, d = i % vdim;
-            float o = O[i] * cor[p];
-            const float *w = S + p * (kGaKeys + 1);
-            for (int j = 0; j < n; j++) o = fmaf(w[j], V[j * vdim + d], o);
-            O[i] = o;
+        __syncthreads();                         /* weights take the keys' place */
+#pragma unroll
+        for (int i = 0; i < TP; i++) {
+            float s[TK], top = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < TK; j++) {
+                const int key = tx + 16 * j;
+                const float2 e = f2_get(acc[i][j]);
+                s[j] = (e.x + e.y) * a.scale;
+                if (a.softcap > 0.0f) s[j] = a.softcap * tanhf(s[j] / a.softcap);
+                if (key >= n || !key_seen(at[i], j0 + key, a.window, a.keep)) s[j] = -INFINITY;
+                top = fmaxf(top, s[j]);
+            }
+#pragma unroll
+            for (int u = 8; u > 0; u >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, u));
+            const float now = fmaxf(mx[i], top), c = mx[i] > -INFINITY ? expf(mx[i] - now) : 0.0f;
+            float sum = 0.0f;
+#pragma unroll
+            for (int j = 0; j < TK; j++) {
+                const float w = s[j] > -INFINITY ? expf(s[j] - now) : 0.0f;
+                P[(ty * TP + i) * kGaLdP + tx + 16 * j] = w;
+                sum += w;
+            }
+#pragma unroll
+            for (int u = 8; u > 0; u >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, u);
+            den[i] = den[i] * c + sum;
+            mx[i] = now;
+#pragma unroll
+            for (int v = 0; v < 2 * NV; v++) o[i][v] = f2_mul(o[i][v], f2_two(c));
+        }
+        __syncwarp();                            /* a pair's weights are read by the half warp that wrote them */
+        for (int j = 0; j < n; j += 4) {         /* rows from n on are zeros */
+            float4 w[TP];
+#pragma unroll
+            for (int i = 0; i < TP; i++) w[i] = *(const float4 *)(P + (ty * TP + i) * kGaLdP + j);
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+#pragma unroll
+                for (int c = 0; c < NV; c++) {
+                    const int col = 64 * c + 4 * tx;
+                    if (col >= ldv) continue;
+                    const ulonglong2 v = *(const ulonglong2 *)(V + (j + u) * ldv + col);
+#pragma unroll
+                    for (int i = 0; i < TP; i++) {
+                        /* zero times what is not finite: only where the key is seen */
+                        if (any_odd && !(j + u < n && key_seen(at[i], j0 + j + u, a.window, a.keep))) continue;
+                        const f2 e = f2_two(u == 0 ? w[i].x : u == 1 ? w[i].y : u == 2 ? w[i].z : w[i].w);
+                        o[i][2 * c] = f2_fma(e, v.x, o[i][2 * c]);
+                        o[i][2 * c + 1] = f2_fma(e, v.y, o[i][2 * c + 1]);
+                    }
+                }
         }
     }
-    __syncthreads();
 
-    float *po = nullptr;
     if (S_eff > 1) {
         /* several CTAs share these pairs: publish the slice, the last arrival merges in slice order */
-        const int stride = vdim + 2;
+        const int stride = ga_stride(vdim);
         const size_t tile = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
-        po = a.scratch + tile * gridDim.z * kGaPairs * stride;
-        float *mine = po + (size_t)sp * kGaPairs * stride;
-        for (int i = tid; i < np * vdim; i += kGaThreads) mine[(i / vdim) * stride + i % vdim] = O[i];
-        if (tid < np) { mine[tid * stride + vdim] = mx[tid]; mine[tid * stride + vdim + 1] = den[tid]; }
+        float *po = a.scratch + tile * gridDim.z * PAIRS * stride;
+#pragma unroll
+        for (int i = 0; i < TP; i++) {
+            float *mine = po + ((size_t)sp * PAIRS + ty * TP + i) * stride;
+#pragma unroll
+            for (int c = 0; c < NV; c++)
+                if (64 * c + 4 * tx < ldv) *(ulonglong2 *)(mine + 64 * c + 4 * tx) = make_ulonglong2(o[i][2 * c], o[i][2 * c + 1]);
+            if (tx == 0) *(float2 *)(mine + ldv) = make_float2(mx[i], den[i]);
+        }
         __threadfence();
         __syncthreads();
         if (tid == 0) {
@@ -213,29 +309,55 @@ __global__ void __launch_bounds__(kGaThreads) lm_attn_generic_kernel(const LmAtt
         __syncthreads();
         if (!last_flag) return;
         __threadfence();
-        if (tid < np) {
+        if (tid < PAIRS) {
             float M0 = -INFINITY, L = 0.0f;
-            for (int u = 0; u < S_eff; u++) M0 = fmaxf(M0, __ldcg(po + ((size_t)u * kGaPairs + tid) * stride + vdim));
+            for (int u = 0; u < S_eff; u++) M0 = fmaxf(M0, __ldcg(po + ((size_t)u * PAIRS + tid) * stride + ldv));
             for (int u = 0; u < S_eff; u++) {
-                const float mu = __ldcg(po + ((size_t)u * kGaPairs + tid) * stride + vdim);
-                const float w = mu > -INFINITY ? expf(mu - M0) : 0.0f;
-                wgt[u * kGaPairs + tid] = w;
-                L += w * __ldcg(po + ((size_t)u * kGaPairs + tid) * stride + vdim + 1);
+                const float2 e = __ldcg((const float2 *)(po + ((size_t)u * PAIRS + tid) * stride + ldv));
+                const float w = e.x > -INFINITY ? expf(e.x - M0) : 0.0f;
+                wgt[u][tid] = w;
+                L += w * e.y;
             }
-            den[tid] = L;
+            total[tid] = L;
         }
         __syncthreads();
-        for (int i = tid; i < np * vdim; i += kGaThreads) {
-            const int p = i / vdim, d = i % vdim;
-            float o = 0.0f;
-            for (int u = 0; u < S_eff; u++) o = fmaf(wgt[u * kGaPairs + p], __ldcg(po + ((size_t)u * kGaPairs + p) * stride + d), o);
-            O[i] = o;
+#pragma unroll
+        for (int i = 0; i < TP; i++) {
+            den[i] = total[ty * TP + i];
+#pragma unroll
+            for (int c = 0; c < 2 * NV; c++) o[i][c] = 0ull;
         }
-        __syncthreads();
+        for (int u = 0; u < S_eff; u++)
+#pragma unroll
+            for (int i = 0; i < TP; i++) {
+                const float *from = po + ((size_t)u * PAIRS + ty * TP + i) * stride;
+                const f2 w = f2_two(wgt[u][ty * TP + i]);
+#pragma unroll
+                for (int c = 0; c < NV; c++) {
+                    if (64 * c + 4 * tx >= ldv) continue;
+                    const ulonglong2 v = __ldcg((const ulonglong2 *)(from + 64 * c + 4 * tx));
+                    o[i][2 * c] = f2_fma(w, v.x, o[i][2 * c]);
+                    o[i][2 * c + 1] = f2_fma(w, v.y, o[i][2 * c + 1]);
+                }
+            }
     }
-    for (int i = tid; i < np * vdim; i += kGaThreads) {
-        const int p = i / vdim, d = i % vdim, P = p0 + p;
-        lm_put(a.out, P / group, (g * group + P % group) * vdim + d, O[i] / den[p]);
+#pragma unroll
+    for (int i = 0; i < TP; i++) {
+        const int p = ty * TP + i, row = (p0 + p) / group, c0 = (g * group + (p0 + p) % group) * vdim;
+        if (p >= np) break;
+#pragma unroll
+        for (int c = 0; c < NV; c++) {
+            const int col = 64 * c + 4 * tx;
+            const float2 x = f2_get(o[i][2 * c]), y = f2_get(o[i][2 * c + 1]);
+            const float e[4] = {x.x / den[i], x.y / den[i], y.x / den[i], y.y / den[i]};
+            if ((vdim & 3) == 0) {
+                if (col < vdim) lm_put4(a.out, row, c0 + col, e);
+            } else {
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (col + u < vdim) lm_put(a.out, row, c0 + col + u, e[u]);
+            }
+        }
     }
 }
 
@@ -633,7 +755,7 @@ constexpr int kStepCtas = 148;           /* one-token kernel: one CTA per SM */
 
 size_t lm_attn_scratch_floats(int heads, int kv_heads, int vdim) {
     (void)heads; (void)kv_heads;
-    return (size_t)kSplitBudget * kLmAttnPairs * (vdim + 2);
+    return std::max((size_t)kSplitBudget * kGaManyPairs * ga_stride(vdim), (size_t)kSplitBudget * kLmAttnPairs * (vdim + 2));
 }
 int lm_attn_ticket_count(int heads, int kv_heads) {
     (void)heads; (void)kv_heads;
@@ -654,21 +776,33 @@ int lm_attn_prepare(const LmAttn &a, int M, cudaStream_t st) {
     return ok(launch_pdl(lm_attn_prepare_kernel, dim3(M), dim3(kPrepThreads), smem, st, a));
 }
 
-int lm_attn_generic(const LmAttn &a, int M, cudaStream_t st) {
-    const size_t smem = ga_smem(a.dim, a.vdim);
+template <int PAIRS, int NV, bool SPLIT>
+static int launch_generic(const LmAttn &a, int M, cudaStream_t st) {
+    const size_t smem = ga_smem(PAIRS, a.dim, a.vdim);
     if (smem > 200 * 1024) return -1;
-    static size_t set = 48 * 1024;
+    static size_t set = 32 * 1024;      /* 48 KB without asking, static arrays included */
     if (smem > set) {
-        if (cudaFuncSetAttribute(lm_attn_generic_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+        if (cudaFuncSetAttribute(lm_attn_generic_kernel<PAIRS, NV, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
             cudaGetLastError();
             return -1;
         }
         set = smem;
     }
-    const int tiles = (M * (a.heads / a.kv_heads) + kGaPairs - 1) / kGaPairs;
+    const int tiles = (M * (a.heads / a.kv_heads) + PAIRS - 1) / PAIRS;
     int splits = kSplitBudget / (tiles * a.kv_heads);
     splits = splits < 1 ? 1 : splits > kLmAttnSplits ? kLmAttnSplits : splits;
-    return ok(launch_pdl(lm_attn_generic_kernel, dim3(tiles, a.kv_heads, splits), dim3(kGaThreads), smem, st, a, M));
+    return ok(launch_pdl(lm_attn_generic_kernel<PAIRS, NV, SPLIT>, dim3(tiles, a.kv_heads, splits), dim3(kGaThreads), smem, st, a, M));
+}
+
+int lm_attn_generic(const LmAttn &a, int M, cudaStream_t st) {
+    if (a.dim > 256 || a.vdim > 256) return -1;
+    const bool many = M * (a.heads / a.kv_heads) > kGaManyPairs / 2, wide = a.vdim > 128;
+    if (many) {
+        if (wide) return a.split ? launch_generic<kGaManyPairs, 4, true>(a, M, st) : launch_generic<kGaManyPairs, 4, false>(a, M, st);
+        return a.split ? launch_generic<kGaManyPairs, 2, true>(a, M, st) : launch_generic<kGaManyPairs, 2, false>(a, M, st);
+    }
+    if (wide) return a.split ? launch_generic<kLmAttnPairs, 4, true>(a, M, st) : launch_generic<kLmAttnPairs, 4, false>(a, M, st);
+    return a.split ? launch_generic<kLmAttnPairs, 2, true>(a, M, st) : launch_generic<kLmAttnPairs, 2, false>(a, M, st);
 }
 
 bool lm_attn_mma_ok(int dim, int vdim) { return dim <= 128 && vdim <= 128 && dim % 8 == 0 && vdim % 8 == 0; }
