@@ -26,7 +26,8 @@ enum { VB200_LM_BF16 = 0, VB200_LM_F32 = 1 };
 
 typedef struct {
     int dtype;        /* VB200_LM_BF16: tensor-core GEMMs on the BF16 weights, fp32 activations as BF16 terms;
-                         VB200_LM_F32: every product on the fp32 pipes */
+                         VB200_LM_F32: no product of a row is rounded (three BF16 terms a value, 24 bits), sums as
+                         exact as the fp32 pipes make them */
     int max_seqs;     /* slots (0: 1) */
     int max_tokens;   /* longest sequence a slot can hold (0: 8192) */
     int block_rows;   /* longest stretch of a portion that runs at once (0: chosen by the library) */

@@ -368,8 +368,8 @@ bool acoustic_tc_ready() { return g_ac.ready; }
  * the launch (eight utterances, 24 frames: 118.4 ms joined, 113.8 ms so). */
 static bool joined(int rows) { return rows <= 16; }
 
-/* The layers on the rows in X6, whose terms are not made yet; `exact` as in TcGemm. */
-static int enqueue_layers(const AcBuffers &b, int ROWS, bool exact) {
+/* The layers on the rows in X6, whose terms are not made yet; `sums` as in TcGemm. */
+static int enqueue_layers(const AcBuffers &b, int ROWS, int sums) {
     const bool join = joined(ROWS);
     const int chunks = join ? D / kTcTileN : tc_prepare_chunks(D);
     const size_t psD = (size_t)ROWS * D;
@@ -383,7 +383,7 @@ static int enqueue_layers(const AcBuffers &b, int ROWS, bool exact) {
         if (l == 0) tc_prepare(b.aD, b.X6, D, ROWS, nullptr, 0, 0, nullptr, nullptr, L.attn_norm, b.ssq, st);
         else if (!join) tc_prepare(b.aD, nullptr, D, ROWS, b.part, t.s_w2, psD, b.X6, b.X6, L.attn_norm, b.ssq, st);
         TcGemm g;
-        g.M = ROWS; g.exact = exact; g.status = b.status;
+        g.M = ROWS; g.sums = sums; g.status = b.status;
         g.epi = TC_EPI_PARTIAL; g.out = b.part;
         g.splits = t.s_qkv; g.ld_out = QKV; g.ssq = b.ssq; g.ssq_chunks = l == 0 ? tc_prepare_chunks(D) : chunks;
         g.eps = VB200_NORM_EPS;
@@ -391,19 +391,19 @@ static int enqueue_layers(const AcBuffers &b, int ROWS, bool exact) {
         launch_pdl(ac_attention_kernel, dim3((ROWS * VB200_HEADS * 32 + 255) / 256), dim3(256), 0, st, b.bQ,
                    (const float *)b.part, t.s_qkv, scale, ROWS, b.rows_pad);
         g = TcGemm();
-        g.M = ROWS; g.exact = exact; g.status = b.status;
+        g.M = ROWS; g.sums = sums; g.status = b.status;
         g.epi = TC_EPI_PARTIAL; g.out = b.part; g.splits = t.s_wo; g.ld_out = D;
         if (join) g.join = {b.X6, b.X6, L.ffn_norm, b.bD, b.rows_pad, b.ssq, nullptr};
         if (tc_gemm(t.wo[l], b.aQ, g, st)) return -1;
         if (!join) tc_prepare(b.aD, nullptr, D, ROWS, b.part, t.s_wo, psD, b.X6, b.X6, L.ffn_norm, b.ssq, st);
         /* FFN half: gate/up with SwiGLU (terms out) -> down */
         g = TcGemm();
-        g.M = ROWS; g.exact = exact; g.status = b.status;
+        g.M = ROWS; g.sums = sums; g.status = b.status;
         g.epi = TC_EPI_SWIGLU_TERMS; g.out_terms = b.bH; g.out_rows_pad = b.rows_pad;
         g.ld_out = HID; g.ssq = b.ssq; g.ssq_chunks = chunks; g.eps = VB200_NORM_EPS;
         if (tc_gemm(t.w13[l], b.aD, g, st)) return -1;
         g = TcGemm();
-        g.M = ROWS; g.exact = exact; g.status = b.status;
+        g.M = ROWS; g.sums = sums; g.status = b.status;
         g.epi = TC_EPI_PARTIAL; g.out = b.part; g.splits = t.s_w2; g.ld_out = D;
         if (join) g.join = {b.X6, b.X6, l + 1 < VB200_AC_LAYERS ? m.ac[l + 1].attn_norm : nullptr, b.bD, b.rows_pad, b.ssq, nullptr};
         if (tc_gemm(t.w2[l], b.aH, g, st)) return -1;
@@ -425,7 +425,7 @@ int acoustic_tc_enqueue_on(const AcBuffers &b, const float *noise_all, int *code
         launch_pdl(ac_tokens_kernel, dim3((D + 127) / 128, b.B), dim3(128), 0, st, b.X6, b.lat, (const float *)b.vel,
                    (const uint16_t *)m.ac_input_proj, (const float *)m.ttok, (const float *)b.ltok, s,
                    VB200_CFG_ALPHA, s > 0 ? m.dt[s - 1] : 0.0f, noise_all, (const VbDyn *)b.dyn, b.sd);
-        if (enqueue_layers(b, ROWS, false)) return -1;
+        if (enqueue_layers(b, ROWS, 2)) return -1;
         launch_pdl(ac_velocity_kernel, dim3(9, 2 * b.B), dim3(512), 0, st, b.vel, (const float *)b.X6, (const float *)b.part,
                    joined(ROWS) ? 0 : t.s_w2, (const float *)m.ac_norm, VB200_NORM_EPS, (const uint16_t *)m.ac_out, ROWS, b.sd.vel);
     }
@@ -507,14 +507,14 @@ static int enqueue_velocity() {
     const int s = tc_pick_splits(D, D, m.sm_count);
     float *const time_part = b.part, *const llm_part = b.part + (size_t)kTcMaxSplits * 2 * D;
     TcGemm g;
-    g.M = 2; g.exact = true; g.status = b.status; g.epi = TC_EPI_PARTIAL; g.splits = s; g.ld_out = D;
+    g.M = 2; g.sums = 4; g.status = b.status; g.epi = TC_EPI_PARTIAL; g.splits = s; g.ld_out = D;
     g.out = time_part;
     if (tc_gemm(t.wtime, b.aD, g, st)) return -1;
     g.out = llm_part;
     if (tc_gemm(t.wllm, b.aD, g, st)) return -1;
     launch_pdl(ac_rows_kernel, dim3((D + 127) / 128), dim3(128), 0, st, b.X6, (const float *)m.d_in->lat[0], (const uint16_t *)m.ac_input_proj,
                (const float *)time_part, (const float *)llm_part, s);
-    if (enqueue_layers(b, 3, true)) return -1;
+    if (enqueue_layers(b, 3, 4)) return -1;
     launch_pdl(ac_velocity_kernel, dim3(9, 1), dim3(512), 0, st, b.vel, (const float *)b.X6, (const float *)nullptr, 0, (const float *)m.ac_norm,
                VB200_NORM_EPS, (const uint16_t *)m.ac_out, 3, b.sd.vel);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;

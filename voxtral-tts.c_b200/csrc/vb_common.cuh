@@ -184,4 +184,10 @@ VB_DEVINL void vb_split3(float v, uint16_t &t0, uint16_t &t1, uint16_t &t2) {
     t2 = __bfloat16_as_ushort(h2);
 }
 
+/* The same where a value may be infinite: its low terms are zeros, not NaN. */
+VB_DEVINL void vb_split3_inf(float v, uint16_t &t0, uint16_t &t1, uint16_t &t2) {
+    vb_split3(v, t0, t1, t2);
+    if ((t0 & 0x7fffu) == 0x7f80u) t1 = t2 = 0;
+}
+
 #endif

@@ -8,8 +8,7 @@
  * or, where one norm feeds mixer and feed-forward,
  *   GEMM of every projection that reads the norm, mixer kernels [, experts], GEMM of the two
  *   out-projections side by side, residual + norm
- * with the GEMMs of vb_tc.cu (split-K partials, summed by the consumer) and, in the 32-bit mode,
- * those of vb_lm_gemm32.cu in their place. One-token steps are captured once as a CUDA graph and
+ * with the GEMMs of vb_tc.cu (split-K partials, summed by the consumer). One-token steps are captured once as a CUDA graph and
  * replayed for every position and slot.
  */
 #include "../../include/voxtral_b200_lm.h"
@@ -64,7 +63,7 @@ struct Source {
 };
 
 struct Linear {
-    uint16_t *W = nullptr;      /* tile-contiguous (tensor cores) or row-major [N][Kp] (fp32) */
+    uint16_t *W = nullptr;      /* tile-contiguous */
     TcWeight tc;
     int N = 0, K = 0, Kp = 0;   /* N padded to a multiple of 4, K padded to whole 64-column blocks */
     bool swiglu = false;
@@ -74,10 +73,9 @@ struct Linear {
     struct Acts *act_acts = nullptr;
 };
 
-/* Rows that feed a GEMM, as BF16 terms or fp32; columns [K, Kp) stay zero. */
+/* Rows that feed a GEMM, as BF16 terms; columns [K, Kp) stay zero. */
 struct Acts {
     uint16_t *terms = nullptr;
-    float *rows = nullptr;
     int K = 0, Kp = 0;
     std::map<int, TcActs> maps;   /* by padded row count */
 };
@@ -115,6 +113,14 @@ enum Variant { STEP_SILENT = 0, STEP_LOGITS = 1, STEP_GREEDY = 2, kVariants = 3 
 constexpr int kHeadRows = 64;     /* rows that go through the head at once */
 constexpr int kLogCap = 1 << 16;  /* generated tokens kept on the device */
 
+/* 32-bit mode: no product is rounded and sums are as exact as on the fp32 pipes. A row is the sum of three BF16 terms
+ * (24 bits), a term's products with BF16 weights are exact, and the tensor cores, which cut their sums off at every
+ * step, add up kF32Segment k-blocks at most where the sizes allow it. A 24-run model of width 2048, seven prompts of 40 to
+ * 390 rows, logits off 64 bits on average: 4.2e-6 on the fp32 pipes, 3.3e-6 with one or two k-blocks, 4.2e-6 with four, 6.7e-6
+ * with eight; 390 rows took 13.9, 12.1, 11.5 and 11.3 ms (37.8 on the fp32 pipes). Up to kF32FewRows rows take the skinny
+ * GEMM, with as many sums as TMEM holds. */
+constexpr int kF32Segment = 2, kF32FewRows = 16;
+
 } // namespace
 
 } // namespace vb
@@ -148,8 +154,6 @@ struct vb200_lm {
     float *x = nullptr, *part_in = nullptr, *part_out = nullptr, *part_head = nullptr, *logits = nullptr;
     float *q = nullptr, *k = nullptr, *v = nullptr, *o = nullptr, *beta = nullptr, *decays = nullptr, *gram = nullptr;
     float *scratch = nullptr, *tap = nullptr;
-    uint16_t *terms = nullptr;           /* 32-bit mode: rows of the GEMM at hand as terms, up to terms_k columns */
-    int terms_k = 0;
     unsigned *tickets = nullptr;
     int *status = nullptr, *log = nullptr, *zero = nullptr;
     /* latent attention */
@@ -204,6 +208,13 @@ private:
     int make_state();
     int make_buffers();
 
+    /* Terms of the rows of a prompt. The 32-bit mode multiplies all three of any row. */
+    int prompt_terms() const { return f32() ? kTcTerms : 2; }
+    int rows_pad(int M) const {
+        if (f32() && M > kF32FewRows) return std::max(256, round_up(M, 128));
+        return M <= 256 ? tc_rows_pad_frame(M) : tc_rows_pad_any(M);
+    }
+    TcGemm plan(int M) const;
     int splits_of(const Linear &l, int M) const;
     bool fused_act(const Linear &l, int M) const { return !f32() && l.act_n0 > 0 && M > 256; }
     size_t part_floats(const Linear &l, int max_rows);
@@ -360,25 +371,20 @@ int vb200_lm::linear(const Source &s, const std::vector<Piece> &pieces, int N, i
         rc = tensor(s, p.name, {p.rows, p.cols}, tmp_, &stage_);
         if (!rc && lm_pack_rows(rows, l->Kp, p.row0, p.step, p.col0, tmp_, p.rows, p.cols, st)) rc = fail("weight packing failed");
     }
-    if (!rc && !f32()) {
+    if (!rc) {
         uint16_t *tiled = nullptr;
         rc = alloc(&tiled, tc_tiled_bytes(l->N, l->Kp) / 2);
         if (!rc && tc_weight_tiled(&l->tc, rows, l->N, l->Kp, tiled, st)) rc = fail("tensor map of a weight matrix could not be made");
         if (!rc) rc = cuda_ok(cudaStreamSynchronize(st), "weight upload");
         l->W = tiled;
-        cudaFree(rows);
         weight_bytes += tc_tiled_bytes(l->N, l->Kp);
-    } else {
-        allocs.push_back(rows);
-        l->W = rows;
-        weight_bytes += elems * 2;
-        if (!rc && tc_weight(&l->tc, rows, l->N, l->Kp)) rc = fail("tensor map of a weight matrix could not be made");
-        terms_k = std::max(terms_k, l->Kp);
     }
+    cudaFree(rows);
     return rc;
 }
 
-/* rows: 0 for as many as a block or the head has; otherwise that many, in two terms (row-block GEMMs only). */
+/* rows: 0 for as many as a block or the head has, in three terms; otherwise that many, in as many terms as prompts have
+ * (row-block GEMMs only). */
 int vb200_lm::make_acts(int K, Acts **out, int rows) {
     acts.emplace_back(new Acts());
     Acts *a = acts.back().get();
@@ -386,9 +392,8 @@ int vb200_lm::make_acts(int K, Acts **out, int rows) {
     a->Kp = round_up(K, kTcBlockK);
     *out = a;
     const int n = rows > 0 ? rows : std::max(block, kHeadRows);
-    if (f32()) return alloc(&a->rows, (size_t)n * a->Kp, true);
-    if (rows > 0) return alloc(&a->terms, (size_t)2 * round_up(std::max(rows, 256), 128) * a->Kp, true);
-    return alloc(&a->terms, tc_acts_bytes(std::max(tc_rows_pad_any(n), 64), a->Kp) / 2, true);
+    if (rows > 0) return alloc(&a->terms, (size_t)prompt_terms() * round_up(std::max(rows, 256), 128) * a->Kp, true);
+    return alloc(&a->terms, tc_acts_bytes(std::max(rows_pad(n), 64), a->Kp) / 2, true);
 }
 
 /* In-projection of an attention or a delta-rule mixer: all of its projections below one another. */
@@ -582,7 +587,11 @@ int vb200_lm::make_state() {
 /* ------------------------------------------------------------------ activations */
 int vb200_lm::splits_of(const Linear &l, int M) const {
     if (l.swiglu || fused_act(l, M)) return 1;
-    if (f32()) return lm_gemm_f32_splits(M, l.N, l.K, n_sm);
+    if (f32() && M > kF32FewRows) return tc_row_splits(l.N, l.Kp, M, n_sm, kTcTerms);
+    if (f32()) {
+        const int kblocks = l.Kp / kTcBlockK, least = (kblocks + kF32Segment * kTcManySums - 1) / (kF32Segment * kTcManySums);
+        return std::max(tc_pick_splits(l.N, l.Kp, n_sm), std::min({least, kblocks, kTcMaxSplits}));
+    }
     if (M <= 64) return tc_pick_splits(l.N, l.Kp, n_sm);
     return tc_row_splits(l.N, l.Kp, M, n_sm);
 }
@@ -660,7 +669,6 @@ int vb200_lm::make_buffers() {
         alloc(&gram, (B + kLmDeltaRows) / kLmDeltaGroup * gn * 2 * kLmDeltaGroup * kLmDeltaGroup) || alloc(&scratch, scr) || alloc(&tickets, (size_t)tick, true) ||
         alloc(&status, 4, true) || alloc(&log, kLogCap, true) || alloc(&zero, 4, true) || alloc(&d_in, 4 + 2 * B, true))
         return -1;
-    if (f32() && alloc(&terms, (size_t)kTcTerms * lm_gemm_f32_rows_pad(std::max(block, kHeadRows)) * terms_k, true)) return -1;
     for (int i = 0; i < 2; i++) {
         LM_CUDA(cudaHostAlloc(&h_in[i], sizeof(int) * (4 + 2 * B), cudaHostAllocDefault));
         LM_CUDA(cudaEventCreateWithFlags(&in_free[i], cudaEventDisableTiming));
@@ -718,7 +726,7 @@ int vb200_lm::init(const Source &src, const vb200_lm_options_t *opt) {
 
 /* ------------------------------------------------------------------ the step */
 TcActs *vb200_lm::map_of(Acts *a, int M) {
-    const int rp = M <= 256 ? tc_rows_pad_frame(M) : tc_rows_pad_any(M);
+    const int rp = rows_pad(M);
     auto it = a->maps.find(rp);
     if (it == a->maps.end()) {
         TcActs t;
@@ -731,30 +739,16 @@ TcActs *vb200_lm::map_of(Acts *a, int M) {
 LmSink vb200_lm::sink(Acts *a, int M) {
     LmSink s = {};
     s.ld = a->Kp;
-    if (f32()) {
-        s.rows = a->rows;
-    } else {
-        s.terms = a->terms;
-        s.rows_pad = M <= 256 ? tc_rows_pad_frame(M) : tc_rows_pad_any(M);
-        s.n_terms = M <= 64 ? 3 : 2;      /* the row-block kernel multiplies two */
-    }
+    s.terms = a->terms;
+    s.rows_pad = rows_pad(M);
+    s.n_terms = M <= 64 ? kTcTerms : prompt_terms();
     return s;
 }
 
 int vb200_lm::gemm(const Linear &l, Acts *in, int M, float *part, Acts *swiglu_out, LmPart *out) {
-    if (f32()) {
-        float *y = l.swiglu ? swiglu_out->rows : part;
-        const int ld = l.swiglu ? swiglu_out->Kp : l.N;
-        const int splits = splits_of(l, M);
-        if (out) *out = {part, splits, l.N, (size_t)M * l.N};
-        if (M > kLmF32FewRows) return lm_gemm_f32_many(y, ld, in->rows, in->Kp, l.tc, terms, M, l.swiglu, st, splits, status);
-        return lm_gemm_f32(y, ld, in->rows, in->Kp, l.W, l.Kp, M, l.N, l.K, l.swiglu ? LM_ACT_SWIGLU : LM_ACT_NONE, st, splits);
-    }
     TcActs *a = map_of(in, M);
     if (!a) return -1;
-    TcGemm g;
-    g.M = M;
-    g.status = status;
+    TcGemm g = plan(M);
     if (l.swiglu) {
         g.epi = TC_EPI_SWIGLU_TERMS;
         g.out_terms = swiglu_out->terms;
@@ -776,6 +770,19 @@ int vb200_lm::gemm(const Linear &l, Acts *in, int M, float *part, Acts *swiglu_o
         *out = {part, g.splits, l.N, (size_t)M * l.N};
     }
     return tc_gemm(l.tc, *a, g, st);
+}
+
+/* A launch for M rows, but for what goes in and out. */
+TcGemm vb200_lm::plan(int M) const {
+    TcGemm g;
+    g.M = M;
+    g.status = status;
+    if (f32()) {
+        if (M <= kF32FewRows) g.sums = kTcManySums;
+        g.terms = kTcTerms;
+        g.segment = kF32Segment;
+    }
+    return g;
 }
 
 /* The in-projection is done up to here; a stretch's keys and values are written out and attended to. */
@@ -838,7 +845,7 @@ int vb200_lm::latent(const Layer &l, const LmLayer &spec, const RunState &s, int
     }
     if (l.mix.in.act_n0 > 0 && !fused_act(l.mix.in, M)) { a.col_ff = l.mix.in.act_n0; a.ff = spec.mlp.ff; a.ff_out = l.mix.in.act_col; }
     a.out = sink(l.mix.acts, M);
-    a.ukv = {l.mix.ukv.W, l.mix.ukv.Kp, f32() ? 0 : 1};
+    a.ukv = {l.mix.ukv.W, l.mix.ukv.Kp};
     a.ql = ql; a.scratch = scratch;
     LM_DO(lm_latent_prepare(a, M, st));
     LM_DO(gemm(l.mix.uq, l.mix.uq_acts, M, part_q, nullptr, &a.q));
@@ -854,8 +861,8 @@ int vb200_lm::experts(const Layer &l, const LmMlp &m, int M, LmMix *mix) {
     LmMoe e = {};
     e.experts = m.experts; e.top = m.top; e.ff = m.ff; e.width = cfg.width;
     e.chosen = route;
-    e.up = {l.up.W, l.up.Kp, f32() ? 0 : 1};
-    e.down = {l.down.W, l.down.Kp, f32() ? 0 : 1};
+    e.up = {l.up.W, l.up.Kp};
+    e.down = {l.down.W, l.down.Kp};
     e.x = sink(x_acts, M);
     e.act = few_act; e.act_ld = round_up(m.ff, kTcBlockK);
     e.table = route_table; e.at = route_at;
@@ -868,27 +875,18 @@ int vb200_lm::experts(const Layer &l, const LmMlp &m, int M, LmMix *mix) {
     const int blocks = lm_moe_blocks(M, m.experts, m.top);
     Acts *ff = expert_acts[m.ff];
     LmSink to = {};
-    to.rows = sorted_acts->rows; to.terms = sorted_acts->terms;
-    to.rows_pad = round_up(std::max(sorted_rows, 256), 128); to.ld = sorted_acts->Kp; to.n_terms = 2;
+    to.terms = sorted_acts->terms;
+    to.rows_pad = round_up(std::max(sorted_rows, 256), 128); to.ld = sorted_acts->Kp; to.n_terms = prompt_terms();
     LM_DO(lm_moe_plan(e, M, st));
     LM_DO(lm_moe_gather(e, to, M, st));
-    if (f32()) {
-        LM_DO(lm_gemm_f32(ff->rows, ff->Kp, to.rows, to.ld, l.up.W, l.up.Kp, blocks * 128, m.ff, cfg.width, LM_ACT_RELU2, st, 1, route_table,
-                          l.expert_rows));
-        LM_DO(lm_gemm_f32(expert_y, y_ld, ff->rows, ff->Kp, l.down.W, l.down.Kp, blocks * 128, cfg.width, m.ff, LM_ACT_NONE, st, 1, route_table,
-                          l.expert_rows_down));
-        return 0;
-    }
     TcActs xa, fa;
     if (tc_acts_blocks(&xa, to.terms, to.rows_pad, to.ld) || tc_acts_blocks(&fa, ff->terms, to.rows_pad, ff->Kp))
         return fail("tensor map of the experts' rows could not be made");
-    TcGemm g;
-    g.status = status;
+    TcGemm g = plan(kHeadRows + 1);
     g.epi = TC_EPI_RELU2_TERMS;
     g.out_terms = ff->terms; g.out_terms_ld = ff->Kp; g.out_rows_pad = to.rows_pad;
     LM_DO(tc_gemm_grouped(l.up.tc, xa, g, m.ff, route_table, blocks, st));
-    g = TcGemm();
-    g.status = status;
+    g = plan(kHeadRows + 1);
     g.epi = TC_EPI_STORE;
     g.out = expert_y; g.ld_out = y_ld;
     LM_DO(tc_gemm_grouped(l.down.tc, fa, g, cfg.width, route_table, blocks, st));

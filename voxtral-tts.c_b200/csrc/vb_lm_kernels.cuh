@@ -4,7 +4,7 @@
  * vb_lm_moe.cu).
  *
  * A kernel reads the result of a GEMM as split-K partials (LmPart), and leaves rows for the next
- * one in an LmSink: BF16 terms for the tensor-core GEMM, or plain fp32 rows for the fp32 one.
+ * one in an LmSink, as BF16 terms for the tensor cores.
  * Everything in between is fp32. Where a sequence stands, and in which slot, is read from device
  * memory (LmDyn), so that a captured graph serves every position and slot.
  */
@@ -77,40 +77,31 @@ VB_DEVINL float4 lm_sum4(const LmPart &g, int m, int c) {
 
 /* Activation rows of the next GEMM. */
 struct LmSink {
-    float *rows;        /* fp32 rows [M][ld], or null */
-    uint16_t *terms;    /* BF16 terms [n_terms][rows_pad][ld], or null */
+    uint16_t *terms;    /* BF16 terms [n_terms][rows_pad][ld] */
     int rows_pad, ld, n_terms;
 };
 
 VB_DEVINL void lm_put(const LmSink &s, int m, int c, float v) {
-    if (s.rows) {
-        s.rows[(size_t)m * s.ld + c] = v;
-    } else {
-        uint16_t t0, t1, t2;
-        vb_split3(v, t0, t1, t2);
-        uint16_t *o = s.terms + (size_t)m * s.ld + c;
-        const size_t term = (size_t)s.rows_pad * s.ld;
-        o[0] = t0;
-        if (s.n_terms > 1) o[term] = t1;
-        if (s.n_terms > 2) o[2 * term] = t2;
-    }
+    uint16_t t0, t1, t2;
+    vb_split3_inf(v, t0, t1, t2);
+    uint16_t *o = s.terms + (size_t)m * s.ld + c;
+    const size_t term = (size_t)s.rows_pad * s.ld;
+    o[0] = t0;
+    if (s.n_terms > 1) o[term] = t1;
+    if (s.n_terms > 2) o[2 * term] = t2;
 }
 
 /* Four columns from c on (a multiple of 4; rows are padded to multiples of 64). */
 VB_DEVINL void lm_put4(const LmSink &s, int m, int c, const float (&v)[4]) {
-    if (s.rows) {
-        *reinterpret_cast<float4 *>(s.rows + (size_t)m * s.ld + c) = make_float4(v[0], v[1], v[2], v[3]);
-    } else {
-        uint16_t t[3][4];
+    uint16_t t[3][4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) vb_split3(v[i], t[0][i], t[1][i], t[2][i]);
-        uint16_t *o = s.terms + (size_t)m * s.ld + c;
-        const size_t term = (size_t)s.rows_pad * s.ld;
+    for (int i = 0; i < 4; i++) vb_split3_inf(v[i], t[0][i], t[1][i], t[2][i]);
+    uint16_t *o = s.terms + (size_t)m * s.ld + c;
+    const size_t term = (size_t)s.rows_pad * s.ld;
 #pragma unroll
-        for (int j = 0; j < 3; j++)
-            if (j < s.n_terms)
-                *reinterpret_cast<uint2 *>(o + j * term) = make_uint2(t[j][0] | ((uint32_t)t[j][1] << 16), t[j][2] | ((uint32_t)t[j][3] << 16));
-    }
+    for (int j = 0; j < 3; j++)
+        if (j < s.n_terms)
+            *reinterpret_cast<uint2 *>(o + j * term) = make_uint2(t[j][0] | ((uint32_t)t[j][1] << 16), t[j][2] | ((uint32_t)t[j][3] << 16));
 }
 
 /* State of one layer run: `base` + slot * `slab` floats. */
@@ -127,14 +118,14 @@ struct LmRing {
 };
 VB_DEVINL int lm_ring_row(const LmRing &r, int p) { return p < r.keep ? p : r.keep + (p - r.keep) % r.ring; }
 
-/* Elements of a weight matrix as it is kept: in tiles of 128 rows x 64 columns for the tensor cores, or row by
- * row. lm_weight_row: 64 columns (block kb of a row of Kp) that lie together. */
+/* Elements of a weight matrix as it is kept, in tiles of 128 rows x 64 columns. lm_weight_row: 64 columns (block kb of a
+ * row of Kp) that lie together. */
 struct LmWeight {
     const uint16_t *W;
-    int Kp, tiled;
+    int Kp;
 };
 VB_DEVINL const uint16_t *lm_weight_row(const LmWeight &w, int n, int kb) {
-    return w.tiled ? w.W + (((size_t)(n >> 7) * (w.Kp >> 6) + kb) * 128 + (n & 127)) * 64 : w.W + (size_t)n * w.Kp + kb * 64;
+    return w.W + (((size_t)(n >> 7) * (w.Kp >> 6) + kb) * 128 + (n & 127)) * 64;
 }
 
 /* Results of the experts of a mixture: row at[m * top + k] of y belongs to the k-th choice of token m. */
@@ -174,23 +165,6 @@ int lm_residual(const LmResidual &a, int M, cudaStream_t st);
 int lm_pack_rows(uint16_t *dst, int Kp, int row0, int step, int col0, const uint16_t *src, int rows, int K, cudaStream_t st);
 int lm_widen(float *dst, const uint16_t *src, int n, cudaStream_t st);
 int lm_fill_random(uint16_t *dst, size_t n, uint32_t seed, float mean, float scale, cudaStream_t st);
-
-/* ---- GEMMs of the 32-bit mode (vb_lm_gemm32.cu) ----
- * y[M][ld_out] = x[M][ldx] . W[N][ldw]^T, BF16 W; columns of x and W from K up to the next multiple of 32 are zero.
- * LM_ACT_SWIGLU: rows of W interleaved (gate, up), y[M][N / 2] = silu(gate) * up. splits > 1 (LM_ACT_NONE): that many
- * partial results, M * ld_out floats apart. With a table of row blocks (as for tc_gemm_grouped, M = 128 times
- * their number) a block uses the matrix that starts at row matrix * group_rows of W.
- * lm_gemm_f32: up to kLmF32FewRows rows, or a table. lm_gemm_f32_many: the rows above, as three terms (`terms`: room for
- * 3 * lm_gemm_f32_rows_pad(M) rows) through the row-block GEMM. */
-enum LmAct { LM_ACT_NONE = 0, LM_ACT_SWIGLU = 1, LM_ACT_RELU2 = 2 };
-constexpr int kLmF32FewRows = 32;
-inline int lm_gemm_f32_rows_pad(int M) { return M <= 256 ? 256 : (M + 127) / 128 * 128; }
-int lm_gemm_f32_splits(int M, int N, int K, int n_sm);
-int lm_gemm_f32(float *y, int ld_out, const float *x, int ldx, const uint16_t *W, int ldw, int M, int N, int K, LmAct act,
-                cudaStream_t st, int splits = 1, const int4 *table = nullptr, int group_rows = 0);
-struct TcWeight;
-int lm_gemm_f32_many(float *y, int ld_out, const float *x, int ldx, const TcWeight &w, uint16_t *terms, int M, bool swiglu, cudaStream_t st,
-                     int splits, int *status);
 
 /* Largest logit of row 0 (first one on a tie) becomes the next token: tokens[0], log[dyn->logged++];
  * the sequence moves on by the `rows` positions just run. */

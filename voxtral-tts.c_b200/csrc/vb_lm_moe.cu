@@ -5,8 +5,7 @@
  *   few rows    a warp multiplies four weight rows of a chosen expert, straight from the tiles the
  *               tensor cores use, in fp32
  *   many rows   tokens are sorted by expert into blocks of 128 rows (plan, gather); the two products
- *               are grouped GEMMs on the tensor cores (tc_gemm_grouped), or fp32 ones in the 32-bit
- *               mode
+ *               are grouped GEMMs on the tensor cores (tc_gemm_grouped)
  */
 #include "vb_lm_kernels.cuh"
 #include "vb_tc.cuh"
@@ -52,8 +51,6 @@ __global__ void __launch_bounds__(kMfThreads) lm_moe_few_kernel(const LmMoe a) {
         pre[i] = i < kblocks ? __ldg(reinterpret_cast<const uint4 *>(lm_weight_row(W, row, i) + c0)) : make_uint4(0u, 0u, 0u, 0u);
     if (DOWN) {
         for (int c = tid; c < W.Kp; c += kMfThreads) xs[c] = c < a.ff ? __ldcg(a.act + (size_t)choice * a.act_ld + c) : 0.0f;
-    } else if (a.x.rows) {
-        for (int c = tid; c < W.Kp; c += kMfThreads) xs[c] = __ldcg(a.x.rows + (size_t)m * a.x.ld + c);
     } else {
         const size_t term = (size_t)a.x.rows_pad * a.x.ld;
         for (int c = tid * 4; c < W.Kp; c += kMfThreads * 4) {
@@ -131,15 +128,10 @@ __global__ void __launch_bounds__(128) lm_moe_gather_kernel(const LmMoe a, const
     pdl_launch_dependents();
     pdl_wait();
     const int i = blockIdx.x, m = i / a.top, r = a.at[i];
-    if (to.rows) {
-        for (int c = threadIdx.x * 4; c < to.ld; c += 512)
-            *reinterpret_cast<float4 *>(to.rows + (size_t)r * to.ld + c) = vb_ldcg4(a.x.rows + (size_t)m * a.x.ld + c);
-    } else {
-        for (int t = 0; t < to.n_terms; t++)
-            for (int c = threadIdx.x * 8; c < to.ld; c += 1024)
-                *reinterpret_cast<uint4 *>(to.terms + ((size_t)t * to.rows_pad + r) * to.ld + c) =
-                    __ldcg(reinterpret_cast<const uint4 *>(a.x.terms + ((size_t)t * a.x.rows_pad + m) * a.x.ld + c));
-    }
+    for (int t = 0; t < to.n_terms; t++)
+        for (int c = threadIdx.x * 8; c < to.ld; c += 1024)
+            *reinterpret_cast<uint4 *>(to.terms + ((size_t)t * to.rows_pad + r) * to.ld + c) =
+                __ldcg(reinterpret_cast<const uint4 *>(a.x.terms + ((size_t)t * a.x.rows_pad + m) * a.x.ld + c));
 }
 
 template <bool DOWN> int launch_few(const LmMoe &a, int M, cudaStream_t st) {

@@ -279,7 +279,7 @@ static int prefill_tc(float *x, const float *cs, int M, int start_pos, int block
         if (tc_map3(&maps.k, t.split.k, 1, keys * 4 * KVD, keys, 4 * KVD, 2 * KVD, kAtKeys) ||
             tc_map3(&maps.v, t.split.v, 1, keys * 4 * KVD, keys, 4 * KVD, 2 * KVD, kAtKeys))
             return -1;
-        const LmSink q_terms = {nullptr, t.bQ, b.rp, QD, b.rp < 256 ? kTcTerms : 2};
+        const LmSink q_terms = {t.bQ, b.rp, QD, b.rp < 256 ? kTcTerms : 2};
         const size_t psD = (size_t)rows * D;
         float *xr = x + (size_t)r0 * D;
         for (int l = 0; l < VB200_DEC_LAYERS; l++) {

@@ -186,7 +186,7 @@ struct TcCfg {
      * frame with one accumulator (and 16 columns read for every row count), 2.709 with two, whose hidden states are 2.0e-5
      * for 2.4e-5 off 64 bits; segments of 512 to 1024 columns that the epilogue fetches under the main loop, with a commit
      * for each, 2.74 to 2.78. A velocity call: 8.7e-6 with one, 4.4e-6 with two, 2.2e-6 with four. */
-    static constexpr int kTmemCols = ACCS * kAccCols <= 128 ? 128 : 256;
+    static constexpr int kTmemCols = ACCS * kAccCols <= 128 ? 128 : ACCS * kAccCols <= 256 ? 256 : 512;
     static_assert(ACCS * kAccCols <= kTmemCols, "accumulators over TMEM");
     static constexpr int kSmemBytes = kStages * kStage + 1024 /* alignment slack */ + 256 /* barriers */ + 4 * NB;
     static_assert(kSmemBytes <= 232448, "over the 227 KB a CTA may use");
@@ -265,6 +265,12 @@ VB_DEVINL void tc_stage_rows(float *to, uint32_t t, int c0, int M, int n_it, int
         const int m = c0 + i;
         if (m < M) to[m * kTcTileN] = rscale ? v[i] * rscale[m] : v[i];
     }
+}
+
+/* the 32-bit mode keeps infinities */
+template <int ACCS> VB_DEVINL void tc_split(float v, uint16_t &t0, uint16_t &t1, uint16_t &t2) {
+    if constexpr (ACCS == kTcManySums) vb_split3_inf(v, t0, t1, t2);
+    else vb_split3(v, t0, t1, t2);
 }
 
 template <int NB, int ST, int MODE, int ACCS>
@@ -450,8 +456,8 @@ vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
                                 *(float2 *)(out + (size_t)m * ld_out + col) = make_float2(res[0], res[1]);
                             } else {
                                 uint16_t q[3][2];
-                                vb_split3(res[0], q[0][0], q[1][0], q[2][0]);
-                                vb_split3(res[1], q[0][1], q[1][1], q[2][1]);
+                                tc_split<ACCS>(res[0], q[0][0], q[1][0], q[2][0]);
+                                tc_split<ACCS>(res[1], q[0][1], q[1][1], q[2][1]);
                                 const size_t o = (size_t)m * ko + col;
 #pragma unroll
                                 for (int j = 0; j < 3; j++) {
@@ -470,7 +476,7 @@ vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
                                     out[(size_t)m * ld_out + col + i] = res[i];
                                 } else {
                                     uint16_t q0, q1, q2;
-                                    vb_split3(res[i], q0, q1, q2);
+                                    tc_split<ACCS>(res[i], q0, q1, q2);
                                     const size_t o = (size_t)m * ko + col + i;
                                     ka.out_terms[o] = q0;
                                     ka.out_terms[(size_t)ka.out_rows_pad * ko + o] = q1;
@@ -631,7 +637,8 @@ static int tc_gemm_join(const TcWeight &w, const TcActs &a, const TcGemm &g, cud
     ka.a_tiled = w.tiled ? 1 : 0;
     ka.N = w.N; ka.K = w.K; ka.M = g.M; ka.rows_pad = a.rows_pad; ka.splits = kTcJoinSplits; ka.status = g.status;
     ka.n_tiles_launch = w.N / kTcTileN;
-    return g.exact ? launch_tc_tp<16, 6, TC_JOIN, 4>(w, a, ka, j, st) : launch_tc_tp<16, 6, TC_JOIN, 2>(w, a, ka, j, st);
+    if (g.sums != 2 && g.sums != 4) return -1;
+    return g.sums == 4 ? launch_tc_tp<16, 6, TC_JOIN, 4>(w, a, ka, j, st) : launch_tc_tp<16, 6, TC_JOIN, 2>(w, a, ka, j, st);
 }
 
 int tc_gemm(const TcWeight &w, const TcActs &a, const TcGemm &g, cudaStream_t st) {
@@ -639,7 +646,7 @@ int tc_gemm(const TcWeight &w, const TcActs &a, const TcGemm &g, cudaStream_t st
     if (g.join.x) return tc_gemm_join(w, a, g, st);
     if (g.splits < 1 || g.splits > kTcMaxSplits || g.splits > w.K / kTcBlockK) return -1;
     if (g.epi != TC_EPI_PARTIAL && g.splits != 1) return -1;
-    if (g.exact && (g.push.n_dst || g.wait.n)) return -1;
+    if (g.sums != 2 && (a.rows_pad == 16 ? g.push.n_dst || g.wait.n || (g.sums != 4 && g.sums != kTcManySums) : a.rows_pad < 256)) return -1;
     if ((g.epi == TC_EPI_SWIGLU || g.epi == TC_EPI_SWIGLU_TERMS) && (w.N & 1)) return -1;
     if (g.epi == TC_EPI_SWIGLU_TERMS && (!g.out_terms || g.out_rows_pad < g.M)) return -1;
     if ((g.epi == TC_EPI_TERMS || g.epi == TC_EPI_RELU2_TERMS) && a.rows_pad < 256) return -1;
@@ -664,7 +671,9 @@ int tc_gemm(const TcWeight &w, const TcActs &a, const TcGemm &g, cudaStream_t st
     tpa.wait = g.wait;
     tpa.wait.status = g.status;
     switch (a.rows_pad) {
-    case 16: return g.exact ? launch_tc_tp<16, 6, TC_PLAIN, 4>(w, a, ka, TcNoTpArgs(), st) : launch_tc<16, 6, 2>(w, a, ka, tpa, st);
+    case 16:
+        if (g.sums == kTcManySums) return launch_tc_tp<16, 6, TC_PLAIN, kTcManySums>(w, a, ka, TcNoTpArgs(), st);
+        return g.sums == 4 ? launch_tc_tp<16, 6, TC_PLAIN, 4>(w, a, ka, TcNoTpArgs(), st) : launch_tc<16, 6, 2>(w, a, ka, tpa, st);
     case 48: return launch_tc<48, 6, 1>(w, a, ka, tpa, st);   /* 8 utterances' acoustic rows: 34 KB stages, six of them */
     case 64: return launch_tc<64, 5, 1>(w, a, ka, tpa, st);
     default: return -1;

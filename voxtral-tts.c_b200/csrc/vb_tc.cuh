@@ -104,12 +104,14 @@ struct TcJoin {
 /* 24 tiles of 3072 columns: clusters of six find room for 22 at once; one utterance, 212 frames: 596 ms with four or five */
 constexpr int kTcJoinSplits = 4;
 
+constexpr int kTcManySums = 10;       /* TcGemm::sums: as many as TMEM holds for 16 rows */
+
 /* One GEMM launch. */
 struct TcGemm {
     int M = 0, splits = 1, epi = TC_EPI_STORE;
     int segment = 32;                 /* 65 rows and more: k-blocks that are summed in TMEM, at most, before registers take over */
     int terms = 2;                    /* the same: terms of the rows that are multiplied, 2 or 3 */
-    bool exact = false;               /* up to 16 rows: four accumulators in place of two (see TcCfg) */
+    int sums = 2;                     /* up to 16 rows: accumulators that share K, 2, 4 or 10 (see TcCfg) */
     float *out = nullptr;
     int ld_out = 0;
     const float *bias = nullptr;

@@ -136,6 +136,12 @@ VB_DEVINL PrTile pr_tile(const RowsArgs &a, int i, int kblocks) {
 
 VB_DEVINL uint32_t pr_pack(uint16_t a, uint16_t b) { return a | ((uint32_t)b << 16); }
 
+/* three terms keep infinities */
+template <int TERMS> VB_DEVINL void pr_split(float v, uint16_t &t0, uint16_t &t1, uint16_t &t2) {
+    if constexpr (TERMS == 3) vb_split3_inf(v, t0, t1, t2);
+    else vb_split3(v, t0, t1, t2);
+}
+
 /* Rows [c0, c0 + 64) of a tile's results, staged as [row][128 columns], to where they belong; `t` is this CTA's weight tile. */
 template <int TERMS>
 VB_DEVINL void pr_store(const RowsArgs &a, const float *stg, const PrTile &tl, int t, int c0, int warp, int lane) {
@@ -155,8 +161,8 @@ VB_DEVINL void pr_store(const RowsArgs &a, const float *stg, const PrTile &tl, i
                 if (both) o[1] = r1;
             } else {
                 uint16_t p[3], q[3];
-                vb_split3(r0, p[0], p[1], p[2]);
-                vb_split3(r1, q[0], q[1], q[2]);
+                pr_split<TERMS>(r0, p[0], p[1], p[2]);
+                pr_split<TERMS>(r1, q[0], q[1], q[2]);
 #pragma unroll
                 for (int j = 0; j < TERMS; j++) {
                     uint16_t *o = a.out_terms + ((size_t)j * a.out_rows_pad + m) * ko + col;
@@ -181,7 +187,7 @@ VB_DEVINL void pr_store(const RowsArgs &a, const float *stg, const PrTile &tl, i
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 if (a.epi == TC_EPI_RELU2_TERMS) { e[i] = fmaxf(e[i], 0.0f); e[i] *= e[i]; }
-                vb_split3(e[i], q[0][i], q[1][i], q[2][i]);
+                pr_split<TERMS>(e[i], q[0][i], q[1][i], q[2][i]);
             }
 #pragma unroll
             for (int j = 0; j < TERMS; j++) {
@@ -461,10 +467,11 @@ long long launch_cost(int M, int pairs, int k_iters, int splits, int clusters, i
     return (tiles + clusters - 1) / clusters * (k_iters * (long long)(std::max(2 * terms * R, 128 * (1 + terms) + terms * R) + 24) + 200) + 24 * R;
 }
 int pick_rows(int M, int pairs, int k_iters, int splits, int clusters, int terms) {
+    const int least = terms == 3 ? 32 : 64;
     int best = 0;
     long long cost = 0;
-    for (int R = terms == 3 ? PrCfg<3>::max_rows : PrCfg<2>::max_rows; R >= 64; R -= 32) {
-        if (R > 64 && R >= M + 32) continue;
+    for (int R = terms == 3 ? PrCfg<3>::max_rows : PrCfg<2>::max_rows; R >= least; R -= 32) {
+        if (R > least && R >= M + 32) continue;
         const long long c = launch_cost(M, pairs, k_iters, splits, clusters, R, terms);
         if (!best || c < cost) { best = R; cost = c; }
     }
@@ -536,7 +543,7 @@ int tc_gemm_rows(const TcWeight &w, const TcActs &a, const TcGemm &g, cudaStream
 int tc_gemm_grouped(const TcWeight &w, const TcActs &a, const TcGemm &g, int n, const int4 *table, int n_blocks, cudaStream_t st) {
     constexpr int kRows = 128;
     const int tiles = (n + kTcTileN - 1) / kTcTileN;
-    if (!w.ok || !w.tiled || !a.ok || w.K != a.K || n < 1 || n_blocks < 1 || !table || g.splits != 1 || g.terms != 2) return -1;
+    if (!w.ok || !w.tiled || !a.ok || w.K != a.K || n < 1 || n_blocks < 1 || !table || g.splits != 1) return -1;
     if (w.N % (tiles * kTcTileN) || (size_t)n_blocks * kRows > (size_t)a.rows_pad || g.act_n0 != 0) return -1;
     if (g.epi == TC_EPI_TERMS || g.epi == TC_EPI_RELU2_TERMS) {
         if (!terms_epilogue_ok(g) || g.out_rows_pad < n_blocks * kRows) return -1;
@@ -552,7 +559,7 @@ int tc_gemm_grouped(const TcWeight &w, const TcActs &a, const TcGemm &g, int n, 
     ra.row_blocks = n_blocks;
     ra.pairs = (tiles + 1) / 2;
     ra.table = table; ra.group_tiles = tiles;
-    return launch_pair<true, 2>(w, a, ra, clusters, st);
+    return g.terms == 3 ? launch_pair<true, 3>(w, a, ra, clusters, st) : launch_pair<true, 2>(w, a, ra, clusters, st);
 }
 
 } // namespace vb
