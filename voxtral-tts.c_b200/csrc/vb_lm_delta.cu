@@ -8,7 +8,7 @@
  *   lm_delta_inputs  convolution, unit norms, step sizes beta, decays: 16 rows per CTA; inner products
  *                    of the scan's groups
  *   lm_delta_scan    the recurrence in fp32, four tokens at a time; columns of S are independent, so a CTA
- *                    owns 16 of a head's value columns, S in registers, eight or more lanes per column
+ *                    owns 16 to 32 of a head's value columns, S in registers, eight or more lanes per pair of columns
  *   lm_delta_gate    head norm and gate of a row; saves the raw convolution inputs of the last rows
  *   lm_delta_step    one token in one launch: a cluster of CTAs per head, 32 value columns each
  *
@@ -31,55 +31,73 @@ VB_DEVINL float softplus(float z) { return fmaxf(z, 0.0f) + log1pf(expf(-fabsf(z
 
 /* ------------------------------------------------------------------ inputs of the recurrence */
 constexpr int kScGroup = kLmDeltaGroup, kGramRow = 2 * kScGroup * kScGroup;
-constexpr int kInThreads = 128, kInRows = kLmDeltaRows;
+constexpr int kInThreads = 256, kInHalf = kInThreads / 2, kInRows = kLmDeltaRows;
 
-/* Short convolution and silu of `size` channels from c0 on, rows [r0, r0 + rows): out[row][ld_out].
- * `raw` is room for the inputs, earlier tokens included. */
+/* Short convolution and silu of `size` channels from c0 on, rows [r0, r0 + rows), by `threads` threads of the CTA (all of
+ * which come here): out[row][ld_out]. `raw` is room for the inputs, earlier tokens included. */
 VB_DEVINL void conv_rows(const LmDelta &a, float *raw, float *out, int ld_out, int c0, int size, int r0, int rows, const float *tail,
-                         int ch, int pos0) {
-    const int tid = threadIdx.x, past = a.taps - 1;
-    auto past_row = [&](int r, int c) {          /* an earlier token's input, zero before the sequence's start */
-        return pos0 + r >= 0 ? tail[(size_t)((pos0 + r) % a.taps) * ch + c] : 0.0f;
-    };
-    if (((c0 | size) & 3) == 0) {
+                         int ch, int pos0, int tid, int threads) {
+    const int past = a.taps - 1;
+    auto past_at = [&](int r) { return tail + (size_t)((pos0 + r) % a.taps) * ch; };   /* an earlier token's inputs */
+    if (((c0 | size | ch) & 3) == 0) {
         const int per = size / 4;
-        for (int i = tid; i < (past + rows) * per; i += kInThreads) {
+#pragma unroll 2
+        for (int i = tid; i < (past + rows) * per; i += threads) {
             const int r = r0 - past + i / per, d = i % per * 4, c = c0 + d;
-            *reinterpret_cast<float4 *>(raw + (i / per) * size + d) =
-                r >= 0 ? lm_sum4(a.in, r, c) : make_float4(past_row(r, c), past_row(r, c + 1), past_row(r, c + 2), past_row(r, c + 3));
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);           /* before the sequence's start */
+            if (r >= 0) v = lm_sum4(a.in, r, c);
+            else if (pos0 + r >= 0) v = *reinterpret_cast<const float4 *>(past_at(r) + c);
+            *reinterpret_cast<float4 *>(raw + (i / per) * size + d) = v;
         }
     } else {
-        for (int i = tid; i < (past + rows) * size; i += kInThreads) {
+        for (int i = tid; i < (past + rows) * size; i += threads) {
             const int r = r0 - past + i / size, c = c0 + i % size;
-            raw[i] = r >= 0 ? lm_sum_batch(a.in, r, c) : past_row(r, c);
+            raw[i] = r >= 0 ? lm_sum_batch(a.in, r, c) : pos0 + r >= 0 ? past_at(r)[c] : 0.0f;
         }
     }
     __syncthreads();
-    /* a thread keeps to its channels, so that their taps stay in registers */
+    /* a thread keeps to its channels, so that their taps stay in registers; spare threads take a part of the rows */
     constexpr int kRegTaps = 4;
-    for (int d = tid; d < size; d += kInThreads) {
+    const int parts = threads > size ? threads / size : 1, part = tid / size;
+    const int first = parts > 1 ? rows * part / parts : 0, end = parts > 1 ? rows * (part + 1) / parts : rows;
+    if (parts > 1 && part >= parts) return;
+    for (int d = parts > 1 ? tid % size : tid; d < size; d += threads) {
         const float *w = a.conv + (size_t)(c0 + d) * a.taps;
-        float wr[kRegTaps];
         if (a.taps <= kRegTaps) {
+            float wr[kRegTaps], x[kRegTaps];
 #pragma unroll
-            for (int j = 0; j < kRegTaps; j++) wr[j] = j < a.taps ? __ldg(w + j) : 0.0f;
-        }
-        for (int r = 0; r < rows; r++) {
-            float v = 0.0f;
-            if (a.taps <= kRegTaps) {
-#pragma unroll
-                for (int j = 0; j < kRegTaps; j++)
-                    if (j < a.taps) v = fmaf(wr[j], raw[(r + j) * size + d], v);
-            } else {
-                for (int j = 0; j < a.taps; j++) v = fmaf(__ldg(w + j), raw[(r + j) * size + d], v);
+            for (int j = 0; j < kRegTaps; j++) {
+                wr[j] = j < a.taps ? __ldg(w + j) : 0.0f;
+                x[j] = j < past ? raw[(first + j) * size + d] : 0.0f;
             }
-            out[(size_t)r * ld_out + d] = silu(v);
+#pragma unroll 4
+            for (int r = first; r < end; r++) {
+                const float now = raw[(r + past) * size + d];
+                float v = 0.0f;
+#pragma unroll
+                for (int j = 0; j < kRegTaps; j++) {
+                    if (j == past) x[j] = now;
+                    if (j < a.taps) v = fmaf(wr[j], x[j], v);
+                }
+#pragma unroll
+                for (int j = 0; j + 1 < kRegTaps; j++) x[j] = x[j + 1];
+                out[(size_t)r * ld_out + d] = silu(v);
+            }
+        } else {
+            for (int r = first; r < end; r++) {
+                float v = 0.0f;
+                for (int j = 0; j < a.taps; j++) v = fmaf(__ldg(w + j), raw[(r + j) * size + d], v);
+                out[(size_t)r * ld_out + d] = silu(v);
+            }
         }
     }
 }
 
-/* grid = (row tiles, kv_heads + heads + 1): q and k of a key head, v of a value head, or (last)
- * step sizes and decays. The q and k CTAs also leave the inner products of the scan's groups. */
+/* grid = (row tiles, kv_heads + heads + 1): q and k of a key head (half of the threads each), v of a value head, or (last)
+ * step sizes and decays. The q and k CTAs also leave the inner products of the scan's groups, a warp those of k or
+ * of q in one group. Bound by the chain of its stages where the rows are few, by its bytes in a prompt. (q after k, an inner
+ * product at a time and the rows of a tile one after another: 26 us for five rows of 16 heads of 128, 70 us for
+ * 2048 of 24.) */
 __global__ void __launch_bounds__(kInThreads) lm_delta_inputs_kernel(const LmDelta a, int M) {
     extern __shared__ __align__(16) float in_smem[];
     pdl_launch_dependents();
@@ -91,8 +109,8 @@ __global__ void __launch_bounds__(kInThreads) lm_delta_inputs_kernel(const LmDel
         for (int i = tid; i < rows * H; i += kInThreads) {
             const int r = r0 + i / H, h = i % H;
             const int cb = ch + H * a.vdim;           /* columns: q, k, v, gate, b, a */
-            a.beta[(size_t)r * H + h] = 1.0f / (1.0f + expf(-lm_sum(a.in, r, cb + h)));
-            a.decays[(size_t)r * H + h] = expf(-__ldg(a.decay + h) * softplus(lm_sum(a.in, r, cb + H + h) + __ldg(a.dt_bias + h)));
+            a.beta[(size_t)r * H + h] = 1.0f / (1.0f + expf(-lm_sum_batch(a.in, r, cb + h)));
+            a.decays[(size_t)r * H + h] = expf(-__ldg(a.decay + h) * softplus(lm_sum_batch(a.in, r, cb + H + h) + __ldg(a.dt_bias + h)));
         }
         return;
     }
@@ -101,46 +119,56 @@ __global__ void __launch_bounds__(kInThreads) lm_delta_inputs_kernel(const LmDel
     if (unit >= G) {
         const int head = unit - G;
         conv_rows(a, in_smem, a.v + (size_t)r0 * H * a.vdim + head * a.vdim, H * a.vdim, 2 * nqk + head * a.vdim, a.vdim, r0, rows, tail, ch,
-                  pos0);
+                  pos0, tid, kInThreads);
         return;
     }
-    const int dim = a.dim;
-    float *qk = in_smem, *raw = qk + 2 * kInRows * dim;         /* [q, k][kInRows][dim], room for the raw rows */
-    for (int kind = 0; kind < 2; kind++) {
-        float *out = qk + kind * kInRows * dim, *dst = kind == 0 ? a.q : a.k;
-        conv_rows(a, raw, out, dim, kind * nqk + unit * dim, dim, r0, rows, tail, ch, pos0);
-        __syncthreads();
-        const float post = kind == 0 ? 1.0f / sqrtf((float)dim) : 1.0f;
-        for (int r = warp; r < kInRows; r += kInThreads / 32) {
-            float s = 0.0f;
-            if (r < rows)
-                for (int d = lane; d < dim; d += 32) s += out[r * dim + d] * out[r * dim + d];
-            s = vb_warp_sum(s);
-            const float f = 1.0f / sqrtf(s + 1e-6f) * post;
-            for (int d = lane; d < dim; d += 32) {
-                const float v = r < rows ? out[r * dim + d] * f : 0.0f;
-                out[r * dim + d] = v;
-                if (r < rows) dst[(size_t)(r0 + r) * nqk + unit * dim + d] = v;
-            }
-        }
-        __syncthreads();
-    }
-    /* inner products inside a group of kScGroup tokens: k_t . k_j and q_t . k_j */
-    const float *Q = qk, *K = qk + kInRows * dim;
-    for (int i = warp; i < kInRows / kScGroup * kGramRow; i += kInThreads / 32) {
-        const int j = i % kScGroup, t = i / kScGroup % kScGroup, isq = i / (kScGroup * kScGroup) % 2, grp = i / kGramRow;
+    const int dim = a.dim, kind = tid / kInHalf, raw_rows = kInRows + a.taps - 1;
+    float *qk = in_smem, *raw = qk + 2 * kInRows * dim + kind * raw_rows * dim;         /* [q, k][kInRows][dim], room for the raw rows of both */
+    float *out = qk + kind * kInRows * dim, *dst = kind == 0 ? a.q : a.k;
+    conv_rows(a, raw, out, dim, kind * nqk + unit * dim, dim, r0, rows, tail, ch, pos0, tid % kInHalf, kInHalf);
+    __syncthreads();
+    const float post = kind == 0 ? 1.0f / sqrtf((float)dim) : 1.0f;
+#pragma unroll
+    for (int r = warp % (kInHalf / 32); r < kInRows; r += kInHalf / 32) {
         float s = 0.0f;
-        if (j <= t) {
-            const float *x = (isq ? Q : K) + (grp * kScGroup + t) * dim, *y = K + (grp * kScGroup + j) * dim;
-            for (int d = lane; d < dim; d += 32) s = fmaf(x[d], y[d], s);
-        }
+        if (r < rows)
+            for (int d = lane; d < dim; d += 32) s += out[r * dim + d] * out[r * dim + d];
         s = vb_warp_sum(s);
-        if (lane == 0) a.gram[((size_t)(r0 / kScGroup + grp) * G + unit) * kGramRow + isq * kScGroup * kScGroup + t * kScGroup + j] = s;
+        const float f = 1.0f / sqrtf(s + 1e-6f) * post;
+        for (int d = lane; d < dim; d += 32) {
+            const float v = r < rows ? out[r * dim + d] * f : 0.0f;
+            out[r * dim + d] = v;
+            if (r < rows) dst[(size_t)(r0 + r) * nqk + unit * dim + d] = v;
+        }
     }
+    __syncthreads();
+    /* inner products inside a group of kScGroup tokens: k_t . k_j and q_t . k_j */
+    static_assert(kInThreads / 32 == 2 * (kInRows / kScGroup), "a warp per group and kind");
+    const int isq = warp & 1, grp = warp >> 1;
+    if (grp * kScGroup >= rows) return;
+    const float *X = qk + (isq ? 0 : kInRows * dim) + grp * kScGroup * dim, *K = qk + (kInRows + grp * kScGroup) * dim;
+    float s[kScGroup][kScGroup] = {};
+    for (int d = lane; d < dim; d += 32) {
+        float x[kScGroup], y[kScGroup];
+#pragma unroll
+        for (int t = 0; t < kScGroup; t++) { x[t] = X[t * dim + d]; y[t] = K[t * dim + d]; }
+#pragma unroll
+        for (int t = 0; t < kScGroup; t++)
+#pragma unroll
+            for (int j = 0; j <= t; j++) s[t][j] = fmaf(x[t], y[j], s[t][j]);
+    }
+    float *to = a.gram + ((size_t)(r0 / kScGroup + grp) * G + unit) * kGramRow + isq * kScGroup * kScGroup;
+#pragma unroll
+    for (int t = 0; t < kScGroup; t++)
+#pragma unroll
+        for (int j = 0; j < kScGroup; j++) {
+            const float v = j <= t ? vb_warp_sum(s[t][j]) : 0.0f;
+            if (lane == 0) to[t * kScGroup + j] = v;
+        }
 }
 
 /* ------------------------------------------------------------------ the recurrence */
-constexpr int kScCols = 16, kScTok = 16, kScGroups = kScTok / kScGroup, kScBufs = 3;
+constexpr int kScMaxCols = 32, kScPer = 2, kScTok = 16, kScCtas = 148, kScGroups = kScTok / kScGroup, kScBufs = 3;
 
 /* two fp32 lanes per instruction */
 VB_DEVINL uint64_t f2_pack(float lo, float hi) {
@@ -190,27 +218,29 @@ struct __align__(16) ScanCoef {
  * sizes, decays and inner products, and the coefficients made of them. */
 template <int DP>
 struct __align__(16) ScanBuf {
-    float k[kScTok][DP], q[kScTok][DP], v[kScTok][kScCols], gram[kScGroups][kGramRow], beta[kScTok], g[kScTok];
+    float k[kScTok][DP], q[kScTok][DP], v[kScTok][kScMaxCols], gram[kScGroups][kGramRow], beta[kScTok], g[kScTok];
     ScanCoef coef[kScGroups];
 };
 
-/* grid = (value column tiles, heads). All warps but the last hold S: LPC lanes per column, each with
+/* grid = (tiles of COLS value columns, heads). All warps but the last hold S: LPC lanes per pair of columns, each with
  * NR rows in groups of four (lane rg takes groups rg, rg + LPC, ...). Four tokens at a time: their
- * eight inner products with S (S^T k_t, S^T q_t) are independent and are summed over the lanes in
+ * eight inner products with a column of S (S^T k_t, S^T q_t) are independent and are summed over the lanes in
  * one halving butterfly, the rest is scalars. The last warp copies the inputs of the next blocks
  * of kScTok tokens (bulk copies where rows start on 16-byte boundaries) and works out their
- * coefficients. */
-template <int LPC, int NR>
-__global__ void __launch_bounds__(kScCols * LPC + 32) lm_delta_scan_kernel(const LmDelta a, int M) {
+ * coefficients.
+ * Bound by the reads of k and q from shared memory (every lane reads its rows of each for all of its columns, a quarter
+ * warp at a time) and the chain of a group; one column a lane and 16 a CTA: 435 us per 2048 tokens of 24 heads of 128. */
+template <int LPC, int NR, int COLS>
+__global__ void __launch_bounds__(COLS / kScPer * LPC + 32) lm_delta_scan_kernel(const LmDelta a, int M) {
     static_assert(kScGroup == 4 && LPC >= 8, "the butterfly spreads eight values over at least eight lanes");
-    constexpr int DP = LPC * NR, kCompute = kScCols * LPC, kThreads = kCompute + 32, NG = NR / 4;
+    constexpr int DP = LPC * NR, kCompute = COLS / kScPer * LPC, kThreads = kCompute + 32, NG = NR / 4;
     extern __shared__ __align__(16) unsigned char scan_smem[];
     __shared__ uint64_t full[kScBufs];
     __shared__ volatile int gave_up;
     ScanBuf<DP> *buf = reinterpret_cast<ScanBuf<DP> *>(scan_smem);
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, h = blockIdx.y, kv = h / (a.heads / a.kv_heads);
-    const int c0 = blockIdx.x * kScCols;
+    const int c0 = blockIdx.x * COLS;
     const int nqk = a.kv_heads * a.dim, nv = a.heads * a.vdim, n_blocks = (M + kScTok - 1) / kScTok;
     const bool bulk = ((a.dim | a.vdim) & 3) == 0;
     /* rows and columns beyond the sizes stay zero in every buffer */
@@ -226,7 +256,7 @@ __global__ void __launch_bounds__(kScCols * LPC + 32) lm_delta_scan_kernel(const
 
     if (tid >= kCompute) {
         /* ---- inputs and coefficients ---- */
-        const int cols = a.vdim - c0 < kScCols ? a.vdim - c0 : kScCols;
+        const int cols = a.vdim - c0 < COLS ? a.vdim - c0 : COLS;
         auto request = [&](int blk) {
             if (blk < n_blocks && !gave_up) {
                 const int b = blk % kScBufs;
@@ -302,7 +332,7 @@ __global__ void __launch_bounds__(kScCols * LPC + 32) lm_delta_scan_kernel(const
             const int nt = M - blk * kScTok, ne = (nt + kScGroup - 1) / kScGroup * kScGroup;
             for (int t = nt; t < ne; t++) {
                 for (int i = lane; i < DP; i += 32) d.k[t][i] = d.q[t][i] = 0.0f;
-                if (lane < kScCols) d.v[t][lane] = 0.0f;
+                if (lane < COLS) d.v[t][lane] = 0.0f;
             }
         };
         request(0);
@@ -321,22 +351,23 @@ __global__ void __launch_bounds__(kScCols * LPC + 32) lm_delta_scan_kernel(const
         return;
     }
 
-    const int rg = tid % LPC, cl = tid / LPC, c = c0 + cl;
-    const bool live = c < a.vdim;
+    const int rg = tid % LPC, cl = tid / LPC * kScPer, c = c0 + cl;      /* this thread's first column, in the tile and in the head */
     float *S = lm_state(a.s, a.dyn) + (size_t)h * a.dim * a.vdim;
-    uint64_t s[NR / 2];
+    uint64_t s[kScPer][NR / 2];
     const bool fresh = a.dyn->pos == 0;
 #pragma unroll
-    for (int i = 0; i < NG; i++) {
-        float x[4];
+    for (int p = 0; p < kScPer; p++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int r = (i * LPC + rg) * 4 + j;
-            x[j] = (!fresh && live && r < a.dim) ? S[(size_t)r * a.vdim + c] : 0.0f;
+        for (int i = 0; i < NG; i++) {
+            float x[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int r = (i * LPC + rg) * 4 + j;
+                x[j] = (!fresh && c + p < a.vdim && r < a.dim) ? S[(size_t)r * a.vdim + c + p] : 0.0f;
+            }
+            s[p][2 * i] = f2_pack(x[0], x[1]);
+            s[p][2 * i + 1] = f2_pack(x[2], x[3]);
         }
-        s[2 * i] = f2_pack(x[0], x[1]);
-        s[2 * i + 1] = f2_pack(x[2], x[3]);
-    }
     auto load = [&](uint64_t (&x)[NR / 2], const float *row) {
 #pragma unroll
         for (int i = 0; i < NG; i++) {
@@ -345,19 +376,19 @@ __global__ void __launch_bounds__(kScCols * LPC + 32) lm_delta_scan_kernel(const
             x[2 * i + 1] = y.y;
         }
     };
-    auto dot = [&](const uint64_t (&x)[NR / 2]) {
+    auto dot = [&](const uint64_t (&y)[NR / 2], const uint64_t (&x)[NR / 2]) {
         uint64_t e0 = 0, e1 = 0;
 #pragma unroll
         for (int i = 0; i < NR / 2; i += 2) {
-            e0 = f2_fma(s[i], x[i], e0);
-            e1 = f2_fma(s[i + 1], x[i + 1], e1);
+            e0 = f2_fma(y[i], x[i], e0);
+            e1 = f2_fma(y[i + 1], x[i + 1], e1);
         }
         return f2_sum(f2_add(e0, e1));
     };
     /* after the butterfly lane rg holds value rg / (LPC / 8): 0 .. 3 are S^T k_t, 4 .. 7 are S^T q_t */
     constexpr int kShare = LPC / 8;
     const int mine = rg / kShare, lane0 = lane & ~(LPC - 1), ot = mine & 3;
-    const bool writes = live && mine >= 4 && rg % kShare == 0;
+    const bool writes = mine >= 4 && rg % kShare == 0;
     float *out = a.o + h * a.vdim + c;
     __syncthreads();                                      /* block 0 is ready */
     for (int blk = 0; blk < n_blocks; blk++) {
@@ -370,69 +401,88 @@ __global__ void __launch_bounds__(kScCols * LPC + 32) lm_delta_scan_kernel(const
         for (int tg = 0; tg < nt; tg += kScGroup) {
             const ScanCoef &x = in.coef[tg / kScGroup];
             uint64_t k[4][NR / 2];
-            float y[8];
+            float y[kScPer][8];
 #pragma unroll
             for (int t = 0; t < 4; t++) {
                 uint64_t qt[NR / 2];
                 load(k[t], in.k[tg + t]);
                 load(qt, in.q[tg + t]);
-                y[t] = dot(k[t]);
-                y[4 + t] = dot(qt);
+#pragma unroll
+                for (int p = 0; p < kScPer; p++) {
+                    y[p][t] = dot(s[p], k[t]);
+                    y[p][4 + t] = dot(s[p], qt);
+                }
             }
             const float4 beta = *reinterpret_cast<const float4 *>(x.beta), ec = *reinterpret_cast<const float4 *>(x.e),
                          u0 = *reinterpret_cast<const float4 *>(x.u), u1 = *reinterpret_cast<const float4 *>(x.u + 4),
                          sc = *reinterpret_cast<const float4 *>(x.s), oc = *reinterpret_cast<const float4 *>(x.o[ot]);
             const float oe = x.c[ot], c3 = x.c[3];
-            const float v0 = beta.x * in.v[tg][cl], v1 = beta.y * in.v[tg + 1][cl], v2 = beta.z * in.v[tg + 2][cl], v3 = beta.w * in.v[tg + 3][cl];
-            /* eight sums over the LPC lanes */
+            float2 v[4];
+#pragma unroll
+            for (int t = 0; t < 4; t++) v[t] = *reinterpret_cast<const float2 *>(&in.v[tg + t][cl]);
+            const uint64_t cc = f2_pack(c3, c3);
+            /* eight sums over the LPC lanes, for each column */
 #pragma unroll
             for (int n = 4, off = LPC / 2; n >= 1; n >>= 1, off >>= 1) {
                 const bool up = (rg & off) != 0;
 #pragma unroll
-                for (int i = 0; i < n; i++) {
-                    const float send = up ? y[i] : y[i + n], keep = up ? y[i + n] : y[i];
-                    y[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-                }
+                for (int p = 0; p < kScPer; p++)
+#pragma unroll
+                    for (int i = 0; i < n; i++) {
+                        const float send = up ? y[p][i] : y[p][i + n], keep = up ? y[p][i + n] : y[p][i];
+                        y[p][i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+                    }
+            }
+            float e[kScPer][4];
+#pragma unroll
+            for (int p = 0; p < kScPer; p++) {
+#pragma unroll
+                for (int off = kShare / 2; off >= 1; off >>= 1) y[p][0] += __shfl_xor_sync(0xffffffffu, y[p][0], off);
+#pragma unroll
+                for (int t = 0; t < 4; t++) e[p][t] = __shfl_sync(0xffffffffu, y[p][0], lane0 + t * kShare);
+#pragma unroll
+                for (int i = 0; i < NR / 2; i++) s[p][i] = f2_mul(s[p][i], cc);
             }
 #pragma unroll
-            for (int off = kShare / 2; off >= 1; off >>= 1) y[0] += __shfl_xor_sync(0xffffffffu, y[0], off);
-            const float e0 = __shfl_sync(0xffffffffu, y[0], lane0), e1 = __shfl_sync(0xffffffffu, y[0], lane0 + kShare),
-                        e2 = __shfl_sync(0xffffffffu, y[0], lane0 + 2 * kShare), e3 = __shfl_sync(0xffffffffu, y[0], lane0 + 3 * kShare);
-            const uint64_t cc = f2_pack(c3, c3);
+            for (int p = 0; p < kScPer; p++) {
+                const float v0 = beta.x * (p ? v[0].y : v[0].x), v1 = beta.y * (p ? v[1].y : v[1].x), v2 = beta.z * (p ? v[2].y : v[2].x),
+                            v3 = beta.w * (p ? v[3].y : v[3].x);
+                const float w0 = fmaf(ec.x, e[p][0], v0);
+                const float w1 = fmaf(u0.x, w0, fmaf(ec.y, e[p][1], v1));
+                const float w2 = fmaf(u0.z, w1, fmaf(u0.y, w0, fmaf(ec.z, e[p][2], v2)));
+                const float w3 = fmaf(u1.y, w2, fmaf(u1.x, w1, fmaf(u0.w, w0, fmaf(ec.w, e[p][3], v3))));
+                const uint64_t d0 = f2_pack(sc.x * w0, sc.x * w0), d1 = f2_pack(sc.y * w1, sc.y * w1), d2 = f2_pack(sc.z * w2, sc.z * w2),
+                               d3 = f2_pack(sc.w * w3, sc.w * w3);
 #pragma unroll
-            for (int i = 0; i < NR / 2; i++) s[i] = f2_mul(s[i], cc);
-            const float w0 = fmaf(ec.x, e0, v0);
-            const float w1 = fmaf(u0.x, w0, fmaf(ec.y, e1, v1));
-            const float w2 = fmaf(u0.z, w1, fmaf(u0.y, w0, fmaf(ec.z, e2, v2)));
-            const float w3 = fmaf(u1.y, w2, fmaf(u1.x, w1, fmaf(u0.w, w0, fmaf(ec.w, e3, v3))));
-            const uint64_t d0 = f2_pack(sc.x * w0, sc.x * w0), d1 = f2_pack(sc.y * w1, sc.y * w1), d2 = f2_pack(sc.z * w2, sc.z * w2),
-                           d3 = f2_pack(sc.w * w3, sc.w * w3);
-#pragma unroll
-            for (int i = 0; i < NR / 2; i++) s[i] = f2_fma(k[3][i], d3, f2_fma(k[2][i], d2, f2_fma(k[1][i], d1, f2_fma(k[0][i], d0, s[i]))));
-            const float o = fmaf(oc.w, w3, fmaf(oc.z, w2, fmaf(oc.y, w1, fmaf(oc.x, w0, oe * y[0]))));
-            if (writes && tg + ot < nt) out[(size_t)(t0 + tg + ot) * nv] = o;
+                for (int i = 0; i < NR / 2; i++)
+                    s[p][i] = f2_fma(k[3][i], d3, f2_fma(k[2][i], d2, f2_fma(k[1][i], d1, f2_fma(k[0][i], d0, s[p][i]))));
+                const float o = fmaf(oc.w, w3, fmaf(oc.z, w2, fmaf(oc.y, w1, fmaf(oc.x, w0, oe * y[p][0]))));
+                if (writes && c + p < a.vdim && tg + ot < nt) out[(size_t)(t0 + tg + ot) * nv + p] = o;
+            }
         }
         __syncthreads();                                  /* block blk is done with, blk + 1 is ready */
     }
 #pragma unroll
-    for (int i = 0; i < NR / 2; i++) {
-        float x[2];
-        asm("mov.b64 {%0, %1}, %2;" : "=f"(x[0]), "=f"(x[1]) : "l"(s[i]));
+    for (int p = 0; p < kScPer; p++)
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int r = ((i / 2) * LPC + rg) * 4 + (i & 1) * 2 + j;
-            if (live && r < a.dim) S[(size_t)r * a.vdim + c] = x[j];
+        for (int i = 0; i < NR / 2; i++) {
+            float x[2];
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(x[0]), "=f"(x[1]) : "l"(s[p][i]));
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const int r = ((i / 2) * LPC + rg) * 4 + (i & 1) * 2 + j;
+                if (c + p < a.vdim && r < a.dim) S[(size_t)r * a.vdim + c + p] = x[j];
+            }
         }
-    }
 }
 
-template <int LPC, int NR>
+template <int LPC, int NR, int COLS>
 int launch_scan(const LmDelta &a, int M, cudaStream_t st) {
     constexpr size_t smem = kScBufs * sizeof(ScanBuf<LPC * NR>);
     static_assert(smem <= 220 * 1024, "over what a CTA may use");
     static bool attr = false;
     if (!attr) {
-        if (cudaFuncSetAttribute(lm_delta_scan_kernel<LPC, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+        if (cudaFuncSetAttribute(lm_delta_scan_kernel<LPC, NR, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
             cudaGetLastError();
             return -1;
         }
@@ -440,8 +490,16 @@ int launch_scan(const LmDelta &a, int M, cudaStream_t st) {
     }
     /* A plain launch: started early, under the tail of the kernel before it, the CTAs would crowd onto the first
      * SMs that have room, and this kernel's time is that of its most crowded SM. */
-    lm_delta_scan_kernel<LPC, NR><<<dim3((a.vdim + kScCols - 1) / kScCols, a.heads), kScCols * LPC + 32, smem, st>>>(a, M);
+    lm_delta_scan_kernel<LPC, NR, COLS><<<dim3((a.vdim + COLS - 1) / COLS, a.heads), COLS / kScPer * LPC + 32, smem, st>>>(a, M);
     return ok(cudaGetLastError());
+}
+
+/* Columns per CTA: the fewest that leave every CTA an SM of its own (the time is that of the most crowded SM); 32 beyond. */
+template <int LPC, int NR>
+int launch_scan(const LmDelta &a, int M, cudaStream_t st) {
+    const int ctas = kScCtas / a.heads;                  /* per head */
+    if (ctas >= (a.vdim + 15) / 16) return launch_scan<LPC, NR, 16>(a, M, st);
+    return ctas >= (a.vdim + 23) / 24 ? launch_scan<LPC, NR, 24>(a, M, st) : launch_scan<LPC, NR, 32>(a, M, st);
 }
 
 /* ------------------------------------------------------------------ head norm, gate, convolution memory */
@@ -631,7 +689,7 @@ int lm_delta_channels(int heads, int kv_heads, int dim, int vdim) { return 2 * k
 bool lm_delta_supported(int dim, int vdim) { return dim >= 1 && dim <= 256 && vdim >= 1; }
 
 int lm_delta_inputs(const LmDelta &a, int M, cudaStream_t st) {
-    const size_t raw = kInRows + a.taps - 1, qk = (raw + 2 * kInRows) * a.dim, v = raw * a.vdim;
+    const size_t raw = kInRows + a.taps - 1, qk = 2 * (raw + kInRows) * a.dim, v = raw * a.vdim;
     const size_t smem = sizeof(float) * (qk > v ? qk : v);
     if (smem > 200 * 1024) return -1;
     static size_t set = 48 * 1024;
