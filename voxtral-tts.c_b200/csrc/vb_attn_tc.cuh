@@ -62,11 +62,33 @@ struct AtCfg {
     static_assert(kAtQ + (kQlTmem ? 2 : 1) * DK * 32 <= kAtTmemCols, "Q does not fit TMEM");
 };
 
-VB_DEVINL void at_mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+/* A descriptor's low word, which holds the address and is what the steps of a product add to; the high word is the same for
+ * all of an operand. (Sums of whole descriptors came out wrong in one of three copies of the score products, heads of
+ * 192, when the kernel around them changed: low halves of the queries read from beyond their place.) */
+struct AtDesc {
+    uint32_t lo, hi;
+    VB_DEVINL explicit AtDesc(uint64_t d) : lo((uint32_t)d), hi((uint32_t)(d >> 32)) {}
+    VB_DEVINL AtDesc at(int units) const {          /* so many 16 bytes on */
+        AtDesc r = *this;
+        r.lo += (uint32_t)units;
+        return r;
+    }
+};
+VB_DEVINL void at_mma_ts(uint32_t d, uint32_t a, AtDesc b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+        "mov.b64 db, {%2, %3};\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(d), "r"(a), "r"(b.lo), "r"(b.hi), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+VB_DEVINL void at_mma_ss(uint32_t d, AtDesc a, AtDesc b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+        "mov.b64 da, {%1, %2};\n\t"
+        "mov.b64 db, {%3, %4};\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(d), "r"(a.lo), "r"(a.hi), "r"(b.lo), "r"(b.hi), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 #define VB_AT_R8(r, o) "r"((r)[o]), "r"((r)[o + 1]), "r"((r)[o + 2]), "r"((r)[o + 3]), "r"((r)[o + 4]), "r"((r)[o + 5]), "r"((r)[o + 6]), "r"((r)[o + 7])
@@ -469,24 +491,24 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const __grid_
         const uint32_t idesc_s = at_idesc(kAtKeys, false), idesc_o = at_idesc((a.vdim + 15) & ~15, true);
         /* descriptors once: the one issuing thread has 32 to 64 clocks per MMA (addresses stay below 2^18, so sums carry
          * into nothing else) */
-        const uint64_t k_desc = umma_desc_k_sw128(k_s), q_desc = umma_desc_k_sw128(ql_s), v_desc = at_desc_mn(vb_smem_u32(v_s));
+        const AtDesc k_desc(umma_desc_k_sw128(k_s)), q_desc(umma_desc_k_sw128(ql_s)), v_desc(at_desc_mn(vb_smem_u32(v_s)));
         bool ok = vb_mbar_wait(q_full, 0u, abort_flag);
         tc_fence_after();
         auto scores = [&](int t) {
             const int slot = t % Cfg::kSlots;
             if (!vb_mbar_wait(&k_full[slot], (uint32_t)(t / Cfg::kSlots) & 1u, abort_flag)) return false;
             tc_fence_after();
-            const uint64_t kd = k_desc + (uint64_t)(slot * (Cfg::kSlotK >> 4));
+            const AtDesc kd = k_desc.at(slot * (Cfg::kSlotK >> 4));
             const uint32_t d = tmem + (uint32_t)((t & 1) * kAtKeys);
 #pragma unroll
             for (int ks = 0; ks < DK * 4; ks++) {
                 if (ks >= k_steps) break;
-                const uint64_t hi = kd + (uint64_t)((ks >> 2) * (kAtBlock >> 4) + 2 * (ks & 3)), lo = hi + DK * (kAtBlock >> 4);
+                const AtDesc hi = kd.at((ks >> 2) * (kAtBlock >> 4) + 2 * (ks & 3)), lo = hi.at(DK * (kAtBlock >> 4));
                 const uint32_t qh = tmem + kAtQ + (uint32_t)(ks * 8);
                 at_mma_ts(d, qh, hi, idesc_s, ks != 0 ? 1u : 0u);
                 at_mma_ts(d, qh, lo, idesc_s, 1u);
                 if constexpr (Cfg::kQlTmem) at_mma_ts(d, qh + DK * 32, hi, idesc_s, 1u);
-                else umma_bf16(d, q_desc + (uint64_t)((ks >> 2) * (kAtRows * 128 >> 4) + 2 * (ks & 3)), hi, idesc_s, 1u);
+                else at_mma_ss(d, q_desc.at((ks >> 2) * (kAtRows * 128 >> 4) + 2 * (ks & 3)), hi, idesc_s, 1u);
             }
             umma_commit(&k_empty[slot]);
             umma_commit(&s_full[t & 1]);
@@ -500,11 +522,11 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const __grid_
                  vb_mbar_wait(&p_full[w], (uint32_t)(t >> 1) & 1u, abort_flag);
             if (!ok) break;
             tc_fence_after();
-            const uint64_t vd = v_desc + (uint64_t)(slot * (Cfg::kSlotV >> 4));
+            const AtDesc vd = v_desc.at(slot * (Cfg::kSlotV >> 4));
             const uint32_t d = tmem + kAtO + (uint32_t)(w * 128);
 #pragma unroll
             for (int ks = 0; ks < kAtKeys / 16; ks++) {
-                const uint64_t hi = vd + (uint64_t)(ks * (2048 >> 4)), lo = hi + DV * (kAtBlock >> 4);
+                const AtDesc hi = vd.at(ks * (2048 >> 4)), lo = hi.at(DV * (kAtBlock >> 4));
                 const uint32_t ph = tmem + (uint32_t)(w * kAtKeys + (ks >> 1) * 32 + (ks & 1) * 8);
                 at_mma_ts(d, ph, hi, idesc_o, (t >> 1 | ks) != 0 ? 1u : 0u);
                 at_mma_ts(d, ph, lo, idesc_o, 1u);
