@@ -38,9 +38,9 @@ static const int NSEM = VB200_SEM_PADDED;
 constexpr int kHD = VB200_HEAD_DIM;        /* 128 */
 constexpr int kGroup = VB200_HEADS / VB200_KV_HEADS;   /* 4 query heads per KV head */
 constexpr int kBtMaxUtt = 8;
-constexpr int kBtKeySplits = 16;           /* CTAs sharing one (utterance, KV head) */
-constexpr int kBtSubsets = 4;              /* warp subsets of a CTA's key range */
-constexpr int kBtAttnThreads = 512;
+constexpr int kBtMaxSplits = 8;            /* CTAs sharing one (utterance, KV head) */
+constexpr int kBtAttnThreads = 256, kBtAttnWarps = 8;
+constexpr int kBtKeys = 8;                 /* keys a warp takes at a time */
 constexpr int kCodeStride = 40;            /* ints per utterance in the codes block */
 
 /* Decoder weights on the tensor-core path (tile-contiguous copies), shared by every context. */
@@ -109,8 +109,6 @@ struct Batch {
     float *part = nullptr, *ssq = nullptr, *logit_part = nullptr;
     float *part_qkv = nullptr, *part_wo = nullptr, *part_w2 = nullptr;   /* = part, or the tensor-parallel arena's */
     bool tp = false;                            /* this context runs tensor-parallel */
-    float *attn_scratch = nullptr;
-    unsigned *tickets = nullptr;
     AcBuffers ac;
     /* the decoder step as one launch of the persistent streaming kernel (vb_stream.cu) */
     bool stream = false, s_tap = false;
@@ -253,218 +251,204 @@ __global__ void bt_embed_kernel(float *X, const uint16_t *table, const int *code
 /* Decode attention for one new token per utterance: split-K reduction of the QKV GEMM's
  * partials, RoPE on q and k, cache append, GQA attention over the utterance's own cache
  * (voxtral_tts_llm.c:221-238; tts_apply_rope / tts_causal_attention,
- * voxtral_tts_kernels.c:403-465, 602-634). grid = (key splits, KV heads, B); a CTA serves the
- * four query heads of its KV head on one slice of the keys; the last CTA of a (utterance,
- * KV head) to finish merges the slices in fixed order and writes the result as the three
- * BF16 terms the O projection's GEMM consumes. */
-template <bool TP, int KP>
-__global__ void __launch_bounds__(kBtAttnThreads)
+ * voxtral_tts_kernels.c:403-465, 602-634). grid = (key splits, KV heads, B), the splits of a KV head form a cluster:
+ * a CTA serves the four query heads of its KV head on one slice of the keys, a warp eight keys at a time for all
+ * four; every CTA sends the slices of the others' columns into their shared memory (asynchronous stores that count on
+ * the receiver's barrier) and merges its own share in fixed order into the three BF16 terms that the O projection's GEMM
+ * consumes.
+ *
+ * Bound by latency: 2.5 MB of keys and values at 300 rows, on a chain of trips to L2. Whatever the kernel before does
+ * not make is fetched before the wait for it: the utterance's state, the rotation angles and the keys and values of
+ * the first pass (the earlier rows of the cache and the state were written before this frame's first kernel, which is a plain
+ * launch: enqueue_decoder). With those behind the wait, a head's keys read by four warps and a merge through global
+ * memory by the last CTA to arrive: 9.8 us a layer at 260 rows. */
+template <bool TP>
+__global__ void __launch_bounds__(kBtAttnThreads, 2)
 bt_attn_kernel(uint16_t *terms, int rows_pad, const float *part, int n_part, size_t part_stride, float *kv_k,
-               float *kv_v, size_t slab, int layer, const VbDyn *dyn, float scale, float theta, float *scratch,
-               unsigned *tickets, int *status, const typename TcWaitSel<TP>::type wait) {
-    __shared__ float cs[kHD];
-    __shared__ __align__(16) float qraw[kGroup * kHD];
-    __shared__ float kraw[kHD], vraw[kHD];
-    __shared__ __align__(16) float qs[kGroup][kHD];
-    __shared__ __align__(16) float attn_o[kBtSubsets][kGroup][kHD];
-    __shared__ float attn_ml[kBtSubsets][kGroup][2];
-    __shared__ float cmb_m[kBtKeySplits * kGroup], cmb_l[kBtKeySplits * kGroup];
-    __shared__ int last_flag;
+               float *kv_v, size_t slab, int layer, const VbDyn *dyn, float scale, float theta, int *status,
+               const typename TcWaitSel<TP>::type wait) {
+    __shared__ __align__(16) float qs[kGroup][kHD], ks[kHD], vs[kHD];
+    __shared__ __align__(16) float warp_o[kBtAttnWarps][kGroup][kHD];
+    __shared__ float2 warp_ml[kBtAttnWarps][kGroup];       /* maximum, sum */
+    __shared__ float4 slices[kBtAttnThreads];              /* [S][columns of this CTA / 2]: two columns, maximum, sum */
+    __shared__ uint64_t arrived;
+    __shared__ volatile int gave_up;
     pdl_launch_dependents();
+    if (threadIdx.x == 0) {
+        vb_mbar_init(&arrived, 1);
+        gave_up = 0;
+        vb_mbar_init_fence();
+        vb_mbar_arrive_expect_tx(&arrived, (uint32_t)sizeof(slices));
+    }
+    __syncthreads();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int sp = blockIdx.x, S = gridDim.x, g = blockIdx.y, b = blockIdx.z;
+    const int pos = __ldcg(&dyn[b].pos), kv_max = __ldcg(&dyn[b].kv_max);
+    const bool done = __ldcg(&dyn[b].done) != 0, in_range = pos >= 0 && pos < kv_max;
+    const int nk = done || !in_range ? 0 : pos + 1;
+    const int j0 = (int)((long long)nk * sp / S), j1 = (int)((long long)nk * (sp + 1) / S);
+    const bool writer = sp == S - 1;   /* its key range ends with the new token */
+    float *Kc = kv_k + (size_t)b * slab + (size_t)layer * kv_max * KVD + g * kHD;
+    float *Vc = kv_v + (size_t)b * slab + (size_t)layer * kv_max * KVD + g * kHD;
+    float4 kq[kBtKeys], vq[kBtKeys];
+    auto fetch = [&](int jb) {         /* keys jb, jb + 8, ...: all requests in flight together; the new token has none */
+#pragma unroll
+        for (int u = 0; u < kBtKeys; u++) {
+            const int j = jb + u * kBtAttnWarps;
+            const bool on = j < j1 && j < pos;
+            kq[u] = on ? vb_ldcg4(Kc + (size_t)j * KVD + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+            vq[u] = on ? vb_ldcg4(Vc + (size_t)j * KVD + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    int jb = j0 + warp;
+    fetch(jb);
+    const int d = tid % (kHD / 2);     /* this thread's pair of dimensions */
+    const float ang = (float)pos * (1.0f / powf(theta, (float)(2 * d) / (float)kHD)), cv = cosf(ang), sv = sinf(ang);
+
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");      /* all barriers of the cluster are set up */
     pdl_wait();
     if constexpr (TP) {   /* tensor parallelism: the QKV partials come from every rank */
-        if (threadIdx.x == 0) tp_wait(wait);
+        if (tid == 0) tp_wait(wait);
         __syncthreads();
     }
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int sp = blockIdx.x, g = blockIdx.y, b = blockIdx.z;
-    const int max_s = gridDim.x, G = gridDim.y;
-    /* The split-K partials of q (and, for the first 128 threads, of the new k and v) are requested
-     * before anything else: they depend on nothing this kernel reads, and the utterance's state
-     * below is a second trip to L2 that now overlaps the first. */
-    const float *row = part + (size_t)b * QKV;
-    const bool kv_lane = tid < kHD;
-    float pq[kTcMaxSplits], pk[kTcMaxSplits], pv[kTcMaxSplits];
-#pragma unroll
-    for (int p = 0; p < kTcMaxSplits; p++) {
-        const bool on = p < n_part;
-        pq[p] = on ? __ldcg(row + p * part_stride + (size_t)g * kGroup * kHD + tid) : 0.0f;
-        pk[p] = (on && kv_lane) ? __ldcg(row + p * part_stride + QD + g * kHD + tid) : 0.0f;
-        pv[p] = (on && kv_lane) ? __ldcg(row + p * part_stride + QD + KVD + g * kHD + tid) : 0.0f;
-    }
-    if (dyn[b].done) return;
-    const int pos = dyn[b].pos, kv_max = dyn[b].kv_max;
-    if (pos < 0 || pos >= kv_max) {
+    if (done) return;
+    if (!in_range) {
         if (tid == 0) atomicCAS(status, 0, (int)VB_ERR_POS_RANGE);
         return;
     }
-    const int nk = pos + 1;
-    int S = (nk + 31) / 32;
-    if (S > max_s) S = max_s;
-    if (S < 1) S = 1;
-    if (sp >= S) return;
-    const int j0 = (int)((long long)nk * sp / S), j1 = (int)((long long)nk * (sp + 1) / S);
-    float *Kc = kv_k + (size_t)b * slab + (size_t)layer * kv_max * KVD;
-    float *Vc = kv_v + (size_t)b * slab + (size_t)layer * kv_max * KVD;
-    const bool writer = sp == S - 1;   /* its key range ends with the new token */
-
     {
-        /* split-K sums in split order */
-        const bool kv = writer && kv_lane;
-        /* the rotation table is worked out while those loads are in flight */
-        if (tid < kHD / 2) {
-            const float freq = 1.0f / powf(theta, (float)(2 * tid) / (float)kHD);
-            const float ang = (float)pos * freq;
-            cs[2 * tid] = cosf(ang);
-            cs[2 * tid + 1] = sinf(ang);
-        }
-        float v = 0.0f, kk = 0.0f, vv = 0.0f;
+        /* a thread sums a pair of q's partials in split order and, in the CTA of the new token, one of k's or v's */
+        const float *row = part + (size_t)b * QKV;
+        const int other = tid / (kHD / 2);                 /* 0: k, 1: v */
+        const bool more = writer && other < 2;
+        float2 pq[kTcMaxSplits], po[kTcMaxSplits], q = make_float2(0.f, 0.f), o = q;
 #pragma unroll
-        for (int p = 0; p < kTcMaxSplits; p++) { v += pq[p]; kk += pk[p]; vv += pv[p]; }
-        qraw[tid] = v;
-        if (kv) { kraw[tid] = kk; vraw[tid] = vv; }
-    }
-    __syncthreads();
-    const int half = kHD / 2;
-    if (tid < kGroup * half) {
-        const int hh = tid / half, d = tid % half;
-        const float a = qraw[hh * kHD + 2 * d], bb = qraw[hh * kHD + 2 * d + 1];
-        const float cv = cs[2 * d], sv = cs[2 * d + 1];
-        qs[hh][2 * d] = a * cv - bb * sv;
-        qs[hh][2 * d + 1] = a * sv + bb * cv;
-    } else if (writer && tid < kGroup * half + half) {
-        const int d = tid - kGroup * half;
-        const float a = kraw[2 * d], bb = kraw[2 * d + 1];
-        const float cv = cs[2 * d], sv = cs[2 * d + 1];
-        float *dst = Kc + (size_t)pos * KVD + g * kHD;
-        dst[2 * d] = a * cv - bb * sv;
-        dst[2 * d + 1] = a * sv + bb * cv;
-        __threadfence();
-    } else if (writer && tid >= 384 && tid < 384 + kHD) {
-        const int d = tid - 384;
-        Vc[(size_t)pos * KVD + g * kHD + d] = vraw[d];
-        __threadfence();
+        for (int p = 0; p < kTcMaxSplits; p++) {
+            const float *at = row + p * part_stride;
+            pq[p] = p < n_part ? __ldcg(reinterpret_cast<const float2 *>(at + (size_t)g * kGroup * kHD) + tid) : make_float2(0.f, 0.f);
+            po[p] = p < n_part && more ? __ldcg(reinterpret_cast<const float2 *>(at + QD + other * KVD + g * kHD) + d) : make_float2(0.f, 0.f);
+        }
+#pragma unroll
+        for (int p = 0; p < kTcMaxSplits; p++) { q.x += pq[p].x; q.y += pq[p].y; o.x += po[p].x; o.y += po[p].y; }
+        *reinterpret_cast<float2 *>(&qs[tid / (kHD / 2)][2 * d]) = make_float2(q.x * cv - q.y * sv, q.x * sv + q.y * cv);
+        if (more) {
+            if (other == 0) o = make_float2(o.x * cv - o.y * sv, o.x * sv + o.y * cv);
+            *reinterpret_cast<float2 *>((other ? vs : ks) + 2 * d) = o;
+            *reinterpret_cast<float2 *>((other ? Vc : Kc) + (size_t)pos * KVD + 2 * d) = o;
+        }
     }
     __syncthreads();
 
-    const int hh = warp & 3, ss = warp >> 2;
-    const float4 q4 = *reinterpret_cast<const float4 *>(&qs[hh][4 * lane]);
-    float mx = -1e30f, den = 0.0f;
-    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-    /* KP keys per pass: their 2 KP loads are in flight together, the running-maximum update then
-     * takes them in key order as the reference does. Eight for a single utterance (one pass instead
-     * of two at 256+ cached rows; its 80 CTAs have an SM each anyway), four for several (82
-     * registers would leave one CTA per SM and a second wave of CTAs) */
-    constexpr int kKeysPerPass = KP;
-    for (int jb = j0 + ss; jb < j1; jb += kKeysPerPass * kBtSubsets) {
-        float4 kq[kKeysPerPass], vq[kKeysPerPass];
+    float4 q4[kGroup], o[kGroup];
 #pragma unroll
-        for (int u = 0; u < kKeysPerPass; u++) {
-            const int j = jb + u * kBtSubsets;
-            if (j < j1) {
-                kq[u] = vb_ldcg4(Kc + (size_t)j * KVD + g * kHD + 4 * lane);
-                vq[u] = vb_ldcg4(Vc + (size_t)j * KVD + g * kHD + 4 * lane);
-            } else {
-                kq[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                vq[u] = kq[u];
-            }
-        }
-        float dq[kKeysPerPass];
-#pragma unroll
-        for (int u = 0; u < kKeysPerPass; u++)
-            dq[u] = q4.x * kq[u].x + q4.y * kq[u].y + q4.z * kq[u].z + q4.w * kq[u].w;
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-#pragma unroll
-            for (int u = 0; u < kKeysPerPass; u++) dq[u] += __shfl_xor_sync(0xffffffffu, dq[u], off);
-        }
-#pragma unroll
-        for (int u = 0; u < kKeysPerPass; u++) {
-            if (jb + u * kBtSubsets >= j1) break;
-            const float d = dq[u] * scale;
-            const float4 vv = vq[u];
-            if (d > mx) {
-                const float corr = expf(mx - d);
-                den = den * corr + 1.0f;
-                o.x = o.x * corr + vv.x; o.y = o.y * corr + vv.y;
-                o.z = o.z * corr + vv.z; o.w = o.w * corr + vv.w;
-                mx = d;
-            } else {
-                const float w = expf(d - mx);
-                den += w;
-                o.x += w * vv.x; o.y += w * vv.y; o.z += w * vv.z; o.w += w * vv.w;
-            }
-        }
+    for (int h = 0; h < kGroup; h++) {
+        q4[h] = *reinterpret_cast<const float4 *>(&qs[h][4 * lane]);
+        o[h] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    *reinterpret_cast<float4 *>(&attn_o[ss][hh][4 * lane]) = o;
-    if (lane == 0) { attn_ml[ss][hh][0] = mx; attn_ml[ss][hh][1] = den; }
+    float mx = -1e30f, den = 0.0f;     /* of head lane / 8 */
+    static_assert(kBtKeys * kGroup == 32, "a lane per key and head");
+    while (jb < j1) {
+        float s[32];                   /* [head][key] */
+#pragma unroll
+        for (int u = 0; u < kBtKeys; u++) {
+            if (writer && jb + u * kBtAttnWarps == pos) {
+                kq[u] = *reinterpret_cast<const float4 *>(ks + 4 * lane);
+                vq[u] = *reinterpret_cast<const float4 *>(vs + 4 * lane);
+            }
+#pragma unroll
+            for (int h = 0; h < kGroup; h++)
+                s[h * kBtKeys + u] = q4[h].x * kq[u].x + q4[h].y * kq[u].y + q4[h].z * kq[u].z + q4[h].w * kq[u].w;
+        }
+        /* 32 sums over the lanes by halving: lane i is left with sum i */
+#pragma unroll
+        for (int n = 16; n > 0; n >>= 1) {
+            const bool up = (lane & n) != 0;
+#pragma unroll
+            for (int i = 0; i < n; i++) {
+                const float send = up ? s[i] : s[i + n], keep = up ? s[i + n] : s[i];
+                s[i] = keep + __shfl_xor_sync(0xffffffffu, send, n);
+            }
+        }
+        const bool on = jb + (lane % kBtKeys) * kBtAttnWarps < j1;
+        const float e = on ? s[0] * scale : -1e30f;
+        float top = e;
+#pragma unroll
+        for (int n = kBtKeys / 2; n > 0; n >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, n));
+        const float now = fmaxf(mx, top), c = expf(mx - now), w = on ? expf(e - now) : 0.0f;
+        float sum = w;
+#pragma unroll
+        for (int n = kBtKeys / 2; n > 0; n >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, n);
+        den = den * c + sum;
+        mx = now;
+#pragma unroll
+        for (int h = 0; h < kGroup; h++) {
+            const float ch = __shfl_sync(0xffffffffu, c, h * kBtKeys);
+            o[h].x *= ch; o[h].y *= ch; o[h].z *= ch; o[h].w *= ch;
+#pragma unroll
+            for (int u = 0; u < kBtKeys; u++) {
+                const float wu = __shfl_sync(0xffffffffu, w, h * kBtKeys + u);
+                o[h].x = fmaf(wu, vq[u].x, o[h].x); o[h].y = fmaf(wu, vq[u].y, o[h].y);
+                o[h].z = fmaf(wu, vq[u].z, o[h].z); o[h].w = fmaf(wu, vq[u].w, o[h].w);
+            }
+        }
+        jb += kBtKeys * kBtAttnWarps;
+        if (jb < j1) fetch(jb);
+    }
+#pragma unroll
+    for (int h = 0; h < kGroup; h++) *reinterpret_cast<float4 *>(&warp_o[warp][h][4 * lane]) = o[h];
+    if (lane % kBtKeys == 0) warp_ml[warp][lane / kBtKeys] = make_float2(mx, den);
     __syncthreads();
 
-    /* merge the four key subsets: thread = (head, dim) */
-    const int th = tid / kHD, td = tid % kHD;
-    float M0 = -1e30f;
+    /* the warps' results, to the CTA that merges these columns: thread = (head, pair of dimensions) */
+    const int share = kBtAttnThreads / S;
+    {
+        const int h = tid / (kHD / 2);
+        float M0 = -1e30f, L = 0.0f;
+        float2 O = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int u = 0; u < kBtSubsets; u++) M0 = fmaxf(M0, attn_ml[u][th][0]);
-    float L = 0.0f, O = 0.0f;
+        for (int u = 0; u < kBtAttnWarps; u++) M0 = fmaxf(M0, warp_ml[u][h].x);
 #pragma unroll
-    for (int u = 0; u < kBtSubsets; u++) {
-        const float w = (attn_ml[u][th][1] > 0.0f) ? expf(attn_ml[u][th][0] - M0) : 0.0f;
-        L += attn_ml[u][th][1] * w;
-        O += attn_o[u][th][td] * w;
+        for (int u = 0; u < kBtAttnWarps; u++) {
+            const float2 ml = warp_ml[u][h], v = *reinterpret_cast<const float2 *>(&warp_o[u][h][2 * d]);
+            const float w = ml.y > 0.0f ? expf(ml.x - M0) : 0.0f;
+            L += ml.y * w;
+            O.x += v.x * w;
+            O.y += v.y * w;
+        }
+        uint32_t to, bar;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(vb_smem_u32(&slices[sp * share + tid % share])), "r"(tid / share));
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(vb_smem_u32(&arrived)), "r"(tid / share));
+        asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(to),
+                     "r"(__float_as_uint(O.x)), "r"(__float_as_uint(O.y)), "r"(__float_as_uint(M0)), "r"(__float_as_uint(L)), "r"(bar)
+                     : "memory");
     }
-    float result;
-    if (S == 1) {
-        result = (L > 0.0f) ? O * (1.0f / L) : 0.0f;
-    } else {
-        /* several CTAs share this KV head: publish the slice, the last arrival merges */
-        const int stride = kHD + 2;
-        float *po = scratch + (size_t)(b * G + g) * max_s * kGroup * stride;   /* [max_s][group][kHD + 2] */
-        float *mine = po + ((size_t)sp * kGroup + th) * stride;
-        mine[td] = O;
-        if (td == 0) { mine[kHD] = M0; mine[kHD + 1] = L; }
-        __threadfence();
-        __syncthreads();
-        if (tid == 0) {
-            const unsigned t = atomicAdd(&tickets[b * G + g], 1u);
-            last_flag = (t == (unsigned)(S - 1));
-            if (last_flag) tickets[b * G + g] = 0u;
-        }
-        __syncthreads();
-        if (!last_flag) return;
-        __threadfence();
-        /* merge the S slices in slice order. All loads are issued before anything waits on them:
-         * the (max, sum) pairs go through shared memory, the S output values of this thread's
-         * (head, dim) are fetched in one unrolled batch. */
-        if (tid < S * kGroup) {
-            const float *pu = po + (size_t)tid * stride;           /* (slice, head) = tid / kGroup, tid % kGroup */
-            cmb_m[tid] = __ldcg(pu + kHD);
-            cmb_l[tid] = __ldcg(pu + kHD + 1);
-        }
-        float ov[kBtKeySplits];
-#pragma unroll
-        for (int u = 0; u < kBtKeySplits; u++)
-            ov[u] = u < S ? __ldcg(po + ((size_t)u * kGroup + th) * stride + td) : 0.0f;
-        __syncthreads();
-        float Mg = -1e30f;
-        for (int u = 0; u < S; u++) Mg = fmaxf(Mg, cmb_m[u * kGroup + th]);
-        float Lg = 0.0f, Og = 0.0f;
-#pragma unroll
-        for (int u = 0; u < kBtKeySplits; u++) {
-            if (u < S) {
-                const float lu = cmb_l[u * kGroup + th];
-                const float w = (lu > 0.0f) ? expf(cmb_m[u * kGroup + th] - Mg) : 0.0f;
-                Lg += lu * w;
-                Og += ov[u] * w;
-            }
-        }
-        result = (Lg > 0.0f) ? Og * (1.0f / Lg) : 0.0f;
+    /* a CTA ends only when it has received everything: nothing is sent to shared memory that is gone */
+    if (!vb_mbar_wait(&arrived, 0u, &gave_up)) {
+        atomicCAS(status, 0, 16);
+        gave_up = 1;
+        return;
     }
-    uint16_t t0, t1, t2;
-    vb_split3(result, t0, t1, t2);
-    const size_t off = (size_t)b * QD + (size_t)(g * kGroup + th) * kHD + td, term = (size_t)rows_pad * QD;
-    terms[off] = t0;
-    terms[term + off] = t1;
-    terms[2 * term + off] = t2;
+    if (tid < share) {
+        const int i = sp * share + tid, h = i / (kHD / 2), c = 2 * (i % (kHD / 2));
+        float2 O = make_float2(0.f, 0.f);
+        float M0 = -1e30f, L = 0.0f;
+        for (int u = 0; u < S; u++) M0 = fmaxf(M0, slices[u * share + tid].z);
+        for (int u = 0; u < S; u++) {
+            const float4 e = slices[u * share + tid];
+            const float w = e.w > 0.0f ? expf(e.z - M0) : 0.0f;
+            L += e.w * w;
+            O.x += e.x * w;
+            O.y += e.y * w;
+        }
+        const float r = L > 0.0f ? 1.0f / L : 0.0f;
+        uint16_t t[3][2];
+        vb_split3(O.x * r, t[0][0], t[1][0], t[2][0]);
+        vb_split3(O.y * r, t[0][1], t[1][1], t[2][1]);
+        const size_t off = (size_t)b * QD + (size_t)(g * kGroup + h) * kHD + c;
+#pragma unroll
+        for (int k = 0; k < 3; k++) *reinterpret_cast<uint32_t *>(terms + k * (size_t)rows_pad * QD + off) = t[k][0] | ((uint32_t)t[k][1] << 16);
+    }
 }
 
 /* End of the decoder step: last residual add (split-K partials of the last down projection),
@@ -967,9 +951,6 @@ static int ctx_open(Batch &t, bool single, int n_utt, int kv_max, int max_frames
     }
     rc |= bt_alloc((void **)&t.ssq, sizeof(float) * 16 * (D / kTcTileN), &t.allocs);
     rc |= bt_alloc((void **)&t.logit_part, sizeof(float) * kTcMaxSplits * B * NSEM, &t.allocs);
-    rc |= bt_alloc((void **)&t.attn_scratch,
-                   sizeof(float) * (size_t)B * VB200_KV_HEADS * kBtKeySplits * kGroup * (kHD + 2), &t.allocs);
-    rc |= bt_alloc((void **)&t.tickets, sizeof(unsigned) * B * VB200_KV_HEADS, &t.allocs);
     if (stream) {
         rc |= bt_alloc((void **)&t.s_qkv, sizeof(stag_t) * QKV, &t.allocs);
         rc |= bt_alloc((void **)&t.s_attn, sizeof(stag_t) * QD, &t.allocs);
@@ -1023,19 +1004,18 @@ static int enqueue_decoder(Batch &t) {
         s_w2 = tc_pick_splits(on * kTcTileN, HID, m.sm_count);
         tp_epoch_kernel<<<1, 1, 0, st>>>(g_tp.epoch);
     }
-    /* Key splits of the decode attention: as many as fit the GPU in one wave. A CTA of this kernel
-     * takes 28 K registers, two fit an SM; beyond that the extra CTAs queue up behind the first
-     * wave (8 utterances x 8 KV heads x 9 splits ran as two waves: 22 us instead of 12 per layer). */
-    int attn_splits = (2 * m.sm_count) / (VB200_KV_HEADS * B);
-    if (attn_splits > kBtKeySplits) attn_splits = kBtKeySplits;
-    if (attn_splits < 1) attn_splits = 1;
+    /* Key splits of the decode attention: clusters of eight while all CTAs fit the GPU in one wave (two an SM: 128
+     * registers a thread), of four for more utterances. */
+    int attn_splits = kBtMaxSplits;
+    while (attn_splits > 1 && attn_splits * VB200_KV_HEADS * B > 2 * m.sm_count) attn_splits /= 2;
     for (int l = 0; l < VB200_DEC_LAYERS; l++) {
         const LayerDev &L = m.dec[l];
         const int NL = VB200_DEC_LAYERS;      /* every exchanged buffer is filled once per layer */
         /* residual-stream taps (single utterance only): after the attention half and after the
          * FFN half of every layer, as the parity tests read them (voxtral_tts_llm.c:245,263) */
         float *const tap_base = (t.single && m.tap_on) ? m.tap : nullptr;
-        if (l == 0) tc_prepare(t.aD, t.X, D, B, nullptr, 0, 0, nullptr, nullptr, L.attn_norm, t.ssq, st);
+        /* a plain launch: what follows it may read what earlier frames left without waiting for its own predecessor */
+        if (l == 0) tc_prepare(t.aD, t.X, D, B, nullptr, 0, 0, nullptr, nullptr, L.attn_norm, t.ssq, st, TcWait(), nullptr, true);
         else if (tp) tc_prepare(t.aD, nullptr, D, B, t.part_w2, s_w2, psD, t.X, t.X, L.attn_norm, t.ssq, st,
                         tp_wait_for(0, TP_W2, NL, l, t.status), tap_base ? tap_base + (size_t)(2 * l - 1) * D : nullptr);
         TcGemm g;
@@ -1044,19 +1024,14 @@ static int enqueue_decoder(Batch &t) {
         g.ssq = t.ssq; g.ssq_chunks = l == 0 ? tc_prepare_chunks(D) : chunksD;
         if (tp) { g.tile0 = q0; g.n_tiles = qn; g.push = tp_push(0, TP_QKV, NL, l + 1); }
         if (tc_gemm(w.wqkv[l], t.aD, g, st)) return -1;
+        const dim3 grid(attn_splits, VB200_KV_HEADS, B);
         if (tp)
-            launch_pdl(bt_attn_kernel<true, 4>, dim3(kBtKeySplits, VB200_KV_HEADS, B), dim3(kBtAttnThreads), 0, st, t.bQ,
-                       16, (const float *)t.part_qkv, s_qkv, psQ, t.kv_k, t.kv_v, t.slab, l, (const VbDyn *)t.dyn,
-                       scale, VB200_ROPE_THETA, t.attn_scratch, t.tickets, t.status,
-                       tp_wait_for(0, TP_QKV, NL, l + 1, t.status));
-        else if (B == 1)   /* one utterance: one CTA per SM at most, so eight keys per pass cost no occupancy */
-            launch_pdl(bt_attn_kernel<false, 8>, dim3(attn_splits, VB200_KV_HEADS, B), dim3(kBtAttnThreads), 0, st, t.bQ,
-                       16, (const float *)t.part_qkv, s_qkv, psQ, t.kv_k, t.kv_v, t.slab, l, (const VbDyn *)t.dyn,
-                       scale, VB200_ROPE_THETA, t.attn_scratch, t.tickets, t.status, TcNoWait());
+            launch_pdl_cluster(bt_attn_kernel<true>, attn_splits, grid, dim3(kBtAttnThreads), 0, st, t.bQ, 16, (const float *)t.part_qkv, s_qkv,
+                               psQ, t.kv_k, t.kv_v, t.slab, l, (const VbDyn *)t.dyn, scale, VB200_ROPE_THETA, t.status,
+                               tp_wait_for(0, TP_QKV, NL, l + 1, t.status));
         else
-            launch_pdl(bt_attn_kernel<false, 4>, dim3(attn_splits, VB200_KV_HEADS, B), dim3(kBtAttnThreads), 0, st, t.bQ,
-                       16, (const float *)t.part_qkv, s_qkv, psQ, t.kv_k, t.kv_v, t.slab, l, (const VbDyn *)t.dyn,
-                       scale, VB200_ROPE_THETA, t.attn_scratch, t.tickets, t.status, TcNoWait());
+            launch_pdl_cluster(bt_attn_kernel<false>, attn_splits, grid, dim3(kBtAttnThreads), 0, st, t.bQ, 16, (const float *)t.part_qkv, s_qkv,
+                               psQ, t.kv_k, t.kv_v, t.slab, l, (const VbDyn *)t.dyn, scale, VB200_ROPE_THETA, t.status, TcNoWait());
         g = TcGemm();
         g.M = B; g.status = t.status; g.eps = VB200_NORM_EPS;
         g.epi = TC_EPI_PARTIAL; g.out = t.part_wo; g.splits = s_wo; g.ld_out = D;
@@ -1214,8 +1189,7 @@ int batch_begin(const float *first_embeds, const int *start_pos, const float *no
         cudaMemcpy(t.X, first_embeds, sizeof(float) * t.B * D, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(t.noise_all, noise, sizeof(float) * (size_t)t.B * t.cap * A, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemset(t.codes_all, 0, sizeof(int) * (size_t)t.B * t.cap * VB200_CODES) != cudaSuccess ||
-        cudaMemset(t.status, 0, sizeof(int) * 4) != cudaSuccess ||
-        cudaMemset(t.tickets, 0, sizeof(unsigned) * t.B * VB200_KV_HEADS) != cudaSuccess)
+        cudaMemset(t.status, 0, sizeof(int) * 4) != cudaSuccess)
         return -1;
     t.launched = 0;
     t.begun = true;
@@ -1438,7 +1412,6 @@ static int one_status(Batch &t) {
     m.last_status = t.h_out->status[0];
     if (m.last_status == 0) return 0;
     fprintf(stderr, "voxtral_b200: a frame kernel gave up with status %d\n", m.last_status);
-    cudaMemsetAsync(t.tickets, 0, sizeof(unsigned) * VB200_KV_HEADS, m.st);
     if (t.s_counters) cudaMemsetAsync(t.s_counters, 0, sizeof(unsigned) * 64, m.st);
     cudaMemsetAsync(t.status, 0, sizeof(int) * 4, m.st);
     cudaStreamSynchronize(m.st);

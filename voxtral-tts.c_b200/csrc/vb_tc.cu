@@ -585,24 +585,6 @@ vb_tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
     }
 }
 
-/* launch_pdl with clusters of so many CTAs (0: none). */
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl_cluster(void (*kernel)(KArgs...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
-    if (cluster == 0) return launch_pdl(kernel, grid, block, smem, st, args...);
-    static const bool no_pdl = getenv("VB200_NO_PDL") != nullptr;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)cluster;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = no_pdl ? 1 : 2;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 template <int NB, int ST, int MODE, int ACCS>
 static int launch_tc_tp(const TcWeight &w, const TcActs &a, const TcKernelArgs &ka, const typename TcTpSel<MODE>::type &arg,
                         cudaStream_t st) {
@@ -755,9 +737,12 @@ int tc_prepare_chunks(int K) { return (K + 1023) / 1024; }
 
 void tc_prepare(const TcActs &acts, const float *x, int ldx, int M, const float *partials, int n_part,
                 size_t part_stride, const float *residual, float *x_out, const float *gain, float *ssq,
-                cudaStream_t st, const TcWait &wait, float *tap) {
+                cudaStream_t st, const TcWait &wait, float *tap, bool plain) {
     if (M <= 0) return;
-    if (wait.n > 0)
+    if (plain)
+        vb_tc_prepare_kernel<false><<<dim3(tc_prepare_chunks(acts.K), M), 256, 0, st>>>(acts.buf, acts.rows_pad, acts.K, x, ldx, partials, n_part,
+                                                                                         part_stride, residual, x_out, gain, ssq, tap, TcNoWait());
+    else if (wait.n > 0)
         launch_pdl(vb_tc_prepare_kernel<true>, dim3(tc_prepare_chunks(acts.K), M), dim3(256), 0, st, acts.buf,
                    acts.rows_pad, acts.K, x, ldx, partials, n_part, part_stride, residual, x_out, gain, ssq, tap, wait);
     else

@@ -145,10 +145,11 @@ int tc_prepare_chunks(int K);                      /* column chunks (and ssq ent
 /* Rows -> BF16 terms in `acts`. Source: x[M, ldx], or residual[M, ldx] + the sum of n_part
  * split-K partial buffers ([M, K] each, part_stride floats apart). x_out (optional) receives the
  * fp32 rows. With `gain` the terms hold row*gain and ssq[m][chunk] the chunk's sum of squares
- * (RMSNorm's scalar is applied by the consuming GEMM). */
+ * (RMSNorm's scalar is applied by the consuming GEMM). plain: without the programmatic launch, so that everything
+ * before this launch is complete once it runs. */
 void tc_prepare(const TcActs &acts, const float *x, int ldx, int M, const float *partials, int n_part,
                 size_t part_stride, const float *residual, float *x_out, const float *gain, float *ssq,
-                cudaStream_t st, const TcWait &wait = TcWait(), float *tap = nullptr);
+                cudaStream_t st, const TcWait &wait = TcWait(), float *tap = nullptr, bool plain = false);
 
 int tc_gemm(const TcWeight &w, const TcActs &acts, const TcGemm &g, cudaStream_t st);
 /* Many rows (vb_tc_rows.cu; two or three terms of the activations are read): what tc_gemm calls from rows_pad = 256 on, and
@@ -187,6 +188,24 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = no_pdl ? 0 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+/* launch_pdl with clusters of so many CTAs (0: none). */
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl_cluster(void (*kernel)(KArgs...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+    if (cluster == 0) return launch_pdl(kernel, grid, block, smem, st, args...);
+    static const bool no_pdl = getenv("VB200_NO_PDL") != nullptr;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = no_pdl ? 1 : 2;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
