@@ -850,7 +850,7 @@ def main():
              "achieved": mean_frame_bytes / (frame_ms / 1000.0) / 1e9,
              "frac": mean_frame_bytes / (frame_ms / 1000.0) / 1e9 / peak}
     if on_tc:
-        # A frame is one CUDA graph of 264 launches; 190 of them are vb_tc_gemm_kernel<16> and
+        # A frame is one CUDA graph of 257 launches; 190 of them are vb_tc_gemm_kernel<16> and
         # carry every weight byte (104 decoder-layer GEMMs, 2 head GEMMs, 84 acoustic-layer
         # GEMMs). Launches inside a graph cannot be bracketed one by one, so the kernel's own
         # launch time is measured live on the decoder's 104 GEMMs launched back to back (every
@@ -874,7 +874,7 @@ def main():
             pass
         roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                     "traffic": traffic,
-                    "kernel": "vb_tc_gemm_kernel<16> (tcgen05 skinny GEMM; 190 of a frame's 264 launches, all weight bytes)",
+                    "kernel": "vb_tc_gemm_kernel<16> (tcgen05 skinny GEMM; 190 of a frame's 257 launches, all weight bytes)",
                     "algorithmic_bytes_per_launch": bytes_per_launch, "launch_ms": launch_ms,
                     "measured_on": f"{sweeps} sweeps of the decoder's {sn.value} layer GEMMs, back to back, CUDA events",
                     "share_of_frame_time": (gemm_bytes_frame / 1e9 / achieved * 1000.0) / frame_ms,

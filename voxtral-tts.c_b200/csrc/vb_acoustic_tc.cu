@@ -42,24 +42,83 @@ __device__ __forceinline__ float euler_step(float x, float vc, float vu, float a
     return __fadd_rn(x, __fmul_rn(v, dt));
 }
 
+/* Weight row of input_proj for column n: static data, fetched before the wait for the previous kernel (6.2 us for a velocity
+ * call's rows with it behind the wait, element by element). */
+struct AcInWeights {
+    uint2 w[A / 4];
+    VB_DEVINL void fetch(const uint16_t *Wip, int n) {
+        static_assert(A % 4 == 0, "rows in pieces of 8 bytes");
+#pragma unroll
+        for (int k = 0; k < A / 4; k++) w[k] = __ldg(reinterpret_cast<const uint2 *>(Wip + (size_t)n * A) + k);
+    }
+    VB_DEVINL float dot(const float *x) const {
+        float acc = 0.0f;
+#pragma unroll
+        for (int k = 0; k < A / 4; k++) {
+            const float e[4] = {vb_bf16_lo(w[k].x), vb_bf16_hi(w[k].x), vb_bf16_lo(w[k].y), vb_bf16_hi(w[k].y)};
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc = __fadd_rn(acc, __fmul_rn(e[j], x[4 * k + j]));
+        }
+        return acc;
+    }
+};
+
+/* Column n of the three tokens of a pass, for rows m0 .. m0 + 2 and, of the unguided branch, m0 + 3 .. m0 + 5, whose third is
+ * zero: residual rows, the first layer's operand (terms of row * gain) and the sums of squares of this CTA's 128 columns.
+ * (The operand was a launch of its own, 7 of a frame's 264: 257 now.) */
+struct AcRowsOut {
+    float *X;
+    uint16_t *terms;
+    int rows_pad;
+    const float *gain;
+    float *ssq;
+};
+VB_DEVINL void ac_rows_out(const AcRowsOut &o, int m0, bool both, int n, const float (&v)[3], float gain, float (&red)[4][3]) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+        uint16_t t[3];
+        vb_split3(v[r] * gain, t[0], t[1], t[2]);
+        for (int c = 0; c < (both ? 2 : 1); c++) {
+            const bool zero = c == 1 && r == 2;
+            const int m = m0 + 3 * c + r;
+            o.X[(size_t)m * D + n] = zero ? 0.0f : v[r];
+#pragma unroll
+            for (int k = 0; k < 3; k++) o.terms[((size_t)k * o.rows_pad + m) * D + n] = zero ? (uint16_t)0 : t[k];
+        }
+        const float ss = vb_warp_sum(v[r] * v[r]);
+        if (lane == 0) red[warp][r] = ss;
+    }
+    __syncthreads();
+    if (threadIdx.x < (both ? 6 : 3)) {
+        const int r = threadIdx.x % 3;
+        o.ssq[(size_t)(m0 + threadIdx.x) * (D / kTcTileN) + blockIdx.x] =
+            threadIdx.x == 5 ? 0.0f : (red[0][r] + red[1][r]) + (red[2][r] + red[3][r]);
+    }
+}
+
 /* Euler update of the latent (step > 0) and the six input rows of a pass
  * (voxtral_tts_acoustic.c:198-212): rows 0,3 input_proj(x_t); 1,4 the precomputed time token;
- * 2 llm_proj(h); 5 zero. */
-__global__ void ac_tokens_kernel(float *X6, float *lat, const float *vel, const uint16_t *Wip, const float *ttok,
-                                 const float *ltok, int step, float alpha, float dt_prev, const float *noise_all,
-                                 const VbDyn *dyn, AcStrides sd) {
-    __shared__ float xs[64];
+ * 2 llm_proj(h); 5 zero. grid = (D / 128, utterances), 128 threads. */
+__global__ void __launch_bounds__(128)
+ac_tokens_kernel(const AcRowsOut out, float *lat, const float *vel, const uint16_t *Wip, const float *ttok, const float *ltok, int step,
+                 float alpha, float dt_prev, const float *noise_all, const VbDyn *dyn, AcStrides sd) {
+    __shared__ __align__(16) float xs[A];
+    __shared__ float red[4][3];
     pdl_launch_dependents();
+    const int n = blockIdx.x * 128 + threadIdx.x;
+    AcInWeights w;
+    w.fetch(Wip, n);
+    const float gain = __ldg(out.gain + n), tt = __ldg(ttok + (size_t)step * D + n);
     pdl_wait();
     /* utterance blockIdx.y of the batch */
     const int b = blockIdx.y;
-    X6 += (size_t)b * ROWS1 * D;
     lat += (size_t)b * sd.lat;
     vel += (size_t)b * sd.vel;
-    ltok += (size_t)b * D;
     dyn += b;
     if (noise_all) noise_all += (size_t)b * sd.noise;
     if (noise_all && dyn->done) return;   /* device-resident run already ended */
+    const float lt = __ldcg(ltok + (size_t)b * D + n);
     if (threadIdx.x < A) {
         float xv;
         if (step == 0) {
@@ -76,41 +135,34 @@ __global__ void ac_tokens_kernel(float *X6, float *lat, const float *vel, const 
         xs[threadIdx.x] = xv;
     }
     __syncthreads();
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= D) return;
-    const uint16_t *wr = Wip + (size_t)n * A;
-    float acc = 0.0f;
-    for (int k = 0; k < A; k++) acc = __fadd_rn(acc, __fmul_rn(__uint_as_float((uint32_t)wr[k] << 16), xs[k]));
-    const float tt = ttok[(size_t)step * D + n];
-    X6[n] = acc;
-    X6[3 * D + n] = acc;
-    X6[1 * D + n] = tt;
-    X6[4 * D + n] = tt;
-    X6[2 * D + n] = ltok[n];
-    X6[5 * D + n] = 0.0f;
+    const float v[3] = {w.dot(xs), tt, lt};
+    ac_rows_out(out, b * ROWS1, true, n, v, gain, red);
 }
 
 /* The three input rows of a single velocity call (voxtral_tts_acoustic.c:198-212): input_proj(x), and the split-K partials
  * [n_part][2][3072] of time_proj on row 1 and of llm_proj on row 0 of (hidden, time embedding). */
-__global__ void ac_rows_kernel(float *X, const float *x, const uint16_t *Wip, const float *time_part, const float *llm_part, int n_part) {
+__global__ void __launch_bounds__(128)
+ac_rows_kernel(const AcRowsOut out, const float *x, const uint16_t *Wip, const float *time_part, const float *llm_part, int n_part) {
+    __shared__ __align__(16) float xs[A];
+    __shared__ float red[4][3];
     pdl_launch_dependents();
+    const int n = blockIdx.x * 128 + threadIdx.x;
+    AcInWeights w;
+    w.fetch(Wip, n);
+    const float gain = __ldg(out.gain + n);
     pdl_wait();
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= D) return;
-    const uint16_t *wr = Wip + (size_t)n * A;
-    float acc = 0.0f;
-    for (int k = 0; k < A; k++) acc = __fadd_rn(acc, __fmul_rn(__uint_as_float((uint32_t)wr[k] << 16), __ldcg(x + k)));
     float a[kTcMaxSplits], b[kTcMaxSplits], ta = 0.0f, tb = 0.0f;
 #pragma unroll
     for (int p = 0; p < kTcMaxSplits; p++) {
         a[p] = p < n_part ? __ldcg(time_part + ((size_t)p * 2 + 1) * D + n) : 0.0f;
         b[p] = p < n_part ? __ldcg(llm_part + (size_t)p * 2 * D + n) : 0.0f;
     }
+    if (threadIdx.x < A) xs[threadIdx.x] = __ldcg(x + threadIdx.x);
+    __syncthreads();
 #pragma unroll
     for (int p = 0; p < kTcMaxSplits; p++) { ta += a[p]; tb += b[p]; }
-    X[n] = acc;
-    X[D + n] = ta;
-    X[2 * D + n] = tb;
+    const float v[3] = {w.dot(xs), ta, tb};
+    ac_rows_out(out, 0, false, n, v, gain, red);
 }
 
 /* Unmasked attention inside each 3-token sequence (tts_bidirectional_attention,
@@ -368,7 +420,7 @@ bool acoustic_tc_ready() { return g_ac.ready; }
  * the launch (eight utterances, 24 frames: 118.4 ms joined, 113.8 ms so). */
 static bool joined(int rows) { return rows <= 16; }
 
-/* The layers on the rows in X6, whose terms are not made yet; `sums` as in TcGemm. */
+/* The layers on the rows in X6, whose terms the kernel that made them left; `sums` as in TcGemm. */
 static int enqueue_layers(const AcBuffers &b, int ROWS, int sums) {
     const bool join = joined(ROWS);
     const int chunks = join ? D / kTcTileN : tc_prepare_chunks(D);
@@ -380,12 +432,11 @@ static int enqueue_layers(const AcBuffers &b, int ROWS, int sums) {
     for (int l = 0; l < VB200_AC_LAYERS; l++) {
         const LayerDev &L = m.ac[l];
         /* attention half: QKV -> attention -> O */
-        if (l == 0) tc_prepare(b.aD, b.X6, D, ROWS, nullptr, 0, 0, nullptr, nullptr, L.attn_norm, b.ssq, st);
-        else if (!join) tc_prepare(b.aD, nullptr, D, ROWS, b.part, t.s_w2, psD, b.X6, b.X6, L.attn_norm, b.ssq, st);
+        if (l > 0 && !join) tc_prepare(b.aD, nullptr, D, ROWS, b.part, t.s_w2, psD, b.X6, b.X6, L.attn_norm, b.ssq, st);
         TcGemm g;
         g.M = ROWS; g.sums = sums; g.status = b.status;
         g.epi = TC_EPI_PARTIAL; g.out = b.part;
-        g.splits = t.s_qkv; g.ld_out = QKV; g.ssq = b.ssq; g.ssq_chunks = l == 0 ? tc_prepare_chunks(D) : chunks;
+        g.splits = t.s_qkv; g.ld_out = QKV; g.ssq = b.ssq; g.ssq_chunks = l == 0 ? D / kTcTileN : chunks;
         g.eps = VB200_NORM_EPS;
         if (tc_gemm(t.wqkv[l], b.aD, g, st)) return -1;
         launch_pdl(ac_attention_kernel, dim3((ROWS * VB200_HEADS * 32 + 255) / 256), dim3(256), 0, st, b.bQ,
@@ -411,6 +462,8 @@ static int enqueue_layers(const AcBuffers &b, int ROWS, int sums) {
     return 0;
 }
 
+static AcRowsOut rows_out(const AcBuffers &b) { return {b.X6, b.bD, b.rows_pad, model().ac[0].attn_norm, b.ssq}; }
+
 /* Enqueues the 7 Euler steps + FSQ on the library's stream. The semantic head, llm token
  * and argmax have already run; the llm token rows are in b.ltok. */
 int acoustic_tc_enqueue_on(const AcBuffers &b, const float *noise_all, int *codes_all, int frame_cap, bool advance,
@@ -422,7 +475,7 @@ int acoustic_tc_enqueue_on(const AcBuffers &b, const float *noise_all, int *code
     const int steps = VB200_FLOW_STEPS - 1;
     const int ROWS = b.rows;
     for (int s = 0; s < steps; s++) {
-        launch_pdl(ac_tokens_kernel, dim3((D + 127) / 128, b.B), dim3(128), 0, st, b.X6, b.lat, (const float *)b.vel,
+        launch_pdl(ac_tokens_kernel, dim3(D / 128, b.B), dim3(128), 0, st, rows_out(b), b.lat, (const float *)b.vel,
                    (const uint16_t *)m.ac_input_proj, (const float *)m.ttok, (const float *)b.ltok, s,
                    VB200_CFG_ALPHA, s > 0 ? m.dt[s - 1] : 0.0f, noise_all, (const VbDyn *)b.dyn, b.sd);
         if (enqueue_layers(b, ROWS, 2)) return -1;
@@ -439,7 +492,7 @@ static int enqueue_direct(const float *noise_all, int *codes_all, int frame_cap,
     return acoustic_tc_enqueue_on(g_ac.one, noise_all, codes_all, frame_cap, advance, ignore_end);
 }
 
-/* The 127 launches of a frame are captured once per argument set as a CUDA graph and
+/* The 120 launches of a frame are captured once per argument set as a CUDA graph and
  * replayed; the first call with a new argument set runs directly (it also sets the
  * kernels' shared-memory attributes, which must not happen inside a capture). */
 struct GraphSlot {
@@ -495,7 +548,7 @@ static int run_slot(GraphSlot &s, const F &enqueue) {
     return cudaGraphLaunch(s.exec, m.st) == cudaSuccess ? 0 : -1;
 }
 
-/* One velocity call on what lies in d_in (latent 0, hidden state, time embedding): 21 launches, against the streaming
+/* One velocity call on what lies in d_in (latent 0, hidden state, time embedding): 20 launches, against the streaming
  * GEMV kernel's one of 0.25 ms; 0.17 ms. */
 static int enqueue_velocity() {
     Model &m = model();
@@ -512,7 +565,7 @@ static int enqueue_velocity() {
     if (tc_gemm(t.wtime, b.aD, g, st)) return -1;
     g.out = llm_part;
     if (tc_gemm(t.wllm, b.aD, g, st)) return -1;
-    launch_pdl(ac_rows_kernel, dim3((D + 127) / 128), dim3(128), 0, st, b.X6, (const float *)m.d_in->lat[0], (const uint16_t *)m.ac_input_proj,
+    launch_pdl(ac_rows_kernel, dim3(D / 128), dim3(128), 0, st, rows_out(b), (const float *)m.d_in->lat[0], (const uint16_t *)m.ac_input_proj,
                (const float *)time_part, (const float *)llm_part, s);
     if (enqueue_layers(b, 3, 4)) return -1;
     launch_pdl(ac_velocity_kernel, dim3(9, 1), dim3(512), 0, st, b.vel, (const float *)b.X6, (const float *)nullptr, 0, (const float *)m.ac_norm,

@@ -516,19 +516,31 @@ bt_argmax_kernel(int *codes, const float *part, int n_part, size_t part_stride, 
                  int valid_end) {
     __shared__ float rv[32];
     __shared__ int ri[32];
+    /* a thread's logits are requested together, the bias before the wait (11 us with one at a time) */
+    constexpr int kPer = (NSEM + 1023) / 1024;
     pdl_launch_dependents();
-    pdl_wait();
     const int b = blockIdx.x, tid = threadIdx.x;
+    float bv[kPer], v[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; u++) bv[u] = bias && tid + u * 1024 < N ? __ldg(bias + tid + u * 1024) : 0.0f;
+    pdl_wait();
     float best = -1e30f;
     int bi = 0;
-    for (int i = tid; i < N; i += 1024) {
-        float v = -1e30f;
-        if (i != 0 && i < valid_end) {
-            v = 0.0f;
-            for (int p = 0; p < n_part; p++) v += __ldcg(part + p * part_stride + (size_t)b * N + i);
-            if (bias) v += __ldg(bias + i);
-        }
-        if (v > best || (v == best && i < bi)) { best = v; bi = i; }
+#pragma unroll
+    for (int u = 0; u < kPer; u++) v[u] = 0.0f;
+    for (int p = 0; p < n_part; p++) {
+        float t[kPer];
+#pragma unroll
+        for (int u = 0; u < kPer; u++) t[u] = tid + u * 1024 < N ? __ldcg(part + p * part_stride + (size_t)b * N + tid + u * 1024) : 0.0f;
+#pragma unroll
+        for (int u = 0; u < kPer; u++) v[u] += t[u];
+    }
+#pragma unroll
+    for (int u = 0; u < kPer; u++) {
+        const int i = tid + u * 1024;
+        if (i == 0 || i >= valid_end) continue;
+        const float e = bias ? v[u] + bv[u] : v[u];
+        if (e > best || (e == best && i < bi)) { best = e; bi = i; }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
