@@ -905,7 +905,7 @@ def main():
                     "traffic": traffic, "kernel": kernel_desc, "algorithmic_bytes_per_launch": eng_bytes,
                     "launch_ms": launch_ms, "share_of_frame_time": launch_ms / frame_ms, "peak_source": peak_src,
                     "whole_frame": whole}
-        launches_per_frame = 1 + (84 + 7 + 21 + 14 + 1 if tc_ac else 0)
+        launches_per_frame = 1 + (84 + 21 + 14 + 1 if tc_ac else 0)
 
     # ---- several utterances per GPU in lock step (weights read once per frame for all) -----------
     batched = None
@@ -960,7 +960,7 @@ def main():
             step_ms = stms.value / 10
             streaming = {"decoder_kernel": "vb_stream_kernel (26 layers + semantic head + llm token + argmax: one launch)",
                          "value": sval, "unit": "frames/s", "steps": Ks, "ms_per_step": smax / Ks,
-                         "launches_per_frame": 1 + (pkg.FLOW_STEPS - 1) * (3 + pkg.AC_LAYERS * 5) + 1,
+                         "launches_per_frame": 1 + (pkg.FLOW_STEPS - 1) * (2 + pkg.AC_LAYERS * 5) + 1,
                          "step_launch_ms": step_ms, "step_cache_row": mid, "step_algorithmic_bytes": stb.value,
                          "step_achieved_gbs": stb.value / (step_ms / 1000.0) / 1e9,
                          "step_frac": stb.value / (step_ms / 1000.0) / 1e9 / peak}

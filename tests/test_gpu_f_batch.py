@@ -59,6 +59,25 @@ def test_batch_equals_single_utterances(pkg, engine, oracle, synth_model, n_utt)
     assert same == n_utt
 
 
+@pytest.mark.parametrize("rows", [[65, 128], [100, 64, 187, 65, 33, 129, 190, 256], [500, 330, 70, 480, 490, 470], [300, 66, 127]])
+def test_prompts_side_by_side(pkg, engine, oracle, synth_model, rows):
+    """Prompts that go through the layers together, in one block or more, beside ones that go alone (up to 64 rows, or up to 64
+    behind a multiple of 256), against each prompt's own prefill. Two-term products whose sums end in other orders: each is
+    up to 5e-5 off."""
+    n = len(rows)
+    x = pkg.synth_f32((sum(rows), 3072), 57, "side.rows", 0.0, 0.5)
+    prompts = [x[sum(rows[:u]):sum(rows[:u + 1])] for u in range(n)]
+    first = synth_model.token_rows([24])[0]
+    noise = np.stack([_noise(oracle, 800 + u, 1) for u in range(n)])
+    want = []
+    for u in range(n):
+        engine.prefill(prompts[u])
+        want.append(engine.frame(first, noise[u, 0], rows[u])[1])
+    _, _, hidden, _ = engine.batch(prompts, np.stack([first] * n), noise)
+    for u in range(n):
+        assert rel_l2(hidden[u], want[u]) < 1e-4, (u, rows[u])
+
+
 def test_full_cache_stops_one_utterance_only(pkg, engine, oracle, synth_model):
     """An utterance whose cache slab fills up stops; the others carry on undisturbed."""
     frames = 6

@@ -99,6 +99,7 @@ def lib():
         "vb200_utterance_run": (C.c_int, [C.c_int]),
         "vb200_batch_open": (C.c_int, [C.c_int, C.c_int, C.c_int]),
         "vb200_batch_prefill": (C.c_int, [C.c_int, C.c_void_p, C.c_int]),
+        "vb200_batch_prefill_all": (C.c_int, [C.c_void_p, C.c_void_p]),
         "vb200_batch_begin": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p]),
         "vb200_batch_run": (C.c_int, [C.c_int]),
         "vb200_batch_end": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, f32p]),
@@ -640,11 +641,10 @@ class Engine:
             kv_max = max(p.shape[0] for p in prompts) + frames + 1
         self._ok("vb200_batch_open", self.L.vb200_batch_open(n, int(kv_max), frames))
         try:
-            start = np.zeros(n, dtype=np.int32)
-            for u, p in enumerate(prompts):
-                p = np.ascontiguousarray(p, dtype=np.float32).reshape(-1, DIM)
-                self._ok("vb200_batch_prefill", self.L.vb200_batch_prefill(u, _ptr(p), p.shape[0]))
-                start[u] = p.shape[0]
+            rows = [np.ascontiguousarray(p, dtype=np.float32).reshape(-1, DIM) for p in prompts]
+            start = np.array([p.shape[0] for p in rows], dtype=np.int32)
+            at = (C.c_void_p * n)(*[p.ctypes.data for p in rows])
+            self._ok("vb200_batch_prefill_all", self.L.vb200_batch_prefill_all(at, _ptr(start)))
             self._ok("vb200_batch_begin", self.L.vb200_batch_begin(_ptr(first_embeds), _ptr(start), _ptr(noise)))
             self._ok("vb200_batch_run", self.L.vb200_batch_run(frames))
             codes = np.zeros((n, frames, CODES), dtype=np.int32)

@@ -164,6 +164,7 @@ int vb200_utterance_run(int n_frames) { return utterance_run(n_frames); }
 
 int vb200_batch_open(int n_utterances, int kv_max, int max_frames) { return batch_open(n_utterances, kv_max, max_frames); }
 int vb200_batch_prefill(int utterance, const float *embeds, int n_rows) { return batch_prefill(utterance, embeds, n_rows); }
+int vb200_batch_prefill_all(const float *const *embeds, const int *n_rows) { return batch_prefill_all(embeds, n_rows); }
 int vb200_batch_begin(const float *first_embeds, const int *start_pos, const float *noise) {
     return batch_begin(first_embeds, start_pos, noise);
 }

@@ -178,6 +178,7 @@ VB_DEVINL uint32_t at_off(int row, int chunk) { return (uint32_t)(row * 128 + ((
  *   tma_keys(...) / tma_values(...)   request a tile by TMA: where AtArgs says so and boxes(j0, n) does, or always (kBoxes:
  *                                what lies beyond the last key is zeros)
  *   start()                      after the wait for the previous kernel: resolves what lies in device memory
+ *   rows(a)                      how many there are: a launch may serve several prompts (blockIdx.z), a.M the most of one
  *   pos0()                       position of row 0
  *   q4(row, head, d)             four query values (zeros beyond the head)
  *   keys(...) / values(...)      otherwise, with cp.async: a loading warp's 16 keys, into blocks of 64 columns, high halves
@@ -197,6 +198,9 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const __grid_
     int *abort_flag = (int *)(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int group = a.heads / a.kv_heads, g = blockIdx.x, pairs = src_arg.rows(a) * group;
+    const int P0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kAtRows;           /* the latest rows see the most keys: they go first */
+    if (P0 >= pairs) return;                                                   /* a shorter prompt beside a longer one */
     if (tid == 0) {
         for (int i = 0; i < Cfg::kSlots; i++) {
             vb_mbar_init(&k_full[i], kAtLoadK);
@@ -227,9 +231,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const __grid_
 
     SRC src = src_arg;
     src.start();
-    const int group = a.heads / a.kv_heads, g = blockIdx.x;
-    const int pairs = a.M * group, pos0 = src.pos0();
-    const int P0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kAtRows;           /* the latest rows see the most keys: they go first */
+    const int pos0 = src.pos0();
     const int last = P0 + kAtRows < pairs ? P0 + kAtRows - 1 : pairs - 1;
     const int imin = pos0 + P0 / group, imax = pos0 + last / group;
     const KeyTiles kt = key_tiles<kAtKeys>(imin, imax, a.window, a.keep);
@@ -548,7 +550,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const __grid_
 }
 
 template <int DK, int DV, class SRC>
-int launch_attn_tc(const AtArgs &a, const SRC &src, cudaStream_t st, const AtMaps &maps = AtMaps()) {
+int launch_attn_tc(const AtArgs &a, const SRC &src, cudaStream_t st, const AtMaps &maps = AtMaps(), int prompts = 1) {
     using Cfg = AtCfg<DK, DV>;
     static bool attr = false;
     if (!attr) {
@@ -559,7 +561,7 @@ int launch_attn_tc(const AtArgs &a, const SRC &src, cudaStream_t st, const AtMap
         attr = true;
     }
     const int tiles = (int)(((long long)a.M * (a.heads / a.kv_heads) + kAtRows - 1) / kAtRows);
-    return launch_pdl(vb_attn_tc_kernel<DK, DV, SRC>, dim3(a.kv_heads, tiles), dim3(kAtThreads), (size_t)Cfg::kSmem, st, maps, a, src) == cudaSuccess
+    return launch_pdl(vb_attn_tc_kernel<DK, DV, SRC>, dim3(a.kv_heads, tiles, prompts), dim3(kAtThreads), (size_t)Cfg::kSmem, st, maps, a, src) == cudaSuccess
                ? 0
                : -1;
 }

@@ -1191,6 +1191,22 @@ int batch_prefill(int utt, const float *embeds, int n_rows) {
     return rc;
 }
 
+/* The prompts of all utterances: side by side where prefill_joint takes them, one by one where it does not. */
+int batch_prefill_all(const float *const *embeds, const int *n_rows) {
+    Batch &t = g_bt;
+    if (!t.open || !embeds || !n_rows) return -1;
+    PfPrompt p[kBtMaxUtt];
+    bool done[kBtMaxUtt];
+    for (int u = 0; u < t.B; u++) {
+        if (!embeds[u] || n_rows[u] < 1 || n_rows[u] > t.kv_max) return -1;
+        p[u] = {embeds[u], n_rows[u], t.kv_k + (size_t)u * t.slab, t.kv_v + (size_t)u * t.slab};
+    }
+    if (prefill_joint(p, t.B, t.kv_max, done)) return -1;
+    for (int u = 0; u < t.B; u++)
+        if (!done[u] && batch_prefill(u, embeds[u], n_rows[u])) return -1;
+    return 0;
+}
+
 int batch_begin(const float *first_embeds, const int *start_pos, const float *noise) {
     Model &m = model();
     Batch &t = g_bt;
@@ -1255,7 +1271,7 @@ int batch_hidden(float *out) {
 }
 
 int batch_launches_per_frame() {
-    const int prepares = g_bt.open && 6 * g_bt.B > 16 ? 2 * VB200_AC_LAYERS : 1;      /* per Euler step; else its GEMMs do it */
+    const int prepares = g_bt.open && 6 * g_bt.B > 16 ? 2 * VB200_AC_LAYERS - 1 : 0;      /* per Euler step; else its GEMMs do it */
     return 2 + VB200_DEC_LAYERS * 5 + 5 + (VB200_FLOW_STEPS - 1) * (2 + prepares + VB200_AC_LAYERS * 5) + 1;
 }
 

@@ -613,6 +613,7 @@ struct AtCache {
     int heads, kv_heads, dim, vdim;
     const float *kc, *vc;
     VB_DEVINL void start() { kc = lm_state(k, dyn); vc = lm_state(v, dyn); }
+    VB_DEVINL int rows(const AtArgs &a) const { return a.M; }
     VB_DEVINL int pos0() const { return dyn->pos; }
     VB_DEVINL float4 q4(int row, int head, int d) const {
         return d < dim ? vb_ldcg4(q + ((size_t)row * heads + head) * dim + d) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -673,6 +674,7 @@ struct AtWide {
     LmSink out;
     int heads, dim, vdim, rot;
     VB_DEVINL void start() { w.cache += (size_t)dyn->slot * w.slab; }
+    VB_DEVINL int rows(const AtArgs &a) const { return a.M; }
     VB_DEVINL int pos0() const { return dyn->pos; }
     VB_DEVINL float4 q4(int row, int head, int d) const {
         if (d >= dim) return make_float4(0.f, 0.f, 0.f, 0.f);

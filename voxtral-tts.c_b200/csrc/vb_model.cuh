@@ -123,6 +123,8 @@ int predict_velocity(float *out_v, const float *x_t, const float *hidden, float 
 int linear(float *y, const float *x, const uint16_t *W_host, int M, int K, int N, const void *W_gpu);
 int linear_device(float *d_y, const float *d_x, const uint16_t *d_W, int M, int K, int N);
 int prefill(const float *embeds, int seq_len, int start_pos);
+struct PfPrompt { const float *embeds; int rows; float *kv_k, *kv_v; };
+int prefill_joint(const PfPrompt *prompts, int n, int kv_max, bool *done);
 int prefill_prompt(const int *text_ids, int n_text, const uint16_t *voice_bf16, int n_voice, int start_pos);
 int prefill_tc_setup();
 void prefill_free_all();
@@ -136,6 +138,7 @@ int acoustic_tc_enqueue(const float *noise_all, int *codes_all, int frame_cap, b
 /* several utterances in lock step (vb_batch.cu) */
 int batch_open(int n_utt, int kv_max, int max_frames);
 int batch_prefill(int utt, const float *embeds, int n_rows);
+int batch_prefill_all(const float *const *embeds, const int *n_rows);
 int batch_begin(const float *first_embeds, const int *start_pos, const float *noise);
 int batch_run(int n);
 int batch_end(int *codes_out, int *frames_done, int *hit_end, float *device_ms);

@@ -14,6 +14,8 @@
 #include "vb_simple.cuh"
 #include "vb_tc.cuh"
 
+#include <algorithm>
+
 #include <math.h>
 #include <stdio.h>
 #include <string.h>
@@ -71,19 +73,45 @@ __global__ void pf_split_kernel(PfSplit to, const float *kc, const float *vc) {
     pf_split(to.v, row, col, __ldcg(reinterpret_cast<const float2 *>(vc + row * KVD + col)));
 }
 
+/* A block of rows is a stretch of one prompt, or several short prompts side by side: their GEMMs are one, each has its own
+ * cache rows, positions and split keys. */
+constexpr int kPfSegs = 8;
+struct PfSeg {
+    int row0, rows;              /* in the block */
+    int pos, cs0;                /* position of its first row, and that row's place in the rotation table */
+    int key0;                    /* where its position 0 lies among the split keys: a multiple of a key tile */
+    int y0;                      /* first of its rows and zero rows in pf_qkv_finish's grid */
+    float *k, *v;                /* its cache, layer 0 */
+    size_t layer;                /* floats from one layer of it to the next */
+};
+struct PfSegs {
+    int n = 0, rows = 0, keys = 0, grid = 0;
+    PfSeg s[kPfSegs] = {};
+    void add(int rows_, int pos, int cs0, float *k, float *v, int kv_max) {
+        const int end = pos + rows_, tiles = (end + kAtKeys - 1) / kAtKeys * kAtKeys;
+        s[n++] = {rows, rows_, pos, cs0, keys, grid, k, v, (size_t)kv_max * KVD};
+        rows += rows_;
+        keys += tiles;
+        grid += tiles - pos;
+    }
+};
+
 /* QKV of a row block: sums the split-K partials in fixed order, rotates the q and k heads
  * (interleaved pairs, voxtral_tts_kernels.c:616-634), leaves q in `qkv` for the attention
- * and writes k and v straight into the cache rows (voxtral_tts_llm.c:318-330) and, split, from row `at` on for the
+ * and writes k and v straight into the cache rows (voxtral_tts_llm.c:318-330) and, split, for the
  * attention, whose tiles of 64 keys end in rows of zeros. One thread per pair of columns. */
-__global__ void pf_qkv_finish_kernel(float *qkv, const float *part, int n_part, size_t part_stride, const float *cs,
-                                     float *k_rows, float *v_rows, PfSplit split, int at, int rows) {
+__global__ void pf_qkv_finish_kernel(float *qkv, const float *part, int n_part, size_t part_stride, const float *cs, PfSplit split,
+                                     const __grid_constant__ PfSegs segs, int layer) {
     pdl_launch_dependents();
     pdl_wait();
-    const int m = blockIdx.y;
+    int i = 0;
+    while (i + 1 < segs.n && (int)blockIdx.y >= segs.s[i + 1].y0) i++;
+    const PfSeg &g = segs.s[i];
+    const int r = (int)blockIdx.y - g.y0, m = g.row0 + r, at = g.key0 + g.pos + r;
     const int col = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
     if (col >= QKV) return;
-    if (m >= rows) {
-        if (col >= QD) pf_split(col < QD + KVD ? split.k : split.v, at + m, col < QD + KVD ? col - QD : col - QD - KVD, make_float2(0.0f, 0.0f));
+    if (r >= g.rows) {
+        if (col >= QD) pf_split(col < QD + KVD ? split.k : split.v, at, col < QD + KVD ? col - QD : col - QD - KVD, make_float2(0.0f, 0.0f));
         return;
     }
     float2 v = make_float2(0.0f, 0.0f);
@@ -93,18 +121,19 @@ __global__ void pf_qkv_finish_kernel(float *qkv, const float *part, int n_part, 
     }
     if (col < QD + KVD) {
         const int d = (col % VB200_HEAD_DIM) >> 1;
-        const float2 t = *reinterpret_cast<const float2 *>(cs + ((size_t)m * (VB200_HEAD_DIM / 2) + d) * 2);
+        const float2 t = *reinterpret_cast<const float2 *>(cs + ((size_t)(g.cs0 + r) * (VB200_HEAD_DIM / 2) + d) * 2);
         const float a = v.x, b = v.y;
         v.x = a * t.x - b * t.y;
         v.y = a * t.y + b * t.x;
     }
+    const size_t row = (size_t)layer * g.layer + (size_t)(g.pos + r) * KVD;
     if (col < QD) *reinterpret_cast<float2 *>(qkv + (size_t)m * QKV + col) = v;
     else if (col < QD + KVD) {
-        *reinterpret_cast<float2 *>(k_rows + (size_t)m * KVD + (col - QD)) = v;
-        pf_split(split.k, at + m, col - QD, v);
+        *reinterpret_cast<float2 *>(g.k + row + (col - QD)) = v;
+        pf_split(split.k, at, col - QD, v);
     } else {
-        *reinterpret_cast<float2 *>(v_rows + (size_t)m * KVD + (col - QD - KVD)) = v;
-        pf_split(split.v, at + m, col - QD - KVD, v);
+        *reinterpret_cast<float2 *>(g.v + row + (col - QD - KVD)) = v;
+        pf_split(split.v, at, col - QD - KVD, v);
     }
 }
 
@@ -114,17 +143,19 @@ struct AtRows {
     static constexpr bool kBoxes = true;
     const float *q;
     LmSink out;                  /* the terms that the O projection reads */
-    int ldq, start_pos;
+    int ldq;
+    struct { int row0, rows, pos, key0; } s[kPfSegs];      /* blockIdx.z chooses: PfSeg */
     VB_DEVINL void start() {}
-    VB_DEVINL int pos0() const { return start_pos; }
+    VB_DEVINL int rows(const AtArgs &) const { return s[blockIdx.z].rows; }
+    VB_DEVINL int pos0() const { return s[blockIdx.z].pos; }
     VB_DEVINL float4 q4(int row, int head, int d) const {
-        return vb_ldcg4(q + (size_t)row * ldq + head * VB200_HEAD_DIM + d);
+        return vb_ldcg4(q + (size_t)(s[blockIdx.z].row0 + row) * ldq + head * VB200_HEAD_DIM + d);
     }
     VB_DEVINL bool boxes(int, int) const { return true; }
     template <int BLOCKS>
     VB_DEVINL void box(const CUtensorMap *map, unsigned char *slot, int g, int j0, uint64_t *bar) const {
 #pragma unroll
-        for (int b = 0; b < 2 * BLOCKS; b++) at_tma(slot + b * kAtBlock, map, (g * 2 * BLOCKS + b) * 64, j0, 0, bar);
+        for (int b = 0; b < 2 * BLOCKS; b++) at_tma(slot + b * kAtBlock, map, (g * 2 * BLOCKS + b) * 64, s[blockIdx.z].key0 + j0, 0, bar);
     }
     template <int BLOCKS>
     VB_DEVINL void tma_keys(const AtArgs &, const AtMaps &m, unsigned char *slot, int g, int j0, uint64_t *bar) const {
@@ -135,7 +166,7 @@ struct AtRows {
         box<BLOCKS>(&m.v, slot, g, j0, bar);
     }
     VB_DEVINL float gate(int, int) const { return 1.0f; }
-    VB_DEVINL void put4(int row, int c, const float (&e)[4]) const { lm_put4(out, row, c, e); }
+    VB_DEVINL void put4(int row, int c, const float (&e)[4]) const { lm_put4(out, s[blockIdx.z].row0 + row, c, e); }
 };
 static_assert(VB200_HEAD_DIM == 128, "two blocks of 64 columns");
 
@@ -223,10 +254,17 @@ static int pf_next_rows(int left, int block) {
     return left > 256 && tail >= 1 && tail <= 64 ? left - tail : left;
 }
 
-static int pf_tc_buffers(int M, int start_pos, int block) {
+static int pf_block_buffers(size_t rows, size_t pad, size_t part, size_t keys) {
     PrefillTc &t = g_pf;
-    const size_t keys = (size_t)(start_pos + M + kAtKeys - 1) / kAtKeys * kAtKeys;
-    if (pf_grow(12, &t.split.k, keys * 4 * KVD) || pf_grow(13, &t.split.v, keys * 4 * KVD)) return -1;
+    return pf_grow(12, &t.split.k, keys * 4 * KVD) || pf_grow(13, &t.split.v, keys * 4 * KVD) || pf_grow(2, &t.qkv, rows * QKV * 4) ||
+                   pf_grow(3, &t.part, part * 4) || pf_grow(4, &t.ssq, rows * tc_prepare_chunks(D) * 4) ||
+                   pf_grow(5, &t.bD, tc_acts_bytes((int)pad, D)) || pf_grow(6, &t.bQ, tc_acts_bytes((int)pad, QD)) ||
+                   pf_grow(7, &t.bH, tc_acts_bytes((int)pad, HID))
+               ? -1
+               : 0;
+}
+
+static int pf_tc_buffers(int M, int start_pos, int block) {
     /* a last block may be split more ways than a full one */
     size_t part = 0, pad = 0, rows = 0;
     for (int left = M, r; left > 0; left -= r) {
@@ -236,11 +274,7 @@ static int pf_tc_buffers(int M, int start_pos, int block) {
         pad = (size_t)b.rp > pad ? b.rp : pad;
         rows = (size_t)r > rows ? r : rows;
     }
-    return pf_grow(2, &t.qkv, rows * QKV * 4) || pf_grow(3, &t.part, part * 4) || pf_grow(4, &t.ssq, rows * tc_prepare_chunks(D) * 4) ||
-                   pf_grow(5, &t.bD, tc_acts_bytes((int)pad, D)) || pf_grow(6, &t.bQ, tc_acts_bytes((int)pad, QD)) ||
-                   pf_grow(7, &t.bH, tc_acts_bytes((int)pad, HID))
-               ? -1
-               : 0;
+    return pf_block_buffers(rows, pad, part, (size_t)(start_pos + M + kAtKeys - 1) / kAtKeys * kAtKeys);
 }
 
 /* Rows that go through a layer at once, with buffers for them: fewer where little memory is left; 0: the streaming
@@ -259,62 +293,74 @@ int prefill_tc_setup() {
     return 0;
 }
 
-/* Prefill with the tcgen05 GEMM (vb_tc.cu, vb_tc_rows.cu), a block of rows and a layer at a time:
+/* Prefill with the tcgen05 GEMM (vb_tc.cu, vb_tc_rows.cu), a block of rows through all layers:
  * gain+terms -> QKV -> RoPE -> cache rows -> causal attention over the cache so far, which leaves terms -> O ->
  * residual+gain+terms -> gate/up with SwiGLU -> down -> residual+gain+terms. */
-static int prefill_tc(float *x, const float *cs, int M, int start_pos, int block) {
+static int prefill_block(float *xr, const float *cs, const PfSegs &segs, const PfBlock &b, int segment) {
     Model &m = model();
     PrefillTc &t = g_pf;
     cudaStream_t st = m.st;
     const float scale = 1.0f / sqrtf((float)VB200_HEAD_DIM);
-    const int chunksD = tc_prepare_chunks(D);
-    /* the row blocks follow one another through all layers: a row sees nothing of later rows */
-    for (int r0 = 0, rows; r0 < M; r0 += rows) {
-        rows = pf_next_rows(M - r0, block);
-        const PfBlock b = pf_block(rows);
-        TcActs aD, aQ, aH;
-        if (tc_acts(&aD, t.bD, b.rp, D) || tc_acts(&aQ, t.bQ, b.rp, QD) || tc_acts(&aH, t.bH, b.rp, HID)) return -1;
-        const uint64_t keys = (uint64_t)(start_pos + r0 + rows + kAtKeys - 1) / kAtKeys * kAtKeys;
-        AtMaps maps = {};
-        if (tc_map3(&maps.k, t.split.k, 1, keys * 4 * KVD, keys, 4 * KVD, 2 * KVD, kAtKeys) ||
-            tc_map3(&maps.v, t.split.v, 1, keys * 4 * KVD, keys, 4 * KVD, 2 * KVD, kAtKeys))
-            return -1;
-        const LmSink q_terms = {t.bQ, b.rp, QD, b.rp < 256 ? kTcTerms : 2};
-        const size_t psD = (size_t)rows * D;
-        float *xr = x + (size_t)r0 * D;
-        for (int l = 0; l < VB200_DEC_LAYERS; l++) {
-            const LayerDev &L = m.dec[l];
-            if (l == 0) tc_prepare(aD, xr, D, rows, nullptr, 0, 0, nullptr, nullptr, L.attn_norm, t.ssq, st);
-            TcGemm g;
-            g.M = rows; g.status = &m.d_out->status; g.epi = TC_EPI_PARTIAL; g.out = t.part; g.ld_out = QKV;
-            g.splits = b.s_qkv; g.ssq = t.ssq; g.ssq_chunks = chunksD; g.eps = VB200_NORM_EPS;
-            if (tc_gemm(t.wqkv[l], aD, g, st)) return -1;
-            float *k0 = m.kv_k + (size_t)l * m.kv_max * KVD, *v0 = m.kv_v + (size_t)l * m.kv_max * KVD;
-            const int at = start_pos + r0, tail = (kAtKeys - (at + rows) % kAtKeys) % kAtKeys;
-            if (at > 0 && launch_pdl(pf_split_kernel, dim3(at, KVD / 512), dim3(256), 0, st, t.split, (const float *)k0, (const float *)v0) != cudaSuccess)
+    const int chunksD = tc_prepare_chunks(D), rows = segs.rows;
+    TcActs aD, aQ, aH;
+    if (tc_acts(&aD, t.bD, b.rp, D) || tc_acts(&aQ, t.bQ, b.rp, QD) || tc_acts(&aH, t.bH, b.rp, HID)) return -1;
+    const uint64_t keys = (uint64_t)segs.keys;
+    AtMaps maps = {};
+    if (tc_map3(&maps.k, t.split.k, 1, keys * 4 * KVD, keys, 4 * KVD, 2 * KVD, kAtKeys) ||
+        tc_map3(&maps.v, t.split.v, 1, keys * 4 * KVD, keys, 4 * KVD, 2 * KVD, kAtKeys))
+        return -1;
+    AtRows rows_of = {t.qkv, {t.bQ, b.rp, QD, b.rp < 256 ? kTcTerms : 2}, QKV, {}};
+    int most = 0;
+    for (int i = 0; i < segs.n; i++) {
+        rows_of.s[i] = {segs.s[i].row0, segs.s[i].rows, segs.s[i].pos, segs.s[i].key0};
+        most = std::max(most, segs.s[i].rows);
+    }
+    const AtArgs args = {most, VB200_HEADS, VB200_KV_HEADS, VB200_HEAD_DIM, VB200_HEAD_DIM, 0, 0, scale, 0.0f, &m.d_out->status, 1};
+    const size_t psD = (size_t)rows * D;
+    for (int l = 0; l < VB200_DEC_LAYERS; l++) {
+        const LayerDev &L = m.dec[l];
+        if (l == 0) tc_prepare(aD, xr, D, rows, nullptr, 0, 0, nullptr, nullptr, L.attn_norm, t.ssq, st);
+        TcGemm g;
+        g.M = rows; g.status = &m.d_out->status; g.epi = TC_EPI_PARTIAL; g.out = t.part; g.ld_out = QKV; g.segment = segment;
+        g.splits = b.s_qkv; g.ssq = t.ssq; g.ssq_chunks = chunksD; g.eps = VB200_NORM_EPS;
+        if (tc_gemm(t.wqkv[l], aD, g, st)) return -1;
+        for (int i = 0; i < segs.n; i++) {       /* earlier rows of a prompt: those of a block of its own alone */
+            const PfSeg &e = segs.s[i];
+            const PfSplit to = {t.split.k + (size_t)e.key0 * 2 * KVD, t.split.v + (size_t)e.key0 * 2 * KVD};
+            if (e.pos > 0 && launch_pdl(pf_split_kernel, dim3(e.pos, KVD / 512), dim3(256), 0, st, to, (const float *)(e.k + l * e.layer),
+                                        (const float *)(e.v + l * e.layer)) != cudaSuccess)
                 return -1;
-            if (launch_pdl(pf_qkv_finish_kernel, dim3(QKV / 2 / 256, rows + tail), dim3(256), 0, st, t.qkv, (const float *)t.part, b.s_qkv,
-                           (size_t)rows * QKV, cs + (size_t)r0 * VB200_HEAD_DIM, k0 + (size_t)at * KVD, v0 + (size_t)at * KVD, t.split, at,
-                           rows) != cudaSuccess)
-                return -1;
-            if (l == VB200_DEC_LAYERS - 1) break;   /* only the cache is kept (voxtral_tts_llm.c:281) */
-            const AtRows rows_of = {t.qkv, q_terms, QKV, at};
-            const AtArgs args = {rows, VB200_HEADS, VB200_KV_HEADS, VB200_HEAD_DIM, VB200_HEAD_DIM, 0, 0, scale, 0.0f, &m.d_out->status, 1};
-            if (launch_attn_tc<2, 2>(args, rows_of, st, maps)) return -1;
-            g.splits = b.s_wo; g.ld_out = D; g.ssq = nullptr; g.ssq_chunks = 0;
-            if (tc_gemm(t.wo[l], aQ, g, st)) return -1;
-            tc_prepare(aD, nullptr, D, rows, t.part, b.s_wo, psD, xr, xr, L.ffn_norm, t.ssq, st);
-            g.epi = TC_EPI_SWIGLU_TERMS; g.out = nullptr; g.out_terms = t.bH; g.out_rows_pad = b.rp; g.splits = 1;
-            g.ld_out = HID; g.ssq = t.ssq; g.ssq_chunks = chunksD;
-            if (tc_gemm(t.w13[l], aD, g, st)) return -1;
-            g.epi = TC_EPI_PARTIAL; g.out = t.part; g.out_terms = nullptr; g.splits = b.s_w2; g.ld_out = D;
-            g.ssq = nullptr; g.ssq_chunks = 0;
-            if (tc_gemm(t.w2[l], aH, g, st)) return -1;
-            /* residual add and the next layer's rows */
-            tc_prepare(aD, nullptr, D, rows, t.part, b.s_w2, psD, xr, xr, m.dec[l + 1].attn_norm, t.ssq, st);
         }
+        if (launch_pdl(pf_qkv_finish_kernel, dim3(QKV / 2 / 256, segs.grid), dim3(256), 0, st, t.qkv, (const float *)t.part, b.s_qkv,
+                       (size_t)rows * QKV, cs, t.split, segs, l) != cudaSuccess)
+            return -1;
+        if (l == VB200_DEC_LAYERS - 1) break;   /* only the cache is kept (voxtral_tts_llm.c:281) */
+        if (launch_attn_tc<2, 2>(args, rows_of, st, maps, segs.n)) return -1;
+        g.splits = b.s_wo; g.ld_out = D; g.ssq = nullptr; g.ssq_chunks = 0;
+        if (tc_gemm(t.wo[l], aQ, g, st)) return -1;
+        tc_prepare(aD, nullptr, D, rows, t.part, b.s_wo, psD, xr, xr, L.ffn_norm, t.ssq, st);
+        g.epi = TC_EPI_SWIGLU_TERMS; g.out = nullptr; g.out_terms = t.bH; g.out_rows_pad = b.rp; g.splits = 1;
+        g.ld_out = HID; g.ssq = t.ssq; g.ssq_chunks = chunksD;
+        if (tc_gemm(t.w13[l], aD, g, st)) return -1;
+        g.epi = TC_EPI_PARTIAL; g.out = t.part; g.out_terms = nullptr; g.splits = b.s_w2; g.ld_out = D;
+        g.ssq = nullptr; g.ssq_chunks = 0;
+        if (tc_gemm(t.w2[l], aH, g, st)) return -1;
+        /* residual add and the next layer's rows */
+        tc_prepare(aD, nullptr, D, rows, t.part, b.s_w2, psD, xr, xr, m.dec[l + 1].attn_norm, t.ssq, st);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+/* The row blocks of a prompt follow one another through all layers: a row sees nothing of later rows. */
+static int prefill_tc(float *x, const float *cs, int M, int start_pos, int block) {
+    Model &m = model();
+    for (int r0 = 0, rows; r0 < M; r0 += rows) {
+        rows = pf_next_rows(M - r0, block);
+        PfSegs segs;
+        segs.add(rows, start_pos + r0, r0, m.kv_k, m.kv_v, m.kv_max);
+        if (prefill_block(x + (size_t)r0 * D, cs, segs, pf_block(rows), TcGemm().segment)) return -1;
+    }
+    return 0;
 }
 
 /* Checks, and the buffers of all rows: g_pf.x for the embeddings, the rotation table. */
@@ -331,6 +377,67 @@ static int prefill_begin(int M, int start_pos) {
 }
 
 static int prefill_run(int M, int start_pos);
+
+/* Waits for what was enqueued; its status, or rc. */
+static int pf_finish(int rc) {
+    Model &m = model();
+    int status = 0;
+    if (cudaMemcpyAsync(&status, &m.d_out->status, sizeof(int), cudaMemcpyDeviceToHost, m.st) != cudaSuccess ||
+        cudaStreamSynchronize(m.st) != cudaSuccess)
+        return -1;
+    if (rc) return rc;
+    m.last_status = status;
+    if (!status) return 0;
+    /* the word is sticky on the device (kernels only set it from 0): clear it so the next call starts clean */
+    cudaMemset(&m.d_out->status, 0, sizeof(int));
+    return -1;
+}
+
+/* Several prompts from position 0 on, each into a cache of its own (kv_max rows a layer): side by side through the layers as
+ * long as a block has room, so that the weights are read once and the GEMMs are wide. Eight prompts of 100 to 187 rows took
+ * 27 ms one after another. Only those that alone would be one block of two-term products; the others, and all where memory
+ * is short, are left for prefill(): done[i] says which are in their caches. K is summed in pieces of 1024 columns: alone,
+ * these prompts have the frame's K splits, of 512 to 1536. */
+constexpr int kPfJointSegment = 16;
+int prefill_joint(const PfPrompt *prompts, int n, int kv_max, bool *done) {
+    Model &m = model();
+    PrefillTc &t = g_pf;
+    if (!m.inited || !m.llm_ready) return -1;
+    std::vector<int> fit;
+    for (int i = 0; i < n; i++) {
+        done[i] = false;
+        const int r = prompts[i].rows;
+        if (r > 64 && r <= kv_max && r <= kPfRows && pf_next_rows(r, kPfRows) == r) fit.push_back(i);
+    }
+    if (!t.ready || fit.size() < 2 || batch_tiled_decoder(&t.wqkv, &t.wo, &t.w13, &t.w2)) return 0;
+    for (size_t i = 0; i < fit.size();) {
+        PfSegs segs;
+        int most = 0;
+        size_t j = i;
+        for (; j < fit.size() && segs.n < kPfSegs && segs.rows + prompts[fit[j]].rows <= kPfRows; j++) {
+            const PfPrompt &p = prompts[fit[j]];
+            segs.add(p.rows, 0, 0, p.kv_k, p.kv_v, kv_max);
+            most = std::max(most, p.rows);
+        }
+        if (segs.n < 2) { i = j; continue; }
+        const PfBlock b = pf_block(segs.rows);
+        const size_t part = std::max({(size_t)b.s_qkv * QKV, (size_t)b.s_wo * D, (size_t)b.s_w2 * D}) * segs.rows;
+        if (pf_grow(0, &t.x, (size_t)segs.rows * D * 4) || pf_grow(1, &t.cs, (size_t)most * VB200_HEAD_DIM * 4) ||
+            pf_block_buffers(segs.rows, b.rp, part, segs.keys)) {
+            pf_release_block();
+            return 0;
+        }
+        rope_table(t.cs, 0, most, VB200_HEAD_DIM, VB200_ROPE_THETA, m.st);
+        for (size_t k = i; k < j; k++)
+            if (cudaMemcpyAsync(t.x + (size_t)segs.s[k - i].row0 * D, prompts[fit[k]].embeds, (size_t)prompts[fit[k]].rows * D * 4, cudaMemcpyDefault,
+                                m.st) != cudaSuccess)
+                return -1;
+        if (pf_finish(prefill_block(t.x, t.cs, segs, b, kPfJointSegment))) return -1;
+        for (size_t k = i; k < j; k++) done[fit[k]] = true;
+        i = j;
+    }
+    return 0;
+}
 
 int prefill(const float *embeds, int seq_len, int start_pos) {
     Model &m = model();
@@ -350,23 +457,7 @@ static int prefill_run(int M, int start_pos) {
     const float scale = 1.0f / sqrtf((float)VB200_HEAD_DIM);
 
     const int block = t.ready && batch_tiled_decoder(&t.wqkv, &t.wo, &t.w13, &t.w2) == 0 ? pf_fit(M, start_pos) : 0;
-    if (block > 0) {
-        rc = prefill_tc(x, cs, M, start_pos, block);
-        int status = 0;
-        if (cudaMemcpyAsync(&status, &m.d_out->status, sizeof(int), cudaMemcpyDeviceToHost, m.st) != cudaSuccess ||
-            cudaStreamSynchronize(m.st) != cudaSuccess)
-            return -1;
-        if (!rc) {
-            m.last_status = status;
-            if (status) {
-                /* the word is sticky on the device (kernels only set it from 0): clear it so the
-                 * next call starts clean */
-                cudaMemset(&m.d_out->status, 0, sizeof(int));
-                rc = -1;
-            }
-        }
-        return rc;
-    }
+    if (block > 0) return pf_finish(prefill_tc(x, cs, M, start_pos, block));
     if (pf_grow(2, &t.qkv, (size_t)M * QKV * 4) || pf_grow(8, &t.attn, (size_t)M * QD * 4) || pf_grow(9, &t.h, (size_t)M * HID * 4)) return -1;
     float *qkv = t.qkv, *attn = t.attn, *h = t.h;
     for (int l = 0; l < VB200_DEC_LAYERS && !rc; l++) {
