@@ -594,6 +594,251 @@ int launch_attn_step(const LmAttn &a, int splits, int lanes_h, cudaStream_t st) 
     return ok(launch_pdl(lm_attn_step_kernel<ND, NV, KP, SPLIT>, dim3(splits, a.kv_heads), dim3(kSaThreads), smem, st, a, lanes_h));
 }
 
+/* ------------------------------------------------------------------ one token, few query heads a key head */
+/* The same for up to four query heads a KV head and heads of up to 128: grid = (key splits, KV heads), the splits of a KV head a
+ * cluster; a warp takes eight keys at a time for all heads of the group, and a CTA sends the others' columns of its
+ * result into their shared memory (asynchronous stores that count on the receiver's barrier), so that each merges its share
+ * in split order. Bound by latency: whatever the kernel before does not make is fetched before the wait for it - the
+ * position, the angles, the gains, the first pass of keys and values (earlier steps are complete: a step's first kernel
+ * is a plain launch). One warp per head and a merge by the last CTA through global memory: 17 us at 220 keys of 8 x 128. */
+constexpr int kSgThreads = 256, kSgWarps = 8, kSgKeys = 8, kSgHeads = 4, kSgDim = 128, kSgSplits = 8, kSgColumns = 8;
+
+template <bool SPLIT>
+__global__ void __launch_bounds__(kSgThreads, 2) lm_attn_step_group_kernel(const LmAttn a) {
+    __shared__ __align__(16) float raw[(kSgHeads + 1) * kSgDim], qs[kSgHeads][kSgDim], ks[kSgDim], vs[kSgDim], cs[kSgDim];
+    __shared__ __align__(16) float warp_o[kSgWarps][kSgHeads][kSgDim];
+    __shared__ float2 warp_ml[kSgWarps][kSgHeads];         /* maximum, sum */
+    __shared__ float4 slices[kSgThreads];                  /* [S][columns of this CTA / 2]: two columns, maximum, sum */
+    __shared__ float red[2][kSgWarps];
+    __shared__ uint64_t arrived;
+    __shared__ volatile int gave_up;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    pdl_launch_dependents();
+    if (tid == 0) {
+        vb_mbar_init(&arrived, 1);
+        gave_up = 0;
+        vb_mbar_init_fence();
+        vb_mbar_arrive_expect_tx(&arrived, (uint32_t)sizeof(slices));
+    }
+    __syncthreads();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    const int dim = a.dim, vdim = a.vdim, group = a.heads / a.kv_heads, half = a.rot / 2;
+    const int nq = a.heads * dim, nk = a.kv_heads * dim, nv = a.kv_heads * vdim;
+    const int sp = blockIdx.x, S = gridDim.x, g = blockIdx.y;
+    const int pos = __ldcg(&a.dyn->pos), slot = __ldcg(&a.dyn->slot);
+    /* visible keys in order: the kept ones, then the window; the new token is the last */
+    const int n_keep = a.window > 0 ? (a.keep < pos + 1 ? a.keep : pos + 1) : 0;
+    const int w0 = a.window > 0 ? (pos - a.window + 1 > n_keep ? pos - a.window + 1 : n_keep) : 0;
+    const int n_keys = n_keep + (pos + 1 - w0);
+    const int x0 = (int)((long long)n_keys * sp / S), x1 = (int)((long long)n_keys * (sp + 1) / S);
+    const bool writer = sp == S - 1;
+    float *Kc = a.k.base + (size_t)slot * a.k.slab + g * dim, *Vc = a.v.base + (size_t)slot * a.v.slab + g * vdim;
+    const int first = w0 > a.ring.keep ? (w0 - a.ring.keep) % a.ring.ring : 0;      /* ring place of the window's first key */
+    float4 kq[kSgKeys], vq[kSgKeys];
+    auto fetch = [&](int xb) {                             /* keys xb, xb + 8, ...: all requests in flight together; the new token has none */
+#pragma unroll
+        for (int u = 0; u < kSgKeys; u++) {
+            const int x = xb + u * kSgWarps;
+            int r = first + x - n_keep;
+            r = x < n_keep ? x : a.ring.keep + (r < a.ring.ring ? r : r - a.ring.ring);
+            const bool on = x < x1 && x < n_keys - 1;
+            kq[u] = on && 4 * lane < dim ? kv_get4<SPLIT>(Kc + (size_t)r * nk, dim, 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+            vq[u] = on && 4 * lane < vdim ? kv_get4<SPLIT>(Vc + (size_t)r * nv, vdim, 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    int xb = x0 + warp;
+    fetch(xb);
+    for (int i = tid; i < half; i += kSgThreads) lm_angle(pos, a.freq[i], a.freq[half + i], a.mag, &cs[i], &cs[half + i]);
+    const int own0 = g * group * dim, k0 = nq + g * dim, total = (writer ? group + 1 : group) * dim;
+    constexpr int kMine = (kSgHeads + 1) * kSgDim / kSgThreads + 1;
+    float gain[kMine];
+#pragma unroll
+    for (int u = 0; u < kMine; u++) {
+        const int i = tid + u * kSgThreads;
+        gain[u] = i >= total ? 0.0f : i < group * dim ? __ldg(a.q_gain + own0 + i) : __ldg(a.k_gain + g * dim + i - group * dim);
+    }
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");             /* all barriers of the cluster are set up */
+    pdl_wait();
+
+    /* every CTA sums the squares of the whole q and k projection itself, up to 8 x 1024 columns requested together */
+    float sq = 0.0f, sk = 0.0f;
+    for (int c0 = tid * 4; c0 < nq + nk; c0 += kSgColumns * kSgThreads * 4) {
+        float4 v[kSgColumns];
+#pragma unroll
+        for (int u = 0; u < kSgColumns; u++) v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+        for (int p = 0; p < a.qkv.n; p++) {
+            const float *at = a.qkv.p + (size_t)p * a.qkv.stride;
+            float4 t[kSgColumns];
+#pragma unroll
+            for (int u = 0; u < kSgColumns; u++) {
+                const int c = c0 + u * kSgThreads * 4;
+                t[u] = c < nq + nk ? vb_ldcg4(at + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int u = 0; u < kSgColumns; u++) { v[u].x += t[u].x; v[u].y += t[u].y; v[u].z += t[u].z; v[u].w += t[u].w; }
+        }
+#pragma unroll
+        for (int u = 0; u < kSgColumns; u++) {
+            const int c = c0 + u * kSgThreads * 4;
+            const float ss = v[u].x * v[u].x + v[u].y * v[u].y + v[u].z * v[u].z + v[u].w * v[u].w;
+            if (c < nq) sq += ss;
+            else if (c < nq + nk) sk += ss;
+            if (c >= own0 && c < own0 + group * dim) *reinterpret_cast<float4 *>(raw + c - own0) = v[u];
+            else if (c >= k0 && c < k0 + dim) *reinterpret_cast<float4 *>(raw + group * dim + c - k0) = v[u];
+        }
+    }
+    const size_t new_row = (size_t)lm_ring_row(a.ring, pos);
+    /* what the cache keeps of the new token is what this step attends to */
+    auto kept = [](float v) {
+        if constexpr (!SPLIT) return v;
+        uint32_t hi, lo;
+        hilo(v, hi, lo);
+        return __uint_as_float(hi << 16) + __uint_as_float(lo << 16);
+    };
+    if (writer && tid < vdim) {
+        const float v = lm_sum_batch(a.qkv, 0, nq + nk + g * vdim + tid);
+        vs[tid] = kept(v);
+        kv_put(Vc + new_row * nv, vdim, tid, v, SPLIT);
+    }
+    sq = vb_warp_sum(sq);
+    sk = vb_warp_sum(sk);
+    if (lane == 0) { red[0][warp] = sq; red[1][warp] = sk; }
+    __syncthreads();
+    sq = sk = 0.0f;
+#pragma unroll
+    for (int w = 0; w < kSgWarps; w++) { sq += red[0][w]; sk += red[1][w]; }
+    const float rq = 1.0f / sqrtf(sq / (float)nq + a.eps), rk = 1.0f / sqrtf(sk / (float)nk + a.eps);
+#pragma unroll
+    for (int u = 0; u < kMine; u++) {
+        const int i = tid + u * kSgThreads;
+        if (i >= total) continue;
+        const bool isq = i < group * dim;
+        const int d = i % dim;
+        const float r = isq ? rq : rk;
+        float v = raw[i] * r * gain[u];
+        if (d < a.rot) {
+            const int j = d < half ? d : d - half, other = d < half ? half : -half;
+            const float y = raw[i + other] * r * __ldg((isq ? a.q_gain + own0 + i : a.k_gain + g * dim + d) + other);
+            v = d < half ? v * cs[j] - y * cs[half + j] : v * cs[j] + y * cs[half + j];
+        }
+        if (isq) {
+            qs[i / dim][d] = v;
+        } else {
+            ks[d] = kept(v);
+            kv_put(Kc + new_row * nk, dim, d, v, SPLIT);
+        }
+    }
+    __syncthreads();
+
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 q4[kSgHeads], o[kSgHeads];
+#pragma unroll
+    for (int h = 0; h < kSgHeads; h++) {
+        q4[h] = h < group && 4 * lane < dim ? *reinterpret_cast<const float4 *>(&qs[h][4 * lane]) : zero;
+        o[h] = zero;
+    }
+    float mx = -INFINITY, den = 0.0f;                      /* of head lane / 8 */
+    static_assert(kSgKeys * kSgHeads == 32, "a lane per key and head");
+    while (xb < x1) {
+        float s[32];                                       /* [head][key] */
+#pragma unroll
+        for (int u = 0; u < kSgKeys; u++) {
+            if (writer && xb + u * kSgWarps == n_keys - 1) {
+                kq[u] = 4 * lane < dim ? *reinterpret_cast<const float4 *>(ks + 4 * lane) : zero;
+                vq[u] = 4 * lane < vdim ? *reinterpret_cast<const float4 *>(vs + 4 * lane) : zero;
+            }
+#pragma unroll
+            for (int h = 0; h < kSgHeads; h++)
+                s[h * kSgKeys + u] = q4[h].x * kq[u].x + q4[h].y * kq[u].y + q4[h].z * kq[u].z + q4[h].w * kq[u].w;
+        }
+        /* 32 sums over the lanes by halving: lane i is left with sum i */
+#pragma unroll
+        for (int n = 16; n > 0; n >>= 1) {
+            const bool up = (lane & n) != 0;
+#pragma unroll
+            for (int i = 0; i < n; i++) {
+                const float send = up ? s[i] : s[i + n], keep = up ? s[i + n] : s[i];
+                s[i] = keep + __shfl_xor_sync(0xffffffffu, send, n);
+            }
+        }
+        float e = s[0] * a.scale;
+        if (a.softcap > 0.0f) e = a.softcap * tanhf(e / a.softcap);
+        if (xb + (lane % kSgKeys) * kSgWarps >= x1) e = -INFINITY;
+        float top = e;
+#pragma unroll
+        for (int n = kSgKeys / 2; n > 0; n >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, n));
+        const float now = fmaxf(mx, top), c = expf(mx - now), w = expf(e - now);      /* the first key of a pass is always there: finite */
+        float sum = w;
+#pragma unroll
+        for (int n = kSgKeys / 2; n > 0; n >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, n);
+        den = den * c + sum;
+        mx = now;
+#pragma unroll
+        for (int h = 0; h < kSgHeads; h++) {
+            const float ch = __shfl_sync(0xffffffffu, c, h * kSgKeys);
+            o[h].x *= ch; o[h].y *= ch; o[h].z *= ch; o[h].w *= ch;
+#pragma unroll
+            for (int u = 0; u < kSgKeys; u++) {
+                const float wu = __shfl_sync(0xffffffffu, w, h * kSgKeys + u);
+                o[h].x = fmaf(wu, vq[u].x, o[h].x); o[h].y = fmaf(wu, vq[u].y, o[h].y);
+                o[h].z = fmaf(wu, vq[u].z, o[h].z); o[h].w = fmaf(wu, vq[u].w, o[h].w);
+            }
+        }
+        xb += kSgKeys * kSgWarps;
+        if (xb < x1) fetch(xb);
+    }
+#pragma unroll
+    for (int h = 0; h < kSgHeads; h++) *reinterpret_cast<float4 *>(&warp_o[warp][h][4 * lane]) = o[h];
+    if (lane % kSgKeys == 0) warp_ml[warp][lane / kSgKeys] = make_float2(mx, den);
+    __syncthreads();
+
+    /* the warps' results, to the CTA that merges these columns: thread = (head, pair of columns) */
+    const int share = kSgThreads / S;
+    {
+        const int h = tid / (kSgDim / 2), d = tid % (kSgDim / 2);
+        float M0 = -INFINITY, L = 0.0f;
+        float2 O = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < kSgWarps; u++) M0 = fmaxf(M0, warp_ml[u][h].x);
+#pragma unroll
+        for (int u = 0; u < kSgWarps; u++) {
+            const float2 ml = warp_ml[u][h], v = *reinterpret_cast<const float2 *>(&warp_o[u][h][2 * d]);
+            const float f = ml.x > -INFINITY ? expf(ml.x - M0) : 0.0f;
+            L = fmaf(ml.y, f, L);
+            O.x = fmaf(v.x, f, O.x);
+            O.y = fmaf(v.y, f, O.y);
+        }
+        uint32_t to, bar;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(vb_smem_u32(&slices[sp * share + tid % share])), "r"(tid / share));
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(vb_smem_u32(&arrived)), "r"(tid / share));
+        asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(to),
+                     "r"(__float_as_uint(O.x)), "r"(__float_as_uint(O.y)), "r"(__float_as_uint(M0)), "r"(__float_as_uint(L)), "r"(bar)
+                     : "memory");
+    }
+    /* a CTA ends only when it has received everything: nothing is sent to shared memory that is gone */
+    if (!vb_mbar_wait(&arrived, 0u, &gave_up)) {
+        atomicCAS(a.status, 0, 53);
+        gave_up = 1;
+        return;
+    }
+    const int i = sp * share + tid, h = i / (kSgDim / 2), c = 2 * (i % (kSgDim / 2));
+    if (tid < share && h < group && c < vdim) {
+        float2 O = make_float2(0.f, 0.f);
+        float M0 = -INFINITY, L = 0.0f;
+        for (int u = 0; u < S; u++) M0 = fmaxf(M0, slices[u * share + tid].z);
+        for (int u = 0; u < S; u++) {
+            const float4 e = slices[u * share + tid];
+            const float f = e.z > -INFINITY ? expf(e.z - M0) : 0.0f;
+            L = fmaf(e.w, f, L);
+            O.x = fmaf(e.x, f, O.x);
+            O.y = fmaf(e.y, f, O.y);
+        }
+        lm_put(a.out, 0, (g * group + h) * vdim + c, O.x / L);
+        lm_put(a.out, 0, (g * group + h) * vdim + c + 1, O.y / L);
+    }
+}
+
 /* ------------------------------------------------------------------ prompts on the tensor cores (vb_attn_tc.cuh) */
 /* Rows of a value tile beyond its keys: their weights are zero, and so must they be. */
 template <int BLOCKS>
@@ -853,6 +1098,12 @@ bool lm_attn_step_ok(const LmAttn &a) {
 
 int lm_attn_step(const LmAttn &a, cudaStream_t st) {
     const int group = a.heads / a.kv_heads;
+    if (group <= kSgHeads && a.dim <= kSgDim && a.vdim <= kSgDim) {
+        int splits = kSgSplits;                  /* as long as a CTA finds an SM of its own */
+        while (splits > 1 && splits * a.kv_heads > kStepCtas) splits /= 2;
+        return ok(launch_pdl_cluster(a.split ? lm_attn_step_group_kernel<true> : lm_attn_step_group_kernel<false>, splits, dim3(splits, a.kv_heads),
+                                     dim3(kSgThreads), 0, st, a));
+    }
     int lanes_h = 1;
     while (lanes_h < group) lanes_h *= 2;
     int splits = kStepCtas / a.kv_heads;

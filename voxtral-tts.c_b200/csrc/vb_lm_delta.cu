@@ -564,22 +564,23 @@ __global__ void __launch_bounds__(kStThreads) lm_delta_step_kernel(const LmDelta
     __shared__ float qs[kStWarps * NR], ks[kStWarps * NR], vs[kStCols], red[2][kStWarps], part[2][kStWarps][kStCols], scal[2], ssq;
     namespace cg = cooperative_groups;
     pdl_launch_dependents();
-    pdl_wait();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int h = blockIdx.y, group = a.heads / a.kv_heads, kv = h / group, H = a.heads;
     const int col0 = blockIdx.x * kStCols, c = col0 + lane;
     const bool live = c < a.vdim;
-    const int pos = a.dyn->pos, nqk = a.kv_heads * a.dim, ch = 2 * nqk + H * a.vdim;
-    float *S = lm_state(a.s, a.dyn) + (size_t)h * a.dim * a.vdim;
-    float *tail = lm_state(a.tail, a.dyn);
+    const int pos = __ldcg(&a.dyn->pos), slot = __ldcg(&a.dyn->slot), nqk = a.kv_heads * a.dim, ch = 2 * nqk + H * a.vdim;
+    float *S = a.s.base + (size_t)slot * a.s.slab + (size_t)h * a.dim * a.vdim;
+    float *tail = a.tail.base + (size_t)slot * a.tail.slab;
 
-    /* the state is requested first: it is the long way */
+    /* The state is requested before the wait for the projection: earlier steps left it, and are complete (a step's first
+     * kernel is a plain launch). 8.7 us a token of 24 heads of 128 with it behind the wait. */
     float s[NR];
 #pragma unroll
     for (int i = 0; i < NR; i++) {
         const int r = warp + kStWarps * i;
         s[i] = (pos > 0 && live && r < a.dim) ? __ldcg(S + (size_t)r * a.vdim + c) : 0.0f;
     }
+    pdl_wait();
     float gate = 0.0f;
     if (warp == 0 && live) gate = lm_sum_batch(a.in, 0, ch + h * a.vdim + c);
     if (warp == 1 && lane < 2) {

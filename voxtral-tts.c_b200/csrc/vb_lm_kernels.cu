@@ -274,19 +274,26 @@ int lm_residual(const LmResidual &a, int M, cudaStream_t st) {
     const bool many = M > 296 && v4 && groups > 256 && groups <= 1024;
     const int threads = many ? 256 : groups >= 1024 ? 1024 : (groups + 31) / 32 * 32, nv = (groups + threads - 1) / threads;
     const dim3 g(M), b(threads);
+    /* The first launch of a step is a plain one: kernels behind it may read what earlier steps left without waiting for
+     * their own predecessor. */
+    auto go = [&](void (*kernel)(const LmResidual)) {
+        if (!a.first) return ok(launch_pdl(kernel, g, b, 0, st, a));
+        kernel<<<g, b, 0, st>>>(a);
+        return ok(cudaGetLastError());
+    };
     if (many) {
-        if (nv <= 2) return ok(launch_pdl(lm_residual_kernel<4, 2, true>, g, b, 0, st, a));
-        if (nv <= 3) return ok(launch_pdl(lm_residual_kernel<4, 3, true>, g, b, 0, st, a));
-        return ok(launch_pdl(lm_residual_kernel<4, 4, true>, g, b, 0, st, a));
+        if (nv <= 2) return go(lm_residual_kernel<4, 2, true>);
+        if (nv <= 3) return go(lm_residual_kernel<4, 3, true>);
+        return go(lm_residual_kernel<4, 4, true>);
     }
     if (v4) {
-        if (nv <= 1) return ok(launch_pdl(lm_residual_kernel<4, 1, false>, g, b, 0, st, a));
-        if (nv <= 2) return ok(launch_pdl(lm_residual_kernel<4, 2, false>, g, b, 0, st, a));
-        if (nv <= 4) return ok(launch_pdl(lm_residual_kernel<4, 4, false>, g, b, 0, st, a));
+        if (nv <= 1) return go(lm_residual_kernel<4, 1, false>);
+        if (nv <= 2) return go(lm_residual_kernel<4, 2, false>);
+        if (nv <= 4) return go(lm_residual_kernel<4, 4, false>);
     } else {
-        if (nv <= 1) return ok(launch_pdl(lm_residual_kernel<1, 1, false>, g, b, 0, st, a));
-        if (nv <= 4) return ok(launch_pdl(lm_residual_kernel<1, 4, false>, g, b, 0, st, a));
-        if (nv <= 16) return ok(launch_pdl(lm_residual_kernel<1, 16, false>, g, b, 0, st, a));
+        if (nv <= 1) return go(lm_residual_kernel<1, 1, false>);
+        if (nv <= 4) return go(lm_residual_kernel<1, 4, false>);
+        if (nv <= 16) return go(lm_residual_kernel<1, 16, false>);
     }
     return -1;
 }
