@@ -277,7 +277,7 @@ int lm_residual(const LmResidual &a, int M, cudaStream_t st) {
     /* The first launch of a step is a plain one: kernels behind it may read what earlier steps left without waiting for
      * their own predecessor. */
     auto go = [&](void (*kernel)(const LmResidual)) {
-        if (!a.first) return ok(launch_pdl(kernel, g, b, 0, st, a));
+        if (!a.first && !a.plain) return ok(launch_pdl(kernel, g, b, 0, st, a));
         kernel<<<g, b, 0, st>>>(a);
         return ok(cudaGetLastError());
     };

@@ -155,6 +155,7 @@ struct LmResidual {
     float *x;                    /* [M][width] residual stream, in and out */
     const int *row_of;           /* optional: output row m takes row row_of[m] of part and x (x is then not stored) */
     float *tap;                  /* optional copy of the new x, [M][width] */
+    bool plain;                  /* an ordinary launch: it follows two streams */
     int next;                    /* LmNext: what goes to the sink */
     const float *next_gain;      /* LM_NEXT_NORM */
     LmSink sink;
