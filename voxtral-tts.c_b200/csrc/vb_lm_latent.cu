@@ -72,9 +72,18 @@ __global__ void __launch_bounds__(kLpThreads, ONE ? 3 : 1) lm_latent_prepare_ker
     extern __shared__ __align__(16) float lp[];
     __shared__ float red[2][kLpWarps];
     pdl_launch_dependents();
-    pdl_wait();
     const int threads = blockDim.x, warps = threads >> 5;
     const int m = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    /* Few rows: position, angle and gains before the wait (earlier steps are complete: a step's first kernel is a plain
+     * launch). One token, 6.3 us with them behind it. */
+    const int pos = __ldcg(&a.dyn->pos) + m, half = a.rot / 2;
+    float cos0 = 0.0f, sin0 = 0.0f;
+    float4 gain0 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!ONE && blockIdx.y == 0) {
+        if (tid < half) lm_angle(pos, a.freq[tid], a.freq[half + tid], a.mag, &cos0, &sin0);
+        if ((a.q_rank & 3) == 0 && tid * 4 < a.q_rank) gain0 = __ldg(reinterpret_cast<const float4 *>(a.q_gain + tid * 4));
+    }
+    pdl_wait();
     auto sum4 = [&](int c) { return ONE ? vb_ldcg4(a.in.p + (size_t)m * a.in.ld + c) : lm_sum4(a.in, m, c); };
     auto sum1 = [&](int c) { return ONE ? vb_ldcg(a.in.p + (size_t)m * a.in.ld + c) : lm_sum_batch(a.in, m, c); };
     if (blockIdx.y > 0) {
@@ -91,13 +100,12 @@ __global__ void __launch_bounds__(kLpThreads, ONE ? 3 : 1) lm_latent_prepare_ker
         }
         return;
     }
-    const int half = a.rot / 2, row = a.rank + a.rot_dim, nq = up4(a.q_rank), nc = a.c_gain ? up4(row) : 0;
+    const int row = a.rank + a.rot_dim, nq = up4(a.q_rank), nc = a.c_gain ? up4(row) : 0;
     float *ql = lp, *cl = ql + nq, *z = cl + nc, *cs = z + a.experts;
-    const int pos = a.dyn->pos + m;
     auto angles = [&]() {
         for (int i = tid; i < half; i += threads) {
-            float c, s;
-            lm_angle(pos, a.freq[i], a.freq[half + i], a.mag, &c, &s);
+            float c = cos0, s = sin0;
+            if (ONE || i != tid) lm_angle(pos, a.freq[i], a.freq[half + i], a.mag, &c, &s);
             cs[i] = c;
             cs[half + i] = s;
             a.cs[(size_t)m * a.rot + i] = c;
@@ -134,7 +142,7 @@ __global__ void __launch_bounds__(kLpThreads, ONE ? 3 : 1) lm_latent_prepare_ker
     const float rq = 1.0f / sqrtf(sq / (float)a.q_rank + a.eps), rc = 1.0f / sqrtf(sc / (float)a.rank + a.eps);
     if ((a.q_rank & 3) == 0) {
         for (int c = tid * 4; c < a.q_rank; c += threads * 4) {
-            const float4 g = __ldg(reinterpret_cast<const float4 *>(a.q_gain + c));
+            const float4 g = !ONE && c == tid * 4 ? gain0 : __ldg(reinterpret_cast<const float4 *>(a.q_gain + c));
             const float e[4] = {ql[c] * rq * g.x, ql[c + 1] * rq * g.y, ql[c + 2] * rq * g.z, ql[c + 3] * rq * g.w};
             lm_put4(a.q_latent, m, c, e);
         }
@@ -257,8 +265,8 @@ inline int attend_splits(int M, int heads) {
 
 /* Key tiles of pairs p0 .. p0 + np - 1 (pair = row * heads + head). */
 template <int KT>
-VB_DEVINL KeyTiles pair_tiles(const LmLatent &a, int M, int p0, int *np) {
-    const int P = M * a.heads, pos0 = a.dyn->pos;
+VB_DEVINL KeyTiles pair_tiles(const LmLatent &a, int pos0, int M, int p0, int *np) {
+    const int P = M * a.heads;
     *np = P - p0 < kLaPairs ? P - p0 : kLaPairs;
     return key_tiles<KT>(pos0 + p0 / a.heads, pos0 + (p0 + *np - 1) / a.heads, a.window, 0);
 }
@@ -309,26 +317,26 @@ __global__ void __launch_bounds__(kLaThreads) lm_latent_attend_kernel(const LmLa
         const int rr = isq ? r % kLaPairs : k % kLaKeys;
         for (int c = per + lane; c < chunks; c += 32) *reinterpret_cast<uint4 *>(plane + swz(rr, c)) = make_uint4(0u, 0u, 0u, 0u);
     }
-    pdl_wait();
     int np;
-    const int p0 = blockIdx.x * kLaPairs, sp = blockIdx.y;
-    const KeyTiles kt = pair_tiles<kLaKeys>(a, M, p0, &np);
+    const int p0 = blockIdx.x * kLaPairs, sp = blockIdx.y, pos0 = __ldcg(&a.dyn->pos), P = M * a.heads;
+    const KeyTiles kt = pair_tiles<kLaKeys>(a, pos0, M, p0, &np);
     const int S_eff = (int)gridDim.y < kt.n_tiles ? (int)gridDim.y : kt.n_tiles;
     if (sp >= S_eff) return;
     const int t0 = (int)((long long)kt.n_tiles * sp / S_eff), t1 = (int)((long long)kt.n_tiles * (sp + 1) / S_eff);
-    const int pos0 = a.dyn->pos, P = M * a.heads;
-    const float *cache = lm_state(a.kv, a.dyn);
-    auto request = [&](int t) {
+    const float *cache = a.kv.base + (size_t)__ldcg(&a.dyn->slot) * a.kv.slab;
+    auto request = [&](int t, bool old, bool now) {          /* rows of earlier steps, of this one */
         int j0, n;
         key_tile<kLaKeys>(kt, t, &j0, &n);
         unsigned char *b = Kb + (stages == 2 ? (t & 1) : 0) * 2 * k_plane;
         for (int key = warp; key < n; key += kLaWarps) {
+            if (j0 + key < pos0 ? !old : !now) continue;
             const uint16_t *src = reinterpret_cast<const uint16_t *>(cache + (size_t)lm_ring_row(a.ring, j0 + key) * row);
             for (int f = lane; f < 2 * per; f += 32) {
                 const int plane = f >= per ? 1 : 0;
                 lm_cp16(b + plane * k_plane + swz(key, f - plane * per), src + f * 8);
             }
         }
+        if (!now) return;
         /* beyond the last key: weights of zero must not meet what an earlier launch left */
         for (int key = n + warp; key < kLaKeys; key += kLaWarps)
             for (int f = lane; f < 2 * per; f += 32) {
@@ -337,7 +345,10 @@ __global__ void __launch_bounds__(kLaThreads) lm_latent_attend_kernel(const LmLa
             }
         lm_cp_commit();
     };
-    request(t0);
+    /* what earlier steps left is complete (a step's first kernel is a plain launch): requested before the wait */
+    request(t0, true, false);
+    pdl_wait();
+    request(t0, false, true);
     for (int p = warp; p < kLaPairs; p += kLaWarps) {
         const float *q = a.ql + (size_t)(p0 + p) * row;
         for (int chunk = lane; chunk < per; chunk += 32) {
@@ -367,11 +378,11 @@ __global__ void __launch_bounds__(kLaThreads) lm_latent_attend_kernel(const LmLa
         key_tile<kLaKeys>(kt, t, &j0, &n);
         if (stages == 1 && t > t0) {
             __syncthreads();
-            request(t);
+            request(t, true, true);
         }
         lm_cp_wait_all();
         __syncthreads();
-        if (stages == 2 && t + 1 < t1) request(t + 1);
+        if (stages == 2 && t + 1 < t1) request(t + 1, true, true);
         const uint32_t sK = vb_smem_u32(Kb + (stages == 2 ? (t & 1) : 0) * 2 * k_plane);
         float s0[4] = {}, s1[4] = {}, s2[4] = {};
 #pragma unroll 4
@@ -474,7 +485,7 @@ __global__ void __launch_bounds__(kLtThreads) lm_latent_attend_f32_kernel(const 
     int np;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int p0 = blockIdx.x * kLaPairs, sp = blockIdx.y, row = a.rank + a.rot_dim, pos0 = a.dyn->pos, P = M * a.heads;
-    const KeyTiles kt = pair_tiles<KT>(a, M, p0, &np);
+    const KeyTiles kt = pair_tiles<KT>(a, a.dyn->pos, M, p0, &np);
     const int S_eff = (int)gridDim.y < kt.n_tiles ? (int)gridDim.y : kt.n_tiles;
     if (sp >= S_eff) return;
     const int t0 = (int)((long long)kt.n_tiles * sp / S_eff), t1 = (int)((long long)kt.n_tiles * (sp + 1) / S_eff);
@@ -557,13 +568,32 @@ __global__ void __launch_bounds__(kLtThreads) lm_latent_readout_kernel(const LmL
 #pragma unroll
     for (int i = 0; i < kPre; i++)
         pre[i] = i < kblocks ? __ldg(reinterpret_cast<const uint4 *>(lm_weight_row(a.ukv, wrow, i) + c0)) : make_uint4(0u, 0u, 0u, 0u);
+    const int pos0 = __ldcg(&a.dyn->pos);
     pdl_wait();
     const size_t P = (size_t)M * a.heads;
     const float2 *stats = attend_stats(a, splits, (int)P);
+    /* One row: its items' splits are requested before their weights are known, and the gate (6 us a launch with one after
+     * the other, 16 heads of 128 out of 512 columns at 350 keys). */
+    constexpr int kAhead = MR == 1 ? 8 : 1;
+    float4 ahead[kAhead];
+    int parts = 1;
+    const int nv = a.rank / 4, items = nr * nv;
+    while (parts < 8 && items * parts * 2 <= kLtThreads) parts *= 2;
+    if (MR == 1 && (a.rank & 3) == 0) {
+        const float *from = a.scratch + ((size_t)m0 * a.heads + h) * a.rank + (tid / parts < items ? tid / parts * 4 : 0);
+#pragma unroll
+        for (int k = 0; k < kAhead; k++) {
+            const int u = tid % parts + k * parts;
+            ahead[k] = u < splits ? vb_ldcg4(from + u * P * a.rank) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    float gate[MR];
+#pragma unroll
+    for (int r = 0; r < MR; r++) gate[r] = r < nr ? __ldcg(a.gate + (size_t)(m0 + r) * a.heads + h) : 0.0f;
     if (warp < nr) {
         const int p = (m0 + warp) * a.heads + h;
         int np;
-        const KeyTiles kt = pair_tiles<KT>(a, M, p / kLaPairs * kLaPairs, &np);
+        const KeyTiles kt = pair_tiles<KT>(a, pos0, M, p / kLaPairs * kLaPairs, &np);
         const int S = splits < kt.n_tiles ? splits : kt.n_tiles;
         float2 st[2];
         float mu[2], top = -INFINITY, L = 0.0f;
@@ -589,9 +619,6 @@ __global__ void __launch_bounds__(kLtThreads) lm_latent_readout_kernel(const LmL
     if ((a.rank & 3) == 0) {
         /* four columns per item; where there are few items, neighbouring lanes share one and take every second,
          * fourth, ... split */
-        const int nv = a.rank / 4, items = nr * nv;
-        int parts = 1;
-        while (parts < 8 && items * parts * 2 <= kLtThreads) parts *= 2;
         for (int i0 = 0; i0 < items; i0 += kLtThreads / parts) {
             const int i = i0 + tid / parts, part = tid % parts;
             const bool in = i < items;
@@ -599,8 +626,17 @@ __global__ void __launch_bounds__(kLtThreads) lm_latent_readout_kernel(const LmL
             const float *s = a.scratch + ((size_t)(m0 + r) * a.heads + h) * a.rank + c;
             const int S = in ? count[r] : 0;
             float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+            int u0 = part;
+            if (MR == 1 && i0 == 0) {
+#pragma unroll
+                for (int k = 0; k < kAhead; k++, u0 += parts) {
+                    if (u0 >= S) continue;
+                    const float w = wgt[r][u0];
+                    o.x = fmaf(w, ahead[k].x, o.x); o.y = fmaf(w, ahead[k].y, o.y); o.z = fmaf(w, ahead[k].z, o.z); o.w = fmaf(w, ahead[k].w, o.w);
+                }
+            }
 #pragma unroll 8
-            for (int u = part; u < S; u += parts) {
+            for (int u = u0; u < S; u += parts) {
                 const float4 t = vb_ldcg4(s + u * P * a.rank);
                 const float w = wgt[r][u];
                 o.x = fmaf(w, t.x, o.x); o.y = fmaf(w, t.y, o.y); o.z = fmaf(w, t.z, o.z); o.w = fmaf(w, t.w, o.w);
@@ -645,7 +681,7 @@ __global__ void __launch_bounds__(kLtThreads) lm_latent_readout_kernel(const LmL
 #pragma unroll
         for (int off = 4; off > 0; off >>= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], off);
         if (r < nr && (lane & 7) == 0 && v < a.vdim)
-            lm_put(a.out, m0 + r, h * a.vdim + v, acc[r] * a.gate[(size_t)(m0 + r) * a.heads + h]);
+            lm_put(a.out, m0 + r, h * a.vdim + v, acc[r] * gate[r]);
     }
 }
 
