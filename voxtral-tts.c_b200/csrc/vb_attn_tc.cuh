@@ -20,7 +20,9 @@
  * What bounds it, by a timeline on the device: the S products, 24 MMAs of 64 columns a tile at 77 clocks (36 of 65 for
  * heads of 192), which is what MMAs of 128 columns take too, then P . V, 12 at 60; 3300 and 4000 clocks a tile. 2048 rows,
  * window 1024, 32 heads: 128 on 8 KV heads 588 us on warp-level MMAs (mma.sync, 16 rows a warp, 44 useful TFLOP/s), 201 with
- * tiles copied 16 bytes a lane, 164 now; 192 + 128 each with its own 830, 282, 225 us.
+ * tiles copied 16 bytes a lane, 164 by TMA; 192 + 128 each with its own 830, 282, 225 us. Short prompts see what comes before
+ * and after the tiles: 58 rows of the speech decoder 17.8 us with queries and results moved a row at a time, 13.1 now, 1203
+ * rows 78.6 -> 66.6, 2048 rows of a language model with window and softcap 175 -> 158.
  */
 #ifndef VB_ATTN_TC_CUH
 #define VB_ATTN_TC_CUH
@@ -35,7 +37,6 @@ constexpr int kAtSoft = 256, kAtLoadK = 128, kAtLoadV = 64, kAtThreads = kAtSoft
 constexpr int kAtMmaWarp = (kAtThreads - 32) / 32;
 constexpr int kAtBlock = kAtKeys * 128;            /* 64 keys x 64 columns */
 constexpr int kAtStatus = 52;
-constexpr int kAtStage = 12;                       /* words of a row in a softmax warp's staging of the queries: 8 columns, and 16 bytes on */
 constexpr uint32_t kAtTmemCols = 512, kAtO = 128, kAtQ = 384;
 
 /* What every use has in common. */
@@ -57,7 +58,10 @@ struct AtCfg {
     static constexpr int kSlots = DK <= 2 ? 3 : 2;
     static constexpr int kSlotK = 2 * DK * kAtBlock, kSlotV = 2 * DV * kAtBlock;
     static constexpr int kQl = kQlTmem ? 0 : DK * kAtRows * 128;
-    static constexpr int kSmem = kQl + kSlots * (kSlotK + kSlotV) + 1024 + 256 + 8 * 32 * kAtStage * 4;
+    static constexpr int kSmem = kQl + kSlots * (kSlotK + kSlotV) + 1024 + 256;
+    /* 16-column steps of the queries that a warp has on their way at once (of 2 * DK): 8 or 16 loads of 16 bytes a lane */
+    static constexpr int kQBatch = DK <= 2 ? 2 * DK : 2;
+    static_assert(2 * DK % kQBatch == 0, "whole batches");
     static_assert(kSmem <= 232448, "over the 227 KB a CTA may use");
     static_assert(kAtQ + (kQlTmem ? 2 : 1) * DK * 32 <= kAtTmemCols, "Q does not fit TMEM");
 };
@@ -110,11 +114,9 @@ VB_DEVINL void at_st32(uint32_t taddr, const uint32_t (&r)[32]) {
         ::VB_AT_R8(r, 0), VB_AT_R8(r, 8), VB_AT_R8(r, 16), VB_AT_R8(r, 24), "r"(taddr)
         : "memory");
 }
-VB_DEVINL void at_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
-        ::VB_AT_R8(r, 0), VB_AT_R8(r, 8), "r"(taddr)
-        : "memory");
+/* 8 columns of 16 TMEM lanes: lane l of the warp has columns 2 (l % 4) and on of rows l / 4 (a, b) and l / 4 + 8 (c, d) */
+VB_DEVINL void at_st_16x8(uint32_t taddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x1.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 VB_DEVINL void at_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 VB_DEVINL void at_proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -178,6 +180,7 @@ VB_DEVINL uint32_t at_off(int row, int chunk) { return (uint32_t)(row * 128 + ((
  *   tma_keys(...) / tma_values(...)   request a tile by TMA: where AtArgs says so and boxes(j0, n) does, or always (kBoxes:
  *                                what lies beyond the last key is zeros)
  *   start()                      after the wait for the previous kernel: resolves what lies in device memory
+ *   here()                       what of it this block is to use
  *   rows(a)                      how many there are: a launch may serve several prompts (blockIdx.z), a.M the most of one
  *   pos0()                       position of row 0
  *   q4(row, head, d)             four query values (zeros beyond the head)
@@ -186,7 +189,7 @@ VB_DEVINL uint32_t at_off(int row, int chunk) { return (uint32_t)(row * 128 + ((
  *   gate(row, head)              factor of a result row
  *   put4(row, column, v)         four results */
 template <int DK, int DV, class SRC>
-__global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const __grid_constant__ AtMaps maps, const AtArgs a, const SRC src_arg) {
+__global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const __grid_constant__ AtMaps maps, const AtArgs a, const __grid_constant__ SRC src_arg) {
     using Cfg = AtCfg<DK, DV>;
     extern __shared__ unsigned char at_smem_raw[];
     unsigned char *base = (unsigned char *)(((uintptr_t)at_smem_raw + 1023) & ~(uintptr_t)1023);
@@ -198,7 +201,9 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const __grid_
     int *abort_flag = (int *)(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int group = a.heads / a.kv_heads, g = blockIdx.x, pairs = src_arg.rows(a) * group;
+    const int group = a.heads / a.kv_heads, g = blockIdx.x;
+    auto src = src_arg.here();
+    const int pairs = src.rows(a) * group;
     const int P0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kAtRows;           /* the latest rows see the most keys: they go first */
     if (P0 >= pairs) return;                                                   /* a shorter prompt beside a longer one */
     if (tid == 0) {
@@ -227,9 +232,29 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const __grid_
     tc_fence_after();
     const uint32_t tmem = *(volatile uint32_t *)tmem_slot;
     pdl_launch_dependents();       /* not before the allocation: a GEMM that starts early must not take columns this kernel needs */
+    /* The queries of a softmax warp's 32 rows, 16 columns a step, the steps in turn by the two warpgroups. Four lanes read 64
+     * bytes of a row, which is how a 16 x 8 TMEM store wants them; the loads of a batch are all on their way before the first
+     * is used; rows past the end repeat the last one. (Two lanes a row, 32 columns at a time, by way of shared memory to the
+     * lane that owns the row: 8000 clocks from the wait to queries in place for 128 x 128, 2200 to 3500 now.) */
+    constexpr bool kEarly = DK <= 2;            /* one batch: before what start() fetches (in two places 147 us, not 138, for heads of 192) */
+    const int w_q = warp >> 2, d_q = (lane & 3) * 4;
+    int qrow[4], qhead[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int x = P0 + (warp & 3) * 32 + (lane >> 2) + 8 * i;
+        qrow[i] = (x < pairs ? x : pairs - 1) / group;
+        qhead[i] = g * group + (x < pairs ? x : pairs - 1) - qrow[i] * group;
+    }
+    float4 qv[Cfg::kQBatch][4];
+    auto q_load = [&](int batch) {
+#pragma unroll
+        for (int u = 0; u < Cfg::kQBatch; u++)
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                qv[u][i] = src.q4(qrow[i], qhead[i], ((batch * Cfg::kQBatch + u) * 2 + w_q) * 16 + d_q);
+    };
     pdl_wait();
-
-    SRC src = src_arg;
+    if (kEarly && warp < 8) q_load(0);
     src.start();
     const int pos0 = src.pos0();
     const int last = P0 + kAtRows < pairs ? P0 + kAtRows - 1 : pairs - 1;
@@ -248,53 +273,36 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const __grid_
         const bool valid = P < pairs;
         const int row = valid ? P / group : 0, head = g * group + (valid ? P - row * group : 0), i = pos0 + row;
         const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16, tS = tmem + lanes + (uint32_t)(w * kAtKeys), tO = tmem + lanes + kAtO + (uint32_t)(w * 128);
-        /* The query rows, 32 columns in turn by the two warpgroups: two lanes read 32 bytes of a row (a lane per row reads 32
-         * rows at once: 18 us for 128 x 192), which then move to the lane that owns the row; halves to TMEM, low ones of
-         * large heads to shared memory. */
-        uint32_t *stage = reinterpret_cast<uint32_t *>((unsigned char *)bars + 256) + warp * 32 * kAtStage;
-        int qrow[2], qhead[2];
-#pragma unroll
-        for (int i2 = 0; i2 < 2; i2++) {
-            const int x = P0 + (warp & 3) * 32 + (lane >> 1) + 16 * i2;
-            qrow[i2] = x < pairs ? x / group : -1;
-            qhead[i2] = g * group + (x < pairs ? x - qrow[i2] * group : 0);
-        }
 #pragma unroll 1
-        for (int u = w; u < 2 * DK; u += 2) {
-            uint32_t hi[16], lo[16];
-            float4 v[4][2];
+        for (int batch = 0; batch < 2 * DK / Cfg::kQBatch; batch++) {
+            if (!kEarly || batch > 0) q_load(batch);
 #pragma unroll
-            for (int c = 0; c < 4; c++)
+            for (int u = 0; u < Cfg::kQBatch; u++) {
+                const int step = (batch * Cfg::kQBatch + u) * 2 + w;
+                uint32_t hi[4][2], lo[4][2];
 #pragma unroll
-                for (int i2 = 0; i2 < 2; i2++)
-                    v[c][i2] = qrow[i2] >= 0 ? src.q4(qrow[i2], qhead[i2], u * 32 + c * 8 + (lane & 1) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                __syncwarp();
-#pragma unroll
-                for (int i2 = 0; i2 < 2; i2++) {
-                    float4 e = v[c][i2];
+                for (int i2 = 0; i2 < 4; i2++) {
+                    float4 e = qv[u][i2];
                     if (a.scale <= 0.0f) {             /* the scores are multiplied by |scale| below, or by one */
                         const float f = a.scale < 0.0f ? -1.0f : 0.0f;
                         e = make_float4(e.x * f, e.y * f, e.z * f, e.w * f);
                     }
-                    uint32_t *to = stage + ((lane >> 1) + 16 * i2) * kAtStage + (lane & 1) * 2;
-                    at_split2(e.x, e.y, to[0], to[4]);
-                    at_split2(e.z, e.w, to[1], to[5]);
+                    at_split2(e.x, e.y, hi[i2][0], lo[i2][0]);
+                    at_split2(e.z, e.w, hi[i2][1], lo[i2][1]);
                 }
-                __syncwarp();
-                const uint4 h4 = *reinterpret_cast<const uint4 *>(stage + lane * kAtStage), l4 = *reinterpret_cast<const uint4 *>(stage + lane * kAtStage + 4);
-                hi[c * 4] = h4.x; hi[c * 4 + 1] = h4.y; hi[c * 4 + 2] = h4.z; hi[c * 4 + 3] = h4.w;
-                lo[c * 4] = l4.x; lo[c * 4 + 1] = l4.y; lo[c * 4 + 2] = l4.z; lo[c * 4 + 3] = l4.w;
-            }
-            at_st16(tmem + lanes + kAtQ + (uint32_t)(u * 16), hi);
-            if constexpr (Cfg::kQlTmem) {
-                at_st16(tmem + lanes + kAtQ + (uint32_t)(DK * 32 + u * 16), lo);
-            } else {
 #pragma unroll
-                for (int c = 0; c < 4; c++)
-                    *reinterpret_cast<uint4 *>(ql_s + (u >> 1) * kAtRows * 128 + at_off(r, (u & 1) * 4 + c)) =
-                        make_uint4(lo[c * 4], lo[c * 4 + 1], lo[c * 4 + 2], lo[c * 4 + 3]);
+                for (int h = 0; h < 2; h++) {
+                    const uint32_t to = tmem + lanes + ((uint32_t)(16 * h) << 16) + kAtQ + (uint32_t)(step * 8);
+                    at_st_16x8(to, hi[2 * h][0], hi[2 * h][1], hi[2 * h + 1][0], hi[2 * h + 1][1]);
+                    if constexpr (Cfg::kQlTmem) at_st_16x8(to + DK * 32, lo[2 * h][0], lo[2 * h][1], lo[2 * h + 1][0], lo[2 * h + 1][1]);
+                }
+                if constexpr (!Cfg::kQlTmem) {
+#pragma unroll
+                    for (int i2 = 0; i2 < 4; i2++)
+                        *reinterpret_cast<uint2 *>(ql_s + (step >> 2) * kAtRows * 128 +
+                                                   at_off((warp & 3) * 32 + (lane >> 2) + 8 * i2, (step & 3) * 2 + ((lane & 3) >> 1)) + (lane & 1) * 8) =
+                            make_uint2(lo[i2][0], lo[i2][1]);
+                }
             }
         }
         at_st_wait();
@@ -421,12 +429,26 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const __grid_
             for (int k = 0; k < 32; k += 4) *reinterpret_cast<uint4 *>(rows + r * kLd + c * 32 + k) = make_uint4(oa[k], oa[k + 1], oa[k + 2], oa[k + 3]);
         }
         vb_named_bar(1, kAtSoft);
-        for (int x = warp; x < kAtRows && P0 + x < pairs; x += kAtSoft / 32) {
-            const int m = (P0 + x) / group, hd = g * group + P0 + x - m * group;
-            for (int c = lane * 4; c < a.vdim; c += 128) {
-                const float4 o = *reinterpret_cast<const float4 *>(rows + x * kLd + c);
-                const float v[4] = {o.x, o.y, o.z, o.w};
-                src.put4(m, hd * a.vdim + c, v);
+        /* Two rows of a warp at a time, whose places each lane has worked out for one: a row at a time, with a division each,
+         * took 8700 clocks of a tile of 128 x 128 with three terms, 5500 now, with two 3500 (four or eight rows: more code, no
+         * faster; terms made above, where a thread has 32 values side by side, and copied from there: 1700 clocks more). */
+        constexpr int kWarps = kAtSoft / 32, kAhead = 2;
+        const int my_pair = P0 + warp + kWarps * (lane % (kAtRows / kWarps)), my_row = my_pair < pairs ? my_pair / group : -1;
+        const int c = lane * 4;
+#pragma unroll 1
+        for (int n = 0; n < kAtRows / kWarps; n += kAhead) {
+            int m[kAhead];
+            float4 o[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; u++) {
+                m[u] = __shfl_sync(0xffffffffu, my_row, n + u);
+                if (c < a.vdim) o[u] = *reinterpret_cast<const float4 *>(rows + (warp + kWarps * (n + u)) * kLd + c);
+            }
+            if (m[0] < 0) break;
+#pragma unroll
+            for (int u = 0; u < kAhead; u++) {
+                const float v[4] = {o[u].x, o[u].y, o[u].z, o[u].w};
+                if (m[u] >= 0 && c < a.vdim) src.put4(m[u], (g * group + P0 + warp + kWarps * (n + u) - m[u] * group) * a.vdim + c, v);
             }
         }
     } else if (warp < kAtMmaWarp) {

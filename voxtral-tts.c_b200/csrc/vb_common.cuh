@@ -184,10 +184,27 @@ VB_DEVINL void vb_split3(float v, uint16_t &t0, uint16_t &t1, uint16_t &t2) {
     t2 = __bfloat16_as_ushort(h2);
 }
 
+/* Two values at once, the first in the low halves: the same terms in half the conversions. */
+VB_DEVINL void vb_split3_pair(float a, float b, uint32_t &t0, uint32_t &t1, uint32_t &t2) {
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(t0) : "f"(b), "f"(a));
+    a -= __uint_as_float(t0 << 16);
+    b -= __uint_as_float(t0 & 0xffff0000u);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(t1) : "f"(b), "f"(a));
+    a -= __uint_as_float(t1 << 16);
+    b -= __uint_as_float(t1 & 0xffff0000u);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(t2) : "f"(b), "f"(a));
+}
 /* The same where a value may be infinite: its low terms are zeros, not NaN. */
 VB_DEVINL void vb_split3_inf(float v, uint16_t &t0, uint16_t &t1, uint16_t &t2) {
     vb_split3(v, t0, t1, t2);
     if ((t0 & 0x7fffu) == 0x7f80u) t1 = t2 = 0;
+}
+/* From here on a value is infinite once rounded to BF16 (halfway between its largest number and 2^128). */
+constexpr float kBf16Inf = 0x1.FFp127f;
+VB_DEVINL void vb_split3_pair_inf(float a, float b, uint32_t &t1, uint32_t &t2) {
+    const uint32_t keep = (fabsf(a) >= kBf16Inf ? 0u : 0xffffu) | (fabsf(b) >= kBf16Inf ? 0u : 0xffff0000u);
+    t1 &= keep;
+    t2 &= keep;
 }
 
 #endif

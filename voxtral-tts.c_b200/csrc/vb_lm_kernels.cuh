@@ -93,15 +93,19 @@ VB_DEVINL void lm_put(const LmSink &s, int m, int c, float v) {
 
 /* Four columns from c on (a multiple of 4; rows are padded to multiples of 64). */
 VB_DEVINL void lm_put4(const LmSink &s, int m, int c, const float (&v)[4]) {
-    uint16_t t[3][4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) vb_split3_inf(v[i], t[0][i], t[1][i], t[2][i]);
+    uint32_t t[3][2];
+    vb_split3_pair(v[0], v[1], t[0][0], t[1][0], t[2][0]);
+    vb_split3_pair(v[2], v[3], t[0][1], t[1][1], t[2][1]);
+    if (fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))) >= kBf16Inf) {
+        vb_split3_pair_inf(v[0], v[1], t[1][0], t[2][0]);
+        vb_split3_pair_inf(v[2], v[3], t[1][1], t[2][1]);
+    }
     uint16_t *o = s.terms + (size_t)m * s.ld + c;
     const size_t term = (size_t)s.rows_pad * s.ld;
 #pragma unroll
     for (int j = 0; j < 3; j++)
         if (j < s.n_terms)
-            *reinterpret_cast<uint2 *>(o + j * term) = make_uint2(t[j][0] | ((uint32_t)t[j][1] << 16), t[j][2] | ((uint32_t)t[j][3] << 16));
+            *reinterpret_cast<uint2 *>(o + j * term) = make_uint2(t[j][0], t[j][1]);
 }
 
 /* State of one layer run: `base` + slot * `slab` floats. */

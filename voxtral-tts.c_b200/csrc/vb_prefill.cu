@@ -139,23 +139,21 @@ __global__ void pf_qkv_finish_kernel(float *qkv, const float *part, int n_part, 
 
 /* Causal attention of prompt rows over the cache prefix (tts_causal_attention, voxtral_tts_kernels.c:403-465) on the
  * tensor cores (vb_attn_tc.cuh). */
-struct AtRows {
+struct AtPrompt {
     static constexpr bool kBoxes = true;
     const float *q;
     LmSink out;                  /* the terms that the O projection reads */
     int ldq;
-    struct { int row0, rows, pos, key0; } s[kPfSegs];      /* blockIdx.z chooses: PfSeg */
+    struct Seg { int row0, rows, pos, key0; } at;          /* PfSeg */
     VB_DEVINL void start() {}
-    VB_DEVINL int rows(const AtArgs &) const { return s[blockIdx.z].rows; }
-    VB_DEVINL int pos0() const { return s[blockIdx.z].pos; }
-    VB_DEVINL float4 q4(int row, int head, int d) const {
-        return vb_ldcg4(q + (size_t)(s[blockIdx.z].row0 + row) * ldq + head * VB200_HEAD_DIM + d);
-    }
+    VB_DEVINL int rows(const AtArgs &) const { return at.rows; }
+    VB_DEVINL int pos0() const { return at.pos; }
+    VB_DEVINL float4 q4(int row, int head, int d) const { return vb_ldcg4(q + (size_t)(at.row0 + row) * ldq + head * VB200_HEAD_DIM + d); }
     VB_DEVINL bool boxes(int, int) const { return true; }
     template <int BLOCKS>
     VB_DEVINL void box(const CUtensorMap *map, unsigned char *slot, int g, int j0, uint64_t *bar) const {
 #pragma unroll
-        for (int b = 0; b < 2 * BLOCKS; b++) at_tma(slot + b * kAtBlock, map, (g * 2 * BLOCKS + b) * 64, s[blockIdx.z].key0 + j0, 0, bar);
+        for (int b = 0; b < 2 * BLOCKS; b++) at_tma(slot + b * kAtBlock, map, (g * 2 * BLOCKS + b) * 64, at.key0 + j0, 0, bar);
     }
     template <int BLOCKS>
     VB_DEVINL void tma_keys(const AtArgs &, const AtMaps &m, unsigned char *slot, int g, int j0, uint64_t *bar) const {
@@ -166,7 +164,16 @@ struct AtRows {
         box<BLOCKS>(&m.v, slot, g, j0, bar);
     }
     VB_DEVINL float gate(int, int) const { return 1.0f; }
-    VB_DEVINL void put4(int row, int c, const float (&e)[4]) const { lm_put4(out, s[blockIdx.z].row0 + row, c, e); }
+    VB_DEVINL void put4(int row, int c, const float (&e)[4]) const { lm_put4(out, at.row0 + row, c, e); }
+};
+/* Several prompts: blockIdx.z chooses. */
+struct AtRows : AtPrompt {
+    Seg s[kPfSegs];
+    VB_DEVINL AtPrompt here() const {
+        AtPrompt r = *this;
+        r.at = s[blockIdx.z];
+        return r;
+    }
 };
 static_assert(VB200_HEAD_DIM == 128, "two blocks of 64 columns");
 
@@ -309,7 +316,7 @@ static int prefill_block(float *xr, const float *cs, const PfSegs &segs, const P
     if (tc_map3(&maps.k, t.split.k, 1, keys * 4 * KVD, keys, 4 * KVD, 2 * KVD, kAtKeys) ||
         tc_map3(&maps.v, t.split.v, 1, keys * 4 * KVD, keys, 4 * KVD, 2 * KVD, kAtKeys))
         return -1;
-    AtRows rows_of = {t.qkv, {t.bQ, b.rp, QD, b.rp < 256 ? kTcTerms : 2}, QKV, {}};
+    AtRows rows_of = {{t.qkv, {t.bQ, b.rp, QD, b.rp < 256 ? kTcTerms : 2}, QKV, {}}, {}};
     int most = 0;
     for (int i = 0; i < segs.n; i++) {
         rows_of.s[i] = {segs.s[i].row0, segs.s[i].rows, segs.s[i].pos, segs.s[i].key0};
