@@ -5,9 +5,9 @@
  *
  *   lm_attn_prepare  one row per CTA: sums the projection's split-K partials, norms and rotates q
  *                    and k, appends k and v to the cache
- *   lm_attn_generic  fp32 pipes: any sizes, short portions and the 32-bit mode (keys split over CTAs,
- *                    last arrival merges)
- *   lm_attn_step     one token, preparation included
+ *   lm_attn_generic  fp32 pipes: any sizes, short portions and the 32-bit mode; a register tile of query rows and keys
+ *                    a thread (keys split over CTAs, last arrival merges)
+ *   lm_attn_step     one token, preparation included; lm_attn_step_group where a cluster per KV head can take it
  *   lm_attn_mma      prompts: tensor cores on hi + lo BF16 halves of q, k, v and the weights (vb_attn_tc.cuh); the
  *                    cache keeps k and v as such halves
  *

@@ -219,7 +219,7 @@ struct TcTpArgs {
 };
 struct TcNoTpArgs {};
 /* TC_JOIN: see TcJoin. The kernel that added up the partial results of these GEMMs before ("prepare") was a launch of its
- * own, 2 of 7 in a layer: a frame had 350 launches, 264 now; 2.86 -> 2.81 ms. */
+ * own, 2 of 7 in a layer: a frame had 350 launches, 264 after it; 2.86 -> 2.81 ms. */
 enum TcMode { TC_PLAIN = 0, TC_TP = 1, TC_JOIN = 2 };
 template <int MODE> struct TcTpSel { using type = TcNoTpArgs; };
 template <> struct TcTpSel<TC_TP> { using type = TcTpArgs; };

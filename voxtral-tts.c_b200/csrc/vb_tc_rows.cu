@@ -24,7 +24,7 @@
  *
  * Three terms: R <= 128, and the two low terms have a sum of their own, so that the high one is cut off a third as often; the
  * stages keep 40 KB (a k-block costs 512 + 3 R clocks of shared memory, 6 R of the tensor pipe). The epilogue adds a
- * segment up within the time of its main loop down to a single k-block (vb_lm_gemm32.cu has the figures).
+ * segment up within the time of its main loop down to a single k-block (kF32Segment in vb_lm.cu has the figures).
  *
  * Warps: 0-15 epilogue (TMEM -> registers -> shared memory -> whole 512-byte row segments), 16 TMA producer, 17 MMA issuer (of the even
  * CTA, for both). Full barriers and the accumulator hand-back live in the even CTA; commits arrive in both. No
