@@ -37,6 +37,19 @@ def velocity():
     assert np.array_equal(calls(), alone)                                 # the same launches on the same weights
 
 
+def step():
+    """The decoder step needs none of the copies (6 GB), and what it gives does not depend on whether they are there."""
+    eng = pkg.Engine(kv_cache_max=64)
+    eng.upload(pkg.SynthModel(seed=77, dec_layers=1), audio_table=True)
+    x = pkg.synth_f32((9, 3072), 5, "mem.rows", 0.0, 0.5)
+    before = free_bytes()
+    alone = [eng.llm_forward(e, p) for p, e in enumerate(x)]
+    assert before - free_bytes() < 64 * MB, (before, free_bytes())
+    eng.prefill(x, 40)
+    for _ in range(3):                                                    # launches, capture, graph, if it were one
+        assert all(np.array_equal(eng.llm_forward(e, p), a) for p, (e, a) in enumerate(zip(x, alone)))
+
+
 def take(eng, leave):
     """All of the device's memory but `leave` bytes."""
     p = eng.L.tts_cuda_alloc(free_bytes() - leave)
@@ -132,5 +145,5 @@ def blocks():
 
 
 if __name__ == "__main__":
-    {"velocity": velocity, "copies": copies, "far": far, "short": short, "blocks": blocks}[sys.argv[1]]()
+    {"velocity": velocity, "step": step, "copies": copies, "far": far, "short": short, "blocks": blocks}[sys.argv[1]]()
     print("OK")

@@ -1,6 +1,7 @@
 """GPU parity of the whole frame in one launch (decoder step + acoustic frame) and of chained
 frames with the re-embedding on the device, against the golden fixture of the reference CPU
 build (three frames: decode -> acoustic -> re-embed, voxtral_tts.c:301-318)."""
+import ctypes as C
 import os
 
 import numpy as np
@@ -86,3 +87,25 @@ def test_device_resident_loop_stops_at_end(pkg, engine, oracle, synth_model):
     finally:
         del synth_model.t[name]
         engine.upload(synth_model, decoder=False, acoustic=True)
+
+
+@pytest.mark.parametrize("runs", [(6,), (2, 4)])
+def test_decoder_step_inside_a_run(pkg, engine, oracle, runs):
+    """A decoder step of the host's at an unrelated cache row, after every run of a device-resident utterance: the utterance is what
+    it is undisturbed, and the step what it is alone."""
+    e, pos, seed, _ = _start(pkg, engine)
+    n = sum(runs)
+    noise = oracle.randn(oracle.seed(seed), 36 * n)[0].reshape(n, 36)
+    want, want_end, _ = engine.utterance(e, pos, noise)
+    row, far = pkg.synth_f32(3072, 61, "step.row", 0.0, 0.5), engine.kv_max - 1
+    alone = engine.llm_forward(row, far)
+    L = engine.L
+    first, noise = np.ascontiguousarray(e, dtype=np.float32), np.ascontiguousarray(noise, dtype=np.float32)
+    codes, done, end = np.zeros((n, 37), dtype=np.int32), np.zeros(1, dtype=np.int32), np.zeros(1, dtype=np.int32)
+    assert L.vb200_utterance_begin(first.ctypes.data, pos, noise.ctypes.data, n) == 0
+    for r in runs:
+        assert L.vb200_utterance_run(r) == 0
+        engine.llm_forward(row, far)
+    assert L.vb200_utterance_end(codes.ctypes.data, C.cast(done.ctypes.data, C.POINTER(C.c_int)), C.cast(end.ctypes.data, C.POINTER(C.c_int)), None) == 0
+    assert done[0] == len(want) and bool(end[0]) == want_end and np.array_equal(codes[:done[0]], want)
+    assert np.array_equal(engine.llm_forward(row, far), alone)

@@ -85,7 +85,6 @@ enum EmbedMode {
 };
 
 constexpr int kVariants = 3;   /* captured graphs: run loop, single frame, single chained frame */
-constexpr int kStep = kVariants, kGraphs = kVariants + 1;   /* and the decoder layers alone */
 
 struct Batch {
     bool open = false, begun = false, single = false;
@@ -122,8 +121,8 @@ struct Batch {
     SOp *s_prog[kVariants] = {};
     SWeights *s_wl[kVariants] = {};             /* the producer's view of each op list: its GEMV weights in order */
     int s_n[kVariants] = {}, s_nw[kVariants] = {};
-    cudaGraphExec_t exec[kGraphs] = {};
-    int direct_calls[kGraphs] = {};
+    cudaGraphExec_t exec[kVariants] = {};
+    int direct_calls[kVariants] = {};
     int graph_cap = 0;                          /* frame cap baked into exec[0] */
     cudaEvent_t e0 = nullptr, e1 = nullptr;
 };
@@ -574,7 +573,7 @@ static void bt_free(std::vector<void *> *owner) {
 }
 
 static void drop_graphs(Batch &t) {
-    for (int v = 0; v < kGraphs; v++) {
+    for (int v = 0; v < kVariants; v++) {
         if (t.exec[v]) cudaGraphExecDestroy(t.exec[v]);
         t.exec[v] = nullptr;
         t.direct_calls[v] = 0;
@@ -994,8 +993,8 @@ static int ctx_open(Batch &t, bool single, int n_utt, int kv_max, int max_frames
     return 0;
 }
 
-/* The decoder layers and the final norm for the rows in t.X, enqueued launch by launch; `sums` as in TcGemm. */
-static int enqueue_decoder(Batch &t, int sums = 2) {
+/* The decoder layers and the final norm for the rows in t.X, enqueued launch by launch. */
+static int enqueue_decoder(Batch &t) {
     Model &m = model();
     const BtWeights &w = g_w;
     cudaStream_t st = m.st;
@@ -1032,7 +1031,7 @@ static int enqueue_decoder(Batch &t, int sums = 2) {
         else if (tp) tc_prepare(t.aD, nullptr, D, B, t.part_w2, s_w2, psD, t.X, t.X, L.attn_norm, t.ssq, st,
                         tp_wait_for(0, TP_W2, NL, l, t.status), tap_base ? tap_base + (size_t)(2 * l - 1) * D : nullptr);
         TcGemm g;
-        g.M = B; g.status = t.status; g.eps = VB200_NORM_EPS; g.sums = sums;
+        g.M = B; g.status = t.status; g.eps = VB200_NORM_EPS;
         g.epi = TC_EPI_PARTIAL; g.out = t.part_qkv; g.splits = s_qkv; g.ld_out = QKV;
         g.ssq = t.ssq; g.ssq_chunks = l == 0 ? tc_prepare_chunks(D) : chunksD;
         if (tp) { g.tile0 = q0; g.n_tiles = qn; g.push = tp_push(0, TP_QKV, NL, l + 1); }
@@ -1046,7 +1045,7 @@ static int enqueue_decoder(Batch &t, int sums = 2) {
             launch_pdl_cluster(bt_attn_kernel<false>, attn_splits, grid, dim3(kBtAttnThreads), 0, st, t.bQ, 16, (const float *)t.part_qkv, s_qkv,
                                psQ, t.kv_k, t.kv_v, t.slab, l, (const VbDyn *)t.dyn, scale, VB200_ROPE_THETA, t.status, TcNoWait());
         g = TcGemm();
-        g.M = B; g.status = t.status; g.eps = VB200_NORM_EPS; g.sums = sums;
+        g.M = B; g.status = t.status; g.eps = VB200_NORM_EPS;
         g.epi = TC_EPI_PARTIAL; g.out = t.part_wo; g.splits = s_wo; g.ld_out = D;
         if (tp) { g.tile0 = o0; g.n_tiles = on; g.push = tp_push(0, TP_WO, NL, l + 1); }
         else g.join = {t.X, t.X, L.ffn_norm, t.bD, 16, t.ssq, tap_base ? tap_base + (size_t)(2 * l) * D : nullptr};
@@ -1054,13 +1053,13 @@ static int enqueue_decoder(Batch &t, int sums = 2) {
         if (tp) tc_prepare(t.aD, nullptr, D, B, t.part_wo, s_wo, psD, t.X, t.X, L.ffn_norm, t.ssq, st,
                    tp_wait_for(0, TP_WO, NL, l + 1, t.status), tap_base ? tap_base + (size_t)(2 * l) * D : nullptr);
         g = TcGemm();
-        g.M = B; g.status = t.status; g.eps = VB200_NORM_EPS; g.sums = sums;
+        g.M = B; g.status = t.status; g.eps = VB200_NORM_EPS;
         g.epi = TC_EPI_SWIGLU_TERMS; g.out_terms = t.bH; g.out_rows_pad = 16;
         g.splits = 1; g.ld_out = HID; g.ssq = t.ssq; g.ssq_chunks = chunksD;
         if (tp) { g.tile0 = h0; g.n_tiles = hn; g.push = tp_push(0, TP_W13, NL, l + 1); }
         if (tc_gemm(w.w13[l], t.aD, g, st)) return -1;
         g = TcGemm();
-        g.M = B; g.status = t.status; g.eps = VB200_NORM_EPS; g.sums = sums;
+        g.M = B; g.status = t.status; g.eps = VB200_NORM_EPS;
         g.epi = TC_EPI_PARTIAL; g.out = t.part_w2; g.splits = s_w2; g.ld_out = D;
         if (tp) {
             g.tile0 = o0; g.n_tiles = on; g.push = tp_push(0, TP_W2, NL, l + 1);
@@ -1115,14 +1114,11 @@ static int enqueue_frame(Batch &t, int embed_mode, bool advance, const float *no
 }
 
 /* Variant v of the frame: 0 = a frame of a device-resident run, 1 = single frame with the
- * host's input row, 2 = single frame re-embedding the previous codes; kStep = the decoder layers alone, with ten sums
- * a GEMM: hidden states of ten prompts of 8 to 300 rows are 2.03e-5 off 64 bits on average on the streaming GEMV kernel,
- * 2.09e-5 with four sums. */
+ * host's input row, 2 = single frame re-embedding the previous codes. */
 static int enqueue_variant(Batch &t, int v) {
     switch (v) {
     case 0: return enqueue_frame(t, EMBED_CODES_AFTER0, true, t.noise_all, t.codes_all, t.cap);
     case 1: return enqueue_frame(t, EMBED_HOST, false, t.noise1, nullptr, 0);
-    case kStep: return enqueue_decoder(t, kTcManySums) || cudaGetLastError() != cudaSuccess ? -1 : 0;
     default: return enqueue_frame(t, EMBED_CODES, false, t.noise1, nullptr, 0);
     }
 }
@@ -1483,35 +1479,6 @@ int single_frame(const float *embed, const float *noise, int pos, float *hidden_
     if (one_status(t)) return -1;
     memcpy(codes, t.h_out->codes, sizeof(int) * VB200_CODES);
     if (hidden_out) memcpy(hidden_out, t.h_out->hidden, sizeof(float) * D);
-    return 0;
-}
-
-/* tts_llm_forward (voxtral_tts_llm.c:171-271) on the frame's GEMMs: 1.4 ms, 1.9 on the streaming GEMV kernel. 1: not on this path. It is
- * where a prefill or a frame has left the decoder's tile-contiguous copies; a program that makes neither is not made to
- * pay 6 GB for them. */
-int single_step(const float *embed, int pos, float *hidden_out) {
-    Model &m = model();
-    static const bool off = getenv("VB200_NO_TC") != nullptr;
-    Batch &t = g_one;
-    if (off || g_tp.on || !g_w.ready || (t.open ? t.stream : stream_wanted()) || one_ready(0)) return 1;
-    t.h_in->dyn.pos = pos; t.h_in->dyn.kv_max = m.kv_max; t.h_in->dyn.frame = 0; t.h_in->dyn.done = 0;
-    memcpy(t.h_in->X, embed, sizeof(float) * D);
-    if (cudaMemcpyAsync(t.d_in, t.h_in, offsetof(OneIn, noise), cudaMemcpyHostToDevice, m.st) != cudaSuccess) return -1;
-    if (m.timing) {
-        flush_launch_time();
-        cudaEventRecord(m.ev0, m.st);
-    }
-    if (launch_variant(t, kStep)) return -1;
-    if (m.timing) {
-        cudaEventRecord(m.ev1, m.st);
-        m.time_pending = true;
-    }
-    if (cudaMemcpyAsync(t.h_out, t.d_out, sizeof(OneOut), cudaMemcpyDeviceToHost, m.st) != cudaSuccess ||
-        cudaStreamSynchronize(m.st) != cudaSuccess)
-        return -1;
-    flush_launch_time();
-    if (one_status(t)) return -1;
-    memcpy(hidden_out, t.h_out->hidden, sizeof(float) * D);
     return 0;
 }
 

@@ -639,8 +639,6 @@ int llm_forward(float *out_hidden, const float *embed, int pos) {
         fprintf(stderr, "voxtral_b200: position %d outside the %d-row cache\n", pos, m.kv_max);
         return -1;
     }
-    const int rc = single_step(embed, pos, out_hidden);
-    if (rc <= 0) return rc;
     m.h_in->dyn.pos = pos; m.h_in->dyn.kv_max = m.kv_max; m.h_in->dyn.frame = 0; m.h_in->dyn.done = 0;
     memcpy(m.h_in->embed, embed, sizeof(float) * D);
     VB_CHECK(cudaMemcpyAsync(m.d_in, m.h_in, offsetof(DevIn, lat), cudaMemcpyHostToDevice, m.st));

@@ -147,7 +147,6 @@ int batch_launches_per_frame();
 /* one utterance on the library's cache, same launches (vb_batch.cu) */
 bool single_tc_usable();
 int single_frame(const float *embed, const float *noise, int pos, float *hidden_out, int *codes, bool chained);
-int single_step(const float *embed, int pos, float *hidden_out);      /* 1: not on this path */
 int single_begin(const float *first_embed, int start_pos, const float *noise_all, int n_frames);
 int single_run(int n);
 int single_end(int *codes_out, int *frames_done, int *hit_end, float *device_ms);

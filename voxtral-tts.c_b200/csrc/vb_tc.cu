@@ -619,12 +619,8 @@ static int tc_gemm_join(const TcWeight &w, const TcActs &a, const TcGemm &g, cud
     ka.a_tiled = w.tiled ? 1 : 0;
     ka.N = w.N; ka.K = w.K; ka.M = g.M; ka.rows_pad = a.rows_pad; ka.splits = kTcJoinSplits; ka.status = g.status;
     ka.n_tiles_launch = w.N / kTcTileN;
-    switch (g.sums) {
-    case 2: return launch_tc_tp<16, 6, TC_JOIN, 2>(w, a, ka, j, st);
-    case 4: return launch_tc_tp<16, 6, TC_JOIN, 4>(w, a, ka, j, st);
-    case kTcManySums: return launch_tc_tp<16, 6, TC_JOIN, kTcManySums>(w, a, ka, j, st);
-    default: return -1;
-    }
+    if (g.sums != 2 && g.sums != 4) return -1;
+    return g.sums == 4 ? launch_tc_tp<16, 6, TC_JOIN, 4>(w, a, ka, j, st) : launch_tc_tp<16, 6, TC_JOIN, 2>(w, a, ka, j, st);
 }
 
 int tc_gemm(const TcWeight &w, const TcActs &a, const TcGemm &g, cudaStream_t st) {
