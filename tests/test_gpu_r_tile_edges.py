@@ -65,6 +65,33 @@ def test_prompt_attention_tiles(pkg, tmp_path, name):
             lm.release(s)
 
 
+@pytest.mark.parametrize("dtype", list(LIMIT))
+@pytest.mark.parametrize("heads,kv_heads,dim,change", [(64, 64, 8, 320), (40, 20, 16, 640), (3, 1, 20, 1280), (80, 80, 8, 160), (10, 2, 16, 160)])
+def test_one_token_attention_changes_kernel(pkg, tmp_path, heads, kv_heads, dim, change, dtype):
+    """Tokens one at a time on both sides of the length from which an unwindowed layer takes the kernel for many keys (none of
+    its own for few in the last two), beside a layer whose window keeps it where it is; the device's own loop makes the
+    change at the same token."""
+    c = Case(pkg, tmp_path, config([attention(heads=heads, kv_heads=kv_heads, dim=dim, vdim=dim, window=0, rot=8, ff=0),
+                                    attention(heads=4, kv_heads=2, dim=16, vdim=16, window=70, keep=3, rot=8, ff=0)]), seed=dim)
+    n = change - 9
+    toks = tokens(c.cfg, n + 20, 12)
+    want = plain.forward(c.w, c.cfg, toks)[0]
+    with c.open(dtype) as lm:
+        s = lm.open()
+        assert error(lm.step(s, toks[:n], [n - 1]), want[n - 1:n]) < LIMIT[dtype]
+        assert error(feed(lm, s, toks[n:], [1]), want[n:]) < LIMIT[dtype]
+        lm.release(s)
+        s = lm.open()
+        loop = lm.generate(s, toks[:n], 20)
+        lm.release(s)
+        s, host = lm.open(), []
+        z = lm.step(s, toks[:n], [n - 1])
+        for _ in range(20):
+            host.append(int(z[0].argmax()))
+            z = lm.step(s, host[-1:], [0])
+        assert loop == host
+
+
 @pytest.mark.parametrize("first,rows", [(1, 64), (65, 31), (100, 129), (7, 300)])
 def test_prefill_attention_tiles(pkg, engine, synth_model, first, rows):
     """A prompt in two calls against the same rows at once. Both are two-term products; a row's sums end in other

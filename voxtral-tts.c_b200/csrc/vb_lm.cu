@@ -166,6 +166,7 @@ struct vb200_lm {
     uint16_t *wide = nullptr;            /* keys and values of a stretch, written out */
     struct { const Acts *acts = nullptr; size_t cache = 0; int first = 0, n = 0; } gathered;   /* what kv_acts hold within a step */
     int pos_now = 0;                     /* position of the first row of the launch sequence being enqueued */
+    int step_near = 1 << 30;             /* a token that sees no more than this takes every layer's kernel for few keys */
     /* mixture of experts */
     Acts *sorted_acts = nullptr;
     std::map<int, Acts *> expert_acts;   /* by expert size */
@@ -185,8 +186,8 @@ struct vb200_lm {
     int *tokens() const { return d_in + 4; }
     int *wanted() const { return d_in + 4 + block; }
 
-    cudaGraphExec_t exec[kVariants] = {};
-    int direct_calls[kVariants] = {};
+    cudaGraphExec_t exec[2][kVariants] = {};      /* near, far: see step_near */
+    int direct_calls[2][kVariants] = {};
     cudaEvent_t ev[3] = {};
     bool timed = false;
 
@@ -220,6 +221,9 @@ private:
         return M <= 256 ? tc_rows_pad_frame(M) : tc_rows_pad_any(M);
     }
     TcGemm plan(int M) const;
+    int most_keys(const LmMixer &m) const {
+        return m.mask.window > 0 ? (int)std::min((long long)m.mask.window + m.mask.keep_first, (long long)max_tokens) : max_tokens;
+    }
     int splits_of(const Linear &l, int M) const;
     bool fused_act(const Linear &l, int M) const { return !f32() && l.act_n0 > 0 && M > 256; }
     size_t part_floats(const Linear &l, int max_rows);
@@ -263,8 +267,9 @@ template <typename T> int vb200_lm::alloc(T **p, size_t n, bool clear) {
 vb200_lm::~vb200_lm() {
     if (st) cudaStreamSynchronize(st);
     if (side) cudaStreamSynchronize(side);
-    for (int i = 0; i < kVariants; i++)
-        if (exec[i]) cudaGraphExecDestroy(exec[i]);
+    for (auto &of : exec)
+        for (cudaGraphExec_t e : of)
+            if (e) cudaGraphExecDestroy(e);
     stage_.close();
     for (int i = 0; i < 2; i++) {
         if (h_in[i]) cudaFreeHost(h_in[i]);
@@ -587,6 +592,11 @@ int vb200_lm::make_state() {
             }
         }
         states.push_back(s);
+    }
+    for (const LmLayer &l : cfg.layers) {
+        const LmMixer &m = l.mixer;
+        const int near = m.kind == LM_MIXER_ATTENTION ? lm_attn_step_near(m.heads, m.kv_heads, m.dim, m.vdim) : 0;
+        if (near > 0 && most_keys(m) > near) step_near = std::min(step_near, near);
     }
     slab = at;
     seqs.resize(max_seqs);
@@ -928,6 +938,7 @@ int vb200_lm::mixer(const Layer &l, const LmLayer &spec, const RunState &s, int 
         a.ring = s.ring;
         a.k = {slabs + s.a, slab}; a.v = {slabs + s.b, slab}; a.slots = (int)seqs.size();
         a.split = !f32() && lm_attn_mma_ok(m.dim, m.vdim);
+        a.most = std::min(most_keys(m), pos_now < step_near ? step_near : max_tokens);
         a.qkv = in; a.q = q; a.scratch = scratch; a.tickets = tickets; a.status = status;
         a.out = sink(l.mix.acts, M);
         if (M == 1 && lm_attn_step_ok(a)) {
@@ -1034,13 +1045,15 @@ int vb200_lm::enqueue(int M, int n_want, float *logits_out, bool greedy) {
     return 0;
 }
 
-/* One-token steps: the first call of a variant runs launch by launch (kernel attributes are set on
+/* One-token steps, near the start of a sequence and beyond: the first call of a variant runs launch by launch (kernel attributes are set on
  * first use, which must not happen inside a capture), the second is captured, later ones replay. */
 int vb200_lm::launch(int M, int n_want, float *logits_out, bool greedy) {
     if (M != 1 || tap_on || f32()) return enqueue(M, n_want, logits_out, greedy);
     const int v = greedy ? STEP_GREEDY : n_want ? STEP_LOGITS : STEP_SILENT;
-    if (!exec[v]) {
-        if (direct_calls[v]++ == 0) return enqueue(M, n_want, logits_out, greedy);
+    const bool far = pos_now >= step_near;
+    cudaGraphExec_t &graph_exec = exec[far][v];
+    if (!graph_exec) {
+        if (direct_calls[far][v]++ == 0) return enqueue(M, n_want, logits_out, greedy);
         cudaGraph_t graph = nullptr;
         LM_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
         const int rc = enqueue(M, n_want, nullptr, greedy);
@@ -1050,14 +1063,14 @@ int vb200_lm::launch(int M, int n_want, float *logits_out, bool greedy) {
             cudaGetLastError();
             return rc ? -1 : fail("the one-token step could not be captured");
         }
-        const cudaError_t ie = cudaGraphInstantiate(&exec[v], graph, 0);
+        const cudaError_t ie = cudaGraphInstantiate(&graph_exec, graph, 0);
         cudaGraphDestroy(graph);
         if (ie != cudaSuccess) {
-            exec[v] = nullptr;
+            graph_exec = nullptr;
             return cuda_ok(ie, "cudaGraphInstantiate");
         }
     }
-    LM_CUDA(cudaGraphLaunch(exec[v], st));
+    LM_CUDA(cudaGraphLaunch(graph_exec, st));
     if (v == STEP_LOGITS && logits_out)
         LM_CUDA(cudaMemcpyAsync(logits_out, logits, sizeof(float) * cfg.vocab, cudaMemcpyDeviceToHost, st));
     return 0;
@@ -1224,6 +1237,7 @@ int vb200_lm_generate(vb200_lm_t *lm, int seq, const int *prompt, int n, int n_n
     cudaEventRecord(lm->ev[1], lm->st);
     /* position, token and log are on the device from here on */
     for (int i = 1; i < n_new; i++) {
+        lm->pos_now = lm->seqs[seq].length;
         if (lm->launch(1, 1, nullptr, true)) return -1;
         lm->seqs[seq].length += 1;
     }

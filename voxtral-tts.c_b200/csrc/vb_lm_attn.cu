@@ -602,6 +602,7 @@ int launch_attn_step(const LmAttn &a, int splits, int lanes_h, cudaStream_t st) 
  * position, the angles, the gains, the first pass of keys and values (earlier steps are complete: a step's first kernel
  * is a plain launch). One warp per head and a merge by the last CTA through global memory: 17 us at 220 keys of 8 x 128. */
 constexpr int kSgThreads = 256, kSgWarps = 8, kSgKeys = 8, kSgHeads = 4, kSgDim = 128, kSgSplits = 8, kSgColumns = 8;
+constexpr int kSgMost = 160;              /* keys a CTA, at most: lm_attn_step_near */
 
 template <bool SPLIT>
 __global__ void __launch_bounds__(kSgThreads, 2) lm_attn_step_group_kernel(const LmAttn a) {
@@ -634,16 +635,19 @@ __global__ void __launch_bounds__(kSgThreads, 2) lm_attn_step_group_kernel(const
     const bool writer = sp == S - 1;
     float *Kc = a.k.base + (size_t)slot * a.k.slab + g * dim, *Vc = a.v.base + (size_t)slot * a.v.slab + g * vdim;
     const int first = w0 > a.ring.keep ? (w0 - a.ring.keep) % a.ring.ring : 0;      /* ring place of the window's first key */
-    float4 kq[kSgKeys], vq[kSgKeys];
-    auto fetch = [&](int xb) {                             /* keys xb, xb + 8, ...: all requests in flight together; the new token has none */
+    uint4 kq[kSgKeys], vq[kSgKeys];
+    /* keys xb, xb + 8, ...: requested without a branch or a conversion between them, so that all are in flight together (16 trips
+     * one after another, 8 us a pass, where each was behind a condition); beyond the slice and for the new token: not used */
+    const int dk = 4 * lane < dim ? 4 * lane : 0, dv = 4 * lane < vdim ? 4 * lane : 0;
+    auto fetch = [&](int xb) {
 #pragma unroll
         for (int u = 0; u < kSgKeys; u++) {
-            const int x = xb + u * kSgWarps;
+            int x = xb + u * kSgWarps;
+            x = x < x1 ? x : x1 > 0 ? x1 - 1 : 0;
             int r = first + x - n_keep;
             r = x < n_keep ? x : a.ring.keep + (r < a.ring.ring ? r : r - a.ring.ring);
-            const bool on = x < x1 && x < n_keys - 1;
-            kq[u] = on && 4 * lane < dim ? kv_get4<SPLIT>(Kc + (size_t)r * nk, dim, 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
-            vq[u] = on && 4 * lane < vdim ? kv_get4<SPLIT>(Vc + (size_t)r * nv, vdim, 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+            kq[u] = kv_raw4<SPLIT>(Kc + (size_t)r * nk, dim, dk);
+            vq[u] = kv_raw4<SPLIT>(Vc + (size_t)r * nv, vdim, dv);
         }
     };
     int xb = x0 + warp;
@@ -744,13 +748,13 @@ __global__ void __launch_bounds__(kSgThreads, 2) lm_attn_step_group_kernel(const
         float s[32];                                       /* [head][key] */
 #pragma unroll
         for (int u = 0; u < kSgKeys; u++) {
-            if (writer && xb + u * kSgWarps == n_keys - 1) {
-                kq[u] = 4 * lane < dim ? *reinterpret_cast<const float4 *>(ks + 4 * lane) : zero;
-                vq[u] = 4 * lane < vdim ? *reinterpret_cast<const float4 *>(vs + 4 * lane) : zero;
-            }
+            const int x = xb + u * kSgWarps;
+            float4 k = kv_value4<SPLIT>(kq[u]);
+            if (writer && x == n_keys - 1) k = *reinterpret_cast<const float4 *>(ks + dk);
+            if (4 * lane >= dim) k = zero;
 #pragma unroll
             for (int h = 0; h < kSgHeads; h++)
-                s[h * kSgKeys + u] = q4[h].x * kq[u].x + q4[h].y * kq[u].y + q4[h].z * kq[u].z + q4[h].w * kq[u].w;
+                s[h * kSgKeys + u] = q4[h].x * k.x + q4[h].y * k.y + q4[h].z * k.z + q4[h].w * k.w;
         }
         /* 32 sums over the lanes by halving: lane i is left with sum i */
 #pragma unroll
@@ -778,11 +782,18 @@ __global__ void __launch_bounds__(kSgThreads, 2) lm_attn_step_group_kernel(const
         for (int h = 0; h < kSgHeads; h++) {
             const float ch = __shfl_sync(0xffffffffu, c, h * kSgKeys);
             o[h].x *= ch; o[h].y *= ch; o[h].z *= ch; o[h].w *= ch;
+        }
 #pragma unroll
-            for (int u = 0; u < kSgKeys; u++) {
+        for (int u = 0; u < kSgKeys; u++) {
+            const int x = xb + u * kSgWarps;
+            float4 v = kv_value4<SPLIT>(vq[u]);
+            if (writer && x == n_keys - 1) v = *reinterpret_cast<const float4 *>(vs + dv);
+            if (x >= x1) v = zero;                         /* whatever lies there: its weight is zero, and so must it be */
+#pragma unroll
+            for (int h = 0; h < kSgHeads; h++) {
                 const float wu = __shfl_sync(0xffffffffu, w, h * kSgKeys + u);
-                o[h].x = fmaf(wu, vq[u].x, o[h].x); o[h].y = fmaf(wu, vq[u].y, o[h].y);
-                o[h].z = fmaf(wu, vq[u].z, o[h].z); o[h].w = fmaf(wu, vq[u].w, o[h].w);
+                o[h].x = fmaf(wu, v.x, o[h].x); o[h].y = fmaf(wu, v.y, o[h].y);
+                o[h].z = fmaf(wu, v.z, o[h].z); o[h].w = fmaf(wu, v.w, o[h].w);
             }
         }
         xb += kSgKeys * kSgWarps;
@@ -1099,11 +1110,27 @@ bool lm_attn_step_ok(const LmAttn &a) {
            a.vdim <= 256;
 }
 
+/* Key splits of lm_attn_step_group_kernel: as long as a CTA finds an SM of its own. */
+static int group_splits(int kv_heads) {
+    int splits = kSgSplits;
+    while (splits > 1 && splits * kv_heads > kStepCtas) splits /= 2;
+    return splits;
+}
+
+/* It is for short sequences and windows: its CTAs are at most 8 a KV head, of 8 warps, where lm_attn_step_kernel has up to 32 of
+ * 16. Layer of an attention-only model, both kernels, at 220, 1000, 2000, 4000 keys: 8 KV heads of 128 with 8 query heads 17.1 /
+ * 21.9, 21.5 / 24.8, 26.2 / 25.4, 37.0 / 28.3 us, with 32 19.5 / 26.2, 23.5 / 30.4, 28.1 / 34.1, 38.9 / 39.8; one of 128 16.1 /
+ * 20.5, 19.4 / 22.7, 23.4 / 22.6, 32.9 / 22.7; 64 of 64 24.3 / 27.8, 47.4 / 34.3, 73.9 / 42.4, 129 / 57; 96 of 32, which
+ * leave one CTA each, 29.7 / 22.1 at 220 already. */
+int lm_attn_step_near(int heads, int kv_heads, int dim, int vdim) {
+    const int splits = group_splits(kv_heads);
+    return heads / kv_heads <= kSgHeads && dim <= kSgDim && vdim <= kSgDim && splits > 1 ? kSgMost * splits : 0;
+}
+
 int lm_attn_step(const LmAttn &a, cudaStream_t st) {
     const int group = a.heads / a.kv_heads;
-    if (group <= kSgHeads && a.dim <= kSgDim && a.vdim <= kSgDim) {
-        int splits = kSgSplits;                  /* as long as a CTA finds an SM of its own */
-        while (splits > 1 && splits * a.kv_heads > kStepCtas) splits /= 2;
+    if (a.most <= lm_attn_step_near(a.heads, a.kv_heads, a.dim, a.vdim)) {
+        const int splits = group_splits(a.kv_heads);
         return ok(launch_pdl_cluster(a.split ? lm_attn_step_group_kernel<true> : lm_attn_step_group_kernel<false>, splits, dim3(splits, a.kv_heads),
                                      dim3(kSgThreads), 0, st, a));
     }

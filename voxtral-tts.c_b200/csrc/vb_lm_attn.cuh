@@ -44,14 +44,22 @@ VB_DEVINL float kv_get(const float *head, int size, int d, int split) {
     const unsigned short *h = reinterpret_cast<const unsigned short *>(head);
     return __uint_as_float((uint32_t)__ldcg(h + d) << 16) + __uint_as_float((uint32_t)__ldcg(h + size + d) << 16);
 }
+/* Four elements as they lie there, and what they are: a load whose result is not looked at yet waits for nothing. */
 template <bool SPLIT>
-VB_DEVINL float4 kv_get4(const float *head, int size, int d) {
-    if constexpr (!SPLIT) return vb_ldcg4(head + d);
+VB_DEVINL uint4 kv_raw4(const float *head, int size, int d) {
+    if constexpr (!SPLIT) return __ldcg(reinterpret_cast<const uint4 *>(head + d));
     const uint16_t *h = reinterpret_cast<const uint16_t *>(head);
     const uint2 hi = __ldcg(reinterpret_cast<const uint2 *>(h + d)), lo = __ldcg(reinterpret_cast<const uint2 *>(h + size + d));
-    return make_float4(vb_bf16_lo(hi.x) + vb_bf16_lo(lo.x), vb_bf16_hi(hi.x) + vb_bf16_hi(lo.x), vb_bf16_lo(hi.y) + vb_bf16_lo(lo.y),
-                       vb_bf16_hi(hi.y) + vb_bf16_hi(lo.y));
+    return make_uint4(hi.x, hi.y, lo.x, lo.y);
 }
+template <bool SPLIT>
+VB_DEVINL float4 kv_value4(uint4 r) {
+    if constexpr (!SPLIT) return make_float4(__uint_as_float(r.x), __uint_as_float(r.y), __uint_as_float(r.z), __uint_as_float(r.w));
+    return make_float4(vb_bf16_lo(r.x) + vb_bf16_lo(r.z), vb_bf16_hi(r.x) + vb_bf16_hi(r.z), vb_bf16_lo(r.y) + vb_bf16_lo(r.w),
+                       vb_bf16_hi(r.y) + vb_bf16_hi(r.w));
+}
+template <bool SPLIT>
+VB_DEVINL float4 kv_get4(const float *head, int size, int d) { return kv_value4<SPLIT>(kv_raw4<SPLIT>(head, size, d)); }
 
 /* Cosine and sine of pos * f: the angle to twice fp32's precision (f as a high and a low part), sine and cosine of its
  * leading part and the remainder as a first-order correction. */

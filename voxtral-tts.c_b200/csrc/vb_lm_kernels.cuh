@@ -189,6 +189,7 @@ struct LmAttn {
     LmRing ring;
     LmState k, v;                /* [ring rows][kv_heads * dim], [..][kv_heads * vdim] */
     int slots;                   /* how many there are */
+    int most;                    /* one token: keys that it may see, at most */
     int split;                   /* 1: a head's part of a cache row is [size] BF16 high halves, then [size] low halves
                                     (hi + lo carry 16 mantissa bits), ready for the tensor cores; 0: fp32 */
     LmPart qkv;
@@ -206,6 +207,7 @@ int lm_attn_prepare(const LmAttn &a, int M, cudaStream_t st);              /* no
 int lm_attn_generic(const LmAttn &a, int M, cudaStream_t st);              /* fp32 pipes, any size */
 bool lm_attn_step_ok(const LmAttn &a);
 int lm_attn_step(const LmAttn &a, cudaStream_t st);                        /* one token: norm, rotation, append, attention */
+int lm_attn_step_near(int heads, int kv_heads, int dim, int vdim);         /* keys up to which it has a kernel of its own for few (0: never) */
 bool lm_attn_mma_ok(int dim, int vdim);                                    /* sizes it runs at; needs split caches */
 int lm_attn_mma(const LmAttn &a, int M, cudaStream_t st);                  /* tensor cores, prompts */
 
