@@ -423,12 +423,7 @@ bt_attn_kernel(uint16_t *terms, int rows_pad, const float *part, int n_part, siz
                      "r"(__float_as_uint(O.x)), "r"(__float_as_uint(O.y)), "r"(__float_as_uint(M0)), "r"(__float_as_uint(L)), "r"(bar)
                      : "memory");
     }
-    /* a CTA ends only when it has received everything: nothing is sent to shared memory that is gone */
-    if (!vb_mbar_wait(&arrived, 0u, &gave_up)) {
-        atomicCAS(status, 0, 16);
-        gave_up = 1;
-        return;
-    }
+    if (!vb_mbar_wait_cluster(&arrived, &gave_up, status, 16)) return;
     if (tid < share) {
         const int i = sp * share + tid, h = i / (kHD / 2), c = 2 * (i % (kHD / 2));
         float2 O = make_float2(0.f, 0.f);

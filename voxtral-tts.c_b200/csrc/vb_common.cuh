@@ -62,6 +62,19 @@ VB_DEVINL bool vb_mbar_wait(uint64_t *bar, uint32_t parity, volatile int *cta_ab
     }
 }
 
+/* The same for what the CTAs of a cluster send into one another's shared memory, called by all threads of a CTA after it has sent its
+ * own. A CTA ends only when it has received everything. Where the wait runs out it reports that and stays for as long
+ * again: a sender held up by a bounded wait of its own, begun with the cluster, is done before that, and what it sends meets
+ * memory that is still there. */
+VB_DEVINL bool vb_mbar_wait_cluster(uint64_t *bar, volatile int *cta_abort, int *status, int code) {
+    if (vb_mbar_wait(bar, 0u, cta_abort)) return true;
+    atomicCAS(status, 0, code);
+    *cta_abort = 1;
+    volatile int stay = 0;
+    vb_mbar_wait(bar, 0u, &stay);
+    return false;
+}
+
 /* 1-D bulk copy global -> shared, completion counted in bytes on an mbarrier.
  * Both addresses 16-byte aligned, size a multiple of 16. No multicast. */
 VB_DEVINL void vb_bulk_g2s(void *smem_dst, const void *gmem_src, uint32_t bytes, uint64_t *bar) {

@@ -827,12 +827,7 @@ __global__ void __launch_bounds__(kSgThreads, 2) lm_attn_step_group_kernel(const
                      "r"(__float_as_uint(O.x)), "r"(__float_as_uint(O.y)), "r"(__float_as_uint(M0)), "r"(__float_as_uint(L)), "r"(bar)
                      : "memory");
     }
-    /* a CTA ends only when it has received everything: nothing is sent to shared memory that is gone */
-    if (!vb_mbar_wait(&arrived, 0u, &gave_up)) {
-        atomicCAS(a.status, 0, 53);
-        gave_up = 1;
-        return;
-    }
+    if (!vb_mbar_wait_cluster(&arrived, &gave_up, a.status, 53)) return;
     const int i = sp * share + tid, h = i / (kSgDim / 2), c = 2 * (i % (kSgDim / 2));
     if (tid < share && h < group && c < vdim) {
         float2 O = make_float2(0.f, 0.f);
