@@ -92,6 +92,21 @@ def test_one_token_attention_changes_kernel(pkg, tmp_path, heads, kv_heads, dim,
         assert loop == host
 
 
+@pytest.mark.parametrize("dtype", list(LIMIT))
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(40, 40, 16, 8), (20, 20, 20, 36), (64, 32, 32, 64), (8, 2, 64, 68), (3, 3, 132, 12), (2, 1, 30, 31)])
+def test_few_rows_tiles(pkg, tmp_path, heads, kv_heads, dim, vdim, dtype):
+    """A few rows at a time: heads of which a warp takes eight, four, two or one at once, whole and with lanes to spare, on both sides
+    of the change from tiles of 32 keys to 64 (at 129 to 193 keys for the first three)."""
+    c = Case(pkg, tmp_path, config([attention(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, window=0, rot=4, ff=0)]), seed=dim)
+    toks = tokens(c.cfg, 215, 13)
+    want = plain.forward(c.w, c.cfg, toks)[0]
+    with c.open(dtype) as lm:
+        for sizes in ([2], [3, 8, 5, 1, 30], [120, 7]):
+            s = lm.open()
+            assert error(feed(lm, s, toks, sizes), want) < LIMIT[dtype], sizes
+            lm.release(s)
+
+
 @pytest.mark.parametrize("first,rows", [(1, 64), (65, 31), (100, 129), (7, 300)])
 def test_prefill_attention_tiles(pkg, engine, synth_model, first, rows):
     """A prompt in two calls against the same rows at once. Both are two-term products; a row's sums end in other

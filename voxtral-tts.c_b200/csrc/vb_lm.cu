@@ -938,7 +938,8 @@ int vb200_lm::mixer(const Layer &l, const LmLayer &spec, const RunState &s, int 
         a.ring = s.ring;
         a.k = {slabs + s.a, slab}; a.v = {slabs + s.b, slab}; a.slots = (int)seqs.size();
         a.split = !f32() && lm_attn_mma_ok(m.dim, m.vdim);
-        a.most = std::min(most_keys(m), pos_now < step_near ? step_near : max_tokens);
+        /* one token: the same for all that a captured step serves */
+        a.most = M > 1 ? std::min(most_keys(m) + M - 1, pos_now + M) : std::min(most_keys(m), pos_now < step_near ? step_near : max_tokens);
         a.qkv = in; a.q = q; a.scratch = scratch; a.tickets = tickets; a.status = status;
         a.out = sink(l.mix.acts, M);
         if (M == 1 && lm_attn_step_ok(a)) {

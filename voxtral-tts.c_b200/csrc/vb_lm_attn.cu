@@ -104,13 +104,13 @@ __global__ void __launch_bounds__(kPrepThreads) lm_attn_prepare_kernel(const LmA
 }
 
 /* ------------------------------------------------------------------ any sizes, fp32 pipes */
-/* PAIRS (row, query head) pairs of a KV head per CTA, 64 keys at a time; a thread holds PAIRS / 16 pairs x 4 keys of the
+/* PAIRS (row, query head) pairs of a KV head per CTA, 32 or 64 keys at a time; a thread holds PAIRS / 16 pairs x 2 or 4 keys of the
  * scores, then the same pairs x 4 * NV columns of the result, as packed fp32 pairs, so that a 16-byte read of shared
  * memory serves 4 to 16 multiply-adds. (Scores by dot products of a lane each, results a column a time through shared
  * memory: 390 rows of 16 heads of 128 took 405 us a layer, five rows at 400 keys 70 us.) 64 pairs for prompts, two
  * CTAs an SM at heads of 128; 16 for a few rows, where the keys are split over CTAs and tiles of 64 pairs would be
  * mostly empty. The last split to arrive merges in split order. */
-constexpr int kGaThreads = 256, kGaKeys = 64, kGaManyPairs = 64;
+constexpr int kGaThreads = 256, kGaKeys = 64, kGaFewKeys = 32, kGaManyPairs = 64;
 
 typedef unsigned long long f2;   /* two packed floats */
 VB_DEVINL f2 f2_fma(f2 a, f2 b, f2 c) {
@@ -137,28 +137,33 @@ VB_DEVINL float2 f2_get(f2 v) {
 /* rows of a multiple of four floats; an odd number of 16-byte pieces, so that eight rows' pieces lie in different banks */
 inline __host__ __device__ int ga_ld(int n) { const int v = (n + 3) / 4 + 1; return 4 * (v | 1); }
 inline __host__ __device__ int ga_stride(int vdim) { return (vdim + 3) / 4 * 4 + 4; }   /* a pair's partial result: columns, maximum, sum */
-constexpr int kGaLdP = kGaKeys + 4;
-inline size_t ga_smem(int pairs, int dim, int vdim) {
-    return sizeof(float) * ((size_t)pairs * ga_ld(dim) + std::max(kGaKeys * ga_ld(dim), pairs * kGaLdP) + (size_t)kGaKeys * ((vdim + 3) / 4 * 4));
+inline size_t ga_smem(int pairs, int keys, int dim, int vdim) {
+    return sizeof(float) * ((size_t)pairs * ga_ld(dim) + std::max(keys * ga_ld(dim), pairs * (keys + 4)) + (size_t)keys * ((vdim + 3) / 4 * 4));
 }
 
-/* n rows of `size` floats or halves into shared memory, rows up to kGaKeys and columns up to a multiple of four as zeros; a warp takes
- * every eighth row. True where a value is not finite. */
-template <bool SPLIT, typename Row>
+/* n rows of `size` floats or halves into shared memory, rows up to KEYS and columns up to a multiple of four as zeros. A warp takes a
+ * row, or the two, four or eight that its lanes have room for (heads of 32 with three lanes in four idle: 25% longer than element
+ * by element, 96 heads). A thread requests its loads together: none behind a condition or a conversion. True where a value is not finite. */
+template <int KEYS, bool SPLIT, typename Row>
 VB_DEVINL bool ga_load(float *to, int ld, int size, int n, const Row &row, int warp, int lane) {
-    const int pieces = (size + 3) / 4;
+    const int pieces = (size + 3) / 4, across = pieces > 16 ? 32 : pieces > 8 ? 16 : pieces > 4 ? 8 : 4, step = kGaThreads / across;
+    const int first = warp * (32 / across) + lane / across;
     bool odd = false;
-    for (int c = lane; c < pieces; c += 32) {
-        float4 v[kGaKeys / 8];
+    for (int c = lane % across; c < pieces; c += across) {
+        float4 v[KEYS / 8];
+        if ((size & 3) == 0) {
+            uint4 raw[KEYS / 8];
 #pragma unroll
-        for (int i = 0; i < kGaKeys / 8; i++) {
-            const int j = warp + 8 * i;
-            v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (j >= n) continue;
-            const float *head = row(j);
-            if ((size & 3) == 0) {
-                v[i] = kv_get4<SPLIT>(head, size, 4 * c);
-            } else {
+            for (int i = 0; i < KEYS / 8; i++) raw[i] = kv_raw4<SPLIT>(row(min(first + step * i, n - 1)), size, 4 * c);
+#pragma unroll
+            for (int i = 0; i < KEYS / 8; i++) v[i] = first + step * i < n ? kv_value4<SPLIT>(raw[i]) : make_float4(0.f, 0.f, 0.f, 0.f);
+        } else {
+#pragma unroll
+            for (int i = 0; i < KEYS / 8; i++) {
+                const int j = first + step * i;
+                v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (j >= n) continue;
+                const float *head = row(j);
                 v[i].x = kv_get(head, size, 4 * c, SPLIT);
                 if (4 * c + 1 < size) v[i].y = kv_get(head, size, 4 * c + 1, SPLIT);
                 if (4 * c + 2 < size) v[i].z = kv_get(head, size, 4 * c + 2, SPLIT);
@@ -166,8 +171,10 @@ VB_DEVINL bool ga_load(float *to, int ld, int size, int n, const Row &row, int w
             }
         }
 #pragma unroll
-        for (int i = 0; i < kGaKeys / 8; i++) {
-            *(float4 *)(to + (size_t)(warp + 8 * i) * ld + 4 * c) = v[i];
+        for (int i = 0; i < KEYS / 8; i++) {
+            const int j = first + step * i;
+            if (j >= KEYS) break;
+            *(float4 *)(to + (size_t)j * ld + 4 * c) = v[i];
             odd |= !(fabsf(v[i].x) < INFINITY && fabsf(v[i].y) < INFINITY && fabsf(v[i].z) < INFINITY && fabsf(v[i].w) < INFINITY);
         }
     }
@@ -175,21 +182,21 @@ VB_DEVINL bool ga_load(float *to, int ld, int size, int n, const Row &row, int w
 }
 
 /* grid = (tiles of pairs, KV heads, key splits) */
-template <int PAIRS, int NV, bool SPLIT>
+template <int PAIRS, int KEYS, int NV, bool SPLIT>
 __global__ void __launch_bounds__(kGaThreads) lm_attn_generic_kernel(const LmAttn a, int M) {
-    constexpr int TP = PAIRS / 16, TK = kGaKeys / 16;
+    constexpr int TP = PAIRS / 16, TK = KEYS / 16, LDP = KEYS + 4;
     extern __shared__ __align__(16) float ga[];
     __shared__ float wgt[kLmAttnSplits][PAIRS], total[PAIRS];
     __shared__ int last_flag;
     pdl_launch_dependents();
     pdl_wait();
     const int dim = a.dim, vdim = a.vdim, group = a.heads / a.kv_heads, ld = ga_ld(dim), ldv = (vdim + 3) / 4 * 4;
-    float *Q = ga, *K = Q + PAIRS * ld, *P = K, *V = K + (kGaKeys * ld > PAIRS * kGaLdP ? kGaKeys * ld : PAIRS * kGaLdP);
+    float *Q = ga, *K = Q + PAIRS * ld, *P = K, *V = K + (KEYS * ld > PAIRS * LDP ? KEYS * ld : PAIRS * LDP);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, tx = tid & 15, ty = tid >> 4;
     const int g = blockIdx.y, p0 = blockIdx.x * PAIRS;
     const int np = M * group - p0 < PAIRS ? M * group - p0 : PAIRS;
     const int pos0 = a.dyn->pos;
-    const KeyTiles kt = key_tiles<kGaKeys>(pos0 + p0 / group, pos0 + (p0 + np - 1) / group, a.window, a.keep);
+    const KeyTiles kt = key_tiles<KEYS>(pos0 + p0 / group, pos0 + (p0 + np - 1) / group, a.window, a.keep);
     const int S_eff = (int)gridDim.z < kt.n_tiles ? (int)gridDim.z : kt.n_tiles;
     const int sp = blockIdx.z;
     if (sp >= S_eff) return;
@@ -214,10 +221,10 @@ __global__ void __launch_bounds__(kGaThreads) lm_attn_generic_kernel(const LmAtt
 
     for (int t = t0; t < t1; t++) {
         int j0, n;
-        key_tile<kGaKeys>(kt, t, &j0, &n);
+        key_tile<KEYS>(kt, t, &j0, &n);
         __syncthreads();                         /* the last tile is read */
-        ga_load<SPLIT>(K, ld, dim, n, [&](int j) { return Kc + ((size_t)lm_ring_row(a.ring, j0 + j) * a.kv_heads + g) * dim; }, warp, lane);
-        const bool odd = ga_load<SPLIT>(V, ldv, vdim, n, [&](int j) { return Vc + ((size_t)lm_ring_row(a.ring, j0 + j) * a.kv_heads + g) * vdim; }, warp, lane);
+        ga_load<KEYS, SPLIT>(K, ld, dim, n, [&](int j) { return Kc + ((size_t)lm_ring_row(a.ring, j0 + j) * a.kv_heads + g) * dim; }, warp, lane);
+        const bool odd = ga_load<KEYS, SPLIT>(V, ldv, vdim, n, [&](int j) { return Vc + ((size_t)lm_ring_row(a.ring, j0 + j) * a.kv_heads + g) * vdim; }, warp, lane);
         const bool any_odd = __syncthreads_or(odd);
         f2 acc[TP][TK] = {};
 #pragma unroll 4
@@ -252,7 +259,7 @@ __global__ void __launch_bounds__(kGaThreads) lm_attn_generic_kernel(const LmAtt
 #pragma unroll
             for (int j = 0; j < TK; j++) {
                 const float w = s[j] > -INFINITY ? expf(s[j] - now) : 0.0f;
-                P[(ty * TP + i) * kGaLdP + tx + 16 * j] = w;
+                P[(ty * TP + i) * LDP + tx + 16 * j] = w;
                 sum += w;
             }
 #pragma unroll
@@ -266,7 +273,7 @@ __global__ void __launch_bounds__(kGaThreads) lm_attn_generic_kernel(const LmAtt
         for (int j = 0; j < n; j += 4) {         /* rows from n on are zeros */
             float4 w[TP];
 #pragma unroll
-            for (int i = 0; i < TP; i++) w[i] = *(const float4 *)(P + (ty * TP + i) * kGaLdP + j);
+            for (int i = 0; i < TP; i++) w[i] = *(const float4 *)(P + (ty * TP + i) * LDP + j);
 #pragma unroll
             for (int u = 0; u < 4; u++)
 #pragma unroll
@@ -1032,13 +1039,13 @@ int lm_attn_prepare(const LmAttn &a, int M, cudaStream_t st) {
     return ok(launch_pdl(lm_attn_prepare_kernel, dim3(M), dim3(kPrepThreads), smem, st, a));
 }
 
-template <int PAIRS, int NV, bool SPLIT>
+template <int PAIRS, int KEYS, int NV, bool SPLIT>
 static int launch_generic(const LmAttn &a, int M, cudaStream_t st) {
-    const size_t smem = ga_smem(PAIRS, a.dim, a.vdim);
+    const size_t smem = ga_smem(PAIRS, KEYS, a.dim, a.vdim);
     if (smem > 200 * 1024) return -1;
     static size_t set = 32 * 1024;      /* 48 KB without asking, static arrays included */
     if (smem > set) {
-        if (cudaFuncSetAttribute(lm_attn_generic_kernel<PAIRS, NV, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+        if (cudaFuncSetAttribute(lm_attn_generic_kernel<PAIRS, KEYS, NV, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
             cudaGetLastError();
             return -1;
         }
@@ -1047,18 +1054,24 @@ static int launch_generic(const LmAttn &a, int M, cudaStream_t st) {
     const int tiles = (M * (a.heads / a.kv_heads) + PAIRS - 1) / PAIRS;
     int splits = kSplitBudget / (tiles * a.kv_heads);
     splits = splits < 1 ? 1 : splits > kLmAttnSplits ? kLmAttnSplits : splits;
-    return ok(launch_pdl(lm_attn_generic_kernel<PAIRS, NV, SPLIT>, dim3(tiles, a.kv_heads, splits), dim3(kGaThreads), smem, st, a, M));
+    return ok(launch_pdl(lm_attn_generic_kernel<PAIRS, KEYS, NV, SPLIT>, dim3(tiles, a.kv_heads, splits), dim3(kGaThreads), smem, st, a, M));
+}
+
+template <int PAIRS, int KEYS>
+static int launch_generic(const LmAttn &a, int M, cudaStream_t st) {
+    if (a.vdim > 128) return a.split ? launch_generic<PAIRS, KEYS, 4, true>(a, M, st) : launch_generic<PAIRS, KEYS, 4, false>(a, M, st);
+    return a.split ? launch_generic<PAIRS, KEYS, 2, true>(a, M, st) : launch_generic<PAIRS, KEYS, 2, false>(a, M, st);
 }
 
 int lm_attn_generic(const LmAttn &a, int M, cudaStream_t st) {
     if (a.dim > 256 || a.vdim > 256) return -1;
-    const bool many = M * (a.heads / a.kv_heads) > kGaManyPairs / 2, wide = a.vdim > 128;
-    if (many) {
-        if (wide) return a.split ? launch_generic<kGaManyPairs, 4, true>(a, M, st) : launch_generic<kGaManyPairs, 4, false>(a, M, st);
-        return a.split ? launch_generic<kGaManyPairs, 2, true>(a, M, st) : launch_generic<kGaManyPairs, 2, false>(a, M, st);
-    }
-    if (wide) return a.split ? launch_generic<kLmAttnPairs, 4, true>(a, M, st) : launch_generic<kLmAttnPairs, 4, false>(a, M, st);
-    return a.split ? launch_generic<kLmAttnPairs, 2, true>(a, M, st) : launch_generic<kLmAttnPairs, 2, false>(a, M, st);
+    const int pairs = M * (a.heads / a.kv_heads);
+    if (pairs > kGaManyPairs / 2) return launch_generic<kGaManyPairs, kGaKeys>(a, M, st);
+    /* Few pairs and few keys: tiles of 32 keys, twice the CTAs, while those of 64 leave SMs without one. Two rows of eight heads of
+     * 128, a layer of an attention-only model at 220 keys: 47.8 us with 64, 39.4 with 32, 38.0 with a tile's loads in flight
+     * together besides; 32 in 32 bits at 1000 keys 51.8, 64 49.4, before the latter. */
+    const long long ctas = (long long)((pairs + kLmAttnPairs - 1) / kLmAttnPairs) * a.kv_heads * ((a.most + kGaKeys - 1) / kGaKeys);
+    return ctas < kStepCtas ? launch_generic<kLmAttnPairs, kGaFewKeys>(a, M, st) : launch_generic<kLmAttnPairs, kGaKeys>(a, M, st);
 }
 
 bool lm_attn_mma_ok(int dim, int vdim) { return dim <= 128 && vdim <= 128 && dim % 8 == 0 && vdim % 8 == 0; }

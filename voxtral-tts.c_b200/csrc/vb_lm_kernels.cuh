@@ -189,7 +189,7 @@ struct LmAttn {
     LmRing ring;
     LmState k, v;                /* [ring rows][kv_heads * dim], [..][kv_heads * vdim] */
     int slots;                   /* how many there are */
-    int most;                    /* one token: keys that it may see, at most */
+    int most;                    /* keys that the rows may see, at most */
     int split;                   /* 1: a head's part of a cache row is [size] BF16 high halves, then [size] low halves
                                     (hi + lo carry 16 mantissa bits), ready for the tensor cores; 0: fp32 */
     LmPart qkv;
