@@ -107,6 +107,21 @@ def test_few_rows_tiles(pkg, tmp_path, heads, kv_heads, dim, vdim, dtype):
             lm.release(s)
 
 
+@pytest.mark.parametrize("dim,rot_dim,vdim", [(128, 64, 128), (64, 16, 64), (40, 8, 72)])
+@pytest.mark.parametrize("q_rank", [56, 200, 700])
+def test_latent_queries_in_parts(pkg, tmp_path, dim, rot_dim, vdim, q_rank):
+    """Portions of 17 to 64 rows, whose queries come in one part, in a few and in as many as a K of eleven blocks is split into."""
+    c = Case(pkg, tmp_path, config([latent(heads=3, dim=dim, rot_dim=rot_dim, vdim=vdim, q_rank=q_rank, kv_rank=64, window=0, scale=0.08, ff=0)]),
+             seed=q_rank)
+    toks = tokens(c.cfg, 200, 14)
+    want = plain.forward(c.w, c.cfg, toks)[0]
+    with c.open("bfloat16") as lm:
+        for sizes in ([64, 17], [33, 24], [130, 70]):
+            s = lm.open()
+            assert error(feed(lm, s, toks, sizes), want) < LIMIT["bfloat16"], sizes
+            lm.release(s)
+
+
 @pytest.mark.parametrize("first,rows", [(1, 64), (65, 31), (100, 129), (7, 300)])
 def test_prefill_attention_tiles(pkg, engine, synth_model, first, rows):
     """A prompt in two calls against the same rows at once. Both are two-term products; a row's sums end in other

@@ -183,7 +183,8 @@ VB_DEVINL uint32_t at_off(int row, int chunk) { return (uint32_t)(row * 128 + ((
  *   here()                       what of it this block is to use
  *   rows(a)                      how many there are: a launch may serve several prompts (blockIdx.z), a.M the most of one
  *   pos0()                       position of row 0
- *   q4(row, head, d)             four query values (zeros beyond the head)
+ *   q4(row, head, d, part)       four query values (zeros beyond the head), or with kParts one of parts() addends of theirs
+ *   turned(row, head, d, v)      those values rotated, where they are not already
  *   keys(...) / values(...)      otherwise, with cp.async: a loading warp's 16 keys, into blocks of 64 columns, high halves
  *                                first
  *   gate(row, head)              factor of a result row
@@ -247,11 +248,25 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const __grid_
     }
     float4 qv[Cfg::kQBatch][4];
     auto q_load = [&](int batch) {
+        auto column = [&](int u) { return ((batch * Cfg::kQBatch + u) * 2 + w_q) * 16 + d_q; };
 #pragma unroll
         for (int u = 0; u < Cfg::kQBatch; u++)
 #pragma unroll
-            for (int i = 0; i < 4; i++)
-                qv[u][i] = src.q4(qrow[i], qhead[i], ((batch * Cfg::kQBatch + u) * 2 + w_q) * 16 + d_q);
+            for (int i = 0; i < 4; i++) qv[u][i] = src.q4(qrow[i], qhead[i], column(u), 0);
+        if constexpr (SRC::kParts) {             /* a part of the whole batch at a time, two on their way */
+#pragma unroll 2
+            for (int p = 1; p < src.parts(); p++) {
+                float4 t[Cfg::kQBatch][4];
+#pragma unroll
+                for (int u = 0; u < Cfg::kQBatch; u++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) t[u][i] = src.q4(qrow[i], qhead[i], column(u), p);
+#pragma unroll
+                for (int u = 0; u < Cfg::kQBatch; u++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) { qv[u][i].x += t[u][i].x; qv[u][i].y += t[u][i].y; qv[u][i].z += t[u][i].z; qv[u][i].w += t[u][i].w; }
+            }
+        }
     };
     pdl_wait();
     if (kEarly && warp < 8) q_load(0);
@@ -282,7 +297,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) vb_attn_tc_kernel(const __grid_
                 uint32_t hi[4][2], lo[4][2];
 #pragma unroll
                 for (int i2 = 0; i2 < 4; i2++) {
-                    float4 e = qv[u][i2];
+                    float4 e = src.turned(qrow[i2], qhead[i2], step * 16 + d_q, qv[u][i2]);
                     if (a.scale <= 0.0f) {             /* the scores are multiplied by |scale| below, or by one */
                         const float f = a.scale < 0.0f ? -1.0f : 0.0f;
                         e = make_float4(e.x * f, e.y * f, e.z * f, e.w * f);

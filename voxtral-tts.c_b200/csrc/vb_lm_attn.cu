@@ -862,7 +862,7 @@ VB_DEVINL void clear_keys(unsigned char *slot, int lw, int lane, int n) {
 
 /* Keys and values from a cache of split rows. */
 struct AtCache {
-    static constexpr bool kBoxes = false;
+    static constexpr bool kBoxes = false, kParts = false;
     const LmDyn *dyn;
     const float *q;
     LmState k, v;
@@ -874,9 +874,10 @@ struct AtCache {
     VB_DEVINL int rows(const AtArgs &a) const { return a.M; }
     VB_DEVINL const AtCache &here() const { return *this; }
     VB_DEVINL int pos0() const { return dyn->pos; }
-    VB_DEVINL float4 q4(int row, int head, int d) const {
+    VB_DEVINL float4 q4(int row, int head, int d, int) const {
         return d < dim ? vb_ldcg4(q + ((size_t)row * heads + head) * dim + d) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+    VB_DEVINL float4 turned(int, int, int, float4 x) const { return x; }
     VB_DEVINL bool boxes(int j0, int n) const { return n == kAtKeys && lm_ring_row(ring, j0 + kAtKeys - 1) - lm_ring_row(ring, j0) == kAtKeys - 1; }
     template <int BLOCKS>
     VB_DEVINL void box(const CUtensorMap *map, int size, unsigned char *slot, int g, int j0, uint64_t *bar) const {
@@ -924,9 +925,11 @@ struct AtCache {
 };
 
 /* Every head has keys and values of its own, read out of a latent (LmWide): a head's own columns of the written-out
- * rows, then the key part that all heads share from the latent's cache row. */
+ * rows, then the key part that all heads share from the latent's cache row. ONE: q comes in one part, as from GEMMs of many rows (without
+ * the code for several 153 -> 138 us, 2048 rows of heads of 192). */
+template <bool ONE>
 struct AtWide {
-    static constexpr bool kBoxes = false;
+    static constexpr bool kBoxes = false, kParts = !ONE;
     const LmDyn *dyn;
     LmWide w;
     LmRing ring;
@@ -936,13 +939,15 @@ struct AtWide {
     VB_DEVINL int rows(const AtArgs &a) const { return a.M; }
     VB_DEVINL const AtWide &here() const { return *this; }
     VB_DEVINL int pos0() const { return dyn->pos; }
-    VB_DEVINL float4 q4(int row, int head, int d) const {
+    VB_DEVINL int parts() const { return w.q.n; }
+    VB_DEVINL float4 q4(int row, int head, int d, int part) const {
         if (d >= dim) return make_float4(0.f, 0.f, 0.f, 0.f);
-        /* one part, as in GEMMs of many rows, without the code for eight: 153 -> 138 us, 2048 rows of heads of 192 */
-        const float4 x = w.q.n == 1 ? vb_ldcg4(w.q.p + (size_t)row * w.q.ld + head * dim + d) : lm_sum4(w.q, row, head * dim + d);
+        return vb_ldcg4(w.q.p + (ONE ? 0 : (size_t)part * w.q.stride) + (size_t)row * w.q.ld + head * dim + d);
+    }
+    VB_DEVINL float4 turned(int row, int, int d, float4 x) const {
         const int half = rot / 2, i0 = (d - (dim - w.rot_dim)) / 2;
         float e[4] = {x.x, x.y, x.z, x.w};
-        if (d >= dim - w.rot_dim) {
+        if (d >= dim - w.rot_dim && d < dim) {
 #pragma unroll
             for (int i = 0; i < 2; i++) {
                 if (i0 + i < half) {
@@ -1095,8 +1100,9 @@ bool lm_attn_wide_ok(int plain, int rot_dim, int vdim) {
     return plain + rot_dim <= 192 && vdim <= 128 && plain % 8 == 0 && rot_dim % 8 == 0 && vdim % 8 == 0;
 }
 
-int lm_attn_wide(const LmAttn &a, const LmWide &w, int M, cudaStream_t st) {
-    AtWide c = {};
+template <bool ONE>
+static int launch_wide(const LmAttn &a, const LmWide &w, int M, cudaStream_t st) {
+    AtWide<ONE> c = {};
     c.dyn = a.dyn; c.w = w; c.ring = a.ring; c.out = a.out;
     c.heads = a.heads; c.dim = a.dim; c.vdim = a.vdim; c.rot = a.rot;
     AtArgs t = at_args(a, M);
@@ -1111,6 +1117,10 @@ int lm_attn_wide(const LmAttn &a, const LmWide &w, int M, cudaStream_t st) {
     if (a.dim <= 64) return v1 ? launch_attn_tc<1, 1>(t, c, st, m) : launch_attn_tc<1, 2>(t, c, st, m);
     if (a.dim <= 128) return v1 ? launch_attn_tc<2, 1>(t, c, st, m) : launch_attn_tc<2, 2>(t, c, st, m);
     return v1 ? launch_attn_tc<3, 1>(t, c, st, m) : launch_attn_tc<3, 2>(t, c, st, m);
+}
+
+int lm_attn_wide(const LmAttn &a, const LmWide &w, int M, cudaStream_t st) {
+    return w.q.n == 1 ? launch_wide<true>(a, w, M, st) : launch_wide<false>(a, w, M, st);
 }
 
 bool lm_attn_step_ok(const LmAttn &a) {

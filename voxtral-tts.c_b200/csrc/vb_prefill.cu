@@ -140,7 +140,7 @@ __global__ void pf_qkv_finish_kernel(float *qkv, const float *part, int n_part, 
 /* Causal attention of prompt rows over the cache prefix (tts_causal_attention, voxtral_tts_kernels.c:403-465) on the
  * tensor cores (vb_attn_tc.cuh). */
 struct AtPrompt {
-    static constexpr bool kBoxes = true;
+    static constexpr bool kBoxes = true, kParts = false;
     const float *q;
     LmSink out;                  /* the terms that the O projection reads */
     int ldq;
@@ -148,7 +148,8 @@ struct AtPrompt {
     VB_DEVINL void start() {}
     VB_DEVINL int rows(const AtArgs &) const { return at.rows; }
     VB_DEVINL int pos0() const { return at.pos; }
-    VB_DEVINL float4 q4(int row, int head, int d) const { return vb_ldcg4(q + (size_t)(at.row0 + row) * ldq + head * VB200_HEAD_DIM + d); }
+    VB_DEVINL float4 q4(int row, int head, int d, int) const { return vb_ldcg4(q + (size_t)(at.row0 + row) * ldq + head * VB200_HEAD_DIM + d); }
+    VB_DEVINL float4 turned(int, int, int, float4 v) const { return v; }
     VB_DEVINL bool boxes(int, int) const { return true; }
     template <int BLOCKS>
     VB_DEVINL void box(const CUtensorMap *map, unsigned char *slot, int g, int j0, uint64_t *bar) const {
