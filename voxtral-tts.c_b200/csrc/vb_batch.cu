@@ -360,16 +360,7 @@ bt_attn_kernel(uint16_t *terms, int rows_pad, const float *part, int n_part, siz
             for (int h = 0; h < kGroup; h++)
                 s[h * kBtKeys + u] = q4[h].x * kq[u].x + q4[h].y * kq[u].y + q4[h].z * kq[u].z + q4[h].w * kq[u].w;
         }
-        /* 32 sums over the lanes by halving: lane i is left with sum i */
-#pragma unroll
-        for (int n = 16; n > 0; n >>= 1) {
-            const bool up = (lane & n) != 0;
-#pragma unroll
-            for (int i = 0; i < n; i++) {
-                const float send = up ? s[i] : s[i + n], keep = up ? s[i + n] : s[i];
-                s[i] = keep + __shfl_xor_sync(0xffffffffu, send, n);
-            }
-        }
+        vb_warp_halve32(s, lane);
         const bool on = jb + (lane % kBtKeys) * kBtAttnWarps < j1;
         const float e = on ? s[0] * scale : -1e30f;
         float top = e;
@@ -416,12 +407,7 @@ bt_attn_kernel(uint16_t *terms, int rows_pad, const float *part, int n_part, siz
             O.x += v.x * w;
             O.y += v.y * w;
         }
-        uint32_t to, bar;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(vb_smem_u32(&slices[sp * share + tid % share])), "r"(tid / share));
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(vb_smem_u32(&arrived)), "r"(tid / share));
-        asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(to),
-                     "r"(__float_as_uint(O.x)), "r"(__float_as_uint(O.y)), "r"(__float_as_uint(M0)), "r"(__float_as_uint(L)), "r"(bar)
-                     : "memory");
+        vb_cluster_send(&slices[sp * share + tid % share], &arrived, tid / share, O.x, O.y, M0, L);
     }
     if (!vb_mbar_wait_cluster(&arrived, &gave_up, status, 16)) return;
     if (tid < share) {

@@ -75,6 +75,56 @@ VB_DEVINL bool vb_mbar_wait_cluster(uint64_t *bar, volatile int *cta_abort, int 
     return false;
 }
 
+/* Two packed floats per instruction. */
+VB_DEVINL uint64_t vb_f2_pack(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+VB_DEVINL float2 vb_f2_get(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+VB_DEVINL uint64_t vb_f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+VB_DEVINL uint64_t vb_f2_add(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+VB_DEVINL uint64_t vb_f2_mul(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+/* 32 sums over the lanes of a warp by halving: lane i is left with sum i, in s[0]. */
+VB_DEVINL void vb_warp_halve32(float (&s)[32], int lane) {
+#pragma unroll
+    for (int n = 16; n > 0; n >>= 1) {
+        const bool up = (lane & n) != 0;
+#pragma unroll
+        for (int i = 0; i < n; i++) {
+            const float send = up ? s[i] : s[i + n], keep = up ? s[i + n] : s[i];
+            s[i] = keep + __shfl_xor_sync(0xffffffffu, send, n);
+        }
+    }
+}
+
+/* 16 bytes to the same place in the shared memory of the cluster's CTA `rank`, counted on its barrier. */
+VB_DEVINL void vb_cluster_send(const void *place, const uint64_t *bar, int rank, float a, float b, float c, float d) {
+    uint32_t to, count;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(vb_smem_u32(place)), "r"(rank));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(count) : "r"(vb_smem_u32(bar)), "r"(rank));
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(to),
+                 "r"(__float_as_uint(a)), "r"(__float_as_uint(b)), "r"(__float_as_uint(c)), "r"(__float_as_uint(d)), "r"(count)
+                 : "memory");
+}
+
 /* 1-D bulk copy global -> shared, completion counted in bytes on an mbarrier.
  * Both addresses 16-byte aligned, size a multiple of 16. No multicast. */
 VB_DEVINL void vb_bulk_g2s(void *smem_dst, const void *gmem_src, uint32_t bytes, uint64_t *bar) {

@@ -112,28 +112,6 @@ __global__ void __launch_bounds__(kPrepThreads) lm_attn_prepare_kernel(const LmA
  * mostly empty. The last split to arrive merges in split order. */
 constexpr int kGaThreads = 256, kGaKeys = 64, kGaFewKeys = 32, kGaManyPairs = 64;
 
-typedef unsigned long long f2;   /* two packed floats */
-VB_DEVINL f2 f2_fma(f2 a, f2 b, f2 c) {
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-VB_DEVINL f2 f2_mul(f2 a, f2 b) {
-    f2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-VB_DEVINL f2 f2_two(float v) {
-    f2 r;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
-    return r;
-}
-VB_DEVINL float2 f2_get(f2 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-
 /* rows of a multiple of four floats; an odd number of 16-byte pieces, so that eight rows' pieces lie in different banks */
 inline __host__ __device__ int ga_ld(int n) { const int v = (n + 3) / 4 + 1; return 4 * (v | 1); }
 inline __host__ __device__ int ga_stride(int vdim) { return (vdim + 3) / 4 * 4 + 4; }   /* a pair's partial result: columns, maximum, sum */
@@ -208,7 +186,7 @@ __global__ void __launch_bounds__(kGaThreads) lm_attn_generic_kernel(const LmAtt
         for (int d = lane; d < (dim + 3) / 4 * 4; d += 32) Q[p * ld + d] = p < np && d < dim ? __ldcg(q + d) : 0.0f;
     }
     float mx[TP], den[TP];
-    f2 o[TP][2 * NV];
+    uint64_t o[TP][2 * NV];
     int at[TP];                                  /* positions of this thread's rows */
 #pragma unroll
     for (int i = 0; i < TP; i++) {
@@ -226,7 +204,7 @@ __global__ void __launch_bounds__(kGaThreads) lm_attn_generic_kernel(const LmAtt
         ga_load<KEYS, SPLIT>(K, ld, dim, n, [&](int j) { return Kc + ((size_t)lm_ring_row(a.ring, j0 + j) * a.kv_heads + g) * dim; }, warp, lane);
         const bool odd = ga_load<KEYS, SPLIT>(V, ldv, vdim, n, [&](int j) { return Vc + ((size_t)lm_ring_row(a.ring, j0 + j) * a.kv_heads + g) * vdim; }, warp, lane);
         const bool any_odd = __syncthreads_or(odd);
-        f2 acc[TP][TK] = {};
+        uint64_t acc[TP][TK] = {};
 #pragma unroll 4
         for (int d = 0; d < dim; d += 4) {
             ulonglong2 q[TP], k[TK];
@@ -237,7 +215,7 @@ __global__ void __launch_bounds__(kGaThreads) lm_attn_generic_kernel(const LmAtt
 #pragma unroll
             for (int i = 0; i < TP; i++)
 #pragma unroll
-                for (int j = 0; j < TK; j++) acc[i][j] = f2_fma(q[i].y, k[j].y, f2_fma(q[i].x, k[j].x, acc[i][j]));
+                for (int j = 0; j < TK; j++) acc[i][j] = vb_f2_fma(q[i].y, k[j].y, vb_f2_fma(q[i].x, k[j].x, acc[i][j]));
         }
         __syncthreads();                         /* weights take the keys' place */
 #pragma unroll
@@ -246,7 +224,7 @@ __global__ void __launch_bounds__(kGaThreads) lm_attn_generic_kernel(const LmAtt
 #pragma unroll
             for (int j = 0; j < TK; j++) {
                 const int key = tx + 16 * j;
-                const float2 e = f2_get(acc[i][j]);
+                const float2 e = vb_f2_get(acc[i][j]);
                 s[j] = (e.x + e.y) * a.scale;
                 if (a.softcap > 0.0f) s[j] = a.softcap * tanhf(s[j] / a.softcap);
                 if (key >= n || !key_seen(at[i], j0 + key, a.window, a.keep)) s[j] = -INFINITY;
@@ -267,7 +245,7 @@ __global__ void __launch_bounds__(kGaThreads) lm_attn_generic_kernel(const LmAtt
             den[i] = den[i] * c + sum;
             mx[i] = now;
 #pragma unroll
-            for (int v = 0; v < 2 * NV; v++) o[i][v] = f2_mul(o[i][v], f2_two(c));
+            for (int v = 0; v < 2 * NV; v++) o[i][v] = vb_f2_mul(o[i][v], vb_f2_pack(c, c));
         }
         __syncwarp();                            /* a pair's weights are read by the half warp that wrote them */
         for (int j = 0; j < n; j += 4) {         /* rows from n on are zeros */
@@ -285,9 +263,10 @@ __global__ void __launch_bounds__(kGaThreads) lm_attn_generic_kernel(const LmAtt
                     for (int i = 0; i < TP; i++) {
                         /* zero times what is not finite: only where the key is seen */
                         if (any_odd && !(j + u < n && key_seen(at[i], j0 + j + u, a.window, a.keep))) continue;
-                        const f2 e = f2_two(u == 0 ? w[i].x : u == 1 ? w[i].y : u == 2 ? w[i].z : w[i].w);
-                        o[i][2 * c] = f2_fma(e, v.x, o[i][2 * c]);
-                        o[i][2 * c + 1] = f2_fma(e, v.y, o[i][2 * c + 1]);
+                        const float wu = u == 0 ? w[i].x : u == 1 ? w[i].y : u == 2 ? w[i].z : w[i].w;
+                        const uint64_t e = vb_f2_pack(wu, wu);
+                        o[i][2 * c] = vb_f2_fma(e, v.x, o[i][2 * c]);
+                        o[i][2 * c + 1] = vb_f2_fma(e, v.y, o[i][2 * c + 1]);
                     }
                 }
         }
@@ -338,13 +317,14 @@ __global__ void __launch_bounds__(kGaThreads) lm_attn_generic_kernel(const LmAtt
 #pragma unroll
             for (int i = 0; i < TP; i++) {
                 const float *from = po + ((size_t)u * PAIRS + ty * TP + i) * stride;
-                const f2 w = f2_two(wgt[u][ty * TP + i]);
+                const float wu = wgt[u][ty * TP + i];
+                const uint64_t w = vb_f2_pack(wu, wu);
 #pragma unroll
                 for (int c = 0; c < NV; c++) {
                     if (64 * c + 4 * tx >= ldv) continue;
                     const ulonglong2 v = __ldcg((const ulonglong2 *)(from + 64 * c + 4 * tx));
-                    o[i][2 * c] = f2_fma(w, v.x, o[i][2 * c]);
-                    o[i][2 * c + 1] = f2_fma(w, v.y, o[i][2 * c + 1]);
+                    o[i][2 * c] = vb_f2_fma(w, v.x, o[i][2 * c]);
+                    o[i][2 * c + 1] = vb_f2_fma(w, v.y, o[i][2 * c + 1]);
                 }
             }
     }
@@ -355,7 +335,7 @@ __global__ void __launch_bounds__(kGaThreads) lm_attn_generic_kernel(const LmAtt
 #pragma unroll
         for (int c = 0; c < NV; c++) {
             const int col = 64 * c + 4 * tx;
-            const float2 x = f2_get(o[i][2 * c]), y = f2_get(o[i][2 * c + 1]);
+            const float2 x = vb_f2_get(o[i][2 * c]), y = vb_f2_get(o[i][2 * c + 1]);
             const float e[4] = {x.x / den[i], x.y / den[i], y.x / den[i], y.y / den[i]};
             if ((vdim & 3) == 0) {
                 if (col < vdim) lm_put4(a.out, row, c0 + col, e);
@@ -763,16 +743,7 @@ __global__ void __launch_bounds__(kSgThreads, 2) lm_attn_step_group_kernel(const
             for (int h = 0; h < kSgHeads; h++)
                 s[h * kSgKeys + u] = q4[h].x * k.x + q4[h].y * k.y + q4[h].z * k.z + q4[h].w * k.w;
         }
-        /* 32 sums over the lanes by halving: lane i is left with sum i */
-#pragma unroll
-        for (int n = 16; n > 0; n >>= 1) {
-            const bool up = (lane & n) != 0;
-#pragma unroll
-            for (int i = 0; i < n; i++) {
-                const float send = up ? s[i] : s[i + n], keep = up ? s[i + n] : s[i];
-                s[i] = keep + __shfl_xor_sync(0xffffffffu, send, n);
-            }
-        }
+        vb_warp_halve32(s, lane);
         float e = s[0] * a.scale;
         if (a.softcap > 0.0f) e = a.softcap * tanhf(e / a.softcap);
         if (xb + (lane % kSgKeys) * kSgWarps >= x1) e = -INFINITY;
@@ -827,12 +798,7 @@ __global__ void __launch_bounds__(kSgThreads, 2) lm_attn_step_group_kernel(const
             O.x = fmaf(v.x, f, O.x);
             O.y = fmaf(v.y, f, O.y);
         }
-        uint32_t to, bar;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(vb_smem_u32(&slices[sp * share + tid % share])), "r"(tid / share));
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(vb_smem_u32(&arrived)), "r"(tid / share));
-        asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(to),
-                     "r"(__float_as_uint(O.x)), "r"(__float_as_uint(O.y)), "r"(__float_as_uint(M0)), "r"(__float_as_uint(L)), "r"(bar)
-                     : "memory");
+        vb_cluster_send(&slices[sp * share + tid % share], &arrived, tid / share, O.x, O.y, M0, L);
     }
     if (!vb_mbar_wait_cluster(&arrived, &gave_up, a.status, 53)) return;
     const int i = sp * share + tid, h = i / (kSgDim / 2), c = 2 * (i % (kSgDim / 2));

@@ -170,32 +170,6 @@ __global__ void __launch_bounds__(kInThreads) lm_delta_inputs_kernel(const LmDel
 /* ------------------------------------------------------------------ the recurrence */
 constexpr int kScMaxCols = 32, kScPer = 2, kScTok = 16, kScCtas = 148, kScGroups = kScTok / kScGroup, kScBufs = 3;
 
-/* two fp32 lanes per instruction */
-VB_DEVINL uint64_t f2_pack(float lo, float hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-VB_DEVINL float f2_sum(uint64_t v) {
-    float lo, hi;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-    return lo + hi;
-}
-VB_DEVINL uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-VB_DEVINL uint64_t f2_add(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-VB_DEVINL uint64_t f2_mul(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 VB_DEVINL void cp_async4(void *smem, const void *gmem) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(vb_smem_u32(smem)), "l"(gmem) : "memory");
 }
@@ -365,8 +339,8 @@ __global__ void __launch_bounds__(COLS / kScPer * LPC + 32) lm_delta_scan_kernel
                 const int r = (i * LPC + rg) * 4 + j;
                 x[j] = (!fresh && c + p < a.vdim && r < a.dim) ? S[(size_t)r * a.vdim + c + p] : 0.0f;
             }
-            s[p][2 * i] = f2_pack(x[0], x[1]);
-            s[p][2 * i + 1] = f2_pack(x[2], x[3]);
+            s[p][2 * i] = vb_f2_pack(x[0], x[1]);
+            s[p][2 * i + 1] = vb_f2_pack(x[2], x[3]);
         }
     auto load = [&](uint64_t (&x)[NR / 2], const float *row) {
 #pragma unroll
@@ -380,10 +354,11 @@ __global__ void __launch_bounds__(COLS / kScPer * LPC + 32) lm_delta_scan_kernel
         uint64_t e0 = 0, e1 = 0;
 #pragma unroll
         for (int i = 0; i < NR / 2; i += 2) {
-            e0 = f2_fma(y[i], x[i], e0);
-            e1 = f2_fma(y[i + 1], x[i + 1], e1);
+            e0 = vb_f2_fma(y[i], x[i], e0);
+            e1 = vb_f2_fma(y[i + 1], x[i + 1], e1);
         }
-        return f2_sum(f2_add(e0, e1));
+        const float2 e = vb_f2_get(vb_f2_add(e0, e1));
+        return e.x + e.y;
     };
     /* after the butterfly lane rg holds value rg / (LPC / 8): 0 .. 3 are S^T k_t, 4 .. 7 are S^T q_t */
     constexpr int kShare = LPC / 8;
@@ -420,7 +395,7 @@ __global__ void __launch_bounds__(COLS / kScPer * LPC + 32) lm_delta_scan_kernel
             float2 v[4];
 #pragma unroll
             for (int t = 0; t < 4; t++) v[t] = *reinterpret_cast<const float2 *>(&in.v[tg + t][cl]);
-            const uint64_t cc = f2_pack(c3, c3);
+            const uint64_t cc = vb_f2_pack(c3, c3);
             /* eight sums over the LPC lanes, for each column */
 #pragma unroll
             for (int n = 4, off = LPC / 2; n >= 1; n >>= 1, off >>= 1) {
@@ -441,7 +416,7 @@ __global__ void __launch_bounds__(COLS / kScPer * LPC + 32) lm_delta_scan_kernel
 #pragma unroll
                 for (int t = 0; t < 4; t++) e[p][t] = __shfl_sync(0xffffffffu, y[p][0], lane0 + t * kShare);
 #pragma unroll
-                for (int i = 0; i < NR / 2; i++) s[p][i] = f2_mul(s[p][i], cc);
+                for (int i = 0; i < NR / 2; i++) s[p][i] = vb_f2_mul(s[p][i], cc);
             }
 #pragma unroll
             for (int p = 0; p < kScPer; p++) {
@@ -451,11 +426,11 @@ __global__ void __launch_bounds__(COLS / kScPer * LPC + 32) lm_delta_scan_kernel
                 const float w1 = fmaf(u0.x, w0, fmaf(ec.y, e[p][1], v1));
                 const float w2 = fmaf(u0.z, w1, fmaf(u0.y, w0, fmaf(ec.z, e[p][2], v2)));
                 const float w3 = fmaf(u1.y, w2, fmaf(u1.x, w1, fmaf(u0.w, w0, fmaf(ec.w, e[p][3], v3))));
-                const uint64_t d0 = f2_pack(sc.x * w0, sc.x * w0), d1 = f2_pack(sc.y * w1, sc.y * w1), d2 = f2_pack(sc.z * w2, sc.z * w2),
-                               d3 = f2_pack(sc.w * w3, sc.w * w3);
+                const uint64_t d0 = vb_f2_pack(sc.x * w0, sc.x * w0), d1 = vb_f2_pack(sc.y * w1, sc.y * w1), d2 = vb_f2_pack(sc.z * w2, sc.z * w2),
+                               d3 = vb_f2_pack(sc.w * w3, sc.w * w3);
 #pragma unroll
                 for (int i = 0; i < NR / 2; i++)
-                    s[p][i] = f2_fma(k[3][i], d3, f2_fma(k[2][i], d2, f2_fma(k[1][i], d1, f2_fma(k[0][i], d0, s[p][i]))));
+                    s[p][i] = vb_f2_fma(k[3][i], d3, vb_f2_fma(k[2][i], d2, vb_f2_fma(k[1][i], d1, vb_f2_fma(k[0][i], d0, s[p][i]))));
                 const float o = fmaf(oc.w, w3, fmaf(oc.z, w2, fmaf(oc.y, w1, fmaf(oc.x, w0, oe * y[p][0]))));
                 if (writes && c + p < a.vdim && tg + ot < nt) out[(size_t)(t0 + tg + ot) * nv + p] = o;
             }
