@@ -123,9 +123,9 @@ def test_portions(mixed, dtype, sizes):
         assert error(feed(lm, s, mixed.toks, sizes), mixed.want) < LIMIT[dtype]
 
 
-@pytest.mark.parametrize("rows", [32, 33, 64, 65, 96, 97, 128, 129, 256, 257, 385])
+@pytest.mark.parametrize("rows", [1, 15, 16, 17, 32, 33, 64, 65, 96, 97, 128, 129, 256, 257, 385])
 def test_32_bit_rows(mixed, rows):
-    """Portions on both sides of the change from streamed weights to the row-block GEMM, and of its tiles."""
+    """Portions on both sides of the change from the skinny GEMM to the row-block one, at 16 and 17 rows, and of its tiles."""
     with mixed.open("float32") as lm:
         s = lm.open()
         assert error(lm.step(s, mixed.toks[:rows], range(rows)), mixed.want[:rows]) < LIMIT["float32"]

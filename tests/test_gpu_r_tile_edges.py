@@ -8,16 +8,31 @@ from lm_models import LIMIT, Case, attention, config, delta, error, feed, latent
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("rows", [1, 7, 8, 9, 32, 33, 64, 65])
+@pytest.mark.parametrize("rows", [1, 7, 8, 9, 16, 17, 32, 33, 64, 65])
 def test_float32_gemm_rows(pkg, tmp_path, rows):
-    """Portions on both sides of the few-rows kernel's and the tile kernel's edges; widths that split K (above 1024)
-    and that end inside a step of 32 columns. The limit is the 32-bit mode's: summation order."""
+    """Portions on both sides of the change from the skinny GEMM to the row-block one (16 and 17 rows) and of what a tile takes;
+    widths that are no whole blocks of 64 columns and that split K. The limit is the 32-bit mode's: summation order."""
     c = Case(pkg, tmp_path, config([delta(ff=1300), attention(ff=60)], width=1100, vocab=301), seed=rows)
     toks = tokens(c.cfg, rows + 70, rows)
     want = plain.forward(c.w, c.cfg, toks)[0]
     with c.open("float32") as lm:
         s = lm.open()
         assert error(feed(lm, s, toks, [rows, 70]), want) < LIMIT["float32"]
+
+
+@pytest.mark.parametrize("width", [5120, 8200])
+def test_float32_wide_few_rows(pkg, tmp_path, width):
+    """A gated feed-forward of the 32-bit mode keeps one K split, so that each of a launch's ten sums takes 8 and 13 blocks of 64
+    columns here. The logits are no further off than in portions of 17 rows, whose sums take two blocks: both within the
+    mode's limit, which is twenty times what they show."""
+    c = Case(pkg, tmp_path, config([delta(heads=2, kv_heads=1, dim=32, vdim=32, ff=200)], width=width, vocab=101), seed=3)
+    toks = tokens(c.cfg, 34, 15)
+    want = plain.forward(c.w, c.cfg, toks)[0]
+    with c.open("float32") as lm:
+        for sizes in ([1], [5], [16], [17]):
+            s = lm.open()
+            assert error(feed(lm, s, toks, sizes), want) < LIMIT["float32"], sizes
+            lm.release(s)
 
 
 @pytest.mark.parametrize("rows", [65, 96, 97, 128, 129, 255, 256, 257, 300])
@@ -60,6 +75,21 @@ def test_prompt_attention_tiles(pkg, tmp_path, name):
     want = plain.forward(c.w, c.cfg, toks)[0]
     with c.open("bfloat16", block_rows=256) as lm:
         for sizes in ([420], [65, 128, 17, 33], [31, 63]):
+            s = lm.open()
+            assert error(feed(lm, s, toks, sizes), want) < LIMIT["bfloat16"], sizes
+            lm.release(s)
+
+
+@pytest.mark.parametrize("dim,rot_dim", [(128, 64), (168, 8), (120, 64)])
+@pytest.mark.parametrize("window", [0, 130])
+def test_heads_of_three_blocks(pkg, tmp_path, dim, rot_dim, window):
+    """Heads of 192, 176 and 184, whose low query halves lie in shared memory: one to seven key tiles, the last of one key, of 63 and
+    whole, by TMA (192) and without, full and nearly empty row tiles."""
+    c = Case(pkg, tmp_path, config([latent(heads=2, dim=dim, rot_dim=rot_dim, vdim=128, kv_rank=64, window=window, scale=0.08, ff=0)]), seed=dim)
+    toks = tokens(c.cfg, 449, 16)
+    want = plain.forward(c.w, c.cfg, toks)[0]
+    with c.open("bfloat16", block_rows=256) as lm:
+        for sizes in ([64], [127, 129], [63, 65, 128], [255, 194], [191, 17, 241]):
             s = lm.open()
             assert error(feed(lm, s, toks, sizes), want) < LIMIT["bfloat16"], sizes
             lm.release(s)
