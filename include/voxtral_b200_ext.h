@@ -84,8 +84,9 @@ double vb200_utterance_engine_ms(int *launches);
  *   hidden:  decoder output rows of the last frame [n, 3072] */
 int vb200_batch_open(int n_utterances, int kv_max, int max_frames);
 int vb200_batch_prefill(int utterance, const float *embeds, int n_rows);
-/* The prompts of all utterances at once, embeds[u] [n_rows[u], 3072]: prompts of a few hundred rows go through the layers side
- * by side, which takes half the time of one after another. */
+/* The prompts of all utterances at once, embeds[u] [n_rows[u], 3072]: those of 65 rows and more go through the layers side by side,
+ * up to 2048 rows together. Against one after another: two of 65 rows 3.3 and 5.9 ms, four of 100 5.6 and 12.4, eight of
+ * 190 15.6 and 29.3, two of 500 11.4 and 12.9. */
 int vb200_batch_prefill_all(const float *const *embeds, const int *n_rows);
 int vb200_batch_begin(const float *first_embeds, const int *start_pos, const float *noise);
 int vb200_batch_run(int n_frames);

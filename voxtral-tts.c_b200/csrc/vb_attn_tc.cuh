@@ -67,8 +67,10 @@ struct AtCfg {
 };
 
 /* A descriptor's low word, which holds the address and is what the steps of a product add to; the high word is the same for
- * all of an operand. (Sums of whole descriptors came out wrong in one of three copies of the score products, heads of
- * 192, when the kernel around them changed: low halves of the queries read from beyond their place.) */
+ * all of an operand. By the source a sum of whole descriptors is the same number: addresses stay below 2^18, 16 bytes a unit, so
+ * nothing carries. Even so, heads of 192 gave wrong scores from the third key tile on with such sums, as if low halves of the
+ * queries had been read from beyond their place, after a change elsewhere in the kernel, and give right ones with these. The cause
+ * is not known. The GEMMs (vb_tc.cu, vb_tc_rows.cu) add whole descriptors in one copy of a loop each. */
 struct AtDesc {
     uint32_t lo, hi;
     VB_DEVINL explicit AtDesc(uint64_t d) : lo((uint32_t)d), hi((uint32_t)(d >> 32)) {}

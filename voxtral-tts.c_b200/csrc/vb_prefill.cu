@@ -405,7 +405,7 @@ static int pf_finish(int rc) {
  * long as a block has room, so that the weights are read once and the GEMMs are wide. Eight prompts of 100 to 187 rows took
  * 27 ms one after another. Only those that alone would be one block of two-term products; the others, and all where memory
  * is short, are left for prefill(): done[i] says which are in their caches. K is summed in pieces of 1024 columns: alone,
- * these prompts have the frame's K splits, of 512 to 1536. */
+ * those of up to 256 rows have the frame's K splits, sums of 704 to 1536 columns (2048 for gate/up). */
 constexpr int kPfJointSegment = 16;
 int prefill_joint(const PfPrompt *prompts, int n, int kv_max, bool *done) {
     Model &m = model();
